@@ -72,6 +72,21 @@ int ensure_me_scratch(h264a_ctx* ctx, size_t n, int queue) {
     return H264A_OK;
 }
 
+int ensure_me_words(h264a_ctx* ctx, size_t n, int queue) {
+    WorkQueue& q = ctx->q[queue];
+    if (n <= q.words_cap) return H264A_OK;
+    if (q.d_words) cudaFree(q.d_words);
+    q.d_words = nullptr;
+    q.words_cap = 0;
+    const size_t cap = n < 4096 ? 4096 : n + n / 4;
+    if (cudaMalloc(&q.d_words, cap * sizeof(unsigned long long)) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(H264A_E_NOMEM, "plain-ME words: cudaMalloc failed");
+    }
+    q.words_cap = cap;
+    return H264A_OK;
+}
+
 int next_epoch(h264a_ctx* ctx, cudaStream_t st, int queue) {
     WorkQueue& q = ctx->q[queue];
     if (q.epoch >= 0x7ffffff0) {  // wrap: clear the flags so stale values never match
@@ -139,8 +154,10 @@ extern "C" int h264a_ctx_destroy(h264a_ctx* ctx) {
     if (ctx->pf_stream) cudaStreamSynchronize(ctx->pf_stream);
     if (ctx->d_counters) cudaFree(ctx->d_counters);
     if (ctx->d_status) cudaFree(ctx->d_status);
-    for (int i = 0; i < NUM_QUEUES; i++)
+    for (int i = 0; i < NUM_QUEUES; i++) {
         if (ctx->q[i].d_flags) cudaFree(ctx->q[i].d_flags);
+        if (ctx->q[i].d_words) cudaFree(ctx->q[i].d_words);
+    }
     if (ctx->pp_buf) cudaFree(ctx->pp_buf);
     if (ctx->cl_buf) cudaFree(ctx->cl_buf);
     if (ctx->me_tab) cudaFree(ctx->me_tab);

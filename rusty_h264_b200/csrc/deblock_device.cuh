@@ -66,52 +66,29 @@ constexpr int CT = 12, CR = 10;   // chroma tile: 10 rows x 12 (stride 12), the 
 __device__ __forceinline__ int clip1(int v) { return v < 0 ? 0 : (v > 255 ? 255 : v); }
 __device__ __forceinline__ int clip3(int lo, int hi, int v) { return v < lo ? lo : (v > hi ? hi : v); }
 
-// filter_luma_line (deblock.rs:67-115) on shared bytes: q0 at q, samples
-// `step` apart.
-__device__ __forceinline__ void luma_line(uint8_t* q, int step, int bs, int alpha, int beta, int tc0) {
-    const int p0 = q[-step], p1 = q[-2 * step], p2 = q[-3 * step], p3 = q[-4 * step];
-    const int q0 = q[0], q1 = q[step], q2 = q[2 * step], q3 = q[3 * step];
+// filter_luma_line (deblock.rs:67-115) on shared bytes, bS 1..2 (no picture of
+// this path has an intra edge): q0 at q, samples `step` apart.
+__device__ __forceinline__ void luma_line(uint8_t* q, int step, int alpha, int beta, int tc0) {
+    const int p0 = q[-step], p1 = q[-2 * step], p2 = q[-3 * step];
+    const int q0 = q[0], q1 = q[step], q2 = q[2 * step];
     if (abs(p0 - q0) >= alpha || abs(p1 - p0) >= beta || abs(q1 - q0) >= beta) return;
     const int ap = abs(p2 - p0), aq = abs(q2 - q0);
-    if (bs < 4) {
-        const int tc = tc0 + (ap < beta) + (aq < beta);
-        const int delta = clip3(-tc, tc, (((q0 - p0) << 2) + (p1 - q1) + 4) >> 3);
-        q[-step] = uint8_t(clip1(p0 + delta));
-        q[0] = uint8_t(clip1(q0 - delta));
-        if (ap < beta) q[-2 * step] = uint8_t(clip1(p1 + clip3(-tc0, tc0, (p2 + ((p0 + q0 + 1) >> 1) - (p1 << 1)) >> 1)));
-        if (aq < beta) q[step] = uint8_t(clip1(q1 + clip3(-tc0, tc0, (q2 + ((p0 + q0 + 1) >> 1) - (q1 << 1)) >> 1)));
-    } else {
-        const bool strong = abs(p0 - q0) < (alpha >> 2) + 2;
-        if (strong && ap < beta) {
-            q[-step] = uint8_t(clip1((p2 + 2 * p1 + 2 * p0 + 2 * q0 + q1 + 4) >> 3));
-            q[-2 * step] = uint8_t(clip1((p2 + p1 + p0 + q0 + 2) >> 2));
-            q[-3 * step] = uint8_t(clip1((2 * p3 + 3 * p2 + p1 + p0 + q0 + 4) >> 3));
-        } else {
-            q[-step] = uint8_t(clip1((2 * p1 + p0 + q1 + 2) >> 2));
-        }
-        if (strong && aq < beta) {
-            q[0] = uint8_t(clip1((q2 + 2 * q1 + 2 * q0 + 2 * p0 + p1 + 4) >> 3));
-            q[step] = uint8_t(clip1((q2 + q1 + q0 + p0 + 2) >> 2));
-            q[2 * step] = uint8_t(clip1((2 * q3 + 3 * q2 + q1 + q0 + p0 + 4) >> 3));
-        } else {
-            q[0] = uint8_t(clip1((2 * q1 + q0 + p1 + 2) >> 2));
-        }
-    }
+    const int tc = tc0 + (ap < beta) + (aq < beta);
+    const int delta = clip3(-tc, tc, (((q0 - p0) << 2) + (p1 - q1) + 4) >> 3);
+    q[-step] = uint8_t(clip1(p0 + delta));
+    q[0] = uint8_t(clip1(q0 - delta));
+    if (ap < beta) q[-2 * step] = uint8_t(clip1(p1 + clip3(-tc0, tc0, (p2 + ((p0 + q0 + 1) >> 1) - (p1 << 1)) >> 1)));
+    if (aq < beta) q[step] = uint8_t(clip1(q1 + clip3(-tc0, tc0, (q2 + ((p0 + q0 + 1) >> 1) - (q1 << 1)) >> 1)));
 }
 
 // filter_chroma_line (deblock.rs:117-137).
-__device__ __forceinline__ void chroma_line(uint8_t* q, int step, int bs, int alpha, int beta, int tc0) {
+__device__ __forceinline__ void chroma_line(uint8_t* q, int step, int alpha, int beta, int tc0) {
     const int p0 = q[-step], p1 = q[-2 * step], q0 = q[0], q1 = q[step];
     if (abs(p0 - q0) >= alpha || abs(p1 - p0) >= beta || abs(q1 - q0) >= beta) return;
-    if (bs < 4) {
-        const int tc = tc0 + 1;
-        const int delta = clip3(-tc, tc, (((q0 - p0) << 2) + (p1 - q1) + 4) >> 3);
-        q[-step] = uint8_t(clip1(p0 + delta));
-        q[0] = uint8_t(clip1(q0 - delta));
-    } else {
-        q[-step] = uint8_t(clip1((2 * p1 + p0 + q1 + 2) >> 2));
-        q[0] = uint8_t(clip1((2 * q1 + q0 + p1 + 2) >> 2));
-    }
+    const int tc = tc0 + 1;
+    const int delta = clip3(-tc, tc, (((q0 - p0) << 2) + (p1 - q1) + 4) >> 3);
+    q[-step] = uint8_t(clip1(p0 + delta));
+    q[0] = uint8_t(clip1(q0 - delta));
 }
 
 // MV and coefficient flag of 4x4 block (bx, by) of MB m (coefficients in the
@@ -146,34 +123,31 @@ __device__ __forceinline__ void deblock_mb_tiles(int lane, uint8_t* lt, uint8_t*
                                                  bool left, bool top, bool has_c, const DbThresh& th) {
     const int pl = (lane >> 3) & 1, li = lane & 7;
     uint8_t* ct = pl ? ct1 : ct0;
-    if (lane < 16) {
-        uint8_t* row = lt + (4 + lane) * LT + 4;
-        for (int e = left ? 0 : 1; e < 4; e++) {
-            const int bs = bsw[e * 4 + (lane >> 2)];
-            if (bs) luma_line(row + 4 * e, 1, bs, th.alpha_y, th.beta_y, th.tc_y[bs - 1]);
+    // both directions through one copy of the filters (the code runs once per
+    // MB among the search's, so its size counts)
+#pragma unroll 1
+    for (int dir = 0; dir < 2; dir++) {
+        const bool first = dir ? top : left;
+        const int* bs4 = bsw + 16 * dir;
+        if (lane < 16) {
+            const int step = dir ? LT : 1;
+            uint8_t* line = lt + 4 * LT + 4 + lane * (dir ? 1 : LT);
+#pragma unroll 1
+            for (int e = first ? 0 : 1; e < 4; e++) {
+                const int bs = bs4[e * 4 + (lane >> 2)];
+                if (bs) luma_line(line + 4 * e * step, step, th.alpha_y, th.beta_y, th.tc_y[bs - 1]);
+            }
+        } else if (has_c) {
+            const int step = dir ? CT : 1;
+            uint8_t* line = ct + 2 * CT + 4 + li * (dir ? 1 : CT);
+#pragma unroll 1
+            for (int ce = first ? 0 : 2; ce < 4; ce += 2) {
+                const int bs = bs4[ce * 4 + (li >> 1)];
+                if (bs) chroma_line(line + 2 * ce * step, step, th.alpha_c, th.beta_c, th.tc_c[bs - 1]);
+            }
         }
-    } else if (has_c) {
-        uint8_t* row = ct + (2 + li) * CT + 4;
-        for (int ce = left ? 0 : 2; ce < 4; ce += 2) {
-            const int bs = bsw[ce * 4 + (li >> 1)];
-            if (bs) chroma_line(row + 2 * ce, 1, bs, th.alpha_c, th.beta_c, th.tc_c[bs - 1]);
-        }
+        __syncwarp();
     }
-    __syncwarp();
-    if (lane < 16) {
-        uint8_t* col = lt + 4 * LT + 4 + lane;
-        for (int e = top ? 0 : 1; e < 4; e++) {
-            const int bs = bsw[16 + e * 4 + (lane >> 2)];
-            if (bs) luma_line(col + 4 * e * LT, LT, bs, th.alpha_y, th.beta_y, th.tc_y[bs - 1]);
-        }
-    } else if (has_c) {
-        uint8_t* col = ct + 2 * CT + 4 + li;
-        for (int ce = top ? 0 : 2; ce < 4; ce += 2) {
-            const int bs = bsw[16 + ce * 4 + (li >> 1)];
-            if (bs) chroma_line(col + 2 * ce * CT, CT, bs, th.alpha_c, th.beta_c, th.tc_c[bs - 1]);
-        }
-    }
-    __syncwarp();
 }
 
 // One lane's word of an MB's left and top strips (the neighbours' samples its

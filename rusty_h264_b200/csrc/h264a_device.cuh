@@ -357,7 +357,7 @@ __device__ __forceinline__ long long lam_cost(double lam, uint32_t rate) {
 // both neighbours lie on earlier diagonals.  Readiness is a per-MB flag set to
 // the launch's epoch with release semantics and polled with acquire loads.
 
-constexpr int SPIN_LIMIT = 1000 * 1000;  // ~0.5 s of polling (a 200 ns sleep per poll)
+constexpr int SPIN_LIMIT = 1000 * 1000;  // ~0.5 s of polling at a 200 ns sleep per poll
 
 // Number of MBs (x, y) of a W x H frame with x + 2y < t: rows y < a are
 // full (t - 2y >= W), rows a <= y < b hold t - 2y MBs.
@@ -391,6 +391,10 @@ __device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
     return old;
 }
+// Add at GPU scope with release semantics, nothing returned.
+__device__ __forceinline__ void red_add_release(int* p, int v) {
+    asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 // Release store at system scope (a word the host polls in mapped memory).
 __device__ __forceinline__ void st_release_sys(int* p, int v) {
     asm volatile("st.release.sys.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
@@ -403,17 +407,18 @@ __device__ __forceinline__ void st_release(int* p, int v) {
     asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Waits (bounded) until flag == epoch; on timeout records `code` in status.
+// Waits (bounded) until flag == epoch, polling every `ns` nanoseconds; on
+// timeout records `code` in status.
 // Once any wait of the launch has timed out (status non-zero, checked every
 // 256 polls) the others give up too, so a failed launch ends promptly.
-static __device__ void wait_flag(const int* flag, int epoch, int* status, int code, int limit) {
+static __device__ void wait_flag(const int* flag, int epoch, int* status, int code, int limit, unsigned ns = 200) {
     for (int it = 0;; it++) {
         if (ld_acquire(flag) == epoch) return;
         if (it >= limit || ((it & 255) == 255 && *reinterpret_cast<volatile int*>(status) != 0)) {
             atomicCAS(status, 0, code);
             return;
         }
-        __nanosleep(200);
+        __nanosleep(ns);
     }
 }
 

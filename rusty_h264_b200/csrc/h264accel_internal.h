@@ -19,6 +19,8 @@ struct WorkQueue {
     int32_t *d_counter = nullptr;  // a word of h264a_ctx::d_counters
     int32_t *d_flags = nullptr;
     size_t flags_cap = 0;
+    unsigned long long *d_words = nullptr;  // the published picks of plain-ME (MV words, cleared per launch)
+    size_t words_cap = 0;
     int32_t epoch = 0;
 };
 // Q_MAIN serves plain-ME, deblocking and the bounded-wait self-test (flags
@@ -104,6 +106,8 @@ int check_launch(const char *what);
 // grows the per-MB done flags of work queue `queue` to at least n entries
 // (zeroed, epoch reset)
 int ensure_me_scratch(h264a_ctx *ctx, size_t n, int queue = Q_MAIN);
+// grows the MV words of work queue `queue` to at least n
+int ensure_me_words(h264a_ctx *ctx, size_t n, int queue);
 // Per-frame outputs of the MC + luma T/Q fused into the plain-ME kernel:
 // coefficients (256 i16 per MB, 16-byte aligned), the QP and dead-zone
 // divisor, and optional row completion words (see FrameDesc in me.cu).
@@ -186,6 +190,7 @@ struct MrTable {
     int nframes = 0, nseg = 0;
     long long total = 0;  // MBs
     size_t b_desc = 0, b_seg = 0;
+    bool lam_ok = true;  // every frame's lambda suits the Balanced searches
 };
 // h264a_mc_tq_frames_multiref on stream st (checks its arguments)
 int mc_tq_mr_run(h264a_ctx *ctx, const h264a_mc_tq_mr_frame *h_frames, int nframes, cudaStream_t st);

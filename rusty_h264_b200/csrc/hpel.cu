@@ -38,7 +38,8 @@ __global__ void __launch_bounds__(32 * HP_WARPS) hpel_build_kernel(const uint8_t
     const int rem = int(wid - per_pic * pic);
     const int band = rem / strips, strip = rem - band * strips;
     const int y0 = band * HP_BAND;
-    hpel_strip_rows(ref + ref_fstride * pic, cw, ch, pad, planes + 4LL * pw * ph * pic, pw, ph, strip, y0,
+    hpel_strip_rows(ref + ref_fstride * pic, cw, ch, pad, planes + 4LL * pw * ph * pic, pw, ph,
+                    strip * HP_STRIP, y0,
                     y0 + HP_BAND < ph ? y0 + HP_BAND : ph, word_in, word_out);
 }
 

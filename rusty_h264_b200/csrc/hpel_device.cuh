@@ -48,21 +48,22 @@ struct HpelRow {
     uint32_t raw, ev, od;  // the source word, its even and odd bytes as 16x2
 };
 
-// Rows [y0, y1) of strip `strip` (plane columns strip * HP_STRIP ..) of the
-// four planes F of picture Y, one warp: see the file comment of hpel.cu.
-// Only the 4-byte words whose plane column lies in [xlo, xhi) are written
-// (xlo, xhi multiples of 4): a strip shared by two column segments is
-// written by each for its own columns.
+// Rows [y0, y1) of the strip of HP_STRIP plane columns from xs (a multiple of
+// 4), those below xhi only, of the four planes F of picture Y, one warp: see
+// the file comment of hpel.cu.
 // CG: read the picture through L2 rather than the read-only path (a picture
 // written during the launch, whose rows below the strip's may still change:
 // the look-ahead loads past y1 must not leave stale lines in L1).
-template <bool CG = false>
+// COMPACT: one row per iteration, the six rows rotated through registers and
+// the next two rows' loads in flight, in a sixth of the code: for the closed
+// loop's kernel, whose instruction footprint bounds it.
+template <bool CG = false, bool COMPACT = false>
 __device__ __forceinline__ void hpel_strip_rows(const uint8_t* __restrict__ Y, int cw, int ch, int pad,
-                                                uint8_t* __restrict__ F, int pw, int ph, int strip, int y0, int y1,
-                                                int word_in, int word_out, int xlo = 0, int xhi = 1 << 30) {
+                                                uint8_t* __restrict__ F, int pw, int ph, int xs, int y0, int y1,
+                                                int word_in, int word_out, int xhi = 1 << 30) {
     const int lane = threadIdx.x & 31;
     const long long ps = (long long)pw * ph;
-    const int X = strip * HP_STRIP + 4 * (lane - 1);  // plane column of the lane's word
+    const int X = xs + 4 * (lane - 1);  // plane column of the lane's word
     const int sx = X - pad;                           // its first picture column
     const bool inner = word_in && sx >= 0 && sx + 3 <= cw - 1;
     const int c0 = clampi(sx, 0, cw - 1), c1 = clampi(sx + 1, 0, cw - 1), c2 = clampi(sx + 2, 0, cw - 1),
@@ -81,7 +82,7 @@ __device__ __forceinline__ void hpel_strip_rows(const uint8_t* __restrict__ Y, i
         return r;
     };
     auto load = [&](int yp) { return mk(ldraw(yp)); };
-    const bool owner = lane >= 1 && lane <= 30 && X < pw && X >= xlo && X < xhi;
+    const bool owner = lane >= 1 && lane <= 30 && X < pw && X < xhi;
     // the four planes' words of row y from the rows y-2 .. y+3
     auto emit = [&](int y, const HpelRow& a, const HpelRow& b, const HpelRow& c, const HpelRow& d, const HpelRow& e,
                     const HpelRow& f) {
@@ -127,6 +128,22 @@ __device__ __forceinline__ void hpel_strip_rows(const uint8_t* __restrict__ Y, i
             }
         }
     };
+    if (COMPACT) {
+        uint32_t n[5];
+#pragma unroll
+        for (int i = 0; i < 5; i++) n[i] = ldraw(y0 - 2 + i);
+        uint32_t pre0 = ldraw(y0 + 3), pre1 = ldraw(y0 + 4);
+        HpelRow a = mk(n[0]), b = mk(n[1]), c = mk(n[2]), d = mk(n[3]), e = mk(n[4]);
+#pragma unroll 1
+        for (int y = y0; y < y1; y++) {
+            const HpelRow f = mk(pre0);
+            pre0 = pre1;
+            pre1 = ldraw(y + 5);  // (rows past the band are clamped reads, discarded)
+            emit(y, a, b, c, d, e, f);
+            a = b; b = c; c = d; d = e; e = f;
+        }
+        return;
+    }
     HpelRow r0 = load(y0 - 2), r1 = load(y0 - 1), r2 = load(y0), r3 = load(y0 + 1), r4 = load(y0 + 2), r5;
     // six rows per iteration, the window rotating through r0..r5 by name
     for (int y = y0; y < y1; y += 6) {

@@ -1,0 +1,1144 @@
+// mb_search.cuh -- the searches of one macroblock (motion_search,
+// crates/rusty_h264-encoder/src/mb16.rs:2433-3302, as best_part runs them,
+// :4921) by one warp: the 16x16, then the four 16x8 / 8x16 partitions side by
+// side, every candidate priced on the tensor cores (satd_mma.cuh).
+//
+// A round prices up to eight candidate slots per group of eight lanes.  Mode 0
+// (16x16): the four groups hold identical state and the warp's eight mma
+// columns are the eight slots, 16 blocks each.  Mode 1: group g searches
+// partition g (0 16x8 top, 1 16x8 bottom, 2 8x16 left, 3 8x16 right; they
+// share the seeds [pmv, mv16], the mvd centre and λ, mb16.rs:8869-8913, so
+// they are independent), and an mma's columns are two slots of each group.
+// Either way 16 mma are one pass: "tile A" and "tile B" of eight blocks,
+// the upper and lower half of the 16x16 candidate, or slots c and c + 2 of
+// the partitions.  A pass costs the same for one candidate as for eight
+// (mode 0) or four per partition (mode 1), so rings are priced whole, and the
+// spare columns of a fixed-centre ring of four price the next rung's ring
+// around the same centre, which the walk needs next whenever the ring does not
+// improve.  Neither changes a decision: only the points the reference evaluates are
+// folded, in its order, and only they are counted.
+//
+// The bound is the wavefront's latency: each MB's rounds depend on one
+// another, and a round is a chain of shared-memory reads, mma and shuffles.
+// Per round, measured against the butterflies on 32 lanes (satd4x4_packed,
+// two 16x16 or one candidate per partition a pass): see me_frames_kernel.
+#pragma once
+
+#include "satd_mma.cuh"
+
+namespace h264a {
+
+constexpr int MET_SATD = 0;
+constexpr int MET_SAD = 1;
+
+// The reference picture's readiness in the pipelined closed loop: its planes
+// are built segment by segment (16 picture rows by segw picture columns;
+// segment (b, s)'s flag == epoch means every segment up and left of it is
+// complete), and a search waits (bounded) for the segment of every pixel it
+// reads.
+struct BandWait {
+    const int* flags;  // nbands x nseg readiness flags, band-major
+    int nbands, nseg, segw, epoch, limit;
+    int* status;
+};
+
+// Waits until the reference's planes (and reconstruction) are final at
+// picture pixel (row, col), clamped into the picture: the flag of the band
+// (16 rows) and column segment (segw columns) holding it.  Segment (b, s) is
+// published after (b-1, s) and (b, s-1), so it stands for every segment up
+// and left of it.  `ready` caches a segment seen ready, packed b << 12 | s
+// (-1: none); any value stored there was seen ready, so a torn update between
+// lanes only loses a shortcut.  Nothing when the search has no BandWait.
+// Out of line: it is called from several places, mostly to find a segment
+// seen ready.
+__device__ __noinline__ void band_wait_at(const BandWait* bw, int* ready, int row, int col) {
+    const int b = min(max(row, 0) >> 4, bw->nbands - 1);
+    const int sg = min(max(col, 0) / bw->segw, bw->nseg - 1);
+    const int c = *reinterpret_cast<volatile int*>(ready);
+    if (c >= 0 && b <= (c >> 12) && sg <= (c & 4095)) return;
+    wait_flag(bw->flags + b * bw->nseg + sg, bw->epoch, bw->status, 1, bw->limit);
+    if (c < 0 || (b >= (c >> 12) && sg >= (c & 4095))) *reinterpret_cast<volatile int*>(ready) = (b << 12) | sg;
+}
+
+__device__ __forceinline__ void band_wait_px(const BandWait* bw, int* ready, int row, int col) {
+    if (bw != nullptr) band_wait_at(bw, ready, row, col);
+}
+
+// Per-warp shared state of an MB's searches (read rarely, or by one lane).
+struct MbScratch {
+    const uint8_t* base;  // the reference's F|H|V|C planes
+    const uint8_t* src;   // the source luma
+    const BandWait* bw;   // the reference's segment readiness, or nullptr (complete)
+    int pw, ph, pad, cw, ch;
+    int wx0, wy0;         // the window's origin in padded-plane coordinates
+    int bready;           // a reference segment seen complete (band_wait_px)
+};
+
+// ---------------------------------------------------------------------------
+// Per-MB reference window in shared memory
+// ---------------------------------------------------------------------------
+// The F|H|V|C planes around the MB's predicted position, copied once per MB by
+// the bulk-copy (TMA) engine: WIN_H rows of WIN_W bytes per plane, every
+// search of the MB (16x16 and its partitions) then reads its candidates from
+// shared memory.  Candidates whose reads leave the window take the plane path
+// (pred_word), which gives the same bytes.  Rows are WIN_STRIDE = 80 bytes
+// (20 banks) apart, so eight consecutive rows start four banks apart and the
+// row words a ring's candidates read together rarely share a bank.
+constexpr int WIN_W = 64, WIN_H = 42, WIN_STRIDE = 80;
+constexpr int WIN_PLANE = WIN_H * WIN_STRIDE;  // bytes per plane (a multiple of 16)
+constexpr int WIN_BYTES = 4 * WIN_PLANE;
+constexpr int WIN_R = 12;  // the window starts this far up/left of the predicted position
+constexpr int WIN_OFF = -(1 << 30);  // window offset of a search without one: below -2^29 for any MV, so every read misses
+
+// Rows of the 4x4 block at window position (wx, wy) (full-pel part of the MV
+// applied) at phase (fx, fy): the same operand table and averaging as
+// pred_rows, read from the staged window at shared address `win`.
+__device__ __forceinline__ void win_rows(uint32_t win, int wx, int wy, int fx, int fy, uint32_t out[4]) {
+    const uint32_t pb = phase_bits(fx, fy);
+    const int pa = int(pb & 3), pbb = int((pb >> 2) & 3);
+    const int xa = wx + int((pb >> 4) & 1), ya = wy + int((pb >> 5) & 1);
+    const uint32_t a = win + uint32_t(pa * WIN_PLANE + ya * WIN_STRIDE + (xa & ~3));
+    const uint32_t sha = uint32_t(xa & 3) * 8u;
+#pragma unroll
+    for (int r = 0; r < 4; r++) out[r] = __funnelshift_r(lds_u32(a + r * WIN_STRIDE), lds_u32(a + r * WIN_STRIDE + 4), sha);
+    if (pbb != 0) {
+        const int xb = wx + int((pb >> 6) & 1), yb = wy + int((pb >> 7) & 1);
+        const uint32_t b = win + uint32_t(pbb * WIN_PLANE + yb * WIN_STRIDE + (xb & ~3));
+        const uint32_t shb = uint32_t(xb & 3) * 8u;
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+            out[r] = avg_up4(out[r], __funnelshift_r(lds_u32(b + r * WIN_STRIDE), lds_u32(b + r * WIN_STRIDE + 4), shb));
+    }
+}
+
+// Both operands of a 4x4 block at window position (wx, wy) lie inside the
+// window: x reads cover the aligned words from (wx + dx) & ~3 to +8, rows
+// wy + dy .. wy + dy + 3, with dx, dy <= 1.
+__device__ __forceinline__ bool win_covers(int wx, int wy) {
+    return wx >= 0 && ((wx + 1) & ~3) <= WIN_W - 8 && wy >= 0 && wy + 5 <= WIN_H;
+}
+
+// The preset's knobs as the general search reads them.
+struct Knobs {
+    const MeParamsDev& p;
+    // the next enabled rung of the diamond ladder after si (5: none)
+    __device__ __forceinline__ int next_rung(int si) const {
+        if (p.fast) return si + 1 >= 2 ? 5 : si + 1;
+        int n = si + 1;
+        while (n < 5 && !(p.dia_mask & (1u << n))) n++;
+        return n;
+    }
+    __device__ __forceinline__ int rung_step(int si) const {
+        return p.fast ? (si == 0 ? 16 : 4) : (64 >> si);  // rungs [64,32,16,8,4] quarter-pel
+    }
+    // rate of an MV against the mvd centre (mb16.rs:2454-2482)
+    __device__ __forceinline__ uint32_t rate(int dx, int dy) const { return mvbits(p.kind, p.tab, dx) + mvbits(p.kind, p.tab, dy); }
+};
+
+// ---------------------------------------------------------------------------
+// Pricing
+// ---------------------------------------------------------------------------
+
+// A lane's view of the MB's searches.  px, py, rw, rh: its group's partition;
+// wox, woy: that partition's origin in window coordinates (WIN_OFF: no
+// window); src: the source words of row lane % 4 of the pass's sixteen blocks.
+struct MbLane {
+    int lane, gl, gb;
+    int px, py, rw, rh, wox, woy, gather;
+    uint32_t winq;
+    HadFrag had;
+    uint32_t src[16];
+};
+
+// The lane's share of the source MB (row lane % 4 of each block row, 16 bytes).
+__device__ __forceinline__ void mb_load_src(MbLane& s, const uint8_t* src, int cw, int lx, int ly) {
+    const int q = threadIdx.x & 3;
+    const uint8_t* p = src + (long long)(ly + q) * cw + lx;
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {  // cw is a multiple of 16
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(p + (long long)(4 * b) * cw));
+            s.src[4 * b] = v.x; s.src[4 * b + 1] = v.y; s.src[4 * b + 2] = v.z; s.src[4 * b + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; i++) s.src[i] = ld4u(p + (long long)(4 * (i >> 2)) * cw + 4 * (i & 3));
+    }
+}
+
+// The partition's place in the staged window (ws.wx0, ws.wy0), or no window.
+__device__ __forceinline__ void mb_lane_window(MbLane& s, const MbScratch& ws, bool win_ok) {
+    s.wox = win_ok ? s.px + ws.pad - ws.wx0 : WIN_OFF;
+    s.woy = win_ok ? s.py + ws.pad - ws.wy0 : WIN_OFF;
+}
+
+// Mode 0: the 16x16 search (source words loaded by mb_load_src).
+__device__ __forceinline__ void mb_lane_16x16(MbLane& s, int lx, int ly, uint32_t win) {
+    const int lane = threadIdx.x & 31;
+    s.lane = lane;
+    s.gl = lane & 7;
+    s.gb = lane & 24;
+    s.px = lx; s.py = ly; s.rw = 16; s.rh = 16;
+    s.winq = win + uint32_t((lane & 3) * WIN_STRIDE);
+    s.gather = (s.gl >> 1) + 16 * (s.gl & 1);
+    s.had = had_frag(lane);
+}
+
+// Mode 1 after mode 0: the lane's group's partition of the same MB.
+__device__ __forceinline__ void mb_lane_parts(MbLane& s) {
+    const int g = s.lane >> 3;
+    const bool tall = g >= 2;  // 8x16
+    const int ox = g == 3 ? 8 : 0, oy = g == 1 ? 8 : 0;
+    s.px += ox; s.py += oy;
+    s.wox += ox; s.woy += oy;
+    s.rw = tall ? 8 : 16;
+    s.rh = tall ? 16 : 8;
+    s.gather = g + 8 * ((s.gl >> 1) & 1) + 16 * (s.gl & 1);
+    uint32_t t[8];
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const uint32_t wide = g == 1 ? s.src[8 + 2 * b + i] : s.src[2 * b + i];
+            const uint32_t high = g == 3 ? s.src[4 * b + 2 + i] : s.src[4 * b + i];
+            t[2 * b + i] = tall ? high : wide;
+        }
+#pragma unroll
+    for (int i = 0; i < 8; i++) s.src[i] = t[i];
+}
+
+// Where candidates are read: the MB's window in shared memory, or (launch
+// shapes without a window) the reference's planes in global memory.
+template <bool STAGE>
+struct RefSrc;
+template <>
+struct RefSrc<true> {
+    using Addr = uint32_t;
+    static __device__ __forceinline__ uint32_t ld(Addr a) { return lds_u32(a); }
+    static __device__ __forceinline__ uint32_t stride(const MbScratch&) { return WIN_STRIDE; }
+    static __device__ __forceinline__ Addr safe(const MbLane& s, const MbScratch&) { return s.winq; }
+};
+template <>
+struct RefSrc<false> {
+    using Addr = const uint8_t*;
+    static __device__ __forceinline__ uint32_t ld(Addr a) { return __ldg(reinterpret_cast<const uint32_t*>(a)); }
+    static __device__ __forceinline__ uint32_t stride(const MbScratch& ws) { return uint32_t(ws.pw); }
+    static __device__ __forceinline__ Addr safe(const MbLane& s, const MbScratch& ws) { return ws.base + (long long)(s.lane & 3) * ws.pw; }
+};
+__device__ __forceinline__ uint32_t align4(uint32_t a) { return a & ~3u; }
+__device__ __forceinline__ const uint8_t* align4(const uint8_t* a) {
+    return reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(a) & ~uintptr_t(3));
+}
+__device__ __forceinline__ uint32_t shift8(uint32_t a) { return a * 8u; }  // the funnel shift takes it modulo 32
+__device__ __forceinline__ uint32_t shift8(const uint8_t* a) { return uint32_t(reinterpret_cast<uintptr_t>(a)) * 8u; }
+
+// A candidate's operands: byte addresses a (and b, equal to a at one-plane
+// phases) of the lane's row of the partition's first block; a safe address
+// when the reads are not covered (the window, or the planes, do not hold them).
+template <bool STAGE>
+struct CandAddr {
+    typename RefSrc<STAGE>::Addr a, b;
+    bool covered;
+};
+template <bool STAGE>
+__device__ __forceinline__ CandAddr<STAGE> cand_addr(const MbLane& s, const MbScratch& ws, uint32_t lut, int mvx, int mvy) {
+    CandAddr<STAGE> t;
+    if constexpr (STAGE) {
+        uint2 ent;
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(ent.x), "=r"(ent.y) : "r"(lut + uint32_t(((mvx & 3) * 4 + (mvy & 3)) * 8)));
+        const int wx = s.wox + (mvx >> 2), wy = s.woy + (mvy >> 2);
+        t.covered = unsigned(wx) <= unsigned(WIN_W - 5 - s.rw) && unsigned(wy) <= unsigned(WIN_H - 1 - s.rh);
+        const uint32_t base = t.covered ? s.winq + uint32_t(wy * WIN_STRIDE + wx) : s.winq;
+        t.a = base + ent.x;
+        t.b = base + ent.y;
+    } else {
+        const uint32_t pb = phase_bits(mvx & 3, mvy & 3);
+        const long long ps = (long long)ws.pw * ws.ph;
+        const int x = s.px + ws.pad + (mvx >> 2), y = s.py + ws.pad + (mvy >> 2);
+        t.covered = x >= 0 && y >= 0 && x + s.rw + 5 <= ws.pw && y + s.rh + 1 <= ws.ph;
+        const uint8_t* base = ws.base + (long long)(s.lane & 3) * ws.pw + (t.covered ? (long long)y * ws.pw + x : 0);
+        t.a = base + ps * (pb & 3u) + ((pb & 32u) ? ws.pw : 0) + ((pb >> 4) & 1u);
+        t.b = ((pb >> 2) & 3u) ? base + ps * ((pb >> 2) & 3u) + ((pb & 128u) ? ws.pw : 0) + ((pb >> 6) & 1u) : t.a;
+    }
+    return t;
+}
+
+// One word (4 pixels of a row) of the prediction at picture position (x, y)
+// for MV (mvx, mvy), from the planes with every coordinate clamped where it
+// leaves them: pred_rows for one row.
+__device__ __noinline__ static uint32_t plane_word(const MbScratch& ws, int x, int y, int mvx, int mvy) {
+    const int fx = mvx & 3, fy = mvy & 3, px = x + (mvx >> 2) + ws.pad, py = y + (mvy >> 2) + ws.pad;
+    const int pw = ws.pw, ph = ws.ph;
+    const long long ps = (long long)pw * ph;
+    const bool cg = ws.bw != nullptr;
+    const uint32_t pb = phase_bits(fx, fy);
+    const int pa = int(pb & 3), pbb = int((pb >> 2) & 3);
+    uint32_t out[2];
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+        const uint8_t* P = ws.base + ps * (k ? pbb : pa);
+        const int xo = px + int((pb >> (k ? 6 : 4)) & 1), yo = py + int((pb >> (k ? 7 : 5)) & 1);
+        const uint8_t* row = P + (long long)clampi(yo, 0, ph - 1) * pw;
+        uint32_t w = 0;
+        if (xo >= 0 && xo + 8 <= pw) {
+            const uintptr_t ad = reinterpret_cast<uintptr_t>(row + xo);
+            const uint32_t* p = reinterpret_cast<const uint32_t*>(ad & ~uintptr_t(3));
+            w = __funnelshift_r(ldw(p, cg), ldw(p + 1, cg), uint32_t(ad & 3) * 8u);
+        } else {
+#pragma unroll 1
+            for (int c = 0; c < 4; c++) w |= uint32_t(ldb(row + clampi(xo + c, 0, pw - 1), cg)) << (8 * c);
+        }
+        out[k] = w;
+        if (pbb == 0) return w;
+    }
+    return avg_up4(out[0], out[1]);
+}
+
+// Rows of the 4x4 block at (x, y) under an MV from the planes (pred_rows), for
+// the MB in a hundred whose pick its window does not cover.
+__device__ __noinline__ static uint4 plane_rows(const MbScratch* ws, int x, int y, int mvx, int mvy) {
+    uint4 r;
+    r.x = plane_word(*ws, x, y, mvx, mvy);
+    r.y = plane_word(*ws, x, y + 1, mvx, mvy);
+    r.z = plane_word(*ws, x, y + 2, mvx, mvy);
+    r.w = plane_word(*ws, x, y + 3, mvx, mvy);
+    return r;
+}
+
+// A pass some of whose candidates' reads are not covered, word by word from
+// the planes; ax, ay / bx, by: the column's MVs in tiles A and B (mode 0: A)
+// of the rw-wide partition at (px, py).  Returns the shares of the column sums
+// as a0 | a1 << 16, b0 | b1 << 16 (each below 2^16: 8 blocks of at most 2 x
+// 4,080), and the row SADs of both tiles.  Out of line, with nothing of the
+// search's state in memory: about one pass in a hundred needs it.
+template <int MODE>
+__device__ __noinline__ int4 slow_pass(MbScratch* ws, int px, int py, int rw, int ax, int ay, int bx, int by, bool wait) {
+    const int lane = threadIdx.x & 31, rh = MODE == 0 ? 16 : 24 - rw;
+    if (wait) band_wait_px(ws->bw, &ws->bready, py + (max(ay, by) >> 2) + rh + 1, px + (max(ax, bx) >> 2) + rw + 1);
+    __syncwarp();
+    const HadFrag had = had_frag(lane);
+    int4 out = make_int4(0, 0, 0, 0);
+#pragma unroll 1
+    for (int j = 0; j < 16; j++) {
+        const bool second = j >= 8;
+        const int k = MODE == 0 ? j : j & 7;
+        // block k of the pass: 16 wide, four a row; 8 wide, two
+        const int xo = MODE == 0 || rw == 16 ? 4 * (k & 3) : 4 * (k & 1), yo = MODE == 0 || rw == 16 ? 4 * (k >> 2) : 4 * (k >> 1);
+        const int x = px + xo, y = py + yo + (lane & 3);
+        const uint32_t sw = ld4u(ws->src + (long long)y * ws->cw + x);
+        const uint32_t pw = plane_word(*ws, x, y, MODE == 1 && second ? bx : ax, MODE == 1 && second ? by : ay);
+        __syncwarp();
+        int t0 = 0, t1 = 0;
+        had_mma(had, pw, sw, t0, t1);
+        const int t = t0 | (t1 << 16), sd = int(__vsadu4(pw, sw));
+        if (second) { out.y += t; out.w += sd; }
+        else { out.x += t; out.z += sd; }
+    }
+    return out;
+}
+
+// The sixteen words of a pass: mode 0 the candidate's (four block rows of
+// five aligned words), mode 1 tile A's and tile B's eight (four pairs of
+// adjacent blocks, three words each).
+template <int MODE, bool STAGE>
+__device__ __forceinline__ void pass_words(const MbLane& s, const MbScratch& ws, typename RefSrc<STAGE>::Addr a0,
+                                           typename RefSrc<STAGE>::Addr b0, uint32_t p[16]) {
+    using R = RefSrc<STAGE>;
+    const auto a = align4(a0);
+    const uint32_t sa = shift8(a0);
+    if constexpr (MODE == 0) {
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            uint32_t w[5];
+#pragma unroll
+            for (int i = 0; i < 5; i++) w[i] = R::ld(a + (r * 4 * R::stride(ws) + 4 * i));
+#pragma unroll
+            for (int i = 0; i < 4; i++) p[4 * r + i] = __funnelshift_r(w[i], w[i + 1], sa);
+        }
+    } else {
+        const auto b = align4(b0);
+        const uint32_t sb = shift8(b0);
+        const uint32_t o1 = s.rw == 8 ? 4 * R::stride(ws) : 8u, o2 = (s.rw == 8 ? 8 : 4) * R::stride(ws);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const auto ad = (k < 4 ? a : b) + ((k & 1) ? o1 : 0u) + ((k & 2) ? o2 : 0u);
+            const uint32_t w0 = R::ld(ad), w1 = R::ld(ad + 4), w2 = R::ld(ad + 8);
+            p[2 * k] = __funnelshift_r(w0, w1, k < 4 ? sa : sb);
+            p[2 * k + 1] = __funnelshift_r(w1, w2, k < 4 ? sa : sb);
+        }
+    }
+}
+
+// One pass: the lane's column's candidates at ta (tile A) and, mode 1, tb
+// (tile B) -- MVs ax, ay and bx, by -- give the lane's shares of
+// the column sums in a0, a1 (columns 2q, 2q+1 of tile A; mode 0: of the whole
+// candidate) and b0, b1 (tile B), and with SADS the lane's row SADs in sa, sb.
+// two: a two-plane phase is possible.  idle: the group has no slots (its
+// addresses are safe and its sums are not used).
+template <int MODE, bool STAGE, bool SADS>
+__device__ __forceinline__ void price_pass(const MbLane& s, MbScratch& ws, const CandAddr<STAGE>& ta, const CandAddr<STAGE>& tb,
+                                           int ax, int ay, int bx, int by, bool two, bool idle, int& a0, int& a1, int& b0,
+                                           int& b1, int& sa, int& sb) {
+    uint32_t p[16];
+    pass_words<MODE, STAGE>(s, ws, ta.a, tb.a, p);
+    if (two) {
+        uint32_t r[16];
+        pass_words<MODE, STAGE>(s, ws, ta.b, tb.b, r);
+#pragma unroll
+        for (int i = 0; i < 16; i++) p[i] = avg_up4(p[i], r[i]);
+    }
+    a0 = a1 = b0 = b1 = sa = sb = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        had_mma(s.had, p[i], s.src[i], a0, a1);
+        had_mma(s.had, p[8 + i], s.src[MODE == 0 ? 8 + i : i], b0, b1);
+    }
+    if (SADS) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            sa += int(__vsadu4(p[i], s.src[i]));
+            sb += int(__vsadu4(p[8 + i], s.src[MODE == 0 ? 8 + i : i]));
+        }
+    }
+    const bool miss = !idle && !(ta.covered && (MODE == 0 || tb.covered));
+    if (__any_sync(0xffffffffu, miss)) {
+        const int4 r = slow_pass<MODE>(&ws, s.px, s.py, s.rw, ax, ay, bx, by, miss);
+        a0 = r.x & 0xffff; a1 = int(uint32_t(r.x) >> 16);
+        b0 = r.y & 0xffff; b1 = int(uint32_t(r.y) >> 16);
+        sa = r.z; sb = r.w;
+    }
+    if (MODE == 0) { a0 += b0; a1 += b1; sa += sb; }
+}
+
+// Distortions of the group's slots 0..n-1 (nmax: the largest n of the
+// groups, nmax <= 8; n = 0: none) under the MVs the lanes hold (lane gl of a
+// group: slot gl), returned to the slots' lanes.  `sad`: this group's metric
+// is SAD.
+template <int MODE>
+__device__ __forceinline__ int price_slots(const MbLane& s, MbScratch& ws, uint32_t lut, int mvx, int mvy, int n, int nmax,
+                                           bool sad) {
+    constexpr bool one = MODE == 0;
+    int out = 0;
+#pragma unroll 1
+    for (int tp = 0; tp < (one ? 1 : (nmax + 3) >> 2); tp++) {
+        // the column's slots in tiles A and B (unused ones repeat slot 0)
+        int ca = one ? s.lane >> 2 : 4 * tp + ((s.lane >> 2) & 1);
+        int cb = ca + 2;
+        ca = ca < n ? ca : 0;
+        cb = cb < n ? cb : 0;
+        const int ax = __shfl_sync(0xffffffffu, mvx, s.gb + ca), ay = __shfl_sync(0xffffffffu, mvy, s.gb + ca);
+        const int bx = __shfl_sync(0xffffffffu, mvx, s.gb + cb), by = __shfl_sync(0xffffffffu, mvy, s.gb + cb);
+        const CandAddr<true> ta = cand_addr<true>(s, ws, lut, ax, ay), tb = cand_addr<true>(s, ws, lut, bx, by);
+        const bool two = __any_sync(0xffffffffu, ta.a != ta.b || (!one && tb.a != tb.b));
+        int a0, a1, b0, b1, sa, sb;
+        price_pass<MODE, true, true>(s, ws, ta, tb, ax, ay, bx, by, two, n == 0, a0, a1, b0, b1, sa, sb);
+        // columns 2q, 2q+1 of tiles A and B, summed over the lanes of each
+        // column: lane bit 4 keeps the odd column, in mode 1 bit 3 tile B
+        const bool hi = (s.lane & 16) != 0, up = (s.lane & 8) != 0;
+        const int ka = (hi ? a1 : a0) + __shfl_xor_sync(0xffffffffu, hi ? a0 : a1, 16);
+        const int kb = one ? ka : (hi ? b1 : b0) + __shfl_xor_sync(0xffffffffu, hi ? b0 : b1, 16);
+        int v = (up ? kb : ka) + __shfl_xor_sync(0xffffffffu, up ? ka : kb, 8);
+        v += __shfl_xor_sync(0xffffffffu, v, 4);
+        v = __shfl_sync(0xffffffffu, v, s.gather);
+        // SAD of a column: its four lanes' rows
+        sa += __shfl_xor_sync(0xffffffffu, sa, 1);
+        sa += __shfl_xor_sync(0xffffffffu, sa, 2);
+        sb += __shfl_xor_sync(0xffffffffu, sb, 1);
+        sb += __shfl_xor_sync(0xffffffffu, sb, 2);
+        const int at = one ? 4 * s.gl : s.gb + 4 * (s.gl & 1);
+        const int va = __shfl_sync(0xffffffffu, sa, at), vb = __shfl_sync(0xffffffffu, sb, at);
+        if (sad) v = one || !(s.gl & 2) ? va : vb;
+        if (one || (s.gl >> 2) == tp) out = v;
+    }
+    return out;
+}
+
+// The eight ring points (dx, dy) in the reference's order: (1,0) (-1,0) (0,1)
+// (0,-1) (1,1) (-1,-1) (1,-1) (-1,1); the four-point diamond is the first four.
+// Packed two bits per point as d+1, so a lane computes its point without a
+// memory lookup.
+constexpr uint32_t kRingXP = 0x2252u, kRingYP = 0x8225u;
+__device__ __forceinline__ int ring_dx(int i) { return int((kRingXP >> (2 * i)) & 3u) - 1; }
+__device__ __forceinline__ int ring_dy(int i) { return int((kRingYP >> (2 * i)) & 3u) - 1; }
+
+// Search phases and what an evaluation round's results are for.
+constexpr int PH_SEEDS = 0, PH_PROP = 1, PH_DIA = 2, PH_REPRICE = 3, PH_SUB = 4, PH_DONE = 5, PH_START = 6;
+constexpr int EV_START = 0, EV_SEEDS = 1, EV_PROP = 2, EV_FIXED = 3, EV_RING = 4, EV_REPRICE = 5;
+// Proposals of the learned search's 16x16 search.
+constexpr int N_PROP = 8;
+constexpr int LOOP_GUARD = 1 << 20;  // iterations of one rung / sub-pel step
+
+struct SearchOut {
+    int x, y, cost, evals;
+};
+
+// motion_search (mb16.rs:2433-3302) of each group's partition, every group at
+// once (mode 0: four copies of one search).  preds p0 (the mvd centre) and,
+// with npred 2, p1.  Returns the reference's evaluation count in evals.
+//
+// One loop around one pricing site: each iteration plans the next slots from
+// the phase state (seeds together with the snaps of sub-pel predictors,
+// diamond ladder, B2 reprice, sub-pel rings), prices them, and folds the
+// result back into the state.
+//  * fixed-centre batches (the FC diamond, sp_fc rings) price all points and
+//    take the first strict minimum, like the reference's argmin loops;
+//  * cascading rings (the centre moves mid-ring) price the remaining points
+//    against the current centre; at the first improvement the centre moves and
+//    the points after it are priced again around the new centre, which is the
+//    order in which the reference evaluates them.
+// Costs are dist + (λ·rate) as i64 held in 32 bits: distortions are below
+// 2^21 and λ·rate below 2^28 for every λ the encoder forms, so the sum never
+// saturates and comparisons match the reference's i64.
+//
+// LEARN with use_prop (the learned-proposal kernels' 16x16 search): after the
+// seeds, the 8 proposals (lane gl: proposal gl in `prop`) are priced with the
+// search's own cost; when the best proposal's distortion exceeds the
+// predictor's by more than prop_t the plain search goes on from the seeds
+// (fell = 1), otherwise it continues as motion_search with the cheapest of
+// predictor and proposals as its start vector (mb16.rs:2445, 2579-2596:
+// refine-only, no full-pel phase).  use_start: a refine-only search from
+// `start`.
+template <int MODE, bool LEARN>
+__device__ __forceinline__ SearchOut mb_search(const MbLane& s, const MeParamsDev& prm, MbScratch& ws, uint32_t lut, int2 p0, int2 p1,
+                                               int npred, double lambda_me, bool use_prop = false,
+                                               int2 prop = make_int2(0, 0), int prop_t = 0, int* fell = nullptr,
+                                               bool use_start = false, int2 start = make_int2(0, 0)) {
+    const Knobs kn{prm};
+    const int gl = s.gl, gb = s.gb;
+    constexpr bool one = MODE == 0;
+    const int rmax = one ? 8 : 4;      // points of a cascading ring priced per round: one pass
+    const bool sadfp = !prm.fast && prm.sadfp;
+    const int m_main = prm.use_sad ? MET_SAD : MET_SATD;
+    const int m_fp = sadfp ? MET_SAD : m_main;
+    const double lam_r = prm.kind != 0 ? lambda_me * 0.25 : lambda_me;  // cost's λ
+    const double lam_fp = lambda_me * (sadfp ? prm.sadfp_lambda : 1.0); // cost_fp's λ under the 16-wide FC diamond
+    const double l_fp = sadfp ? lam_fp : lam_r;
+    const bool fc = !prm.fast && prm.fc;
+    const int spat = prm.subpel_pat >= 0 ? prm.subpel_pat : (prm.sp_single_pass ? 2 : 0);
+    const bool sp_fc = prm.sp_fc && !prm.fast;
+    const int sp_nring = (spat & 1) ? 4 : 8;
+    const int rw = s.rw, rh = s.rh, cw = ws.cw, ch = ws.ch;
+
+    // Seed slots: 0 the zero MV, 1 p0, 2 p1 when it differs, then with the
+    // integer snap on the snapped positions of the sub-pel predictors
+    // (mb16.rs:2597-2607); equal positions share a slot (equal costs).
+    const bool two = npred > 1 && (p1.x != p0.x || p1.y != p0.y);
+    const int2 q0 = make_int2(((p0.x + 2) >> 2) * 4, ((p0.y + 2) >> 2) * 4);
+    const int2 q1 = make_int2(((p1.x + 2) >> 2) * 4, ((p1.y + 2) >> 2) * 4);
+    const bool snap0 = prm.me_snap && ((p0.x | p0.y) & 3) != 0;
+    const bool snap1 = two && prm.me_snap && ((p1.x | p1.y) & 3) != 0;
+    const int i_q0 = two ? 3 : 2;
+    const bool q_same = snap0 && q0.x == q1.x && q0.y == q1.y;
+    const int i_q1 = q_same ? i_q0 : i_q0 + (snap0 ? 1 : 0);
+    const int n_seed = i_q0 + (snap0 ? 1 : 0) + (snap1 && !q_same ? 1 : 0);
+    auto inside = [&](int x, int y, int step) {  // every point of the ring at full-pel distance inside the picture
+        const int st = step >> 2, px = s.px + (x >> 2), py = s.py + (y >> 2);
+        return px - st >= 0 && py - st >= 0 && px + st + rw <= cw && py + st + rh <= ch;
+    };
+
+    int evals = 0;
+    int bx = 0, by = 0, seed_x = 0, seed_y = 0;
+    int best_c = 0, seed_c = 0;
+    int cp = 0, dp = 0;  // the predictor's cost and distortion (learned search)
+    int phase = use_start ? PH_START : PH_SEEDS;
+    int si = -1, sk = -1, loops = 0, iter = 0, step = 0;
+    bool ring_open = false, ring_improved = false;
+    int ring_i = 0, ring_n = 0;
+    for (;;) {
+        // ---------- plan (per group) ----------
+        int kind = -1, n = 0, metric = m_main;
+        int mx = bx, my = by;  // the lane's slot
+        double lam = lam_r;
+        while (kind < 0 && phase != PH_DONE) {
+            if (phase == PH_SEEDS) {
+                kind = EV_SEEDS; n = n_seed; metric = m_fp; lam = l_fp;
+                mx = my = 0;
+                if (gl == 1) { mx = p0.x; my = p0.y; }
+                if (two && gl == 2) { mx = p1.x; my = p1.y; }
+                if (snap0 && gl == i_q0) { mx = q0.x; my = q0.y; }
+                else if (snap1 && gl == i_q1) { mx = q1.x; my = q1.y; }
+            } else if (LEARN && phase == PH_PROP) {
+                mx = prop.x; my = prop.y;
+                kind = EV_PROP; n = N_PROP;
+            } else if (phase == PH_START) {
+                mx = start.x; my = start.y;
+                kind = EV_START; n = 1;
+            } else if (phase == PH_DIA) {
+                if (ring_open) {
+                    kind = EV_RING; n = min(ring_n - ring_i, rmax); metric = m_fp; lam = l_fp;
+                    break;
+                }
+                if (si < 0 || loops >= LOOP_GUARD) {
+                    const int nsi = kn.next_rung(si);
+                    if (nsi >= 5) {
+                        phase = PH_REPRICE;
+                        continue;
+                    }
+                    si = nsi;
+                    step = kn.rung_step(si);
+                    loops = 0;
+                }
+                loops++;
+                if (fc && ((bx | by) & 3) == 0 && inside(bx, by, step)) {
+                    kind = EV_FIXED; n = 4;
+                    metric = rw == 16 ? (sadfp ? MET_SAD : MET_SATD) : m_fp;
+                    lam = rw == 16 ? lam_fp : l_fp;
+                    mx = bx + ring_dx(gl & 3) * step;
+                    my = by + ring_dy(gl & 3) * step;
+                } else {
+                    ring_open = true; ring_improved = false; ring_i = 0; ring_n = 4;
+                    kind = EV_RING; n = 4; metric = m_fp; lam = l_fp;
+                }
+            } else if (phase == PH_REPRICE) {
+                if (sadfp) {
+                    if (gl == 1) { mx = seed_x; my = seed_y; }
+                    kind = EV_REPRICE; n = 2;
+                } else {
+                    phase = PH_SUB;
+                }
+            } else {  // PH_SUB
+                if (ring_open) {
+                    kind = EV_RING; n = min(ring_n - ring_i, rmax);
+                    break;
+                }
+                if (!prm.subpel) {
+                    phase = PH_DONE;
+                    continue;
+                }
+                if (sk < 0 || loops >= LOOP_GUARD) {
+                    if (++sk >= 2) {
+                        phase = PH_DONE;
+                        continue;
+                    }
+                    step = sk == 0 ? 2 : 1;
+                    loops = 0;
+                    iter = 0;
+                }
+                loops++;
+                iter++;
+                if (sp_fc && (spat & 1) == 0 && (step == 1 || ((bx | by) & 3) == 0)) {
+                    // hpel_qpel_refs / hpel_ref resolve every ring point (inter.rs:1015, 1060):
+                    // inside the +1-slack window, and at step 1 a quarter phase
+                    bool all = true;
+                    for (int i = 0; i < 8; i++) {
+                        const int rx = bx + ring_dx(i) * step, ry = by + ring_dy(i) * step;
+                        const int px = s.px + (rx >> 2) + ws.pad, py = s.py + (ry >> 2) + ws.pad;
+                        all = all && px >= 0 && py >= 0 && px + rw + 1 <= ws.pw && py + rh + 1 <= ws.ph &&
+                              (step == 2 || ((rx | ry) & 1));
+                    }
+                    if (all) {
+                        mx = bx + ring_dx(gl) * step;
+                        my = by + ring_dy(gl) * step;
+                        kind = EV_FIXED; n = 8;
+                        metric = rw == 16 ? MET_SATD : m_main;
+                        lam = rw == 16 ? lambda_me : lam_r;
+                        break;
+                    }
+                }
+                ring_open = true; ring_improved = false; ring_i = 0; ring_n = sp_nring;
+                kind = EV_RING; n = min(sp_nring, rmax);
+            }
+        }
+        if (kind == EV_RING && gl < n) {
+            mx = bx + ring_dx(ring_i + gl) * step;
+            my = by + ring_dy(ring_i + gl) * step;
+        }
+        if (kind < 0) n = 0;
+        if (__all_sync(0xffffffffu, kind < 0)) break;
+        const int nmax = one ? n : __reduce_max_sync(0xffffffffu, n);
+        // which collectives this round's folds need (warp-uniform)
+        const bool need_min = __any_sync(0xffffffffu, kind == EV_FIXED || kind == EV_PROP);
+        const bool need_hit = __any_sync(0xffffffffu, kind == EV_RING);
+        const bool need_seed = __any_sync(0xffffffffu, kind == EV_SEEDS || kind == EV_REPRICE || kind == EV_START);
+
+        // ---------- price ----------
+        const long long rc = lam_cost(lam, kn.rate(mx - p0.x, my - p0.y));
+        const int d = price_slots<MODE>(s, ws, lut, mx, my, n, nmax, metric == MET_SAD);
+        int cc = INT_MAX;  // dist + λ·rate of the lane's slot
+        if (gl < n) {
+            const long long c = (long long)d + rc;
+            cc = c > INT_MAX - 1 ? INT_MAX - 1 : int(c);
+        }
+        // group-wide collectives, taken by every lane: the first minimum of
+        // slots 0..3 and of 4..7, the first improving slot, the seed slots
+        int m0 = INT_MAX, m1 = INT_MAX;
+        unsigned at = 0;
+        if (need_min) {
+            int t = min(cc, __shfl_xor_sync(0xffffffffu, cc, 1));
+            t = min(t, __shfl_xor_sync(0xffffffffu, t, 2));
+            m0 = __shfl_sync(0xffffffffu, t, gb);
+            m1 = __shfl_sync(0xffffffffu, t, gb + 4);
+            at = (__ballot_sync(0xffffffffu, cc == t) >> gb) & 0xffu;
+        }
+        unsigned hit = 0;
+        int jhit = 0, cj = 0;
+        if (need_hit) {
+            hit = (__ballot_sync(0xffffffffu, gl < n && cc < best_c) >> gb) & 0xffu;
+            jhit = hit ? __ffs(hit) - 1 : 0;
+            cj = __shfl_sync(0xffffffffu, cc, gb + jhit);
+        }
+        int c_seed[5] = {0, 0, 0, 0, 0};
+        if (need_seed) {
+#pragma unroll
+            for (int i = 0; i < 5; i++) c_seed[i] = __shfl_sync(0xffffffffu, cc, gb + i);
+            if (LEARN) dp = __shfl_sync(0xffffffffu, d, gb + 1);
+        }
+
+        // ---------- fold (per group) ----------
+        if (kind == EV_SEEDS) {
+            // sequential strict-< scan: (0,0) first, then the predictors in order
+            best_c = c_seed[0];
+            bx = 0; by = 0;
+            int wi = 0;
+            if (c_seed[1] < best_c) { best_c = c_seed[1]; bx = p0.x; by = p0.y; wi = 1; }
+            if (two && c_seed[2] < best_c) { best_c = c_seed[2]; bx = p1.x; by = p1.y; wi = 2; }
+            cp = c_seed[1];
+            evals += npred + 1;
+            seed_x = bx; seed_y = by; seed_c = best_c;
+            if ((wi == 1 && snap0) || (wi == 2 && snap1)) {
+                // the winner is a sub-pel predictor: take its snap, priced in this round
+                bx = wi == 1 ? q0.x : q1.x;
+                by = wi == 1 ? q0.y : q1.y;
+                const int k = wi == 1 ? i_q0 : i_q1;
+                best_c = k == 2 ? c_seed[2] : (k == 3 ? c_seed[3] : c_seed[4]);
+                evals += 1;
+            }
+            phase = LEARN && use_prop ? PH_PROP : PH_DIA;
+        } else if (kind == EV_START) {
+            // a refine-only search (mb16.rs:2580-2582): the start vector
+            // priced with `cost`, no full-pel phase, the sub-pel steps from it
+            best_c = c_seed[0];
+            bx = start.x;
+            by = start.y;
+            seed_x = bx; seed_y = by; seed_c = best_c;
+            evals += 1;
+            phase = PH_SUB;
+        } else if (LEARN && kind == EV_PROP) {
+            // the cheapest proposal (first wins) and its distortion against the predictor's
+            const int m = min(m0, m1);
+            const unsigned bits = m0 == m ? at & 0xfu : at & 0xf0u;
+            const int bi = __ffs(bits) - 1;
+            const int dprop = __shfl_sync(0xffffffffu, d, gb + bi);  // mode 0: every lane is here
+            const int vx = __shfl_sync(0xffffffffu, prop.x, gb + bi), vy = __shfl_sync(0xffffffffu, prop.y, gb + bi);
+            const bool fb = (long long)dprop > (long long)dp + prop_t;
+            if (fell) *fell = fb ? 1 : 0;
+            evals += fb ? N_PROP + 1 : N_PROP + 1 - evals;
+            if (fb) {
+                phase = PH_DIA;  // the plain search goes on from its seeds
+            } else {
+                best_c = cp;
+                bx = p0.x; by = p0.y;
+                if (m < best_c) { best_c = m; bx = vx; by = vy; }
+                seed_x = bx; seed_y = by; seed_c = best_c;
+                phase = PH_SUB;  // a start vector: no full-pel phase, no B2 reprice
+            }
+        } else if (kind == EV_REPRICE) {
+            best_c = c_seed[0];
+            seed_c = c_seed[1];
+            evals += 2;
+            phase = PH_SUB;
+        } else if (kind == EV_FIXED) {
+            if (phase == PH_DIA) {
+                evals += 4;
+                if (m0 < best_c) {
+                    const int bi = __ffs(at & 0xfu) - 1;
+                    best_c = m0;
+                    bx += ring_dx(bi) * step;
+                    by += ring_dy(bi) * step;
+                } else {
+                    loops = LOOP_GUARD;  // rung done
+                }
+            } else {
+                evals += n;
+                const int m = min(m0, m1);
+                const int bi = m < best_c ? __ffs(m0 == m ? at & 0xfu : at & 0xf0u) - 1 : -1;
+                if (bi >= 0) {
+                    best_c = m;
+                    bx += ring_dx(bi) * step;
+                    by += ring_dy(bi) * step;
+                }
+                if (bi < 0 || !prm.me_subpel_iter || (spat & 2) || (prm.sp_maxit != 0 && iter >= prm.sp_maxit))
+                    loops = LOOP_GUARD;
+            }
+        } else if (kind == EV_RING) {
+            if (hit == 0) {
+                evals += n;
+                ring_i += n;
+            } else {
+                best_c = cj;
+                evals += jhit + 1;
+                bx += ring_dx(ring_i + jhit) * step;
+                by += ring_dy(ring_i + jhit) * step;
+                ring_improved = true;
+                ring_i += jhit + 1;
+            }
+            ring_open = ring_i < ring_n;
+            if (!ring_open) {
+                if (phase == PH_DIA) {
+                    if (!ring_improved) loops = LOOP_GUARD;
+                } else if (!ring_improved || !prm.me_subpel_iter || (spat & 2) ||
+                           (prm.sp_maxit != 0 && iter >= prm.sp_maxit)) {
+                    loops = LOOP_GUARD;
+                }
+            }
+        }
+        __syncwarp();
+    }
+    // ---- seed restore (mb16.rs:3297-3300) ----
+    if (prm.me_snap && seed_c < best_c) {
+        bx = seed_x; by = seed_y; best_c = seed_c;
+    }
+    return SearchOut{bx, by, best_c, evals};
+}
+
+// ---------------------------------------------------------------------------
+// The Balanced preset's searches
+// ---------------------------------------------------------------------------
+// mb_search above runs any preset.  The Balanced preset's 16x16 search, which
+// every MB runs and the wavefront waits for, has its own form, in which every
+// decision is warp-uniform: costs are compared through redux and ballots, a
+// lane forms its column's candidate from the round's centre, step and ring
+// index, the operand addresses come from a 16-entry table and the
+// λ·rate products from a table per λ, and one pass's column sums cross the
+// lanes through shared memory.  Host rule (balanced_search_ok): the preset's
+// knobs and 0 <= λ < 2^23, so that every table entry and cost fits 31 bits.
+
+constexpr int LAM_TAB = 48;  // (λ·rate) as i64 for rates below LAM_TAB
+
+// Per-warp tables and scratch of the Balanced searches.
+struct BalScratch {
+    double lam;             // the λ the table holds (NaN: none)
+    int lamtab[LAM_TAB];
+    int red[2][8][8];       // column sums' shares: [tile][lane / 4][column]
+};
+// Per-CTA operand table: byte offsets in the window of both operands of each
+// quarter phase fx * 4 + fy (equal at one-plane phases).
+struct PhaseTab {
+    uint2 e[16];
+};
+__device__ __forceinline__ void phase_tab_init(PhaseTab& t, int i) {
+    if (i >= 16) return;
+    const uint32_t pb = phase_bits(i >> 2, i & 3);
+    const uint32_t a = (pb & 3u) * WIN_PLANE + ((pb >> 5) & 1u) * WIN_STRIDE + ((pb >> 4) & 1u);
+    const uint32_t b = ((pb >> 2) & 3u) * WIN_PLANE + ((pb >> 7) & 1u) * WIN_STRIDE + ((pb >> 6) & 1u);
+    t.e[i] = make_uint2(a, ((pb >> 2) & 3u) ? b : a);
+}
+__device__ __forceinline__ void bal_lambda(BalScratch& b, double lambda_me) {
+    if (b.lam == lambda_me) return;  // warp-uniform
+    __syncwarp();
+    for (int r = int(threadIdx.x & 31); r < LAM_TAB; r += 32) b.lamtab[r] = int(lam_cost(lambda_me, uint32_t(r)));
+    if ((threadIdx.x & 31) == 0) b.lam = lambda_me;
+    __syncwarp();
+}
+// Exp-Golomb bits of an mvd component (mb16.rs:2454-2482, kind 0)
+__device__ __forceinline__ uint32_t eg_bits(int d) {
+    const uint32_t v = uint32_t(d > 0 ? 2 * d : 1 - 2 * d);
+    return 63u - 2u * uint32_t(__clz(int(v)));
+}
+__device__ __forceinline__ int bal_rate_cost(const BalScratch& b, double lam, int dx, int dy) {
+    const uint32_t r = eg_bits(dx) + eg_bits(dy);
+    return r < LAM_TAB ? b.lamtab[r] : int(lam_cost(lam, r));
+}
+
+// The 16x16 search of the Balanced preset (predictor p0 the mvd centre), warp-uniform.
+// LEARN with use_prop: as mb_search's.  propc / propg: proposals lane / 4 and
+// lane % 8.
+template <bool LEARN, bool STAGE>
+__device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws, BalScratch& bs, uint32_t lut, int2 p0,
+                                                  double lambda_me, bool use_prop, int2 propc, int2 propg, int prop_t,
+                                                  int* fell) {
+    constexpr int SEED = 0, DIA = 1, RING = 2, PROP = 3;
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = s.lane, gl = s.gl, col = lane >> 2;
+    const int px = s.px, py = s.py, cw = ws.cw, ch = ws.ch;
+    bal_lambda(bs, lambda_me);
+    auto inside = [&](int x, int y, int st) {  // the ring's points at full-pel distance st inside the picture
+        const int ox = px + (x >> 2), oy = py + (y >> 2);
+        return ox - st >= 0 && oy - st >= 0 && ox + st + 16 <= cw && oy + st + 16 <= ch;
+    };
+    const int2 q0 = make_int2(((p0.x + 2) >> 2) * 4, ((p0.y + 2) >> 2) * 4);  // its integer snap
+    const bool sub = ((p0.x | p0.y) & 3) != 0;
+    const bool seed_ring = !(LEARN && use_prop) && inside(q0.x, q0.y, 4);
+    int evals = 0, best = 0, seed_c = 0, seed_x = 0, seed_y = 0, cp = 0, dp = 0;
+    int cx = q0.x, cy = q0.y, step = 16, kind = SEED, ri = 0, rn = 4;
+    bool improved = false;
+    for (;;) {
+        // the candidates of the lane's mma column and of its cost slot: SEED
+        // 0 the zero MV, 1 p0, 2 its snap, 4..7 the first rung's ring around
+        // the snap; DIA this rung's ring and the next's; RING the points from ri
+        int mx, my, rx, ry;
+        {
+            const int ic = kind == RING ? min(ri + col, 7) : col & 3, ig = kind == RING ? min(ri + gl, 7) : gl & 3;
+            const int sc = kind == DIA && col >= 4 ? step >> 1 : step, sg = kind == DIA && gl >= 4 ? step >> 1 : step;
+            mx = cx + ring_dx(ic) * sc; my = cy + ring_dy(ic) * sc;
+            rx = cx + ring_dx(ig) * sg; ry = cy + ring_dy(ig) * sg;
+            if (kind == SEED) {
+                if (col < 4 || !seed_ring) { mx = col == 0 ? 0 : (col == 1 ? p0.x : q0.x); my = col == 0 ? 0 : (col == 1 ? p0.y : q0.y); }
+                if (gl < 4 || !seed_ring) { rx = gl == 0 ? 0 : (gl == 1 ? p0.x : q0.x); ry = gl == 0 ? 0 : (gl == 1 ? p0.y : q0.y); }
+            }
+            if (LEARN && kind == PROP) { mx = propc.x; my = propc.y; rx = propg.x; ry = propg.y; }
+        }
+        const CandAddr<STAGE> ta = cand_addr<STAGE>(s, ws, lut, mx, my);
+        const int rc = bal_rate_cost(bs, lambda_me, rx - p0.x, ry - p0.y);
+        int a0, a1, b0, b1, sa, sb;
+        // a two-plane phase is possible among the seeds, at quarter-pel steps
+        // and, from a start vector, around a quarter-pel centre
+        const bool two = kind == SEED || step == 1 || (LEARN && (kind == PROP || ((cx | cy) & 1)));
+        price_pass<0, STAGE, false>(s, ws, ta, ta, mx, my, mx, my, two, false, a0, a1, b0, b1, sa, sb);
+        // column sums through shared memory: slot gl's eight shares
+        *reinterpret_cast<int2*>(&bs.red[0][col][2 * (lane & 3)]) = make_int2(a0, a1);
+        __syncwarp();
+        int d = 0;
+#pragma unroll
+        for (int g = 0; g < 8; g++) d += bs.red[0][g][gl];
+        const int cc = d + rc;
+        if (kind == RING) {
+            const unsigned hit = __ballot_sync(FULL, gl < rn - ri && cc < best) & 0xffu;
+            if (hit) {
+                const int j = __ffs(hit) - 1;
+                best = __reduce_min_sync(FULL, gl == j ? cc : INT_MAX);
+                evals += j + 1;
+                cx += ring_dx(ri + j) * step;
+                cy += ring_dy(ri + j) * step;
+                improved = true;
+                ri += j + 1;
+            } else {
+                evals += rn - ri;
+                ri = rn;
+            }
+            if (ri < rn) continue;  // the rest of the ring around the moved centre
+            if (!(step >= 4 && improved)) step >>= 1;
+        } else {
+            // the minima of slots 0..3 and 4..7 and their first slots
+            const int m0 = __reduce_min_sync(FULL, gl < 4 ? cc : INT_MAX), m1 = __reduce_min_sync(FULL, gl < 4 ? INT_MAX : cc);
+            const unsigned at = __ballot_sync(FULL, cc == (gl < 4 ? m0 : m1)) & 0xffu;
+            const int j0 = __ffs(at) - 1, j1 = __ffs(at >> 4) - 1;
+            if (kind == DIA) {
+                evals += 4;
+                if (m0 < best) {
+                    best = m0;
+                    cx += ring_dx(j0) * step;
+                    cy += ring_dy(j0) * step;
+                } else {
+                    step >>= 1;
+                    if (step >= 4) {  // the next rung's first ring, priced beside it
+                        evals += 4;
+                        if (m1 < best) {
+                            best = m1;
+                            cx += ring_dx(j1) * step;
+                            cy += ring_dy(j1) * step;
+                        } else {
+                            step >>= 1;
+                        }
+                    }
+                }
+            } else if (kind == SEED) {
+                // sequential strict-< scan: (0,0), then the predictor; the
+                // winner's integer snap is the centre
+                const int c0 = __reduce_min_sync(FULL, gl == 0 ? cc : INT_MAX), c1 = __reduce_min_sync(FULL, gl == 1 ? cc : INT_MAX),
+                          c2 = __reduce_min_sync(FULL, gl == 2 ? cc : INT_MAX);
+                if (LEARN) {
+                    cp = c1;
+                    dp = __reduce_min_sync(FULL, gl == 1 ? d : INT_MAX);
+                }
+                evals = 2;
+                if (c1 < c0) {
+                    best = seed_c = c1;
+                    seed_x = p0.x; seed_y = p0.y;
+                    if (sub) {
+                        best = c2;
+                        evals = 3;
+                    }
+                } else {
+                    best = seed_c = c0;
+                    cx = cy = 0;
+                }
+                if (LEARN && use_prop) {
+                    kind = PROP;
+                    continue;
+                }
+                if (seed_ring && cx == q0.x && cy == q0.y) {
+                    evals += 4;
+                    if (m1 < best) {
+                        best = m1;
+                        cx += ring_dx(j1) * 16;
+                        cy += ring_dy(j1) * 16;
+                    } else {
+                        step = 8;
+                    }
+                }
+            } else {  // PROP: the cheapest proposal (first wins) against the predictor
+                const int m = min(m0, m1), j = m0 == m ? j0 : 4 + j1;
+                const int dprop = __reduce_min_sync(FULL, gl == j ? d : INT_MAX);
+                const bool fb = dprop - dp > prop_t;
+                *fell = fb ? 1 : 0;
+                if (fb) {
+                    evals += N_PROP + 1;  // the plain search goes on from its seeds
+                } else {
+                    evals = N_PROP + 1;
+                    best = cp;
+                    cx = p0.x; cy = p0.y;
+                    if (m < cp) {
+                        best = m;
+                        cx = __shfl_sync(FULL, propg.x, j);
+                        cy = __shfl_sync(FULL, propg.y, j);
+                    }
+                    seed_c = best; seed_x = cx; seed_y = cy;
+                    step = 2;  // a start vector: the sub-pel steps only
+                }
+            }
+        }
+        if (step == 0) break;
+        improved = false;
+        ri = 0;
+        rn = step >= 4 ? 4 : 8;
+        kind = step >= 4 && inside(cx, cy, step >> 2) ? DIA : RING;
+    }
+    // ---- seed restore (mb16.rs:3297-3300) ----
+    if (seed_c < best) {
+        cx = seed_x; cy = seed_y; best = seed_c;
+    }
+    return SearchOut{cx, cy, best, evals};
+}
+
+// The four partitions of the Balanced preset, group g of eight lanes searching
+// partition g (mode 1): seeds (0,0), p0 (the mvd centre), p1, then as
+// search16_bal, four slots a round.  use_start: refine-only from `start`.
+template <bool LEARN, bool STAGE>
+__device__ __forceinline__ SearchOut search_parts_bal(const MbLane& s, MbScratch& ws, BalScratch& bs, uint32_t lut, int2 p0,
+                                                      int2 p1, double lambda_me, bool use_start, int2 start) {
+    constexpr int SEED = 0, DIA = 1, RING = 2, SNAP = 3, START = 4, DONE = 5;
+    constexpr unsigned FULL = 0xffffffffu;
+    const int gl = s.gl, gb = s.gb, sl = gl & 3, grp = gb >> 3, half = (s.lane >> 2) & 1;
+    const int px = s.px, py = s.py, cw = ws.cw, ch = ws.ch;
+    bal_lambda(bs, lambda_me);
+    auto inside = [&](int x, int y, int st) {
+        const int ox = px + (x >> 2), oy = py + (y >> 2);
+        return ox - st >= 0 && oy - st >= 0 && ox + st + s.rw <= cw && oy + st + s.rh <= ch;
+    };
+    auto snap = [](int v) { return ((v + 2) >> 2) * 4; };
+    const bool two = p1.x != p0.x || p1.y != p0.y;  // equal predictors: p1 cannot win
+    // seed slots: 0 the zero MV, 1 p0, 2 p1, 3 the snap of p1 (the likely winner)
+    const int2 q0 = make_int2(snap(p0.x), snap(p0.y)), q1 = make_int2(snap(p1.x), snap(p1.y));
+    const bool sub1 = ((p1.x | p1.y) & 3) != 0;
+    int evals = 0, best = 0, seed_c = 0, seed_x = 0, seed_y = 0;
+    int cx = 0, cy = 0, step = 16, kind = SEED, ri = 0, rn = 4;
+    bool improved = false;
+    if (LEARN && use_start) {
+        kind = START;
+        cx = seed_x = start.x;
+        cy = seed_y = start.y;
+    }
+    while (!__all_sync(FULL, kind == DONE)) {
+        // the MV of slot i of this round
+        auto slot_mv = [&](int i, int& x, int& y) {
+            const int ir = kind == RING ? min(ri + i, 7) : i;
+            x = cx + ring_dx(ir) * step;
+            y = cy + ring_dy(ir) * step;
+            if (kind == SEED) {
+                x = i == 0 ? 0 : (i == 1 ? p0.x : (i == 2 ? p1.x : q1.x));
+                y = i == 0 ? 0 : (i == 1 ? p0.y : (i == 2 ? p1.y : q1.y));
+            } else if (kind >= SNAP) {  // (DONE: a position the window covers)
+                x = cx;
+                y = cy;
+            }
+        };
+        int ax, ay, bx, by, rx, ry;
+        slot_mv(half, ax, ay);
+        slot_mv(half + 2, bx, by);
+        slot_mv(sl, rx, ry);
+        const CandAddr<STAGE> ta = cand_addr<STAGE>(s, ws, lut, ax, ay), tb = cand_addr<STAGE>(s, ws, lut, bx, by);
+        const int rc = bal_rate_cost(bs, lambda_me, rx - p0.x, ry - p0.y);
+        const bool planes2 = __any_sync(FULL, ta.a != ta.b || tb.a != tb.b);
+        int a0, a1, b0, b1, sa, sb;
+        price_pass<1, STAGE, false>(s, ws, ta, tb, ax, ay, bx, by, planes2, kind == DONE, a0, a1, b0, b1, sa, sb);
+        // column sums through shared memory: columns 2g, 2g+1 of tile A are
+        // slots 0, 1 of group g, of tile B slots 2, 3
+        *reinterpret_cast<int2*>(&bs.red[0][s.lane >> 2][2 * (s.lane & 3)]) = make_int2(a0, a1);
+        *reinterpret_cast<int2*>(&bs.red[1][s.lane >> 2][2 * (s.lane & 3)]) = make_int2(b0, b1);
+        __syncwarp();
+        int d = 0;
+#pragma unroll
+        for (int g = 0; g < 8; g++) d += bs.red[sl >> 1][g][2 * grp + (sl & 1)];
+        const int cc = d + rc;
+        // collectives of every group's fold
+        const int n = rn - ri < 4 ? rn - ri : 4;
+        const unsigned hit = (__ballot_sync(FULL, sl < n && cc < best) >> gb) & 0xfu;
+        const int jh = hit ? __ffs(hit) - 1 : 0;
+        int m = min(cc, __shfl_xor_sync(FULL, cc, 1));
+        m = min(m, __shfl_xor_sync(FULL, m, 2));
+        const int jm = __ffs((__ballot_sync(FULL, cc == m) >> gb) & 0xfu) - 1;
+        const int cj = __shfl_sync(FULL, cc, gb + jh);
+        const int c0 = __shfl_sync(FULL, cc, gb), c1 = __shfl_sync(FULL, cc, gb + 1), c2 = __shfl_sync(FULL, cc, gb + 2),
+                  c3 = __shfl_sync(FULL, cc, gb + 3);
+        __syncwarp();
+        bool next = false;  // the round's ring or rung is done
+        if (kind == RING) {
+            if (hit) {
+                best = cj;
+                evals += jh + 1;
+                cx += ring_dx(ri + jh) * step;
+                cy += ring_dy(ri + jh) * step;
+                improved = true;
+                ri += jh + 1;
+            } else {
+                evals += n;
+                ri += n;
+            }
+            next = ri >= rn;
+            if (next && !(step >= 4 && improved)) step >>= 1;
+        } else if (kind == DIA) {
+            evals += 4;
+            if (m < best) {
+                best = m;
+                cx += ring_dx(jm) * step;
+                cy += ring_dy(jm) * step;
+            } else {
+                step >>= 1;
+            }
+            next = true;
+        } else if (kind == SEED) {
+            // sequential strict-< scan: (0,0), p0, p1; a sub-pel winner's
+            // integer snap is the centre
+            evals = 3;
+            best = seed_c = c0;
+            next = true;
+            if (c1 < best) { best = seed_c = c1; cx = seed_x = p0.x; cy = seed_y = p0.y; }
+            if (two && c2 < best) { best = seed_c = c2; cx = seed_x = p1.x; cy = seed_y = p1.y; }
+            if (best == c2 && two && cx == p1.x && cy == p1.y && sub1) {
+                best = c3;
+                cx = q1.x; cy = q1.y;
+                evals = 4;
+            } else if ((cx | cy) & 3) {  // p0 won
+                evals = 4;
+                cx = q0.x; cy = q0.y;
+                if (cx == q1.x && cy == q1.y) {
+                    best = c3;
+                } else {
+                    kind = SNAP;  // price its snap
+                    next = false;
+                }
+            }
+        } else if (kind == SNAP) {
+            best = c0;
+            next = true;
+        } else if (LEARN && kind == START) {
+            best = seed_c = c0;
+            evals = 1;
+            step = 2;
+            next = true;
+        }
+        if (next) {
+            improved = false;
+            ri = 0;
+            rn = step >= 4 ? 4 : 8;
+            kind = step == 0 ? DONE : (step >= 4 && inside(cx, cy, step >> 2) ? DIA : RING);
+        }
+    }
+    if (seed_c < best) {
+        cx = seed_x; cy = seed_y; best = seed_c;
+    }
+    return SearchOut{cx, cy, best, evals};
+}
+
+}  // namespace h264a

@@ -1,12 +1,13 @@
 // me.cu -- a10/a11/a12: motion_search (crates/rusty_h264-encoder/src/mb16.rs:
 // 2433-3302), best_part (:4921) and the plain-ME frame pass.
 //
-// One warp runs one search.  Each lane owns one 4x4 sub-block of the
-// partition (its source rows stay in registers for the whole search), so a
-// pass over 32 lanes prices 32/nb candidates at once (nb = sub-blocks per
-// partition); a candidate's distortion is the sum of its lanes' blocks, added
-// with shared-memory atomics.  Control flow is warp-uniform and replays the
-// reference exactly:
+// One warp runs one search.  The frame kernels price an MB's 16x16 and its
+// four partitions on the tensor cores (mb_search.cuh).  h264a_me_search's jobs
+// (any shape and preset) run motion_search_warp below: each lane owns one 4x4
+// sub-block of the partition, so a pass over 32 lanes prices 32/nb candidates
+// at once (nb = sub-blocks per partition); a candidate's distortion is the sum
+// of its lanes' blocks, added with shared-memory atomics.  Control flow
+// replays the reference exactly:
 //  * fixed-centre diamond passes and batched rings price their 4/8 candidates
 //    together, then take the first strict-minimum like the reference's argmin;
 //  * cascading rings (the centre moves mid-ring) are priced speculatively
@@ -27,52 +28,18 @@
 
 #include "deblock_device.cuh"
 #include "hpel_device.cuh"
+#include "mb_search.cuh"
 #include "tq_device.cuh"
+
 
 namespace h264a {
 
-constexpr int MET_SATD = 0;
-constexpr int MET_SAD = 1;
-// Warps per CTA of the narrow frame kernel (one MB per warp) and of the wide
-// one (one MB per CTA: the 16x16 search by all its warps, each partition by
-// one warp).  Four: one warp per SM sub-partition, since the warps of a team
-// repeat the same control code and two of them on one sub-partition would
-// share its issue slots.
+// Warps per CTA of the frame kernels (one MB per warp).
 constexpr int ME_WARPS = 4;
-constexpr int ME_WIDE_WARPS = 4;
-constexpr int ME_PART_TEAM = ME_WIDE_WARPS / 4;  // warps per partition search
 
-// The reference picture's readiness in the pipelined closed loop: its planes
-// are built segment by segment (16 picture rows by segw picture columns;
-// segment (b, s)'s flag == epoch means every segment up and left of it is
-// complete), and a search waits (bounded) for the segment of every pixel it
-// reads.
-struct BandWait {
-    const int* flags;  // nbands x nseg readiness flags, band-major
-    int nbands, nseg, segw, epoch, limit;
-    int* status;
-};
-
-// Waits until the reference's planes (and reconstruction) are final at
-// picture pixel (row, col), clamped into the picture: the flag of the band
-// (16 rows) and column segment (segw columns) holding it.  Segment (b, s) is
-// published after (b-1, s) and (b, s-1), so it stands for every segment up
-// and left of it.  `ready` caches a segment seen ready, packed b << 12 | s
-// (-1: none); any value stored there was seen ready, so a torn update between
-// lanes only loses a shortcut.  Nothing when the search has no BandWait.
-__device__ __forceinline__ void band_wait_px(const BandWait* bw, int* ready, int row, int col) {
-    if (bw == nullptr) return;
-    const int b = min(max(row, 0) >> 4, bw->nbands - 1);
-    const int sg = min(max(col, 0) / bw->segw, bw->nseg - 1);
-    const int c = *reinterpret_cast<volatile int*>(ready);
-    if (c >= 0 && b <= (c >> 12) && sg <= (c & 4095)) return;
-    wait_flag(bw->flags + b * bw->nseg + sg, bw->epoch, bw->status, 1, bw->limit);
-    if (c < 0 || (b >= (c >> 12) && sg >= (c & 4095))) *reinterpret_cast<volatile int*>(ready) = (b << 12) | sg;
-}
-
-// Per-warp shared state: the round's candidates and distortions, and the
-// search's cold parameters (read a few times per round, so they live here
-// rather than in registers).
+// Per-warp shared state of an h264a_me_search job: the round's candidates and
+// distortions, and the search's cold parameters (read a few times per round,
+// so they live here rather than in registers).
 struct WarpScratch {
     int2 cand[32];
     int dist[32];
@@ -82,76 +49,19 @@ struct WarpScratch {
     double lam_r;         // cost's λ (λ/4 for the table kinds)
     double lam_fp;        // cost_fp's λ (λ·RFF_ME_SADL under B2, else λ)
     double lam_me;        // λ itself (the batched sub-pel arms)
-    int win_ok;           // the MB's reference window is staged in shared memory
-    int wx0, wy0;         // its origin in padded-plane coordinates
-    const BandWait* bw;   // the reference's band readiness, or nullptr (complete)
-    int bready;           // a reference segment seen complete (band_wait_px)
 };
-
-// ---------------------------------------------------------------------------
-// Per-MB reference window in shared memory
-// ---------------------------------------------------------------------------
-// The F|H|V|C planes around the MB's predicted position, copied once per MB by
-// the bulk-copy (TMA) engine: WIN_H rows of WIN_W bytes per plane, every
-// search of the MB (16x16 and its partitions) then reads its candidates from
-// shared memory.  Candidates whose reads leave the window take the plane path
-// (pred_rows), which gives the same bytes.  Rows are WIN_STRIDE = 80 bytes
-// apart: a block's four rows are then load-immediate offsets of its first, and
-// the rows one candidate's 16 lanes read together (four apart) fall in at most
-// two lanes per bank.
-constexpr int WIN_W = 64, WIN_H = 42, WIN_STRIDE = 80;
-constexpr int WIN_PLANE = WIN_H * WIN_STRIDE;  // bytes per plane (a multiple of 16)
-constexpr int WIN_BYTES = 4 * WIN_PLANE;
-constexpr int WIN_R = 12;  // the window starts this far up/left of the predicted position
-constexpr int WIN_OFF = -(1 << 30);  // window offset of a search without one: below -2^29 for any MV, so every read misses
-
-// Rows of the 4x4 block at window position (wx, wy) (full-pel part of the MV
-// applied) at phase (fx, fy): the same operand table and averaging as
-// pred_rows, read from the staged window at shared address `win`.
-__device__ __forceinline__ void win_rows(uint32_t win, int wx, int wy, int fx, int fy, uint32_t out[4]) {
-    const uint32_t pb = phase_bits(fx, fy);
-    const int pa = int(pb & 3), pbb = int((pb >> 2) & 3);
-    const int xa = wx + int((pb >> 4) & 1), ya = wy + int((pb >> 5) & 1);
-    const uint32_t a = win + uint32_t(pa * WIN_PLANE + ya * WIN_STRIDE + (xa & ~3));
-    const uint32_t sha = uint32_t(xa & 3) * 8u;
-#pragma unroll
-    for (int r = 0; r < 4; r++) out[r] = __funnelshift_r(lds_u32(a + r * WIN_STRIDE), lds_u32(a + r * WIN_STRIDE + 4), sha);
-    if (pbb != 0) {
-        const int xb = wx + int((pb >> 6) & 1), yb = wy + int((pb >> 7) & 1);
-        const uint32_t b = win + uint32_t(pbb * WIN_PLANE + yb * WIN_STRIDE + (xb & ~3));
-        const uint32_t shb = uint32_t(xb & 3) * 8u;
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-            out[r] = avg_up4(out[r], __funnelshift_r(lds_u32(b + r * WIN_STRIDE), lds_u32(b + r * WIN_STRIDE + 4), shb));
-    }
-}
-
-// Both operands of a block at window position (wx, wy) lie inside the window:
-// x reads cover the aligned words from (wx + dx) & ~3 to +8, rows wy + dy ..
-// wy + dy + 3, with dx, dy <= 1.
-__device__ __forceinline__ bool win_covers(int wx, int wy) {
-    return wx >= 0 && ((wx + 1) & ~3) <= WIN_W - 8 && wy >= 0 && wy + 5 <= WIN_H;
-}
-
-// Passes whose plane loads are issued together before their SATD: one, since
-// the window reads are shared-memory loads and batching passes only costs
-// registers.
-constexpr int ME_MAX_PASS = 1;
 
 // Register-resident part of one search (every function below is inlined, so
 // nothing of it is ever addressed in local memory); the rest is in the
 // warp's WarpScratch.
 struct SearchGeom {
     int lx, ly, lg_nb, lane, bxo, byo;
-    int wox, woy;             // this lane's block at MV (0,0) in window coordinates (WIN_OFF: no window)
-    uint32_t win;             // shared address of the warp's window
     uint32_t spa[4], spb[4];  // this lane's source 4x4 rows, split into column pairs
 };
 
 __device__ __forceinline__ void geom_init(SearchGeom& g, WarpScratch& ws, const h264a_picture& pc, int x, int y, int w,
-                                          int h, uint32_t win) {
+                                          int h) {
     g.lx = x; g.ly = y;
-    g.win = win;
     g.lane = threadIdx.x & 31;
     if (g.lane == 0) {
         ws.base = pc.d_planes;
@@ -168,13 +78,6 @@ __device__ __forceinline__ void geom_init(SearchGeom& g, WarpScratch& ws, const 
     const int blk = g.lane & ((1 << g.lg_nb) - 1);
     g.bxo = (blk % nbx) * 4;
     g.byo = (blk / nbx) * 4;
-    if (ws.win_ok) {
-        g.wox = x + g.bxo + pc.pad - ws.wx0;
-        g.woy = y + g.byo + pc.pad - ws.wy0;
-    } else {
-        g.wox = WIN_OFF;
-        g.woy = WIN_OFF;
-    }
     uint32_t srow[4];
     // x + bxo is a multiple of 4 and the row lies inside the picture: aligned loads
 #pragma unroll
@@ -184,51 +87,28 @@ __device__ __forceinline__ void geom_init(SearchGeom& g, WarpScratch& ws, const 
     __syncwarp();
 }
 
-// Distortions of ws.cand[0..n) under `metric` into ws.dist.  All the round's
-// plane loads are issued before any is consumed, so a round pays one memory
-// latency however many passes it takes.
-// Distortions of ws.cand[0..n) added into ws.dist (zeroed by the caller) by
-// shared-memory atomics of the lanes' 4x4 blocks.
+// Distortions of ws.cand[0..n) under `metric` added into ws.dist (zeroed by
+// the caller) by shared-memory atomics of the lanes' 4x4 blocks.
 __device__ __forceinline__ void eval_round(const SearchGeom& g, WarpScratch& ws, int n, int metric) {
     const int npass = ((n << g.lg_nb) + 31) >> 5;
-    for (int k0 = 0; k0 < npass; k0 += ME_MAX_PASS) {
-    uint32_t pr4[ME_MAX_PASS][4];
-#pragma unroll
-    for (int kk = 0; kk < ME_MAX_PASS; kk++) {
-        const int k = k0 + kk;
+    for (int k = 0; k < npass; k++) {
         const int c = (32 * k + g.lane) >> g.lg_nb;
-        if (k < npass && c < n) {
-            const int2 mv = ws.cand[c];
-            const int dx = mv.x >> 2, dy = mv.y >> 2;
-            const int wx = g.wox + dx, wy = g.woy + dy;
-            if (win_covers(wx, wy)) {
-                win_rows(g.win, wx, wy, mv.x & 3, mv.y & 3, pr4[kk]);
-            } else {
-                Planes P;
-                P.base = ws.base; P.pw = ws.pw; P.ph = ws.ph; P.pad = ws.pad; P.ps = (long long)ws.pw * ws.ph;
-                pred_rows(P, g.lx + g.bxo + dx, g.ly + g.byo + dy, mv.x & 3, mv.y & 3, pr4[kk]);
-            }
-        }
-    }
+        if (c >= n) continue;
+        const int2 mv = ws.cand[c];
+        Planes P;
+        P.base = ws.base; P.pw = ws.pw; P.ph = ws.ph; P.pad = ws.pad; P.ps = (long long)ws.pw * ws.ph;
+        uint32_t p4[4];
+        pred_rows(P, g.lx + g.bxo + (mv.x >> 2), g.ly + g.byo + (mv.y >> 2), mv.x & 3, mv.y & 3, p4);
+        int d;
+        if (metric == MET_SAD) {
+            uint32_t srow[4];
 #pragma unroll
-    for (int kk = 0; kk < ME_MAX_PASS; kk++) {
-        const int k = k0 + kk;
-        if (k < npass) {
-            const int c = (32 * k + g.lane) >> g.lg_nb;
-            int d = 0;
-            if (c < n) {
-                if (metric == MET_SAD) {
-                    uint32_t srow[4];
-#pragma unroll
-                    for (int r = 0; r < 4; r++) srow[r] = g.spa[r] | (g.spb[r] << 8);
-                    d = sad4x4_rows(srow, pr4[kk]);
-                } else {
-                    d = satd4x4_packed(g.spa, g.spb, pr4[kk]);
-                }
-            }
-            if (c < n) atomicAdd(&ws.dist[c], d);  // the candidate's blocks, summed in shared memory
+            for (int r = 0; r < 4; r++) srow[r] = g.spa[r] | (g.spb[r] << 8);
+            d = sad4x4_rows(srow, p4);
+        } else {
+            d = satd4x4_packed(g.spa, g.spb, p4);
         }
-    }
+        atomicAdd(&ws.dist[c], d);  // the candidate's blocks, summed in shared memory
     }
     __syncwarp();
 }
@@ -249,14 +129,6 @@ __device__ __forceinline__ int lane_cost(const MeParamsDev& pr, const WarpScratc
     return c > INT_MAX - 1 ? INT_MAX - 1 : int(c);
 }
 
-// The eight ring points (dx, dy) in the reference's order: (1,0) (-1,0) (0,1)
-// (0,-1) (1,1) (-1,-1) (1,-1) (-1,1); the four-point diamond is the first four.
-// Packed two bits per point as d+1, so a lane computes its point without a
-// memory lookup.
-constexpr uint32_t kRingXP = 0x2252u, kRingYP = 0x8225u;
-__device__ __forceinline__ int ring_dx(int i) { return int((kRingXP >> (2 * i)) & 3u) - 1; }
-__device__ __forceinline__ int ring_dy(int i) { return int((kRingYP >> (2 * i)) & 3u) - 1; }
-
 __device__ __forceinline__ bool in_plane_window(const SearchGeom& g, const WarpScratch& ws, int mvx, int mvy) {
     const int px = g.lx + (mvx >> 2) + ws.pad, py = g.ly + (mvy >> 2) + ws.pad;
     return px >= 0 && py >= 0 && px + ws.rw + 1 <= ws.pw && py + ws.rh + 1 <= ws.ph;
@@ -267,14 +139,6 @@ __device__ __forceinline__ long long cand_cost64(const MeParamsDev& pr, const Wa
     const int2 mv = ws.cand[i];
     return (long long)ws.dist[i] + lam_cost(lam, rate_of(pr, ws, mv.x, mv.y));
 }
-
-// Search phases and what an evaluation round's results are for.
-constexpr int PH_SEEDS = 0, PH_PROP = 1, PH_DIA = 2, PH_REPRICE = 3, PH_SUB = 4, PH_DONE = 5, PH_START = 6;
-constexpr int EV_START = 0, EV_SEEDS = 1, EV_PROP = 2, EV_FIXED = 3, EV_RING = 4, EV_REPRICE = 5;
-// Candidates of the learned search's proposal round: the median predictor
-// and the network's 8 proposals.
-constexpr int N_PROP = 8;
-constexpr int LOOP_GUARD = 1 << 20;  // iterations of one rung / sub-pel step
 
 // Points of a cascading ring priced per round: the first round prices
 // RING_FIRST of them, later rounds (after the centre moved, or none improved)
@@ -564,564 +428,12 @@ __device__ __forceinline__ void motion_search_warp(const SearchGeom& g, const Me
     }
     out_x = bx; out_y = by; out_c = best_c;
 }
-
-// ---------------------------------------------------------------------------
-// Searches of one MB in lane groups
-// ---------------------------------------------------------------------------
-// The plain-ME frame pass runs best_part's searches of an MB with this one
-// search body: first the 16x16 search with the whole warp as one group (one
-// lane per 4x4 block, two candidates per pass); then, when the 16x16 J
-// exceeds the gate, the four partition searches (16x8 top, 16x8 bottom,
-// 8x16 left, 8x16 right) side by side, lane group g = lane / 8 searching
-// partition g with one candidate per pass.  The partitions share their seeds
-// [pmv, mv16], mvd centre and λ (mb16.rs:8869-8913), so the four searches are
-// independent; each group carries its own copy of the search state (the
-// state machine of motion_search_warp, every decision taken per group) and
-// the warp loops until every group is done.  Candidates and distortions of a
-// group live in its slots ws.cand / ws.dist [gb, gb + group size).
-
-struct GroupGeom {
-    SearchGeom s;     // the lane's partition origin, its 4x4 block, window offsets, source rows
-    int rw, rh;       // partition size
-    int gb;           // first slot of the lane's group
-    int gl;           // lane within the group
-    int lg;           // log2 lanes per group (5: one group, 3: four groups)
-    unsigned gmask;   // the group's bits in a ballot, shifted down to bit 0
-};
-
-// mode 0: the MB's 16x16 search (one group); mode 1: its four partitions,
-// one lane group of 8 each; mode 2: partition `part` (0 16x8 top, 1 16x8
-// bottom, 2 8x16 left, 3 8x16 right) with the whole warp as one group, four
-// candidates per pass.
-// pre: for mode 0, the lane's source rows already loaded (block lane & 15).
-__device__ __forceinline__ void group_geom_init(GroupGeom& q, WarpScratch& ws, const h264a_picture& pc, int mx, int my,
-                                                int mode, uint32_t win, const uint32_t* pre, int part = 0,
-                                                const BandWait* bw = nullptr, int bready = 0) {
-    const int lane = threadIdx.x & 31;
-    SearchGeom& g = q.s;
-    int x = mx, y = my;
-    if (mode == 2) {
-        q.gb = 0;
-        q.gl = lane;
-        q.lg = 5;
-        q.gmask = 0xffffffffu;
-        q.rw = part < 2 ? 16 : 8;
-        q.rh = part < 2 ? 8 : 16;
-        g.lg_nb = 3;
-        x += part == 3 ? 8 : 0;
-        y += part == 1 ? 8 : 0;
-    } else if (mode == 0) {
-        q.gb = 0;
-        q.gl = lane;
-        q.lg = 5;
-        q.gmask = 0xffffffffu;
-        q.rw = 16;
-        q.rh = 16;
-        g.lg_nb = 4;
-    } else {
-        const int grp = lane >> 3;
-        q.gb = grp * 8;
-        q.gl = lane & 7;
-        q.lg = 3;
-        q.gmask = 0xffu;
-        q.rw = grp < 2 ? 16 : 8;
-        q.rh = grp < 2 ? 8 : 16;
-        g.lg_nb = 3;
-        x += grp == 3 ? 8 : 0;
-        y += grp == 1 ? 8 : 0;
-    }
-    if (lane == 0) {
-        ws.bw = bw;
-        ws.bready = bready;
-        ws.base = pc.d_planes;
-        ws.pad = pc.pad;
-        ws.pw = pc.cw + 2 * pc.pad;
-        ws.ph = pc.ch + 2 * pc.pad;
-        ws.cw = pc.cw;
-        ws.ch = pc.ch;
-    }
-    g.lx = x; g.ly = y;
-    g.win = win;
-    g.lane = lane;
-    const int blk = q.gl & ((1 << g.lg_nb) - 1);
-    const int nbx = q.rw >> 2;
-    g.bxo = (blk % nbx) * 4;
-    g.byo = (blk / nbx) * 4;
-    if (ws.win_ok) {
-        g.wox = x + g.bxo + pc.pad - ws.wx0;
-        g.woy = y + g.byo + pc.pad - ws.wy0;
-    } else {
-        g.wox = WIN_OFF;
-        g.woy = WIN_OFF;
-    }
-    uint32_t srow[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) srow[r] = pre ? pre[r] : ld4u(pc.d_src + (long long)(y + g.byo + r) * pc.cw + x + g.bxo);
-    split_pairs(srow, g.spa, g.spb);
-    __syncwarp();
-}
-
-// Distortions of each group's candidates ws.cand[gb..gb+n) (n and metric per
-// group) added into ws.dist, which the caller has zeroed: each lane adds its
-// 4x4 block's distortion to its candidate's slot with a shared-memory atomic
-// (exact, so the order does not matter), which has a shorter dependency chain
-// than a shuffle tree over the candidate's lanes.  A group prices
-// 2^(lg - lg_nb) candidates per pass; passes run to the largest need over the
-// groups.  SATD_ONLY: the caller's preset never prices with SAD (Balanced).
-// TW > 1 (a search run by a team of TW warps with the same state, the wide
-// kernel's): warp tw of the team prices, in each pass, the candidates
-// [tw * cpw, (tw + 1) * cpw) of that pass's TW * cpw (cpw = the warp's
-// candidates per pass), into the team's shared slots `dist` (its own slots
-// only).
-template <int TW>
-__device__ __forceinline__ int team_cand(int k, int cpw, int sub) {
-    return (k * TW + int(threadIdx.x >> 5) % TW) * cpw + sub;
-}
-
-template <bool SATD_ONLY, int TW = 1>
-__device__ __forceinline__ void eval_round_group(const GroupGeom& q, WarpScratch& ws, int n, int metric,
-                                                 int* dist = nullptr) {
-    constexpr bool COOP = TW > 1;
-    const SearchGeom& g = q.s;
-    const int cps = q.lg - g.lg_nb;  // log2 candidates per pass of a group
-    const int npass = COOP ? (n + (TW << cps) - 1) / (TW << cps)
-                           : __reduce_max_sync(0xffffffffu, (n + (1 << cps) - 1) >> cps);
-    const int sub = q.gl >> g.lg_nb;  // which of the pass's candidates the lane serves
-    for (int k0 = 0; k0 < npass; k0 += ME_MAX_PASS) {
-        uint32_t pr4[ME_MAX_PASS][4];
-#pragma unroll
-        for (int kk = 0; kk < ME_MAX_PASS; kk++) {
-            const int c = COOP ? team_cand<TW>(k0 + kk, 1 << cps, sub) : ((k0 + kk) << cps) + sub;
-            if (k0 + kk < npass && c < n) {
-                const int2 mv = ws.cand[q.gb + c];
-                const int dx = mv.x >> 2, dy = mv.y >> 2;
-                const int wx = g.wox + dx, wy = g.woy + dy;
-                if (win_covers(wx, wy)) {
-                    win_rows(g.win, wx, wy, mv.x & 3, mv.y & 3, pr4[kk]);
-                } else {
-                    band_wait_px(ws.bw, &ws.bready, g.ly + g.byo + dy + 5, g.lx + g.bxo + dx + 5);
-                    Planes P;
-                    P.base = ws.base; P.pw = ws.pw; P.ph = ws.ph; P.pad = ws.pad; P.ps = (long long)ws.pw * ws.ph;
-                    P.cg = ws.bw != nullptr;
-                    pred_rows(P, g.lx + g.bxo + dx, g.ly + g.byo + dy, mv.x & 3, mv.y & 3, pr4[kk]);
-                }
-            }
-        }
-#pragma unroll
-        for (int kk = 0; kk < ME_MAX_PASS; kk++) {
-            const int k = k0 + kk;
-            if (k < npass) {
-                const int c = COOP ? team_cand<TW>(k, 1 << cps, sub) : (k << cps) + sub;
-                int d = 0;
-                if (c < n) {
-                    if (!SATD_ONLY && metric == MET_SAD) {
-                        uint32_t srow[4];
-#pragma unroll
-                        for (int r = 0; r < 4; r++) srow[r] = g.spa[r] | (g.spb[r] << 8);
-                        d = sad4x4_rows(srow, pr4[kk]);
-                    } else {
-                        d = satd4x4_packed(g.spa, g.spb, pr4[kk]);
-                    }
-                }
-                if (c < n) atomicAdd(COOP ? &dist[c] : &ws.dist[q.gb + c], d);  // the candidate's blocks, summed in shared memory
-            }
-        }
-    }
-    __syncwarp();
-}
-
-__device__ __forceinline__ bool group_in_plane_window(const GroupGeom& q, const WarpScratch& ws, int mvx, int mvy) {
-    const int px = q.s.lx + (mvx >> 2) + ws.pad, py = q.s.ly + (mvy >> 2) + ws.pad;
-    return px >= 0 && py >= 0 && px + q.rw + 1 <= ws.pw && py + q.rh + 1 <= ws.ph;
-}
-
-// motion_search (mb16.rs:2433-3302) of the lane's partition, every group at
-// once; same phases, order and pricing as motion_search_warp.
-// The search's knobs: read from the parameters, or, for the Balanced preset
-// (BAL, h264a_me_params_default), compile-time constants, so that the control
-// logic of every round folds to the preset's path.
-template <bool BAL>
-struct Knobs {
-    const MeParamsDev& p;
-    __device__ __forceinline__ bool fast() const { return BAL ? false : p.fast != 0; }
-    __device__ __forceinline__ bool use_sad() const { return BAL ? false : p.use_sad != 0; }
-    __device__ __forceinline__ bool sadfp() const { return BAL ? false : p.sadfp != 0; }
-    __device__ __forceinline__ int kind() const { return BAL ? 0 : p.kind; }
-    __device__ __forceinline__ bool me_snap() const { return BAL ? true : p.me_snap != 0; }
-    __device__ __forceinline__ bool fc() const { return BAL ? true : p.fc != 0; }
-    __device__ __forceinline__ uint32_t dia_mask() const { return BAL ? 0x1cu : p.dia_mask; }
-    __device__ __forceinline__ bool subpel() const { return BAL ? true : p.subpel != 0; }
-    __device__ __forceinline__ int subpel_pat() const { return BAL ? -1 : p.subpel_pat; }
-    __device__ __forceinline__ bool sp_single_pass() const { return BAL ? true : p.sp_single_pass != 0; }
-    __device__ __forceinline__ bool me_subpel_iter() const { return BAL ? true : p.me_subpel_iter != 0; }
-    __device__ __forceinline__ int sp_maxit() const { return BAL ? 0 : p.sp_maxit; }
-    __device__ __forceinline__ bool sp_fc() const { return BAL ? false : p.sp_fc != 0; }
-    __device__ __forceinline__ double sadfp_lambda() const { return p.sadfp_lambda; }
-    // rate of an MV against the search's mvd centre (mb16.rs:2454-2482)
-    __device__ __forceinline__ uint32_t rate(const WarpScratch& ws, int mvx, int mvy) const {
-        return mvbits(kind(), p.tab, mvx - ws.cx) + mvbits(kind(), p.tab, mvy - ws.cy);
-    }
-};
-
-// LEARN (the learned-proposal kernels) with use_prop (their 16x16 search): the
-// search first prices the median predictor preds[0..1] and the 8 proposals
-// (lane gl of the group holds proposal gl - 1 in `prop`) with the search's
-// own cost; when the best proposal's distortion exceeds the predictor's by
-// more than prop_t it falls back to the plain search (fell = 1), otherwise it
-// continues as motion_search with the cheapest of the nine as its start
-// vector (mb16.rs:2445, 2579-2596: refine-only, no full-pel phase).
-//
-// RF / RR: the ring batches (RING_FIRST / RING_REST) of this search; wider
-// batches where a pass prices more candidates at once.  TW > 1: the search is
-// run by a team of TW consecutive warps with identical state (each warp its
-// own `ws`, the same plan and fold), the pricing split between them
-// (eval_round_group) into the team's shared distortions cdist[2][32], one
-// named barrier (1 + the team's index) per round, the two halves alternating
-// by round.
-// Named barrier `id` (1..4) over a team of TW warps.  The barrier index is
-// an immediate in each branch, so the compiler reserves barriers 1..4 only
-// (an index in a register reserves all 16, and the barrier count then caps
-// the CTAs per SM).
-template <int TW>
-__device__ __forceinline__ void team_sync(int id) {
-    switch (id) {
-        case 1: asm volatile("bar.sync 1, %0;" ::"n"(32 * TW) : "memory"); break;
-        case 2: asm volatile("bar.sync 2, %0;" ::"n"(32 * TW) : "memory"); break;
-        case 3: asm volatile("bar.sync 3, %0;" ::"n"(32 * TW) : "memory"); break;
-        default: asm volatile("bar.sync 4, %0;" ::"n"(32 * TW) : "memory"); break;
-    }
-}
-
-template <bool BAL, bool LEARN = false, int RF = RING_FIRST, int RR = RING_REST, int TW = 1>
-__device__ __forceinline__ void motion_search_group(const GroupGeom& q, const MeParamsDev& prm, WarpScratch& ws,
-                                                    const int* preds, int npred, double lambda_me, int& out_x,
-                                                    int& out_y, long long& out_c, int& evals, bool use_prop = false,
-                                                    int2 prop = make_int2(0, 0), int prop_t = 0, int* fell = nullptr,
-                                                    int* cdist = nullptr, bool use_start = false,
-                                                    int2 start = make_int2(0, 0)) {
-    const Knobs<BAL> pr{prm};
-    const int gl = q.gl, gb = q.gb;
-    const bool sadfp = !pr.fast() && pr.sadfp();
-    const int m_main = pr.use_sad() ? MET_SAD : MET_SATD;
-    if (q.s.lane == 0) {
-        ws.cx = preds[0];
-        ws.cy = preds[1];
-        ws.lam_me = lambda_me;
-        ws.lam_r = pr.kind() != 0 ? lambda_me * 0.25 : lambda_me;
-        ws.lam_fp = lambda_me * (sadfp ? pr.sadfp_lambda() : 1.0);
-    }
-    // seeds and the snaps of sub-pel predictors (as motion_search_warp), per group
-    int qx = 0, qy = 0;
-    const bool mine = gl >= 1 && gl <= npred;
-    if (mine) {  // npred <= 2: lane 1 the first predictor, lane 2 the second
-        qx = gl == 1 ? preds[0] : preds[2];
-        qy = gl == 1 ? preds[1] : preds[3];
-        ws.cand[gb + gl] = make_int2(qx, qy);
-    }
-    const unsigned snaps =
-        (__ballot_sync(0xffffffffu, pr.me_snap() && mine && ((qx & 3) != 0 || (qy & 3) != 0)) >> gb) & q.gmask;
-    if ((snaps >> gl) & 1u)
-        ws.cand[gb + npred + 1 + __popc(snaps & ((1u << gl) - 1u))] = make_int2(((qx + 2) >> 2) * 4, ((qy + 2) >> 2) * 4);
-    __syncwarp();
-    const int m_fp = sadfp ? MET_SAD : m_main;
-    const double l_fp = sadfp ? ws.lam_fp : ws.lam_r;
-    const int rw = q.rw, rh = q.rh;
-    const bool fc = !pr.fast() && pr.fc();  // 16x16, 16x8 and 8x16 are x4 shapes
-    const uint32_t dmask = pr.fast() ? 0u : pr.dia_mask();
-    const int spat = pr.subpel_pat() >= 0 ? pr.subpel_pat() : (pr.sp_single_pass() ? 2 : 0);
-    const bool sp_fc = pr.sp_fc() && !pr.fast();
-    const int sp_nring = (spat & 1) ? 4 : 8;
-
-    evals = 0;
-    int bx = 0, by = 0, seed_x = 0, seed_y = 0;
-    int best_c = 0, seed_c = 0;  // costs below 2^30 (lane_cost), compared as i32
-    int phase = (LEARN && use_prop) ? PH_PROP : (use_start ? PH_START : PH_SEEDS);
-    int si = -1, sk = -1, loops = 0, iter = 0, step = 0;
-    bool ring_open = false, ring_improved = false;
-    int ring_i = 0, ring_n = 0;
-    constexpr bool COOP = TW > 1;
-    const int team_bar = 1 + int(threadIdx.x >> 5) / TW;
-    int round = 0;
-    for (;;) {
-        // the round's distortion slots: the warp's own, or the team's half
-        // for this round
-        int* const dist = COOP ? cdist + 32 * (round & 1) : ws.dist + gb;
-        round++;
-        // ---------- plan (per group) ----------
-        int kind = -1, n = 0, metric = m_main;
-        double lam = ws.lam_r;
-        while (kind < 0 && phase != PH_DONE) {
-            if (phase == PH_SEEDS) {
-                if (gl == 0) ws.cand[gb] = make_int2(0, 0);
-                kind = EV_SEEDS; n = npred + 1 + __popc(snaps); metric = m_fp; lam = l_fp;
-            } else if (LEARN && phase == PH_PROP) {
-                if (gl <= N_PROP) ws.cand[gb + gl] = gl == 0 ? make_int2(preds[0], preds[1]) : prop;
-                kind = EV_PROP; n = N_PROP + 1; metric = m_main; lam = ws.lam_r;
-            } else if (phase == PH_START) {
-                if (gl == 0) ws.cand[gb] = start;
-                kind = EV_START; n = 1; metric = m_main; lam = ws.lam_r;
-            } else if (phase == PH_DIA) {
-                if (ring_open) {
-                    kind = EV_RING; n = min(ring_n - ring_i, RR); metric = m_fp; lam = l_fp;
-                    if (gl < n)
-                        ws.cand[gb + gl] = make_int2(bx + ring_dx(ring_i + gl) * step, by + ring_dy(ring_i + gl) * step);
-                    break;
-                }
-                if (si < 0 || loops >= LOOP_GUARD) {
-                    int nsi = si + 1;
-                    if (pr.fast()) nsi = nsi >= 2 ? 5 : nsi;
-                    else
-                        while (nsi < 5 && !(dmask & (1u << nsi))) nsi++;
-                    if (nsi >= 5) {
-                        phase = PH_REPRICE;
-                        continue;
-                    }
-                    si = nsi;
-                    step = pr.fast() ? (si == 0 ? 16 : 4) : (64 >> si);
-                    loops = 0;
-                }
-                loops++;
-                bool fixed = false;
-                if (fc && (bx & 3) == 0 && (by & 3) == 0) {
-                    const int st = step >> 2;
-                    const int px = q.s.lx + (bx >> 2), py = q.s.ly + (by >> 2);
-                    fixed = px - st >= 0 && py - st >= 0 && px + st + rw <= ws.cw && py + st + rh <= ws.ch;
-                }
-                if (gl < 4) ws.cand[gb + gl] = make_int2(bx + ring_dx(gl) * step, by + ring_dy(gl) * step);
-                if (fixed) {
-                    kind = EV_FIXED; n = 4;
-                    metric = rw == 16 ? (sadfp ? MET_SAD : MET_SATD) : m_fp;
-                    lam = rw == 16 ? ws.lam_fp : l_fp;
-                } else {
-                    ring_open = true; ring_improved = false; ring_i = 0; ring_n = 4;
-                    kind = EV_RING; n = 4; metric = m_fp; lam = l_fp;
-                }
-            } else if (phase == PH_REPRICE) {
-                if (sadfp) {
-                    if (gl == 0) {
-                        ws.cand[gb] = make_int2(bx, by);
-                        ws.cand[gb + 1] = make_int2(seed_x, seed_y);
-                    }
-                    kind = EV_REPRICE; n = 2; metric = m_main; lam = ws.lam_r;
-                } else {
-                    phase = PH_SUB;
-                }
-            } else {  // PH_SUB
-                if (ring_open) {
-                    kind = EV_RING; n = min(ring_n - ring_i, RR); metric = m_main; lam = ws.lam_r;
-                    if (gl < n)
-                        ws.cand[gb + gl] = make_int2(bx + ring_dx(ring_i + gl) * step, by + ring_dy(ring_i + gl) * step);
-                    break;
-                }
-                if (!pr.subpel()) {
-                    phase = PH_DONE;
-                    continue;
-                }
-                if (sk < 0 || loops >= LOOP_GUARD) {
-                    if (++sk >= 2) {
-                        phase = PH_DONE;
-                        continue;
-                    }
-                    step = sk == 0 ? 2 : 1;
-                    loops = 0;
-                    iter = 0;
-                }
-                loops++;
-                if (sp_fc && (spat & 1) == 0 && (step == 1 || ((bx & 3) == 0 && (by & 3) == 0))) {
-                    bool all = true;
-                    for (int i = 0; i < 8; i++) {
-                        const int qx2 = bx + ring_dx(i) * step, qy2 = by + ring_dy(i) * step;
-                        all = all && group_in_plane_window(q, ws, qx2, qy2) && (step == 2 || ((qx2 | qy2) & 1));
-                    }
-                    if (all) {
-                        iter++;
-                        if (gl < 8) ws.cand[gb + gl] = make_int2(bx + ring_dx(gl) * step, by + ring_dy(gl) * step);
-                        kind = EV_FIXED; n = 8;
-                        metric = rw == 16 ? MET_SATD : m_main;
-                        lam = rw == 16 ? ws.lam_me : ws.lam_r;
-                        break;
-                    }
-                }
-                iter++;
-                n = min(sp_nring, RF);
-                if (gl < n) ws.cand[gb + gl] = make_int2(bx + ring_dx(gl) * step, by + ring_dy(gl) * step);
-                ring_open = true; ring_improved = false; ring_i = 0; ring_n = sp_nring;
-                kind = EV_RING; metric = m_main; lam = ws.lam_r;
-            }
-        }
-        if (kind < 0) n = 0;
-        if (__all_sync(0xffffffffu, kind < 0)) break;
-        // which collectives this round's folds need, decided before the pricing
-        // (votes off the critical path): the group minimum for fixed-centre
-        // rings, the first improvement for cascading rings, the seed costs for
-        // the seed and reprice rounds
-        const bool need_min = __any_sync(0xffffffffu, kind == EV_FIXED);
-        const bool need_hit = __any_sync(0xffffffffu, kind == EV_RING);
-        const bool need_seed = __any_sync(0xffffffffu, kind == EV_SEEDS || kind == EV_REPRICE || kind == EV_START);
-        if (COOP) {
-            // the warp zeroes the slots of the candidates it prices (lane gl
-            // < 8: pass gl / cpw, candidate gl % cpw of the warp's share)
-            const int cpw = 1 << (q.lg - q.s.lg_nb);
-            const int zc = team_cand<TW>(gl / cpw, cpw, gl % cpw);
-            if (gl < 8 && zc < n) dist[zc] = 0;
-        } else if (gl < n) {
-            dist[gl] = 0;  // the pricing adds each lane's block into its candidate's slot
-        }
-        __syncwarp();
-        __syncwarp();
-
-        // ---------- price ----------
-        eval_round_group<BAL, TW>(q, ws, n, metric, dist);
-        if (COOP) team_sync<TW>(team_bar);
-        int cc = INT_MAX;  // dist + λ·rate of slot gb + gl, as lane_cost prices it
-        if (gl < n) {
-            const int2 mv = ws.cand[gb + gl];
-            const long long c = (long long)dist[gl] + lam_cost(lam, pr.rate(ws, mv.x, mv.y));
-            cc = c > INT_MAX - 1 ? INT_MAX - 1 : int(c);
-        }
-        // group-wide collectives, taken by every lane (each only in rounds
-        // where some group's fold reads it; the conditions are warp-uniform)
-        int gmin = cc;
-        unsigned at = 0;
-        if (need_min) {
-            for (int o = 1; o < (1 << q.lg); o <<= 1) gmin = min(gmin, __shfl_xor_sync(0xffffffffu, gmin, o));
-            at = (__ballot_sync(0xffffffffu, cc == gmin) >> gb) & q.gmask;
-        }
-        unsigned hit = 0;
-        int jhit = 0, cj = 0;
-        if (need_hit) {
-            hit = (__ballot_sync(0xffffffffu, gl < n && cc < best_c) >> gb) & q.gmask;
-            jhit = hit ? __ffs(hit) - 1 : 0;
-            cj = __shfl_sync(0xffffffffu, cc, gb + jhit);
-        }
-        int c_seed[3] = {0, 0, 0};
-        if (need_seed) {
-#pragma unroll
-            for (int i = 0; i < 3; i++) c_seed[i] = __shfl_sync(0xffffffffu, cc, gb + i);
-        }
-
-        // ---------- fold (per group) ----------
-        if (kind == EV_SEEDS) {
-            best_c = c_seed[0];
-            bx = 0; by = 0;
-            int wi = 0;
-#pragma unroll
-            for (int i = 1; i < 3; i++) {
-                const int ci = c_seed[i];
-                if (i <= npred && ci < best_c) {
-                    best_c = ci;
-                    bx = ws.cand[gb + i].x;
-                    by = ws.cand[gb + i].y;
-                    wi = i;
-                }
-            }
-            evals += npred + 1;
-            seed_x = bx; seed_y = by; seed_c = best_c;
-            if ((snaps >> wi) & 1u) {
-                const int sl = gb + npred + 1 + __popc(snaps & ((1u << wi) - 1u));
-                bx = ws.cand[sl].x; by = ws.cand[sl].y;
-                best_c = int(((long long)dist[sl - gb] + lam_cost(lam, pr.rate(ws, ws.cand[sl].x, ws.cand[sl].y))));
-                evals += 1;
-            }
-            phase = PH_DIA;
-        } else if (kind == EV_START) {
-            // a refine-only search (mb16.rs:2580-2582): the start vector
-            // priced with `cost`, no full-pel phase, the sub-pel steps from it
-            best_c = c_seed[0];
-            bx = start.x;
-            by = start.y;
-            seed_x = bx; seed_y = by; seed_c = best_c;
-            evals += 1;
-            phase = PH_SUB;
-        } else if (LEARN && kind == EV_PROP) {
-            // the cheapest of the nine (first wins, the predictor first), and
-            // the cheapest proposal's distortion against the predictor's
-            int bi = 0, bp = 1;
-            long long cbest = 0, cprop = 0;
-            for (int i = 0; i <= N_PROP; i++) {
-                const int2 mv = ws.cand[gb + i];
-                const long long c = (long long)dist[i] + lam_cost(lam, pr.rate(ws, mv.x, mv.y));
-                if (i == 0 || c < cbest) { cbest = c; bi = i; }
-                if (i == 1 || (i > 1 && c < cprop)) { cprop = c; bp = i; }
-            }
-            evals += N_PROP + 1;
-            const bool fb = (long long)dist[bp] > (long long)dist[0] + prop_t;
-            if (fell) *fell = fb ? 1 : 0;
-            if (fb) {
-                // the plain search's seed slots again (the round above used
-                // them; fb is the same in every lane of the 16x16 group)
-                __syncwarp();
-                if (mine) ws.cand[gb + gl] = make_int2(qx, qy);
-                if ((snaps >> gl) & 1u)
-                    ws.cand[gb + npred + 1 + __popc(snaps & ((1u << gl) - 1u))] =
-                        make_int2(((qx + 2) >> 2) * 4, ((qy + 2) >> 2) * 4);
-                phase = PH_SEEDS;
-            } else {
-                bx = ws.cand[gb + bi].x;
-                by = ws.cand[gb + bi].y;
-                best_c = cbest > INT_MAX - 1 ? INT_MAX - 1 : int(cbest);
-                seed_x = bx; seed_y = by; seed_c = best_c;
-                phase = PH_SUB;  // a start vector: no full-pel phase, no B2 reprice
-            }
-        } else if (kind == EV_REPRICE) {
-            best_c = int(((long long)dist[0] + lam_cost(lam, pr.rate(ws, ws.cand[gb].x, ws.cand[gb].y))));
-            seed_c = int(((long long)dist[1] + lam_cost(lam, pr.rate(ws, ws.cand[gb + 1].x, ws.cand[gb + 1].y))));
-            evals += 2;
-            phase = PH_SUB;
-        } else if (kind == EV_FIXED) {
-            evals += n;
-            const int bi = gmin < best_c ? __ffs(at) - 1 : -1;
-            if (bi >= 0) {
-                best_c = gmin;
-                bx += ring_dx(bi) * step;
-                by += ring_dy(bi) * step;
-            }
-            if (phase == PH_DIA) {
-                if (bi < 0) loops = LOOP_GUARD;
-            } else {
-                const bool stop = bi < 0 || !pr.me_subpel_iter() || (spat & 2) || (pr.sp_maxit() != 0 && iter >= pr.sp_maxit());
-                if (stop) loops = LOOP_GUARD;
-            }
-        } else if (kind == EV_RING) {
-            if (hit == 0) {
-                evals += n;
-                ring_i += n;
-                ring_open = ring_i < ring_n;
-            } else {
-                best_c = cj;
-                const int2 mv = ws.cand[gb + jhit];
-                evals += jhit + 1;
-                bx = mv.x;
-                by = mv.y;
-                ring_improved = true;
-                ring_i += jhit + 1;
-                ring_open = ring_i < ring_n;
-            }
-            if (!ring_open) {
-                if (phase == PH_DIA) {
-                    if (!ring_improved) loops = LOOP_GUARD;
-                } else if (!ring_improved || !pr.me_subpel_iter() || (spat & 2) ||
-                           (pr.sp_maxit() != 0 && iter >= pr.sp_maxit())) {
-                    loops = LOOP_GUARD;
-                }
-            }
-        }
-        __syncwarp();
-    }
-    if (pr.me_snap() && seed_c < best_c) {
-        bx = seed_x; by = seed_y; best_c = seed_c;
-    }
-    out_x = bx; out_y = by; out_c = best_c;
-}
-
 __device__ __forceinline__ bool job_shape_ok(int w, int h) {
     return (w == 16 && (h == 16 || h == 8)) || (w == 8 && (h == 16 || h == 8 || h == 4)) ||
            (w == 4 && (h == 8 || h == 4));
 }
 
-#ifndef ME_MIN_BLOCKS
-#define ME_MIN_BLOCKS 4
-#endif
+constexpr int ME_MIN_BLOCKS = 4;  // CTAs per SM of the frame kernels (their windows fill the shared memory)
 
 __global__ void __launch_bounds__(32 * ME_WARPS) me_search_kernel(const h264a_picture* __restrict__ pics, int npics,
                                                                  const __grid_constant__ MeParamsDev prm,
@@ -1145,10 +457,8 @@ __global__ void __launch_bounds__(32 * ME_WARPS) me_search_kernel(const h264a_pi
         if ((threadIdx.x & 31) == 0) out[j] = res;
         return;
     }
-    if ((threadIdx.x & 31) == 0) scratch[w].win_ok = 0;
-    __syncwarp();
     SearchGeom g;
-    geom_init(g, scratch[w], pc, job.x, job.y, job.w, job.h, 0u);
+    geom_init(g, scratch[w], pc, job.x, job.y, job.w, job.h);
     int mx, my, evals;
     long long c;
     motion_search_warp(g, prm, scratch[w], job.preds, job.npred, job.has_start ? job.start : nullptr, job.lambda_me, mx,
@@ -1206,19 +516,23 @@ struct FrameDesc {
 // lie on earlier diagonals, so a window of resident warps always holds MBs
 // that are ready, and no MB ever waits on a ticket dealt after its own.
 constexpr int ME_MAXF = 96;
-// Launches of at most this many frames run the wide kernel (a CTA per MB):
-// one frame's wavefront has at most a few dozen ready MBs, far fewer than the
-// resident warps, so each MB's own latency is what counts.
-constexpr int ME_WIDE_MAXF = 2;
-// The pipelined closed loop: the width of a band's column segments in MBs,
-// and the number of CTA pools (frames dealt round-robin to them).
-#ifndef PIPE_SEGW_MBS
-#define PIPE_SEGW_MBS 16
-#endif
-#ifndef PIPE_POOL_COUNT
-#define PIPE_POOL_COUNT 8
-#endif
-constexpr int PIPE_SEGW = PIPE_SEGW_MBS, PIPE_POOLS = PIPE_POOL_COUNT;
+// Launches of at most this many frames use the work queue of the closed loop
+// (Q_WIDE), larger ones Q_MAIN.
+constexpr int ME_FEW_FRAMES = 2;
+// The pipelined closed loop: the width of a band's column segments in MBs (112
+// pixels: one strip of the plane builder; the next frame follows closer than
+// with 16 MBs: 46.1 -> 43.7 ms for 59 1080p P frames when it was changed) and
+// the number of warp pools (frames dealt round-robin to them).  The launch
+// takes as many CTAs per SM as give a pool about one warp per ready MB of its
+// frame's wavefront: more only hold MBs that wait, and slow the warps that
+// run (59 1080p P frames at 1, 2, 3, 4 CTAs per SM: 27.1, 29.2, 31.0, 32.4 ms,
+// with 10, 12, 12, 16 pools; at one CTA, 8 pools take 28.7 and 16 pools more).
+constexpr int PIPE_SEGW = 7, PIPE_POOLS = 10;
+static inline int pipe_ctas_per_sm(int mb_w, int mb_h, int pools, int num_sms, int most) {
+    const int wave = std::min((mb_w + 1) / 2, mb_h);  // MBs of the longest anti-diagonal
+    const int n = (pools * wave + ME_WARPS * num_sms - 1) / (ME_WARPS * num_sms);
+    return std::min(std::max(n, 1), most);
+}
 struct FrameBatch {
     FrameDesc f[ME_MAXF];
     long long seg_start[ME_MAXF + 1];
@@ -1271,218 +585,16 @@ __device__ __forceinline__ int2 predict_mv_ref0(bool aa, int2 a, bool ba, int2 b
     return make_int2(med(mva.x, mvb.x, mvc.x), med(mva.y, mvb.y, mvc.y));
 }
 
-// The persistent plain-ME kernel.  Each warp takes MB tickets dealt in
-// wavefront order (frames interleaved), waits (bounded, status 1) until the
-// MB's left and top-right neighbours are published, derives the median
-// predictor from their picks, stages the reference window around it in
-// shared memory (one TMA tensor copy, or bulk copies row by row when the
-// planes have no tensor map; status 3 if they do not land), runs best_part
-// for 16x16 and, when its J exceeds the gate, for the four 16x8/8x16
-// partitions (mb16.rs:8869-8913), and publishes the pick (then, for
-// h264a_me_tq_frames, the MB's MC + T/Q).  BAL: the Balanced preset's knobs
-// as constants.  Dynamic shared memory: ME_WARPS windows of WIN_BYTES.
-template <bool BAL, bool LEARN, class TAB>
-__device__ __forceinline__ void me_frames_body(const TAB& tab, long long total, const MeParamsDev& prm,
-                                               int* __restrict__ counter, int* __restrict__ flags, int epoch,
-                                               int* __restrict__ status, int spin_limit) {
-    __shared__ WarpScratch scratch[ME_WARPS];
-    __shared__ __align__(8) unsigned long long win_bar[ME_WARPS];
-    extern __shared__ __align__(128) uint8_t me_win[];
-    const int w = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const uint32_t win = uint32_t(__cvta_generic_to_shared(me_win)) + uint32_t(w * WIN_BYTES);
-    const uint32_t bar = uint32_t(__cvta_generic_to_shared(&win_bar[w]));
-    if (lane == 0) {
-        mbar_init(bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
-    uint32_t parity = 0;
-    for (;;) {
-        int t = 0;
-        if (lane == 0) t = atomicAdd(counter, 1);
-        t = __shfl_sync(0xffffffffu, t, 0);
-        if (t >= total) return;
-        // the ticket's segment (dealt in order), frame and wavefront position
-        int s = 0;
-        while (s + 1 < tab.nseg() && tab.seg(s + 1) <= t) s++;
-        const int j = tab.segj(s);
-        const long long u = t - tab.seg(s);
-        const int nxt = j + 1 < tab.n() ? tab.fr(j + 1).mb_w * tab.fr(j + 1).mb_h : 0;
-        const FrameDesc& fd = tab.fr(int(u % (j + 1)));
-        const int k = nxt + int(u / (j + 1));  // position in the frame's wavefront order
-        int mbx, mby;
-        wave_mb(fd.mb_w, fd.mb_h, k, mbx, mby);
-        const int m = mby * fd.mb_w + mbx;
-        int* fl = flags + fd.flag_base;
-        const int lx = mbx * 16, ly = mby * 16;
-        // the source rows of the lane's 4x4 block in the 16x16 search (block
-        // lane & 15), loaded before the neighbour wait: the source is an input
-        uint32_t src4[4];
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-            src4[r] = ld4u(fd.pic.d_src + (long long)(ly + ((lane >> 2) & 3) * 4 + r) * fd.pic.cw + lx + (lane & 3) * 4);
-        // the learned search's proposal (lanes 1..8), also an input
-        int2 prop = make_int2(0, 0);
-        if (LEARN && lane >= 1 && lane <= N_PROP) {
-            const int32_t* pp = fd.props + 16LL * m + 2 * (lane - 1);
-            prop = make_int2(__ldg(pp), __ldg(pp + 1));
-        }
-        // dependencies: left, and top-right (or top at the right edge)
-        if (lane == 0) {
-            if (mbx > 0) wait_flag(fl + m - 1, epoch, status, 1, spin_limit);
-            if (mby > 0) wait_flag(fl + m - fd.mb_w + (mbx < fd.mb_w - 1 ? 1 : 0), epoch, status, 1, spin_limit);
-        }
-        __syncwarp();
-        // neighbours of the MB's top-left 4x4 block (mv_neighbors_block, mb16.rs:1871)
-        const bool aa = mbx > 0, ba = mby > 0, ca = mby > 0 && mbx < fd.mb_w - 1, da = mbx > 0 && mby > 0;
-        const int2 a = aa ? pick_mv_at(fd.picks, m - 1, 3, 0) : make_int2(0, 0);
-        const int2 bb = ba ? pick_mv_at(fd.picks, m - fd.mb_w, 0, 3) : make_int2(0, 0);
-        int2 c = ca ? pick_mv_at(fd.picks, m - fd.mb_w + 1, 0, 3) : make_int2(0, 0);
-        bool cav = ca;
-        if (!ca) {
-            cav = da;
-            c = da ? pick_mv_at(fd.picks, m - fd.mb_w - 1, 3, 3) : make_int2(0, 0);
-        }
-        const int2 pmv = predict_mv_ref0(aa, a, ba, bb, cav, c);
-        // stage the window: WIN_R rows/columns up-left of the predicted
-        // position, the x origin on a 16-byte boundary (bulk-copy alignment)
-        const h264a_picture& pc = fd.pic;
-        const int pw = pc.cw + 2 * pc.pad, ph = pc.ch + 2 * pc.pad;
-        const bool win_ok = ((reinterpret_cast<uintptr_t>(pc.d_planes) | uintptr_t(pw)) & 15) == 0 && pw >= WIN_W &&
-                            ph >= WIN_H;
-        if (win_ok) {
-            const int wx0 = min(max((lx + pc.pad + (pmv.x >> 2) - WIN_R) & ~15, 0), pw - WIN_W);
-            const int wy0 = min(max(ly + pc.pad + (pmv.y >> 2) - WIN_R, 0), ph - WIN_H);
-            if (lane == 0) {
-                scratch[w].wx0 = wx0;
-                scratch[w].wy0 = wy0;
-                // the previous MB's window reads are complete (the warp is converged here)
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                if (fd.tmap_ok) {  // the whole window in one tensor copy
-                    mbar_expect_tx(bar, uint32_t(WIN_BYTES));
-                    // a tensor map written to device memory by the host since an
-                    // earlier launch read that address: acquire it for the copy
-                    if (TAB::kGlobal)
-                        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&fd.tmap)
-                                     : "memory");
-                    tma_load_3d(win, &fd.tmap, wx0, wy0, 0, bar);
-                } else {
-                    mbar_expect_tx(bar, uint32_t(4 * WIN_H * WIN_W));
-                }
-            }
-            __syncwarp();
-            if (!fd.tmap_ok) {  // a bulk copy per plane row
-                const long long ps = (long long)pw * ph;
-                for (int i = lane; i < 4 * WIN_H; i += 32) {
-                    const int pl = i / WIN_H, r = i - pl * WIN_H;
-                    bulk_g2s(win + uint32_t(pl * WIN_PLANE + r * WIN_STRIDE),
-                             pc.d_planes + ps * pl + (long long)(wy0 + r) * pw + wx0, WIN_W, bar);
-                }
-            }
-        }
-        if (lane == 0) scratch[w].win_ok = win_ok;
-        __syncwarp();
-        int preds[4] = {pmv.x, pmv.y, 0, 0};
-        // best_part for 16x16 (the warp as one group), then, J above the gate,
-        // the four partitions seeded with [pmv, mv16] side by side; one call
-        // site, so the search body exists once in the kernel.
-        int evals = 0, shape = 0, mv0x = 0, mv0y = 0, mv1x = 0, mv1y = 0, fell = 0;
-        long long c16 = 0, best = 0;
-        for (int mode = 0; mode < 2; mode++) {
-            if (mode == 1 && !(fd.split_gate >= 0 && c16 > fd.split_gate)) break;
-            GroupGeom qg;
-            group_geom_init(qg, scratch[w], pc, lx, ly, mode, win, mode == 0 ? src4 : nullptr);
-            if (mode == 0 && win_ok) {
-                wait_window(bar, parity, status, 3, spin_limit);
-                parity ^= 1u;
-            }
-            int rx, ry, ev;
-            long long rc;
-            // the learned search's partitions, when its 16x16 search took a
-            // proposal: refine-only from the 16x16 MV
-            const bool lstart = LEARN && mode == 1 && !fell;
-            motion_search_group<BAL, LEARN>(qg, prm, scratch[w], preds, mode == 0 ? 1 : 2, fd.lambda_me, rx, ry, rc, ev,
-                                            LEARN && mode == 0, prop, fd.prop_t, mode == 0 ? &fell : nullptr, nullptr,
-                                            lstart, make_int2(preds[2], preds[3]));
-            if (mode == 0) {
-                evals = ev << 4;  // 4x4-block evaluations
-                c16 = rc; best = rc;
-                mv0x = mv1x = rx; mv0y = mv1y = ry;
-                preds[2] = rx; preds[3] = ry;
-            } else {
-                int px[4], py[4];
-                long long pcost[4];
-#pragma unroll
-                for (int gi = 0; gi < 4; gi++) {
-                    px[gi] = __shfl_sync(0xffffffffu, rx, 8 * gi);
-                    py[gi] = __shfl_sync(0xffffffffu, ry, 8 * gi);
-                    pcost[gi] = __shfl_sync(0xffffffffu, rc, 8 * gi);
-                    evals += __shfl_sync(0xffffffffu, ev, 8 * gi) << 3;
-                }
-                if (pcost[0] + pcost[1] < best) {  // 16x8 top + bottom
-                    best = pcost[0] + pcost[1]; shape = 1;
-                    mv0x = px[0]; mv0y = py[0]; mv1x = px[1]; mv1y = py[1];
-                }
-                if (pcost[2] + pcost[3] < best) {  // 8x16 left + right
-                    best = pcost[2] + pcost[3]; shape = 2;
-                    mv0x = px[2]; mv0y = py[2]; mv1x = px[3]; mv1y = py[3];
-                }
-            }
-        }
-        if (lane == 0) {
-            int32_t* p = fd.picks + 6 * m;
-            p[0] = shape; p[1] = mv0x; p[2] = mv0y; p[3] = mv1x; p[4] = mv1y; p[5] = evals;
-            fd.costs[2 * m] = best;
-            fd.costs[2 * m + 1] = c16;
-            if (LEARN && fd.fallback) fd.fallback[m] = fell;
-            st_release(fl + m, epoch);  // orders the pick's stores before the flag
-        }
-        // MC + luma T/Q of the MB under its pick (mb16.rs:3436-3450, as
-        // mc_tq_frames_kernel): after the publish, so off the wavefront's
-        // path; lane = 4x4 block, the prediction from the staged window
-        // when it covers the block's MV.
-        if (fd.coeffs != nullptr && lane < 16) {
-            const int bx = (lane & 3) * 4, by = (lane >> 2) * 4;
-            const int part = shape == 1 ? (by >= 8) : (shape == 2 ? (bx >= 8) : 0);
-            const int mvx = part ? mv1x : mv0x, mvy = part ? mv1y : mv0y;
-            const int x = lx + bx, y = ly + by;
-            uint32_t pr[4];
-            const uint32_t* sr = src4;  // lane < 16: the same block as the 16x16 search
-            const int wx = x + pc.pad - scratch[w].wx0 + (mvx >> 2), wy = y + pc.pad - scratch[w].wy0 + (mvy >> 2);
-            if (win_ok && win_covers(wx, wy)) {
-                win_rows(win, wx, wy, mvx & 3, mvy & 3, pr);
-            } else {
-                Planes P;
-                P.base = pc.d_planes; P.pw = pw; P.ph = ph; P.pad = pc.pad; P.ps = (long long)pw * ph;
-                pred_rows(P, x + (mvx >> 2), y + (mvy >> 2), mvx & 3, mvy & 3, pr);
-            }
-            const int qi = (by >= 8 ? 2 : 0) + (bx >= 8 ? 1 : 0), k = ((by & 4) ? 2 : 0) + ((bx & 4) ? 1 : 0);
-            tq4x4_store(sr, pr, fd.qff, fd.qmf, fd.coeffs + (long long)m * 256 + qi * 64 + k * 16);
-        }
-        __syncwarp();  // the lanes' stores ordered before lane 0's count
-        if (fd.row_count != nullptr && lane == 0 && atom_add_acq_rel(fd.row_count + mby, 1) == fd.mb_w - 1)
-            st_release_sys(fd.row_done + mby, fd.row_token);  // the row's last MB: tell the host
-        __syncwarp();
-    }
-}
+// ---------------------------------------------------------------------------
+// One MB of the frame kernels
+// ---------------------------------------------------------------------------
 
-// The wide variant for launches of few frames (the closed loop's one frame
-// at a time), where the wavefront has far fewer ready MBs than resident warps
-// and an MB's own latency is the whole cost: a CTA of ME_WARPS (4) warps takes
-// one MB.  Warp 0 waits for the neighbours, stages the window and runs the
-// 16x16 search exactly as the narrow kernel does; when the gate opens, warp w
-// searches partition w with all 32 lanes (four candidates per pass instead of
-// one per 8-lane group), each warp with its own copy of the search state and
-// the same seeds, centre and lambda, so every partition's result equals the
-// narrow kernel's.  Warp 0 then picks the shape and publishes, as before.
-// Dynamic shared memory: one window of WIN_BYTES.
-// The closed loop's reconstruction of a frame, fused into the wide kernel:
-// after an MB's pick is published, its luma MC + T/Q + reconstruction (warp
-// 0), chroma MC + T/Q + reconstruction (warp 1), then the in-loop deblocking
-// of the MB (warp 2) in shared tiles, once the deblocking of its left and
-// top-right neighbours is done (bounded waits on a second run of flags, the
-// same wavefront order as the search).
+// The closed loop's reconstruction of a frame, fused into the frame kernels:
+// after an MB's pick is published, the same warp runs its luma and chroma MC +
+// T/Q + reconstruction and then the in-loop deblocking of the MB in shared
+// tiles, once the deblocking of its left and top-right neighbours is done
+// (bounded waits on a second run of flags, the same wavefront order as the
+// search).
 struct RecDesc {
     const uint8_t* src_c[2];  // the frame's chroma source (U, V)
     const uint8_t* ref_c[2];  // the chroma reconstruction of the previous frame
@@ -1491,46 +603,34 @@ struct RecDesc {
     int16_t* ccoeffs;         // chroma levels, 128 per MB
     int qp, qpc;              // luma and chroma QP
     int16_t cff[8], cmf[8];   // the chroma QP's quant row (inter dead-zone)
-    int dflag_base;           // the deblocking flags' offset in the flag array
+    int dflag_base, nz_base;  // the deblocking flags' and coefficient masks' offsets in the flag array
     DbThresh th;
 };
 
-// The wide kernel's frame table (at most ME_WIDE_MAXF frames), passed by value.
-struct WideBatch {
-    FrameDesc f[ME_WIDE_MAXF];
-    RecDesc rec[ME_WIDE_MAXF];
-    long long seg_start[ME_WIDE_MAXF + 1];
-    int seg_j[ME_WIDE_MAXF];
-    int n, nseg;
-};
-struct WideTable {
-    const WideBatch& b;
-    __device__ __forceinline__ int n() const { return b.n; }
-    __device__ __forceinline__ int nseg() const { return b.nseg; }
-    __device__ __forceinline__ long long seg(int s) const { return b.seg_start[s]; }
-    __device__ __forceinline__ int segj(int s) const { return b.seg_j[s]; }
-    __device__ __forceinline__ const FrameDesc& fr(int i) const { return b.f[i]; }
-    __device__ __forceinline__ const RecDesc& rd(int i) const { return b.rec[i]; }
-};
-
-// The wide kernel publishes each MB's pick to the wavefront as three 64-bit
-// words, each the launch's epoch (high half) and one MV (x, y as i16, low
-// half): the MVs of its blocks (3,0), (0,3) and (3,3), which are what its
+// Where pictures allow it an MB's pick is published to the wavefront as three
+// 64-bit words, each the launch's epoch (high half) and one MV (x, y as i16,
+// low half): the MVs of its blocks (3,0), (0,3) and (3,3), which are what its
 // right, lower (and lower-left) and lower-right neighbours' median predictors
 // read (mv_neighbors_block, mb16.rs:1871).  A waiting MB polls the words it
 // needs until their epoch is the launch's, so the flag and the data arrive in
 // one load and no release fence orders anything else.  MVs fit i16 because
-// the search keeps every block inside the padded picture (at most 8191
-// samples wide or high here).
+// the search keeps every block inside the padded picture, at most 8191 samples
+// wide or high; larger pictures, and launches whose scratch holds one flag per
+// MB (h264a_me_frames_noalloc), publish a flag after the pick instead.
 constexpr int EW_PER_MB = 3;
+// Nanoseconds between polls of a warp diagonals ahead of the wavefront, and of
+// one waiting for its left or top-right neighbour.
+constexpr unsigned POLL_FAR_NS = 1000, POLL_NEAR_NS = 40;
+constexpr int EW_MAX_SIDE = 8191;
 __device__ __forceinline__ unsigned long long mv_word(int epoch, int x, int y) {
     return ((unsigned long long)(unsigned)epoch << 32) | (uint32_t(uint16_t(x)) | (uint32_t(uint16_t(y)) << 16));
 }
 __device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned long long v) {
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-// Waits (bounded; status 1 on timeout) for the word to carry `epoch`; returns its MV.
-__device__ __forceinline__ int2 wait_mv_word(const unsigned long long* p, int epoch, int* status, int limit) {
+// Waits (bounded; status 1 on timeout) for the word to carry `epoch`, polling
+// every `ns` nanoseconds; returns its MV.
+__device__ __forceinline__ int2 wait_mv_word(const unsigned long long* p, int epoch, int* status, int limit, unsigned ns) {
     unsigned long long v = 0;
     for (int it = 0;; it++) {
         asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -1539,383 +639,379 @@ __device__ __forceinline__ int2 wait_mv_word(const unsigned long long* p, int ep
             atomicCAS(status, 0, 1);
             break;
         }
-        if (it >= 32) __nanosleep(64);
+        __nanosleep(ns);
     }
     return make_int2(int(int16_t(v & 0xffffu)), int(int16_t((v >> 16) & 0xffffu)));
 }
 
-struct WideMb {
-    int pmvx, pmvy;         // the median predictor
-    int bready;             // a reference segment seen complete (pipelined loop, band_wait_px)
-    long long c16;          // 16x16 J
-    int mv16x, mv16y, ev16;
-    int px[4], py[4], pev[4];
-    long long pc[4];
+// The launch's synchronisation as one MB sees it: the frame's MV words (or
+// null: its flags), its deblocking flags and coefficient masks, the reference's segment readiness
+// (pipelined closed loop, or null) and the bounded waits' parameters.
+struct MbSync {
+    unsigned long long* ew;
+    int* flags;
+    int* dfl;
+    int* nz;  // REC: each MB's mask of luma blocks with coefficients (raster order), stored before its deblocking flag
+    const BandWait* bw;
+    int epoch;
+    int* status;
+    int limit;
 };
 
-// One MB of the wide kernels (a CTA per MB): the search (16x16 by all warps,
-// the partitions one warp each), the pick published to the wavefront as MV
-// words, and for h264a_me_tq_frames-style launches the MB's MC + T/Q; REC:
-// its reconstruction and deblocking (RecDesc).  ew_frame: the frame's MV
-// words; dfl: its deblocking flags; bw: the reference's band readiness
-// (pipelined closed loop) or nullptr.  The caller's CTA barrier after the
-// call frees the window and the shared state for the next MB.
-template <bool BAL, bool LEARN, bool REC>
-__device__ __forceinline__ void wide_mb(const FrameDesc& fd, const RecDesc& rd, int mbx, int mby,
-                                        const MeParamsDev& prm, unsigned long long* __restrict__ ew_frame,
-                                        int* __restrict__ dfl, const BandWait* bw, int epoch, int* __restrict__ status,
-                                        int spin_limit, uint32_t win, uint32_t bar, uint32_t& parity,
-                                        bool tmap_global = false) {
-    __shared__ WarpScratch scratch[ME_WIDE_WARPS];
-    __shared__ WideMb mb;
-    __shared__ int coop_dist[2][32];     // the team-wide 16x16 search's distortions
-    __shared__ int part_dist[4][2][32];  // each partition team's
-    // REC: the MB's reconstruction tiles (deblock_device.cuh's layout), its
-    // luma blocks' coefficient flags (raster order) and the edges' bS
-    __shared__ __align__(16) uint8_t rec_lt[REC ? LT * LT : 4];
-    __shared__ __align__(16) uint8_t rec_ct[2][REC ? CR * CT : 4];
-    __shared__ int rec_nz[16];
-    __shared__ int rec_bs[32];
-    const int w = threadIdx.x >> 5;
+// The reconstruction tiles of an MB (deblock_device.cuh's layout) and its
+// edges' bS.  They live in the MB's window buffer once its motion compensation
+// has read the window.
+struct RecTiles {
+    uint8_t lt[LT * LT];
+    uint8_t ct[2][CR * CT];
+    int bs[32];
+};
+static_assert(sizeof(RecTiles) <= WIN_BYTES && alignof(RecTiles) <= 16, "the tiles fit the window buffer");
+
+// Stages the reference window around MV `mv` of the MB at (lx, ly): WIN_R rows
+// and columns up-left of the position, the x origin on a 16-byte boundary
+// (bulk-copy alignment); one TMA tensor copy, or a bulk copy per plane row
+// when the planes have no tensor map.  Returns whether a window is on its way
+// (wait_window on `bar`).  The warp is converged; its earlier accesses to the
+// buffer are ordered before the copy.
+__device__ __forceinline__ bool stage_window(MbScratch& ws, const CUtensorMap* tmap, bool tmap_ok, bool tmap_global,
+                                             int lx, int ly, int2 mv, uint32_t win, uint32_t bar) {
     const int lane = threadIdx.x & 31;
-    const int m = mby * fd.mb_w + mbx;
-    unsigned long long* const ew = ew_frame + EW_PER_MB * m;
-    const int lx = mbx * 16, ly = mby * 16;
-    const h264a_picture& pc = fd.pic;
-    const int pw = pc.cw + 2 * pc.pad, ph = pc.ch + 2 * pc.pad;
-    const bool win_ok = ((reinterpret_cast<uintptr_t>(pc.d_planes) | uintptr_t(pw)) & 15) == 0 && pw >= WIN_W &&
-                        ph >= WIN_H;
-    int preds[4] = {0, 0, 0, 0};
-    int fell = 0;
-    // every warp's source rows of its lane's 4x4 block in the 16x16 search
-    // (block lane & 15) and, for the learned search, its proposal (lane
-    // gl holds proposal gl - 1), loaded before the neighbour wait
-    uint32_t src4[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++)
-        src4[r] = ld4u(pc.d_src + (long long)(ly + ((lane >> 2) & 3) * 4 + r) * pc.cw + lx + (lane & 3) * 4);
-    int2 prop = make_int2(0, 0);
-    if (LEARN && lane >= 1 && lane <= N_PROP) {
-        const int32_t* pp = fd.props + 16LL * m + 2 * (lane - 1);
-        prop = make_int2(__ldg(pp), __ldg(pp + 1));
-    }
-    if (w == 0) {
-        // the neighbours' published MVs: lane 0 the left MB's (3,0), lane
-        // 1 the top MB's (0,3), lane 2 the top-right MB's (0,3), lane 3
-        // the top-left MB's (3,3) when there is no top-right
-        const bool aa = mbx > 0, ba = mby > 0, ca = mby > 0 && mbx < fd.mb_w - 1, da = mbx > 0 && mby > 0;
-        const bool need = lane < 4 && (lane == 0 ? aa : (lane == 1 ? ba : (lane == 2 ? ca : (!ca && da))));
-        const int dm = lane == 0 ? -EW_PER_MB
-                                 : EW_PER_MB * (lane == 1 ? -fd.mb_w : (lane == 2 ? 1 - fd.mb_w : -1 - fd.mb_w));
-        const unsigned long long* word = ew + dm + (lane == 0 ? 0 : (lane == 3 ? 2 : 1));
-        // The neighbours above were published a row earlier, so the window's
-        // origin is guessed from the top MB's MV and its copy overlaps the
-        // wait for the left MB (on the wavefront's path).  Any origin gives
-        // the same results: candidates the window misses read the planes.
-        int2 nv = make_int2(0, 0);
-        if (need && (lane > 0 || !ba)) nv = wait_mv_word(word, epoch, status, spin_limit);
-        __syncwarp();
-        const int2 bb = make_int2(__shfl_sync(0xffffffffu, nv.x, 1), __shfl_sync(0xffffffffu, nv.y, 1));
-        const int2 c = make_int2(__shfl_sync(0xffffffffu, nv.x, ca ? 2 : 3), __shfl_sync(0xffffffffu, nv.y, ca ? 2 : 3));
-        const int2 guess = ba ? bb : predict_mv_ref0(aa, make_int2(__shfl_sync(0xffffffffu, nv.x, 0),
-                                                                   __shfl_sync(0xffffffffu, nv.y, 0)),
-                                                     false, bb, false, c);
-        if (lane == 0) {
-            mb.bready = -1;
-            scratch[0].win_ok = win_ok;
+    const bool ok = ((reinterpret_cast<uintptr_t>(ws.base) | uintptr_t(ws.pw)) & 15) == 0 && ws.pw >= WIN_W && ws.ph >= WIN_H;
+    if (!ok) return false;
+    const int wx0 = min(max((lx + ws.pad + (mv.x >> 2) - WIN_R) & ~15, 0), ws.pw - WIN_W);
+    const int wy0 = min(max(ly + ws.pad + (mv.y >> 2) - WIN_R, 0), ws.ph - WIN_H);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) {
+        ws.wx0 = wx0;
+        ws.wy0 = wy0;
+        // the window's reference rows are built (pipelined loop), and the
+        // generic-proxy writes of them are visible to the copy
+        band_wait_px(ws.bw, &ws.bready, wy0 - ws.pad + WIN_H - 1, wx0 - ws.pad + WIN_W - 1);
+        if (ws.bw != nullptr) asm volatile("fence.proxy.async.global;" ::: "memory");
+        if (tmap_ok) {
+            mbar_expect_tx(bar, uint32_t(WIN_BYTES));
+            // a tensor map written to device memory by the host since an
+            // earlier launch read that address: acquire it for the copy
+            if (tmap_global) asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmap) : "memory");
+            tma_load_3d(win, tmap, wx0, wy0, 0, bar);
+        } else {
+            mbar_expect_tx(bar, uint32_t(4 * WIN_H * WIN_W));
         }
-        if (win_ok) {
-            const int wx0 = min(max((lx + pc.pad + (guess.x >> 2) - WIN_R) & ~15, 0), pw - WIN_W);
-            const int wy0 = min(max(ly + pc.pad + (guess.y >> 2) - WIN_R, 0), ph - WIN_H);
-            if (lane == 0) {
-                scratch[0].wx0 = wx0;
-                scratch[0].wy0 = wy0;
-                // the window's reference rows are built (pipelined loop), and
-                // the generic-proxy writes of them are visible to the copy
-                band_wait_px(bw, &mb.bready, wy0 - pc.pad + WIN_H - 1, wx0 - pc.pad + WIN_W - 1);
-                if (bw != nullptr) asm volatile("fence.proxy.async.global;" ::: "memory");
-                // every warp's reads of the previous MB's window are
-                // complete (the CTA barrier at the end of the last MB)
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                if (fd.tmap_ok) {
-                    mbar_expect_tx(bar, uint32_t(WIN_BYTES));
-                    if (tmap_global)  // a tensor map in device memory, as above (once per frame and CTA)
-                        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&fd.tmap)
-                                     : "memory");
-                    tma_load_3d(win, &fd.tmap, wx0, wy0, 0, bar);
-                } else {
-                    mbar_expect_tx(bar, uint32_t(4 * WIN_H * WIN_W));
-                }
-            }
-            __syncwarp();
-            if (!fd.tmap_ok) {
-                const long long ps = (long long)pw * ph;
-                for (int i = lane; i < 4 * WIN_H; i += 32) {
-                    const int pl = i / WIN_H, r = i - pl * WIN_H;
-                    bulk_g2s(win + uint32_t(pl * WIN_PLANE + r * WIN_STRIDE),
-                             pc.d_planes + ps * pl + (long long)(wy0 + r) * pw + wx0, WIN_W, bar);
-                }
-            }
-        }
-        if (need && lane == 0 && ba) nv = wait_mv_word(word, epoch, status, spin_limit);
-        __syncwarp();
-        const int2 a = make_int2(__shfl_sync(0xffffffffu, nv.x, 0), __shfl_sync(0xffffffffu, nv.y, 0));
-        const int2 pmv = predict_mv_ref0(aa, a, ba, bb, ca || da, c);
-        if (lane == 0) {
-            mb.pmvx = pmv.x;
-            mb.pmvy = pmv.y;
-        }
-    }
-    __syncthreads();  // the predictor and the window's origin are in shared memory
-    if (lane == 0 && w > 0) {
-        scratch[w].win_ok = scratch[0].win_ok;
-        scratch[w].wx0 = scratch[0].wx0;
-        scratch[w].wy0 = scratch[0].wy0;
     }
     __syncwarp();
-    preds[0] = mb.pmvx;
-    preds[1] = mb.pmvy;
-    // the 16x16 search by all warps together (2 * ME_WIDE_WARPS candidates
-    // per pass)
-    int rx16, ry16, ev16;
-    long long c16;
-    {
-        GroupGeom qg;
-        group_geom_init(qg, scratch[w], pc, lx, ly, 0, win, src4, 0, bw, mb.bready);
-        if (win_ok) wait_window(bar, parity, status, 3, spin_limit);
-        if (win_ok) parity ^= 1u;
-        motion_search_group<BAL, LEARN, 2 * ME_WIDE_WARPS, 2 * ME_WIDE_WARPS, ME_WIDE_WARPS>(
-            qg, prm, scratch[w], preds, 1, fd.lambda_me, rx16, ry16, c16, ev16, LEARN, prop, fd.prop_t, &fell,
-            &coop_dist[0][0]);
-    }
-    if (w == 0 && lane == 0) {
-        mb.c16 = c16;
-        mb.mv16x = rx16;
-        mb.mv16y = ry16;
-        mb.ev16 = ev16 << 4;
-    }
-    // every warp holds the same 16x16 result: the gate and the partition
-    // searches' seeds need no barrier
-    const bool gated = fd.split_gate >= 0 && c16 > fd.split_gate;
-    if (gated) {
-        // partition w / ME_PART_TEAM by its team of warps
-        const int part = w / ME_PART_TEAM;
-        preds[2] = rx16;
-        preds[3] = ry16;
-        GroupGeom qg;
-        group_geom_init(qg, scratch[w], pc, lx, ly, 2, win, nullptr, part, bw, mb.bready);
-        int rx, ry, ev;
-        long long rc;
-        // the learned search's partitions, when its 16x16 search took a
-        // proposal: refine-only from the 16x16 MV
-        motion_search_group<BAL, false, 4 * ME_PART_TEAM, 4 * ME_PART_TEAM, ME_PART_TEAM>(
-            qg, prm, scratch[w], preds, 2, fd.lambda_me, rx, ry, rc, ev, false, make_int2(0, 0), 0, nullptr,
-            &part_dist[part][0][0], LEARN && !fell, make_int2(rx16, ry16));
-        if (lane == 0 && w % ME_PART_TEAM == 0) {
-            mb.px[part] = rx;
-            mb.py[part] = ry;
-            mb.pc[part] = rc;
-            mb.pev[part] = ev << 3;
+    if (!tmap_ok) {
+        const long long ps = (long long)ws.pw * ws.ph;
+        for (int i = lane; i < 4 * WIN_H; i += 32) {
+            const int pl = i / WIN_H, r = i - pl * WIN_H;
+            bulk_g2s(win + uint32_t(pl * WIN_PLANE + r * WIN_STRIDE),
+                     ws.base + ps * pl + (long long)(wy0 + r) * ws.pw + wx0, WIN_W, bar);
         }
     }
-    __syncthreads();
-    // the shape decision (mb16.rs:8869-8913), taken by every warp from
-    // the shared results
-    int evals = ev16 << 4, shape = 0;
-    int mv0x = rx16, mv0y = ry16, mv1x = rx16, mv1y = ry16;
-    long long best = c16;
-    if (gated) {
-        evals += mb.pev[0] + mb.pev[1] + mb.pev[2] + mb.pev[3];
-        if (mb.pc[0] + mb.pc[1] < best) {  // 16x8 top + bottom
-            best = mb.pc[0] + mb.pc[1]; shape = 1;
-            mv0x = mb.px[0]; mv0y = mb.py[0]; mv1x = mb.px[1]; mv1y = mb.py[1];
-        }
-        if (mb.pc[2] + mb.pc[3] < best) {  // 8x16 left + right
-            best = mb.pc[2] + mb.pc[3]; shape = 2;
-            mv0x = mb.px[2]; mv0y = mb.py[2]; mv1x = mb.px[3]; mv1y = mb.py[3];
-        }
-    }
-    if (w == 0) {
-        if (lane == 0) {
-            int32_t* p = fd.picks + 6 * m;
-            p[0] = shape; p[1] = mv0x; p[2] = mv0y; p[3] = mv1x; p[4] = mv1y; p[5] = evals;
-            fd.costs[2 * m] = best;
-            fd.costs[2 * m + 1] = c16;
-            if (LEARN && fd.fallback) fd.fallback[m] = fell;
-        }
-        // the pick to the wavefront: blocks (3,0), (0,3), (3,3)
-        if (lane < EW_PER_MB) {
-            const bool second = lane == 0 ? shape == 2 : (lane == 1 ? shape == 1 : shape != 0);
-            st_relaxed_u64(ew + lane, mv_word(epoch, second ? mv1x : mv0x, second ? mv1y : mv0y));
-        }
-        if (fd.coeffs != nullptr && lane < 16) {
-            const int bx = (lane & 3) * 4, by = (lane >> 2) * 4;
-            const int part = shape == 1 ? (by >= 8) : (shape == 2 ? (bx >= 8) : 0);
-            const int mvx = part ? mv1x : mv0x, mvy = part ? mv1y : mv0y;
-            const int x = lx + bx, y = ly + by;
-            uint32_t sr[4], pr[4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) sr[r] = ld4u(pc.d_src + (long long)(y + r) * pc.cw + x);
-            const int wx = x + pc.pad - scratch[0].wx0 + (mvx >> 2), wy = y + pc.pad - scratch[0].wy0 + (mvy >> 2);
-            if (win_ok && win_covers(wx, wy)) {
-                win_rows(win, wx, wy, mvx & 3, mvy & 3, pr);
-            } else {
-                band_wait_px(bw, &scratch[0].bready, y + (mvy >> 2) + 5, x + (mvx >> 2) + 5);
-                Planes P;
-                P.base = pc.d_planes; P.pw = pw; P.ph = ph; P.pad = pc.pad; P.ps = (long long)pw * ph;
-                P.cg = bw != nullptr;
-                pred_rows(P, x + (mvx >> 2), y + (mvy >> 2), mvx & 3, mvy & 3, pr);
-            }
-            const int qi = (by >= 8 ? 2 : 0) + (bx >= 8 ? 1 : 0), kk = ((by & 4) ? 2 : 0) + ((bx & 4) ? 1 : 0);
-            int16_t* co = fd.coeffs + (long long)m * 256 + qi * 64 + kk * 16;
-            if (REC) {
-                // mb16.rs:3575-3605: the luma reconstruction into the tile
-                int lv[16];
-                tq4x4_store(sr, pr, fd.qff, fd.qmf, co, lv);
-                int any = 0;
-#pragma unroll
-                for (int i = 0; i < 16; i++) any |= lv[i];
-                rec_nz[lane] = any != 0;
-                uint32_t r4[4];
-                rec4x4(lv, pr, rd.qp, r4);
-#pragma unroll
-                for (int r = 0; r < 4; r++)
-                    *reinterpret_cast<uint32_t*>(rec_lt + (4 + by + r) * LT + 4 + bx) = r4[r];
-            } else {
-                tq4x4_store(sr, pr, fd.qff, fd.qmf, co);
-            }
-        }
-        __syncwarp();
-        if (fd.row_count != nullptr && lane == 0 && atom_add_acq_rel(fd.row_count + mby, 1) == fd.mb_w - 1)
-            st_release_sys(fd.row_done + mby, fd.row_token);
-    }
-    if (REC) {
-        const int cx0 = mbx * 8, cy0 = mby * 8;
-        if (w == 1) {
-            // chroma: lanes 0..7 are (plane, block k); lanes 8..31 shadow
-            // them so that the quads' shuffles run over the full warp
-            const int c = (lane >> 2) & 1, kb = lane & 3;
-            const int bx = (kb & 1) * 4, by = (kb >> 1) * 4;
-            const int part = shape == 1 ? (by >= 4) : (shape == 2 ? (bx >= 4) : 0);
-            const int mvx = part ? mv1x : mv0x, mvy = part ? mv1y : mv0y;
-            // the previous reconstruction's chroma rows it reads are final
-            // (pipelined loop: band b complete means MB rows 0..b+1 deblocked)
-            band_wait_px(bw, &scratch[1].bready, 2 * min(cy0 + by + 4 + (mvy >> 3), pc.ch / 2 - 1) + 1,
-                         2 * min(cx0 + bx + 4 + (mvx >> 3), pc.cw / 2 - 1) + 1);
-            uint32_t r4[4];
-            chroma_tq_rec(rd.src_c[c], rd.ref_c[c], pc.cw / 2, pc.ch / 2, cx0 + bx, cy0 + by, mvx, mvy, kb, rd.qpc,
-                          rd.cff, rd.cmf, lane < 8 ? rd.ccoeffs + (long long)m * 128 + c * 64 + kb * 16 : nullptr,
-                          r4, bw != nullptr);
-            if (lane < 8) {
-#pragma unroll
-                for (int r = 0; r < 4; r++)
-                    *reinterpret_cast<uint32_t*>(&rec_ct[c][(2 + by + r) * CT + 4 + bx]) = r4[r];
-            }
-        }
-        const bool left = mbx > 0, top = mby > 0;
-        const DbStrips strips(lane, rd.rec_y, pc.cw, lx, ly, rd.rec_c, cx0, cy0, rec_lt, rec_ct[0], rec_ct[1], left,
-                              top, true);
-        int nmx = 0, nmy = 0;
-        bool nnz = false;
-        if (w == 2) {
-            // the left and top-right neighbours' deblocking (so the top
-            // neighbour's too), then the strips their edges reach and the
-            // neighbours' blocks on this MB's edges
-            if (lane == 0 && left) wait_flag(dfl + m - 1, epoch, status, 1, spin_limit);
-            if (lane == 1 && top)
-                wait_flag(dfl + m - fd.mb_w + (mbx < fd.mb_w - 1 ? 1 : 0), epoch, status, 1, spin_limit);
-            __syncwarp();
-            strips.load();
-            if (lane < 4 && left) block_state_at(fd.picks, fd.coeffs, m - 1, 3, lane, nmx, nmy, nnz);
-            if (lane >= 16 && lane < 20 && top)
-                block_state_at(fd.picks, fd.coeffs, m - fd.mb_w, lane - 16, 3, nmx, nmy, nnz);
-        }
-        __syncthreads();  // the MB's tiles and coefficient flags are complete
-        if (w == 2) {
-            // bS: lanes 0..15 the vertical edges (edge e, block row sg),
-            // lanes 16..31 the horizontal ones (edge e, block column sg)
-            const int hor = lane >> 4, e = (lane >> 2) & 3, sg = lane & 3;
-            const int qbx = hor ? sg : e, qby = hor ? e : sg;
-            auto own = [&](int bx4, int by4, int& mx, int& my) {
-                const int part = shape == 1 ? (by4 >= 2) : (shape == 2 ? (bx4 >= 2) : 0);
-                mx = part ? mv1x : mv0x;
-                my = part ? mv1y : mv0y;
-            };
-            int bs = 0;
-            if (e > 0 || (hor ? top : left)) {
-                int pmx = nmx, pmy = nmy, qmx, qmy;
-                bool pnz = nnz;
-                if (e > 0) {
-                    const int pbx = hor ? sg : e - 1, pby = hor ? e - 1 : sg;
-                    own(pbx, pby, pmx, pmy);
-                    pnz = rec_nz[pby * 4 + pbx] != 0;
-                }
-                own(qbx, qby, qmx, qmy);
-                bs = bs_of(pnz, rec_nz[qby * 4 + qbx] != 0, pmx, pmy, qmx, qmy);
-            }
-            rec_bs[lane] = bs;
-            __syncwarp();
-            deblock_mb_tiles(lane, rec_lt, rec_ct[0], rec_ct[1], rec_bs, left, top, true, rd.th);
-            db_store_mb(lane, rec_lt, rec_ct[0], rec_ct[1], rd.rec_y, pc.cw, lx, ly, rd.rec_c, cx0, cy0, true);
-            strips.store();
-            __syncwarp();  // every lane's stores ordered before lane 0's release
-            if (lane == 0) st_release(dfl + m, epoch);
-        }
-    }
+    return true;
 }
 
-template <bool BAL, bool LEARN, bool REC>
-__device__ __forceinline__ void me_frames_body_wide(const WideTable& tab, long long total, const MeParamsDev& prm,
-                                                    int* __restrict__ counter, int* __restrict__ flags, int epoch,
-                                                    int* __restrict__ status, int spin_limit) {
-    __shared__ __align__(8) unsigned long long win_bar;
-    __shared__ int ticket;
-    extern __shared__ __align__(128) uint8_t me_win[];
-    const uint32_t win = uint32_t(__cvta_generic_to_shared(me_win));
-    const uint32_t bar = uint32_t(__cvta_generic_to_shared(&win_bar));
-    if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
+// A warp's window buffer (dynamic shared memory), its mbarrier and the CTA's
+// operand table (shared address).
+struct WarpWindow {
+    uint8_t* p;
+    uint32_t win, bar, lut;
+};
+__device__ __forceinline__ WarpWindow warp_window(uint8_t* dyn, unsigned long long* bars, PhaseTab& pt, BalScratch* bs) {
+    const int w = threadIdx.x >> 5;
+    WarpWindow o;
+    o.p = dyn + w * WIN_BYTES;
+    o.win = uint32_t(__cvta_generic_to_shared(o.p));
+    o.bar = uint32_t(__cvta_generic_to_shared(bars + w));
+    o.lut = uint32_t(__cvta_generic_to_shared(&pt));
+    phase_tab_init(pt, int(threadIdx.x));
+    if ((threadIdx.x & 31) == 0) {
+        bs[w].lam = __longlong_as_double(0x7ff8000000000000ll);  // NaN: no table yet
+        mbar_init(o.bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    return o;
+}
+
+// One MB by one warp: the predictor from the neighbours' picks, the reference
+// window, best_part for 16x16 and, when its J exceeds the gate, for the four
+// partitions (mb16.rs:8869-8913), the pick published to the wavefront, then
+// off its path the MB's MC + T/Q when the frame has coefficients, and with
+// REC its reconstruction and deblocking.
+//
+// The neighbours above were published a row earlier; only the left one is on
+// the wavefront's path.  So the window's origin comes from the top MB's MV
+// and its copy overlaps the wait for the left MB; any origin gives the same
+// picks, as candidates the window misses read the planes.
+template <bool BAL, bool LEARN, bool REC>
+__device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp, int mbx, int mby,
+                                         const MeParamsDev& prm, const MbSync& sy, MbScratch& ws, BalScratch& bs,
+                                         const WarpWindow& ww, uint32_t& parity, bool tmap_global) {
+    const uint32_t win = ww.win, bar = ww.bar;
+    uint8_t* const winp = ww.p;
+    const int lane = threadIdx.x & 31;
+    const int mb_w = fd.mb_w, m = mby * mb_w + mbx;
+    const int lx = mbx * 16, ly = mby * 16;
+    const h264a_picture pc = fd.pic;
+    const int pw = pc.cw + 2 * pc.pad, ph = pc.ch + 2 * pc.pad;
+    MbLane s;
+    mb_load_src(s, pc.d_src, pc.cw, lx, ly);  // inputs: before any wait
+    int2 prop = make_int2(0, 0), propc = prop;  // proposals lane % 8 and lane / 4
+    if (LEARN) {
+        prop = make_int2(__ldg(fd.props + 16LL * m + 2 * (lane & 7)), __ldg(fd.props + 16LL * m + 2 * (lane & 7) + 1));
+        propc = make_int2(__ldg(fd.props + 16LL * m + 2 * (lane >> 2)), __ldg(fd.props + 16LL * m + 2 * (lane >> 2) + 1));
+    }
+    if (lane == 0) {
+        ws.base = pc.d_planes;
+        ws.src = pc.d_src;
+        ws.bw = sy.bw;
+        ws.pw = pw; ws.ph = ph; ws.pad = pc.pad; ws.cw = pc.cw; ws.ch = pc.ch;
+        ws.bready = -1;
+    }
+    // the neighbours' MVs: lane 0 the left MB's block (3,0), lane 1 the top
+    // MB's (0,3), lane 2 the top-right MB's (0,3), lane 3 the top-left MB's
+    // (3,3) when there is no top-right (mv_neighbors_block, mb16.rs:1871)
+    const bool aa = mbx > 0, ba = mby > 0, ca = mby > 0 && mbx < mb_w - 1, da = mbx > 0 && mby > 0;
+    const bool need = lane < 4 && (lane == 0 ? aa : (lane == 1 ? ba : (lane == 2 ? ca : (!ca && da))));
+    const int nb = m + (lane == 0 ? -1 : (lane == 1 ? -mb_w : (lane == 2 ? 1 - mb_w : -1 - mb_w)));
+    auto fetch = [&](unsigned ns) {
+        if (sy.ew != nullptr)
+            return wait_mv_word(sy.ew + EW_PER_MB * (long long)nb + (lane == 0 ? 0 : (lane == 3 ? 2 : 1)), sy.epoch, sy.status,
+                                sy.limit, ns);
+        wait_flag(sy.flags + nb, sy.epoch, sy.status, 1, sy.limit);
+        return pick_mv_at(fd.picks, nb, lane == 0 || lane == 3 ? 3 : 0, lane == 0 ? 0 : 3);
+    };
+    // most resident warps hold MBs some diagonals ahead of the wavefront: they
+    // wait for the top MB (two diagonals back) with long sleeps, so that their
+    // polling does not slow the warps on the path
+    int2 nv = make_int2(0, 0);
+    if (need && (lane == 1 || !ba)) nv = fetch(ba ? POLL_FAR_NS : POLL_NEAR_NS);
+    __syncwarp();
+    const int2 top = make_int2(__shfl_sync(0xffffffffu, nv.x, 1), __shfl_sync(0xffffffffu, nv.y, 1));
+    const int2 first = make_int2(__shfl_sync(0xffffffffu, nv.x, 0), __shfl_sync(0xffffffffu, nv.y, 0));
+    const int2 guess = ba ? top : first;  // (the first row predicts from the left MB alone)
+    const bool win_ok = stage_window(ws, &fd.tmap, fd.tmap_ok != 0, tmap_global, lx, ly, guess, win, bar);
+    if (need && lane != 1 && ba) nv = fetch(POLL_NEAR_NS);
+    __syncwarp();
+    const int2 left = make_int2(__shfl_sync(0xffffffffu, nv.x, 0), __shfl_sync(0xffffffffu, nv.y, 0));
+    const int2 corner = make_int2(__shfl_sync(0xffffffffu, nv.x, ca ? 2 : 3), __shfl_sync(0xffffffffu, nv.y, ca ? 2 : 3));
+    const int2 pmv = predict_mv_ref0(aa, left, ba, top, ca || da, corner);
+    mb_lane_16x16(s, lx, ly, win);
+    mb_lane_window(s, ws, win_ok);
+    if (win_ok) {
+        wait_window(bar, parity, sy.status, 3, sy.limit);
+        parity ^= 1u;
+    }
+    // best_part for 16x16, then, J above the gate, the four partitions seeded
+    // [pmv, mv16] side by side
+    int shape = 0, fell = 0;
+    SearchOut r16;
+    if constexpr (BAL)
+        r16 = search16_bal<LEARN, true>(s, ws, bs, ww.lut, pmv, fd.lambda_me, LEARN, propc, prop, fd.prop_t, &fell);
+    else
+        r16 = mb_search<0, LEARN>(s, prm, ws, ww.lut, pmv, pmv, 1, fd.lambda_me, LEARN, prop, fd.prop_t, &fell);
+    int evals = r16.evals << 4;  // 4x4-block evaluations
+    const int c16 = r16.cost;
+    long long best = c16;
+    int mv0x = r16.x, mv0y = r16.y, mv1x = r16.x, mv1y = r16.y;
+    if (fd.split_gate >= 0 && c16 > fd.split_gate) {
+        mb_lane_parts(s);
+        // the learned search's partitions, when its 16x16 search took a
+        // proposal: refine-only from the 16x16 MV
+        const int2 mv16 = make_int2(mv0x, mv0y);
+        SearchOut r;
+        if constexpr (BAL)
+            r = search_parts_bal<LEARN, true>(s, ws, bs, ww.lut, pmv, mv16, fd.lambda_me, LEARN && !fell, mv16);
+        else
+            r = mb_search<1, LEARN>(s, prm, ws, ww.lut, pmv, mv16, 2, fd.lambda_me, false, prop, 0, nullptr, LEARN && !fell, mv16);
+        int px[4], py[4];
+        long long pcost[4];
+#pragma unroll
+        for (int gi = 0; gi < 4; gi++) {
+            px[gi] = __shfl_sync(0xffffffffu, r.x, 8 * gi);
+            py[gi] = __shfl_sync(0xffffffffu, r.y, 8 * gi);
+            pcost[gi] = __shfl_sync(0xffffffffu, r.cost, 8 * gi);
+            evals += __shfl_sync(0xffffffffu, r.evals, 8 * gi) << 3;
+        }
+        if (pcost[0] + pcost[1] < best) {  // 16x8 top + bottom
+            best = pcost[0] + pcost[1]; shape = 1;
+            mv0x = px[0]; mv0y = py[0]; mv1x = px[1]; mv1y = py[1];
+        }
+        if (pcost[2] + pcost[3] < best) {  // 8x16 left + right
+            best = pcost[2] + pcost[3]; shape = 2;
+            mv0x = px[2]; mv0y = py[2]; mv1x = px[3]; mv1y = py[3];
+        }
+    }
+    if (sy.ew != nullptr && lane < EW_PER_MB) {
+        // the pick to the wavefront: blocks (3,0), (0,3), (3,3)
+        const bool second = lane == 0 ? shape == 2 : (lane == 1 ? shape == 1 : shape != 0);
+        st_relaxed_u64(sy.ew + EW_PER_MB * (long long)m + lane, mv_word(sy.epoch, second ? mv1x : mv0x, second ? mv1y : mv0y));
+    }
+    if (lane == 0) {
+        int32_t* p = fd.picks + 6LL * m;
+        p[0] = shape; p[1] = mv0x; p[2] = mv0y; p[3] = mv1x; p[4] = mv1y; p[5] = evals;
+        fd.costs[2LL * m] = best;
+        fd.costs[2LL * m + 1] = c16;
+        if (LEARN && fd.fallback) fd.fallback[m] = fell;
+        if (sy.ew == nullptr) st_release(sy.flags + m, sy.epoch);  // orders the pick's stores before the flag
+    }
+    // MC + T/Q of the MB under its pick (mb16.rs:3436-3450): lanes 0..15 the
+    // luma 4x4 blocks, the prediction from the staged window when it covers
+    // the block's MV; with REC, lanes 16..23 the chroma blocks (plane, block k
+    // in SUBBLOCKS order; lanes 24..31 shadow them) and the reconstruction of both
+    if (!REC && fd.coeffs == nullptr) return;
+    const bool chroma = REC && lane >= 16;
+    const int bx = (lane & 3) * 4, by = ((lane >> 2) & 3) * 4;             // luma block
+    const int cpl = (lane >> 2) & 1, kb = lane & 3, cbx = (kb & 1) * 4, cby = (kb >> 1) * 4;  // chroma block
+    const bool hi_y = chroma ? cby >= 4 : by >= 8, hi_x = chroma ? cbx >= 4 : bx >= 8;
+    const bool part = shape == 1 ? hi_y : (shape == 2 ? hi_x : false);
+    const int mvx = part ? mv1x : mv0x, mvy = part ? mv1y : mv0y;
+    const int cx0 = mbx * 8, cy0 = mby * 8;
+    uint32_t sr[4], prd[4];
+    if (chroma) {
+        const int ccw = pc.cw / 2, cch = pc.ch / 2;
+        const uint8_t* sp = rdp->src_c[cpl] + (long long)(cy0 + cby) * ccw + cx0 + cbx;
+#pragma unroll
+        for (int r = 0; r < 4; r++) sr[r] = __ldg(reinterpret_cast<const uint32_t*>(sp + (long long)r * ccw));
+        // the previous reconstruction's chroma rows it reads are final
+        band_wait_px(sy.bw, &ws.bready, 2 * min(cy0 + cby + 4 + (mvy >> 3), cch - 1) + 1,
+                     2 * min(cx0 + cbx + 4 + (mvx >> 3), ccw - 1) + 1);
+        chroma_rows(rdp->ref_c[cpl], ccw, cch, cx0 + cbx + (mvx >> 3), cy0 + cby + (mvy >> 3), mvx & 7, mvy & 7, prd);
+    } else if (lane < 16) {
+        const int x = lx + bx, y = ly + by;
+#pragma unroll
+        for (int r = 0; r < 4; r++) sr[r] = ld4u(pc.d_src + (long long)(y + r) * pc.cw + x);
+        const int wx = x + pc.pad - ws.wx0 + (mvx >> 2), wy = y + pc.pad - ws.wy0 + (mvy >> 2);
+        if (win_ok && win_covers(wx, wy)) {
+            win_rows(win, wx, wy, mvx & 3, mvy & 3, prd);
+        } else {
+            band_wait_px(sy.bw, &ws.bready, y + (mvy >> 2) + 5, x + (mvx >> 2) + 5);
+            const uint4 r = plane_rows(&ws, x, y, mvx, mvy);
+            prd[0] = r.x; prd[1] = r.y; prd[2] = r.z; prd[3] = r.w;
+        }
+    }
+    __syncwarp();  // the window is read: REC's tiles take its place
+    const int qi = (by >= 8 ? 2 : 0) + (bx >= 8 ? 1 : 0), kk = ((by & 4) ? 2 : 0) + ((bx & 4) ? 1 : 0);
+    int16_t* const co = fd.coeffs + (long long)m * 256 + qi * 64 + kk * 16;
+    if (!REC) {
+        if (lane < 16) tq4x4_store(sr, prd, fd.qff, fd.qmf, co);
+        if (fd.row_count != nullptr) {
+            __syncwarp();  // the lanes' stores ordered before lane 0's count
+            if (lane == 0 && atom_add_acq_rel(fd.row_count + mby, 1) == mb_w - 1)
+                st_release_sys(fd.row_done + mby, fd.row_token);  // the row's last MB: tell the host
+        }
+    }
+    if constexpr (REC) {
+        const RecDesc& rd = *rdp;
+        RecTiles& rt = *reinterpret_cast<RecTiles*>(winp);
+        const BlockQuant bq = block_quant(chroma ? rd.cff : fd.qff, chroma ? rd.cmf : fd.qmf, chroma ? rd.qpc : rd.qp);
+        uint32_t r4[4];
+        const bool any = mb_code_block(sr, prd, bq, chroma, kb,
+                                       chroma ? (lane < 24 ? rd.ccoeffs + (long long)m * 128 + cpl * 64 + kb * 16 : nullptr) : co, r4);
+        const unsigned nz = __ballot_sync(0xffffffffu, any) & 0xffffu;
+        if (lane < 24) {
+            uint8_t* const t = chroma ? &rt.ct[cpl][(2 + cby) * CT + 4 + cbx] : rt.lt + (4 + by) * LT + 4 + bx;
+#pragma unroll
+            for (int r = 0; r < 4; r++) *reinterpret_cast<uint32_t*>(t + r * (chroma ? CT : LT)) = r4[r];
+        }
+        if (lane == 0) sy.nz[m] = int(nz);
+        // the left and top-right neighbours' deblocking (so the top
+        // neighbour's too), then the strips their edges reach, and on lanes
+        // 0..3 and 16..19 the left and top MBs' blocks at this MB's edges:
+        // their MVs from the published words, their coefficient masks
+        const DbStrips strips(lane, rd.rec_y, pc.cw, lx, ly, rd.rec_c, cx0, cy0, rt.lt, rt.ct[0], rt.ct[1], aa, ba, true);
+        if (lane == 0 && aa) wait_flag(sy.dfl + m - 1, sy.epoch, sy.status, 1, sy.limit);
+        if (lane == 1 && ba) wait_flag(sy.dfl + m - mb_w + (mbx < mb_w - 1 ? 1 : 0), sy.epoch, sy.status, 1, sy.limit);
+        __syncwarp();
+        // bS: lanes 0..15 the vertical edges (edge e, block row sg),
+        // lanes 16..31 the horizontal ones (edge e, block column sg)
+        const int hor = lane >> 4, e = (lane >> 2) & 3, sg = lane & 3;
+        const bool edge = e > 0 || (hor ? ba : aa);
+        unsigned long long nw = 0;
+        unsigned nnz = 0;
+        if (e == 0 && edge) {
+            const int n = hor ? m - mb_w : m - 1;
+            nw = __ldcg(sy.ew + EW_PER_MB * (long long)n + (sg >= 2 ? 2 : hor));
+            nnz = (unsigned(__ldcg(sy.nz + n)) >> (hor ? 12 + sg : 4 * sg + 3)) & 1u;
+        }
+        strips.load();
+        auto own = [&](int bx4, int by4) {
+            const bool second = shape == 1 ? by4 >= 2 : (shape == 2 ? bx4 >= 2 : false);
+            return second ? make_int2(mv1x, mv1y) : make_int2(mv0x, mv0y);
+        };
+        int bs = 0;
+        if (edge) {
+            const int qbx = hor ? sg : e, qby = hor ? e : sg;
+            int2 pm = make_int2(int(int16_t(nw & 0xffffu)), int(int16_t((nw >> 16) & 0xffffu)));
+            if (e > 0) {
+                const int pbx = hor ? sg : e - 1, pby = hor ? e - 1 : sg;
+                pm = own(pbx, pby);
+                nnz = (nz >> (4 * pby + pbx)) & 1u;
+            }
+            const int2 qm = own(qbx, qby);
+            bs = bs_of(nnz != 0, ((nz >> (4 * qby + qbx)) & 1u) != 0, pm.x, pm.y, qm.x, qm.y);
+        }
+        rt.bs[lane] = bs;
+        __syncwarp();
+        deblock_mb_tiles(lane, rt.lt, rt.ct[0], rt.ct[1], rt.bs, aa, ba, true, rd.th);
+        db_store_mb(lane, rt.lt, rt.ct[0], rt.ct[1], rd.rec_y, pc.cw, lx, ly, rd.rec_c, cx0, cy0, true);
+        strips.store();
+        __syncwarp();  // every lane's stores ordered before lane 0's release
+        if (lane == 0) st_release(sy.dfl + m, sy.epoch);
+    }
+    __syncwarp();
+}
+
+// The persistent plain-ME kernel.  Each warp takes MB tickets dealt in
+// wavefront order (frames interleaved) and runs frame_mb on them.  words: the
+// launch's MV words (EW_PER_MB per MB), or null to use its flags.  Dynamic
+// shared memory: ME_WARPS windows of WIN_BYTES.
+template <bool BAL, bool LEARN, bool REC, class TAB>
+__device__ __forceinline__ void me_frames_body(const TAB& tab, long long total, const MeParamsDev& prm,
+                                               int* __restrict__ counter, int* __restrict__ flags,
+                                               unsigned long long* __restrict__ words, int epoch,
+                                               int* __restrict__ status, int spin_limit) {
+    __shared__ MbScratch scratch[ME_WARPS];
+    __shared__ __align__(16) BalScratch bal[ME_WARPS];
+    __shared__ PhaseTab ptab;
+    __shared__ __align__(8) unsigned long long win_bar[ME_WARPS];
+    extern __shared__ __align__(128) uint8_t me_win[];
+    const WarpWindow ww = warp_window(me_win, win_bar, ptab, bal);
+    MbScratch& ws = scratch[threadIdx.x >> 5];
     uint32_t parity = 0;
     for (;;) {
-        if (threadIdx.x == 0) ticket = atomicAdd(counter, 1);
-        __syncthreads();
-        const int t = ticket;
+        int t = 0;
+        if ((threadIdx.x & 31) == 0) t = atomicAdd(counter, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= total) return;
-        int s = 0;
-        while (s + 1 < tab.nseg() && tab.seg(s + 1) <= t) s++;
-        const int j = tab.segj(s);
-        const long long u = t - tab.seg(s);
+        // the ticket's segment (dealt in order), frame and wavefront position
+        int sg = 0;
+        while (sg + 1 < tab.nseg() && tab.seg(sg + 1) <= t) sg++;
+        const int j = tab.segj(sg);
+        const long long u = t - tab.seg(sg);
         const int nxt = j + 1 < tab.n() ? tab.fr(j + 1).mb_w * tab.fr(j + 1).mb_h : 0;
         const int fi = int(u % (j + 1));
         const FrameDesc& fd = tab.fr(fi);
-        const int k = nxt + int(u / (j + 1));
+        const int k = nxt + int(u / (j + 1));  // position in the frame's wavefront order
         int mbx, mby;
         wave_mb(fd.mb_w, fd.mb_h, k, mbx, mby);
-        const RecDesc& rd = tab.rd(fi);
-        wide_mb<BAL, LEARN, REC>(fd, rd, mbx, mby, prm,
-                                 reinterpret_cast<unsigned long long*>(flags) + EW_PER_MB * fd.flag_base,
-                                 flags + rd.dflag_base, nullptr, epoch, status, spin_limit, win, bar, parity);
-        __syncthreads();  // the MB's window and shared state are free for the next ticket
+        const RecDesc* rd = nullptr;
+        if constexpr (REC) rd = tab.rec(fi);
+        const MbSync sy{words ? words + EW_PER_MB * (long long)fd.flag_base : nullptr, flags + fd.flag_base,
+                        REC ? flags + rd->dflag_base : nullptr, REC ? flags + rd->nz_base : nullptr, nullptr, epoch,
+                        status, spin_limit};
+        frame_mb<BAL, LEARN, REC>(fd, rd, mbx, mby, prm, sy, ws, bal[threadIdx.x >> 5], ww, parity, TAB::kGlobal);
     }
-}
-
-template <bool BAL, bool LEARN, bool REC>
-__global__ void __launch_bounds__(32 * ME_WIDE_WARPS, ME_MIN_BLOCKS)
-    me_frames_wide_kernel(const __grid_constant__ WideBatch batch, long long total,
-                          const __grid_constant__ MeParamsDev prm, int* __restrict__ counter, int* __restrict__ flags,
-                          int epoch, int* __restrict__ status, int spin_limit) {
-    me_frames_body_wide<BAL, LEARN, REC>(WideTable{batch}, total, prm, counter, flags, epoch, status, spin_limit);
 }
 
 template <bool BAL, bool LEARN = false>
 __global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
     me_frames_kernel(const __grid_constant__ FrameBatch batch, long long total, const __grid_constant__ MeParamsDev prm,
-                     int* __restrict__ counter, int* __restrict__ flags, int epoch, int* __restrict__ status,
-                     int spin_limit) {
-    me_frames_body<BAL, LEARN>(ParamTable{batch}, total, prm, counter, flags, epoch, status, spin_limit);
+                     int* __restrict__ counter, int* __restrict__ flags, unsigned long long* __restrict__ words,
+                     int epoch, int* __restrict__ status, int spin_limit) {
+    me_frames_body<BAL, LEARN, false>(ParamTable{batch}, total, prm, counter, flags, words, epoch, status, spin_limit);
 }
 
 // The same kernel over a frame table in device memory (more than ME_MAXF
@@ -1925,13 +1021,38 @@ __global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
     me_frames_dkernel(const FrameDesc* __restrict__ frames, const long long* __restrict__ seg_start,
                       const int* __restrict__ seg_j, int nframes, int nseg, long long total,
                       const __grid_constant__ MeParamsDev prm, int* __restrict__ counter, int* __restrict__ flags,
-                      int epoch, int* __restrict__ status, int spin_limit) {
-    me_frames_body<BAL, LEARN>(DeviceTable{frames, seg_start, seg_j, nframes, nseg}, total, prm, counter, flags, epoch,
-                               status, spin_limit);
+                      unsigned long long* __restrict__ words, int epoch, int* __restrict__ status, int spin_limit) {
+    me_frames_body<BAL, LEARN, false>(DeviceTable{frames, seg_start, seg_j, nframes, nseg}, total, prm, counter, flags,
+                                      words, epoch, status, spin_limit);
 }
 
-// One warp waits on a flag that nothing sets; the bounded wait must give up
-// after `limit` polls and record status code 2.
+// One or two P frames with the fused reconstruction (h264a_closed_step_frame):
+// the frame table with its reconstruction descriptors, by value.
+struct StepBatch {
+    FrameDesc f[ME_FEW_FRAMES];
+    RecDesc rec[ME_FEW_FRAMES];
+    long long seg_start[ME_FEW_FRAMES + 1];
+    int seg_j[ME_FEW_FRAMES];
+    int n, nseg;
+};
+struct StepTable {
+    static constexpr bool kGlobal = false;
+    const StepBatch& b;
+    __device__ __forceinline__ int n() const { return b.n; }
+    __device__ __forceinline__ int nseg() const { return b.nseg; }
+    __device__ __forceinline__ long long seg(int s) const { return b.seg_start[s]; }
+    __device__ __forceinline__ int segj(int s) const { return b.seg_j[s]; }
+    __device__ __forceinline__ const FrameDesc& fr(int i) const { return b.f[i]; }
+    __device__ __forceinline__ const RecDesc* rec(int i) const { return &b.rec[i]; }
+};
+template <bool BAL, bool LEARN>
+__global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
+    me_step_kernel(const __grid_constant__ StepBatch batch, long long total, const __grid_constant__ MeParamsDev prm,
+                   int* __restrict__ counter, int* __restrict__ flags, unsigned long long* __restrict__ words, int epoch,
+                   int* __restrict__ status, int spin_limit) {
+    me_frames_body<BAL, LEARN, true>(StepTable{batch}, total, prm, counter, flags, words, epoch, status, spin_limit);
+}
+
 // ---------------------------------------------------------------------------
 // The pipelined closed loop: every P frame of a clip in one launch
 // ---------------------------------------------------------------------------
@@ -1955,13 +1076,13 @@ __global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
 // and a segment ticket of frame h first waits until frame h-nbuf+1, the last
 // reader of the buffer's previous picture, has finished every MB.
 //
-// Deadlock freedom: the CTAs form `pools` pools, block i taking frames
+// Deadlock freedom: the warps form `pools` pools, warp i taking frames
 // 1 + i % pools, 1 + i % pools + pools, ..., each pool its frames in order, a
-// CTA moving to the pool's next frame only once the current frame's tickets
+// warp moving to the pool's next frame only once the current frame's tickets
 // are all dealt.  A ticket waits only on earlier tickets of its own frame, on
 // frame h-1 and on frame h-nbuf+1's completion; the oldest unfinished frame
 // therefore depends on nothing unfinished, its tickets are all dealt or held
-// by CTAs of its own pool that are not blocked by a later frame, and it
+// by warps of its own pool that are not blocked by a later frame, and it
 // always progresses.  Every wait is still bounded, and after the first
 // timeout the others give up (status 1).
 struct PipeParams {
@@ -1971,7 +1092,7 @@ struct PipeParams {
     int nitems, n, mb_w, mb_h, nbands, nseg, segw, nbuf, pools;
     int* flags;            // per frame fstride ints: MV words, deblocking flags, segment flags
     long long fstride;
-    int ew_off, dfl_off, band_off;
+    int ew_off, dfl_off, nz_off, band_off;
     int* ctr;              // n ticket counters and n completed-MB counters, zeroed
     int* done;
     const uint8_t* rec_y;  // frame h's luma reconstruction at h * fs
@@ -1988,13 +1109,15 @@ struct PipeParams {
 // Segment (b, s) of frame h: the planes of its reconstruction for padded rows
 // [pad + 16b, pad + 16b + 16) (band 0 from row 0, the last band to the end)
 // and padded columns [pad + 16*segw*s, pad + 16*segw*(s+1)) (segment 0 from
-// column 0, the last segment to the end), into buffer h % nbuf.
+// column 0, the last segment to the end), into buffer h % nbuf.  One warp,
+// in strips of HP_STRIP columns from the segment's first.
 __device__ __forceinline__ void pipe_band(const PipeParams& pp, int h, int b, int sg, int epoch, int* status,
                                           int limit) {
     int* const ff = pp.flags + pp.fstride * h;
-    if (threadIdx.x == 0) {
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) {
         const int r = min(b + 1, pp.mb_h - 1), x = min(pp.segw * (sg + 1), pp.mb_w - 1);
-        wait_flag(ff + pp.dfl_off + r * pp.mb_w + x, epoch, status, 1, limit);
+        wait_flag(ff + pp.dfl_off + r * pp.mb_w + x, epoch, status, 1, limit, POLL_FAR_NS);
         if (h - pp.nbuf + 1 >= 1) {
             const int nmb = pp.mb_w * pp.mb_h;
             for (int it = 0; ld_acquire(pp.done + h - pp.nbuf + 1) < nmb; it++) {
@@ -2006,104 +1129,94 @@ __device__ __forceinline__ void pipe_band(const PipeParams& pp, int h, int b, in
             }
         }
     }
-    __syncthreads();
+    __syncwarp();
     const int pw = pp.cw + 2 * pp.pad, ph = pp.ch + 2 * pp.pad;
     const int y0 = b == 0 ? 0 : pp.pad + 16 * b;
     const int y1 = b == pp.nbands - 1 ? ph : pp.pad + 16 * b + 16;
     const int x0 = sg == 0 ? 0 : pp.pad + 16 * pp.segw * sg;
     const int x1 = sg == pp.nseg - 1 ? pw : pp.pad + 16 * pp.segw * (sg + 1);
-    for (int st = x0 / HP_STRIP + int(threadIdx.x >> 5); st * HP_STRIP < x1; st += ME_WIDE_WARPS)
-        hpel_strip_rows<true>(pp.rec_y + pp.fs * h, pp.cw, pp.ch, pp.pad, pp.planes + pp.pbytes * (h % pp.nbuf), pw,
-                              ph, st, y0, y1, pp.word_in, pp.word_out, x0, x1);
+    for (int xs = x0; xs < x1; xs += HP_STRIP)
+        hpel_strip_rows<true, true>(pp.rec_y + pp.fs * h, pp.cw, pp.ch, pp.pad, pp.planes + pp.pbytes * (h % pp.nbuf), pw,
+                              ph, xs, y0, y1, pp.word_in, pp.word_out, x1);
     // the planes' generic-proxy writes, visible to the readers' bulk copies
     asm volatile("fence.proxy.async.global;" ::: "memory");
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    __syncwarp();
+    if (lane == 0) {
         int* const sf = ff + pp.band_off + b * pp.nseg + sg;
         if (b > 0) wait_flag(sf - pp.nseg, epoch, status, 1, limit);
         if (sg > 0) wait_flag(sf - 1, epoch, status, 1, limit);
         st_release(sf, epoch);
     }
+    __syncwarp();
 }
 
-#ifndef PIPE_MIN_BLOCKS
-#define PIPE_MIN_BLOCKS ME_MIN_BLOCKS
-#endif
 template <bool BAL, bool LEARN>
-__global__ void __launch_bounds__(32 * ME_WIDE_WARPS, PIPE_MIN_BLOCKS)
+__global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
     closed_pipe_kernel(const __grid_constant__ PipeParams pp, const __grid_constant__ MeParamsDev prm, int epoch,
                        int* __restrict__ status, int spin_limit) {
-    __shared__ __align__(8) unsigned long long win_bar;
-    __shared__ int ticket;
-    __shared__ BandWait bwait;
+    __shared__ MbScratch scratch[ME_WARPS];
+    __shared__ __align__(16) BalScratch bal[ME_WARPS];
+    __shared__ PhaseTab ptab;
+    __shared__ __align__(8) unsigned long long win_bar[ME_WARPS];
+    __shared__ BandWait bwait[ME_WARPS];
     extern __shared__ __align__(128) uint8_t me_win[];
-    const uint32_t win = uint32_t(__cvta_generic_to_shared(me_win));
-    const uint32_t bar = uint32_t(__cvta_generic_to_shared(&win_bar));
-    if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const WarpWindow ww = warp_window(me_win, win_bar, ptab, bal);
     uint32_t parity = 0;
-    int fenced = -1;   // the frame whose tensor maps this CTA has acquired
-    int arrived = -1;  // the frame whose sources this CTA has seen uploaded
-    int h = 1 + int(blockIdx.x % unsigned(pp.pools));  // this CTA's pool: frames h, h + pools, ...
+    int fenced = -1;   // the frame whose tensor map this warp has acquired and whose sources it has seen
+    int h = 1 + int((blockIdx.x * ME_WARPS + w) % unsigned(pp.pools));  // this warp's pool: frames h, h + pools, ...
     while (h < pp.n) {
-        if (threadIdx.x == 0) ticket = atomicAdd(pp.ctr + h, 1);
-        __syncthreads();
-        const int t = ticket;
+        int t = 0;
+        if (lane == 0) t = atomicAdd(pp.ctr + h, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= pp.nitems) {
             h += pp.pools;  // every ticket of frame h is dealt: the pool's next frame
-            __syncthreads();
             continue;
         }
         const int item = __ldg(pp.items + t);
-        int* const ff = pp.flags + pp.fstride * h;
-        if (item >= 0) {
-            if (threadIdx.x == 0) {
-                if (pp.arrive != nullptr && arrived != h) {
-                    // the frame's sources are still being uploaded beside the launch
-                    for (int it = 0; ld_acquire(pp.arrive + h) != pp.atoken; it++) {
-                        if (it >= spin_limit ||
-                            ((it & 255) == 255 && *reinterpret_cast<volatile int*>(status) != 0)) {
-                            atomicCAS(status, 0, 1);
-                            break;
-                        }
-                        __nanosleep(200);
-                    }
-                }
-                bwait.flags = pp.flags + pp.fstride * (h - 1) + pp.band_off;
-                bwait.nbands = pp.nbands;
-                bwait.nseg = pp.nseg;
-                bwait.segw = 16 * pp.segw;
-                bwait.epoch = epoch;
-                bwait.limit = spin_limit;
-                bwait.status = status;
-            }
-            __syncthreads();
-            // frame 1's reference (frame 0) is built before the launch
-            wide_mb<BAL, LEARN, true>(pp.fds[h], pp.rds[h], item % pp.mb_w, item / pp.mb_w, prm,
-                                      reinterpret_cast<unsigned long long*>(ff + pp.ew_off), ff + pp.dfl_off,
-                                      h > 1 ? &bwait : nullptr, epoch, status, spin_limit, win, bar, parity,
-                                      fenced != h);
-            fenced = h;
-            arrived = h;
-            __syncthreads();  // every read and write of the MB is done
-            if (threadIdx.x == 0) {
-                const int c = atom_add_acq_rel(pp.done + h, 1);
-                if (c == pp.mb_w * pp.mb_h - 1 && pp.frame_words != nullptr) {
-                    // the frame's last MB: its outputs are final, for the host
-                    __threadfence_system();
-                    st_release_sys(pp.frame_words + h, pp.ftoken);
-                }
-            }
-        } else {
+        if (item < 0) {
             pipe_band(pp, h, (-item - 1) / pp.nseg, (-item - 1) % pp.nseg, epoch, status, spin_limit);
+            continue;
         }
-        __syncthreads();  // the window and shared state are free for the next ticket
+        int* const ff = pp.flags + pp.fstride * h;
+        if (lane == 0) {
+            if (pp.arrive != nullptr && fenced != h) {
+                // the frame's sources are still being uploaded beside the launch
+                for (int it = 0; ld_acquire(pp.arrive + h) != pp.atoken; it++) {
+                    if (it >= spin_limit || ((it & 255) == 255 && *reinterpret_cast<volatile int*>(status) != 0)) {
+                        atomicCAS(status, 0, 1);
+                        break;
+                    }
+                    __nanosleep(200);
+                }
+            }
+            if (fenced != h)
+                bwait[w] = BandWait{pp.flags + pp.fstride * (h - 1) + pp.band_off, pp.nbands, pp.nseg, 16 * pp.segw, epoch,
+                                    spin_limit, status};
+        }
+        __syncwarp();
+        // frame 1's reference (frame 0) is built before the launch
+        const MbSync sy{reinterpret_cast<unsigned long long*>(ff + pp.ew_off), nullptr, ff + pp.dfl_off, ff + pp.nz_off,
+                        h > 1 ? &bwait[w] : nullptr, epoch, status, spin_limit};
+        frame_mb<BAL, LEARN, true>(pp.fds[h], pp.rds + h, item % pp.mb_w, item / pp.mb_w, prm, sy, scratch[w], bal[w], ww,
+                                   parity, fenced != h);
+        fenced = h;
+        if (lane == 0 && pp.frame_words == nullptr) {
+            red_add_release(pp.done + h, 1);
+        } else if (lane == 0) {
+            const int c = atom_add_acq_rel(pp.done + h, 1);
+            if (c == pp.mb_w * pp.mb_h - 1) {
+                // the frame's last MB: its outputs are final, for the host
+                __threadfence_system();
+                st_release_sys(pp.frame_words + h, pp.ftoken);
+            }
+        }
+        __syncwarp();
     }
 }
 
+// One warp waits on a flag that nothing sets; the bounded wait must give up
+// after `limit` polls and record status code 2.
 __global__ void bounded_wait_selftest_kernel(const int* flag, int* status, int limit) {
     if (threadIdx.x == 0) wait_flag(flag, 1, status, 2, limit);
 }
@@ -2181,6 +1294,10 @@ static int me_frames_setup_once(int& per_sm, bool learn) {
     H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     H264A_CUDA(cudaFuncSetAttribute(me_frames_dkernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     H264A_CUDA(cudaFuncSetAttribute(me_frames_dkernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     per_sm = 0;
     if (learn)
         H264A_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, me_frames_kernel<false, true>, 32 * ME_WARPS,
@@ -2191,10 +1308,15 @@ static int me_frames_setup_once(int& per_sm, bool learn) {
     return H264A_OK;
 }
 
-// True when the parameters are the Balanced preset's (h264a_me_params_default):
-// the frame kernel then runs its instance with those knobs as constants.
-static bool balanced_preset(const MeParamsDev& p) {
-    return p.fast == 0 && p.use_sad == 0 && p.sadfp == 0 && p.kind == 0 && p.me_snap == 1 && p.fc == 1 &&
+// A λ that the Balanced searches' tables hold: every (λ·rate) as i64 (rates
+// up to 126) and every cost (distortions below 2^21) fits 31 bits.  The
+// encoder's are below 1,500; others run the general search.
+static bool balanced_lambda(double lam) { return lam >= 0.0 && lam < 8388608.0; }
+// True when the parameters are the Balanced preset's (h264a_me_params_default)
+// and the frames' λ allow it (lam_ok): the frame kernels then run the searches
+// written for it.
+static bool balanced_preset(const MeParamsDev& p, bool lam_ok) {
+    return lam_ok && p.fast == 0 && p.use_sad == 0 && p.sadfp == 0 && p.kind == 0 && p.me_snap == 1 && p.fc == 1 &&
            p.dia_mask == 0x1cu && p.subpel == 1 && p.subpel_pat == -1 && p.sp_single_pass == 1 &&
            p.me_subpel_iter == 1 && p.sp_maxit == 0 && p.sp_fc == 0;
 }
@@ -2229,111 +1351,49 @@ static long long fill_segments(FrameBatch& fb) {
 
 static void launch_me_frames_dtab(const MeParamsDev& prm, unsigned blocks, cudaStream_t st, const FrameDesc* frames,
                                   const long long* seg_start, const int* seg_j, int nframes, int nseg, long long total,
-                                  int* counter, int* flags, int epoch, int* status, bool learn = false) {
+                                  int* counter, int* flags, unsigned long long* words, int epoch, int* status,
+                                  bool lam_ok, bool learn = false) {
     const size_t sm = ME_WARPS * WIN_BYTES;
-    const bool bal = balanced_preset(prm);
+    const bool bal = balanced_preset(prm, lam_ok);
     if (learn && bal)
         me_frames_dkernel<true, true><<<blocks, 32 * ME_WARPS, sm, st>>>(frames, seg_start, seg_j, nframes, nseg, total,
-                                                                        prm, counter, flags, epoch, status, SPIN_LIMIT);
+                                                                        prm, counter, flags, words, epoch, status, SPIN_LIMIT);
     else if (learn)
         me_frames_dkernel<false, true><<<blocks, 32 * ME_WARPS, sm, st>>>(frames, seg_start, seg_j, nframes, nseg, total,
-                                                                         prm, counter, flags, epoch, status, SPIN_LIMIT);
+                                                                         prm, counter, flags, words, epoch, status, SPIN_LIMIT);
     else if (bal)
         me_frames_dkernel<true><<<blocks, 32 * ME_WARPS, sm, st>>>(frames, seg_start, seg_j, nframes, nseg, total, prm,
-                                                                  counter, flags, epoch, status, SPIN_LIMIT);
+                                                                  counter, flags, words, epoch, status, SPIN_LIMIT);
     else
         me_frames_dkernel<false><<<blocks, 32 * ME_WARPS, sm, st>>>(frames, seg_start, seg_j, nframes, nseg, total, prm,
-                                                                   counter, flags, epoch, status, SPIN_LIMIT);
+                                                                   counter, flags, words, epoch, status, SPIN_LIMIT);
 }
 
-// CTAs per SM of the wide kernel (one window per CTA), cached per device
-static int me_wide_setup_once(int& per_sm);
-static int me_wide_setup(int& per_sm) {
-    constexpr int kMaxDev = 64;
-    static int cached[kMaxDev];
-    static std::mutex mu;
-    int dev = 0;
-    H264A_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDev) return me_wide_setup_once(per_sm);
-    std::lock_guard<std::mutex> lock(mu);
-    if (!cached[dev]) {
-        const int rc = me_wide_setup_once(per_sm);
-        if (rc) return rc;
-        cached[dev] = per_sm + 1;
-    }
-    per_sm = cached[dev] - 1;
-    return H264A_OK;
-}
-
-template <bool BAL, bool LEARN, bool REC>
-static int wide_attr(int smem) {
-    H264A_CUDA(cudaFuncSetAttribute(me_frames_wide_kernel<BAL, LEARN, REC>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    return H264A_OK;
-}
-
-static int me_wide_setup_once(int& per_sm) {
-    const int smem = WIN_BYTES;
-    int rc = wide_attr<false, false, false>(smem) | wide_attr<true, false, false>(smem) |
-             wide_attr<false, true, false>(smem) | wide_attr<true, true, false>(smem) |
-             wide_attr<false, false, true>(smem) | wide_attr<true, false, true>(smem) |
-             wide_attr<false, true, true>(smem) | wide_attr<true, true, true>(smem);
-    if (rc) return rc;
-    // the residency of the largest variant bounds the grid of every one
-    per_sm = 0;
-    H264A_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, me_frames_wide_kernel<false, true, true>,
-                                                             32 * ME_WIDE_WARPS, smem));
-    int p2 = 0;
-    H264A_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p2, me_frames_wide_kernel<false, true, false>,
-                                                             32 * ME_WIDE_WARPS, smem));
-    if (p2 < per_sm) per_sm = p2;
-    if (per_sm < 1) per_sm = 1;
-    return H264A_OK;
-}
-
-template <bool REC>
-static void launch_wide_t(const MeParamsDev& prm, unsigned blocks, cudaStream_t st, const WideBatch& wb,
-                          long long total, int* counter, int* flags, int epoch, int* status, bool learn) {
-    const size_t sm = WIN_BYTES;
-    const bool bal = balanced_preset(prm);
-    if (learn && bal)
-        me_frames_wide_kernel<true, true, REC><<<blocks, 32 * ME_WIDE_WARPS, sm, st>>>(wb, total, prm, counter, flags,
-                                                                                 epoch, status, SPIN_LIMIT);
-    else if (learn)
-        me_frames_wide_kernel<false, true, REC><<<blocks, 32 * ME_WIDE_WARPS, sm, st>>>(wb, total, prm, counter, flags,
-                                                                                  epoch, status, SPIN_LIMIT);
-    else if (bal)
-        me_frames_wide_kernel<true, false, REC><<<blocks, 32 * ME_WIDE_WARPS, sm, st>>>(wb, total, prm, counter, flags,
-                                                                                  epoch, status, SPIN_LIMIT);
-    else
-        me_frames_wide_kernel<false, false, REC><<<blocks, 32 * ME_WIDE_WARPS, sm, st>>>(wb, total, prm, counter, flags,
-                                                                                   epoch, status, SPIN_LIMIT);
-}
-
-static void launch_me_frames_wide(const MeParamsDev& prm, unsigned blocks, cudaStream_t st, const WideBatch& wb,
-                                  long long total, int* counter, int* flags, int epoch, int* status, bool learn,
-                                  bool rec) {
-    if (rec)
-        launch_wide_t<true>(prm, blocks, st, wb, total, counter, flags, epoch, status, learn);
-    else
-        launch_wide_t<false>(prm, blocks, st, wb, total, counter, flags, epoch, status, learn);
+static void launch_me_step(const MeParamsDev& prm, unsigned blocks, cudaStream_t st, const StepBatch& sb, long long total,
+                           int* counter, int* flags, unsigned long long* words, int epoch, int* status, bool lam_ok,
+                           bool learn) {
+    const size_t sm = ME_WARPS * WIN_BYTES;
+    auto kern = balanced_preset(prm, lam_ok) ? (learn ? me_step_kernel<true, true> : me_step_kernel<true, false>)
+                                     : (learn ? me_step_kernel<false, true> : me_step_kernel<false, false>);
+    kern<<<blocks, 32 * ME_WARPS, sm, st>>>(sb, total, prm, counter, flags, words, epoch, status, SPIN_LIMIT);
 }
 
 static void launch_me_frames(const MeParamsDev& prm, unsigned blocks, cudaStream_t st, const FrameBatch& fb,
-                             long long total, int* counter, int* flags, int epoch, int* status, bool learn = false) {
+                             long long total, int* counter, int* flags, unsigned long long* words, int epoch,
+                             int* status, bool lam_ok, bool learn = false) {
     const size_t sm = ME_WARPS * WIN_BYTES;
-    const bool bal = balanced_preset(prm);
+    const bool bal = balanced_preset(prm, lam_ok);
     if (learn && bal)
-        me_frames_kernel<true, true><<<blocks, 32 * ME_WARPS, sm, st>>>(fb, total, prm, counter, flags, epoch, status,
+        me_frames_kernel<true, true><<<blocks, 32 * ME_WARPS, sm, st>>>(fb, total, prm, counter, flags, words, epoch, status,
                                                                        SPIN_LIMIT);
     else if (learn)
-        me_frames_kernel<false, true><<<blocks, 32 * ME_WARPS, sm, st>>>(fb, total, prm, counter, flags, epoch, status,
+        me_frames_kernel<false, true><<<blocks, 32 * ME_WARPS, sm, st>>>(fb, total, prm, counter, flags, words, epoch, status,
                                                                         SPIN_LIMIT);
     else if (bal)
-        me_frames_kernel<true><<<blocks, 32 * ME_WARPS, sm, st>>>(fb, total, prm, counter, flags, epoch, status,
+        me_frames_kernel<true><<<blocks, 32 * ME_WARPS, sm, st>>>(fb, total, prm, counter, flags, words, epoch, status,
                                                                  SPIN_LIMIT);
     else
-        me_frames_kernel<false><<<blocks, 32 * ME_WARPS, sm, st>>>(fb, total, prm, counter, flags, epoch, status,
+        me_frames_kernel<false><<<blocks, 32 * ME_WARPS, sm, st>>>(fb, total, prm, counter, flags, words, epoch, status,
                                                                   SPIN_LIMIT);
 }
 
@@ -2397,7 +1457,7 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
                          const MeRecIn* rec) {
     if (!ctx || !h_frames || !params) return fail(H264A_E_ARG, "me_frames: null pointer");
     if (nframes < 1) return fail(H264A_E_ARG, "me_frames: need at least one frame");
-    if (rec && (!tq || nframes > ME_WIDE_MAXF))
+    if (rec && (!tq || nframes > ME_FEW_FRAMES))
         return fail(H264A_E_ARG, "me_frames: the fused reconstruction needs T/Q outputs and at most two frames");
     if ((params->mv_cost_kind == 1 || params->mv_cost_kind == 2) && !params->d_mv_cost_tab)
         return fail(H264A_E_ARG, "me_frames: mv cost kinds 1 and 2 need d_mv_cost_tab");
@@ -2424,12 +1484,14 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
     });
     std::vector<FrameDesc> desc(nframes);
     memset(desc.data(), 0, sizeof(FrameDesc) * nframes);
-    RecDesc rdesc[ME_WIDE_MAXF];
+    RecDesc rdesc[ME_FEW_FRAMES];
     memset(rdesc, 0, sizeof rdesc);
     long long total = 0;
+    bool lam_ok = true;
     for (int k = 0; k < nframes; k++) {
         const h264a_me_frame& f = h_frames[order[k]];
         FrameDesc& d = desc[k];
+        lam_ok = lam_ok && balanced_lambda(f.lambda_me);
         d.pic = f.pic;
         d.tmap_ok = encode_window_map(&d.tmap, f.pic.d_planes, f.pic.cw + 2 * f.pic.pad, f.pic.ch + 2 * f.pic.pad);
         d.lambda_me = f.lambda_me;
@@ -2483,60 +1545,57 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
     std::vector<int> segj(nframes);
     const int nseg = make_segments(desc.data(), nframes, seg.data(), segj.data());
     if (seg[nseg] != total) return fail(H264A_E_ARG, "me_frames: internal queue layout error");
-    // The wide kernel (launches of at most ME_WIDE_MAXF frames) publishes MV
-    // words (2 * EW_PER_MB ints per MB), then the fused reconstruction's
-    // deblocking flags, in its own queue's flag space (cleared per launch);
-    // its MVs are packed as i16, so the padded pictures must be at most 8191
-    // samples wide and high.
-    bool wide = nframes <= ME_WIDE_MAXF;
+    // Launches of few frames run on the closed loop's queue, larger ones on the
+    // main one.  Picks go to the wavefront as MV words where the pictures'
+    // sides allow it and the words stay below 400 MB, else by flags.  The
+    // words, and the few-frame queue's flags (which also hold other layouts),
+    // are cleared ahead of the launch.
+    const bool few = nframes <= ME_FEW_FRAMES;
+    bool words_ok = total <= (1LL << 24);
     for (int k = 0; k < nframes; k++)
-        if (desc[k].pic.cw + 2 * desc[k].pic.pad > 8191 || desc[k].pic.ch + 2 * desc[k].pic.pad > 8191) wide = false;
-    if (rec && !wide) return fail(H264A_E_ARG, "me_frames: the fused reconstruction needs pictures of at most 8191 - 2 pad samples");
-    if (wide) {
-        // few frames: a CTA per MB, the partitions one warp each
-        const size_t nflags = size_t(2 * EW_PER_MB + (rec ? 1 : 0)) * size_t(total);
-        int rc = ensure_me_scratch(ctx, nflags, Q_WIDE);
-        if (rc) return rc;
-        WorkQueue& qw = ctx->q[Q_WIDE];
-        H264A_CUDA(cudaMemsetAsync(qw.d_counter, 0, sizeof(int32_t), st));
-        H264A_CUDA(cudaMemsetAsync(qw.d_flags, 0, sizeof(int32_t) * nflags, st));
-        const int epoch = next_epoch(ctx, st, Q_WIDE);
-        if (epoch < 0) return H264A_E_CUDA;
-        int wide_sm = 0;
-        rc0 = me_wide_setup(wide_sm);
-        if (rc0) return rc0;
-        long long wblocks = (long long)ctx->num_sms * wide_sm;
-        if (wblocks > total) wblocks = total;
-        WideBatch wb;
-        memset(&wb, 0, sizeof wb);
-        wb.n = nframes;
-        memcpy(wb.f, desc.data(), sizeof(FrameDesc) * nframes);
-        for (int k = 0; k < nframes; k++) {
-            wb.rec[k] = rdesc[k];
-            wb.rec[k].dflag_base = int(2 * EW_PER_MB * total) + desc[k].flag_base;
-        }
-        wb.nseg = make_segments(wb.f, wb.n, wb.seg_start, wb.seg_j);
-        if (wb.seg_start[wb.nseg] != total) return fail(H264A_E_ARG, "me_frames: internal queue layout error");
-        launch_me_frames_wide(prm, unsigned(wblocks), st, wb, total, qw.d_counter, qw.d_flags, epoch, ctx->d_status,
-                              learn != nullptr, rec != nullptr);
-        return check_launch("me_frames_wide_kernel");
-    }
-    int rc = ensure_me_scratch(ctx, size_t(total));
+        if (desc[k].pic.cw + 2 * desc[k].pic.pad > EW_MAX_SIDE || desc[k].pic.ch + 2 * desc[k].pic.pad > EW_MAX_SIDE)
+            words_ok = false;
+    if (rec && !words_ok)
+        return fail(H264A_E_ARG, "me_frames: the fused reconstruction needs pictures of at most 8191 - 2 pad samples");
+    const int qi = few ? Q_WIDE : Q_MAIN;
+    WorkQueue& qw = ctx->q[qi];
+    const size_t nflags = size_t(rec ? 3 * total : total);  // with rec: then deblocking flags and coefficient masks
+    int rc = ensure_me_scratch(ctx, nflags, qi);
+    if (!rc && words_ok) rc = ensure_me_words(ctx, size_t(EW_PER_MB) * size_t(total), qi);
     if (rc) return rc;
-    H264A_CUDA(cudaMemsetAsync(ctx->q[Q_MAIN].d_counter, 0, sizeof(int32_t), st));
-    const int epoch = next_epoch(ctx, st);
+    H264A_CUDA(cudaMemsetAsync(qw.d_counter, 0, sizeof(int32_t), st));
+    if (few) H264A_CUDA(cudaMemsetAsync(qw.d_flags, 0, sizeof(int32_t) * nflags, st));
+    unsigned long long* words = words_ok ? qw.d_words : nullptr;
+    if (words) H264A_CUDA(cudaMemsetAsync(words, 0, sizeof(unsigned long long) * EW_PER_MB * size_t(total), st));
+    const int epoch = next_epoch(ctx, st, qi);
     if (epoch < 0) return H264A_E_CUDA;
     long long blocks = (long long)ctx->num_sms * per_sm;
     const long long need = (total + ME_WARPS - 1) / ME_WARPS;
     if (blocks > need) blocks = need;
+    if (rec) {
+        StepBatch sb;
+        memset(&sb, 0, sizeof sb);
+        sb.n = nframes;
+        memcpy(sb.f, desc.data(), sizeof(FrameDesc) * nframes);
+        for (int k = 0; k < nframes; k++) {
+            sb.rec[k] = rdesc[k];
+            sb.rec[k].dflag_base = int(total) + desc[k].flag_base;
+            sb.rec[k].nz_base = int(2 * total) + desc[k].flag_base;
+        }
+        sb.nseg = make_segments(sb.f, sb.n, sb.seg_start, sb.seg_j);
+        if (sb.seg_start[sb.nseg] != total) return fail(H264A_E_ARG, "me_frames: internal queue layout error");
+        launch_me_step(prm, unsigned(blocks), st, sb, total, qw.d_counter, qw.d_flags, words, epoch, ctx->d_status,
+                       lam_ok, learn != nullptr);
+        return check_launch("me_step_kernel");
+    }
     if (nframes <= ME_MAXF) {
         FrameBatch fb;
         memset(&fb, 0, sizeof fb);
         fb.n = nframes;
         memcpy(fb.f, desc.data(), sizeof(FrameDesc) * nframes);
         if (fill_segments(fb) != total) return fail(H264A_E_ARG, "me_frames: internal queue layout error");
-        launch_me_frames(prm, unsigned(blocks), st, fb, total, ctx->q[Q_MAIN].d_counter, ctx->q[Q_MAIN].d_flags, epoch,
-                         ctx->d_status, learn != nullptr);
+        launch_me_frames(prm, unsigned(blocks), st, fb, total, qw.d_counter, qw.d_flags, words, epoch, ctx->d_status,
+                         lam_ok, learn != nullptr);
         return check_launch("me_frames_kernel");
     }
     // the table, its segment starts and j values in one device buffer
@@ -2553,8 +1612,8 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
     char* dv = static_cast<char*>(ctx->me_tab);
     launch_me_frames_dtab(prm, unsigned(blocks), st, reinterpret_cast<const FrameDesc*>(dv),
                           reinterpret_cast<const long long*>(dv + b_desc), reinterpret_cast<const int*>(dv + b_desc + b_seg),
-                          nframes, nseg, total, ctx->q[Q_MAIN].d_counter, ctx->q[Q_MAIN].d_flags, epoch, ctx->d_status,
-                          learn != nullptr);
+                          nframes, nseg, total, qw.d_counter, qw.d_flags, words, epoch, ctx->d_status,
+                          lam_ok, learn != nullptr);
     rc = check_launch("me_frames_dkernel");
     if (rc) return rc;
     return table_done(ctx, st);
@@ -2686,9 +1745,11 @@ extern "C" int h264a_me_frames_noalloc(const h264a_me_frame* h_frames, int nfram
     memset(&fb, 0, sizeof fb);
     fb.n = nframes;
     total = 0;
+    bool lam_ok = true;
     for (int k = 0; k < nframes; k++) {
         const h264a_me_frame& f = h_frames[order[k]];
         FrameDesc& d = fb.f[k];
+        lam_ok = lam_ok && balanced_lambda(f.lambda_me);
         d.pic = f.pic;
         d.tmap_ok = encode_window_map(&d.tmap, f.pic.d_planes, f.pic.cw + 2 * f.pic.pad, f.pic.ch + 2 * f.pic.pad);
         d.lambda_me = f.lambda_me;
@@ -2715,7 +1776,7 @@ extern "C" int h264a_me_frames_noalloc(const h264a_me_frame* h_frames, int nfram
     const long long need = (total + ME_WARPS - 1) / ME_WARPS;
     if (blocks > need) blocks = need;
     const MeParamsDev prm = to_dev(*params);
-    launch_me_frames(prm, unsigned(blocks), st, fb, total, scratch, scratch + 1, kNoallocFlag, d_status);
+    launch_me_frames(prm, unsigned(blocks), st, fb, total, scratch, scratch + 1, nullptr, kNoallocFlag, d_status, lam_ok);
     return check_launch("me_frames_kernel (no-alloc)");
 }
 
@@ -2724,7 +1785,7 @@ extern "C" int h264a_me_frames_noalloc(const h264a_me_frame* h_frames, int nfram
 // ---------------------------------------------------------------------------
 
 static int closed_pipe_setup_once() {
-    const int smem = WIN_BYTES;
+    const int smem = ME_WARPS * WIN_BYTES;
     H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -2745,7 +1806,7 @@ static int closed_pipe_setup(int& per_sm) {
         if (rc) return rc;
         int p = 0;
         H264A_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, closed_pipe_kernel<false, true>,
-                                                                 32 * ME_WIDE_WARPS, WIN_BYTES));
+                                                                 32 * ME_WARPS, ME_WARPS * WIN_BYTES));
         if (p < 1) p = 1;
         if (dev < 0 || dev >= kMaxDev) {
             per_sm = p;
@@ -2775,7 +1836,7 @@ int h264a::closed_pipe_run(h264a_ctx* ctx, const ClosedPipeIn& in, const h264a_m
     memset(fds.data(), 0, sizeof(FrameDesc) * n);
     memset(rds.data(), 0, sizeof(RecDesc) * n);
     // the plane buffers (frame h's planes in buffer h % nbuf), the column
-    // segments of the bands, the CTA pools
+    // segments of the bands, the warp pools
     const int nbuf = std::min(n, H264A_CLOSED_PLANE_PICTURES);
     const int segw = PIPE_SEGW, nseg = (mb_w + segw - 1) / segw;
     const int pools = std::min(PIPE_POOLS, n - 1);
@@ -2846,7 +1907,7 @@ int h264a::closed_pipe_run(h264a_ctx* ctx, const ClosedPipeIn& in, const h264a_m
     if (rc) return rc;
     char* dv = static_cast<char*>(ctx->me_tab);
     // flags: n ticket counters, n completed-MB counters, then per frame its
-    // MV words, deblocking flags and band flags (an even count per frame)
+    // MV words, deblocking flags, coefficient masks and band flags (an even count per frame)
     PipeParams pp;
     memset(&pp, 0, sizeof pp);
     pp.fds = reinterpret_cast<const FrameDesc*>(dv);
@@ -2863,7 +1924,8 @@ int h264a::closed_pipe_run(h264a_ctx* ctx, const ClosedPipeIn& in, const h264a_m
     pp.pools = pools;
     pp.ew_off = 0;
     pp.dfl_off = 2 * EW_PER_MB * nmb;
-    pp.band_off = pp.dfl_off + nmb;
+    pp.nz_off = pp.dfl_off + nmb;
+    pp.band_off = pp.nz_off + nmb;
     pp.fstride = (pp.band_off + (long long)nbands * nseg + 1) & ~1LL;
     const long long head = (2LL * n + 1) & ~1LL;
     const long long need = head + pp.fstride * n;
@@ -2892,23 +1954,11 @@ int h264a::closed_pipe_run(h264a_ctx* ctx, const ClosedPipeIn& in, const h264a_m
     H264A_CUDA(cudaMemsetAsync(fl, 0, sizeof(int) * size_t(need), st));
     const int epoch = next_epoch(ctx, st, Q_WIDE);
     if (epoch < 0) return H264A_E_CUDA;
-    long long blocks = (long long)ctx->num_sms * per_sm;
-    blocks -= blocks % pools;  // an equal share of CTAs per pool
-    if (blocks < pools) blocks = pools;
-    const bool bal = balanced_preset(prm), learn = in.props != nullptr;
-    const size_t sm = WIN_BYTES;
-    if (learn && bal)
-        closed_pipe_kernel<true, true><<<unsigned(blocks), 32 * ME_WIDE_WARPS, sm, st>>>(pp, prm, epoch, ctx->d_status,
-                                                                                        SPIN_LIMIT);
-    else if (learn)
-        closed_pipe_kernel<false, true><<<unsigned(blocks), 32 * ME_WIDE_WARPS, sm, st>>>(pp, prm, epoch, ctx->d_status,
-                                                                                         SPIN_LIMIT);
-    else if (bal)
-        closed_pipe_kernel<true, false><<<unsigned(blocks), 32 * ME_WIDE_WARPS, sm, st>>>(pp, prm, epoch, ctx->d_status,
-                                                                                         SPIN_LIMIT);
-    else
-        closed_pipe_kernel<false, false><<<unsigned(blocks), 32 * ME_WIDE_WARPS, sm, st>>>(pp, prm, epoch,
-                                                                                          ctx->d_status, SPIN_LIMIT);
+    const long long blocks = (long long)ctx->num_sms * pipe_ctas_per_sm(mb_w, mb_h, pools, ctx->num_sms, per_sm);
+    const bool bal = balanced_preset(prm, balanced_lambda(in.lambda_me)), learn = in.props != nullptr;
+    auto kern = bal ? (learn ? closed_pipe_kernel<true, true> : closed_pipe_kernel<true, false>)
+                    : (learn ? closed_pipe_kernel<false, true> : closed_pipe_kernel<false, false>);
+    kern<<<unsigned(blocks), 32 * ME_WARPS, ME_WARPS * WIN_BYTES, st>>>(pp, prm, epoch, ctx->d_status, SPIN_LIMIT);
     rc = check_launch("closed_pipe_kernel");
     if (rc) return rc;
     return table_done(ctx, st);
@@ -2977,28 +2027,24 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW)
                         const int* __restrict__ seg_j, int nf, int ns, long long total,
                         const __grid_constant__ MeParamsDev prm, int* __restrict__ counter, int* __restrict__ flags,
                         int epoch, int* __restrict__ status, int spin_limit) {
-    __shared__ WarpScratch scratch[NW];
+    __shared__ MbScratch scratch[NW];
+    __shared__ __align__(16) BalScratch bal[NW];
+    __shared__ PhaseTab ptab;
     __shared__ __align__(8) unsigned long long win_bar[NW];
     extern __shared__ __align__(128) uint8_t me_win[];
-    const int w = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const uint32_t win = uint32_t(__cvta_generic_to_shared(me_win)) + uint32_t(w * WIN_BYTES);
-    const uint32_t bar = uint32_t(__cvta_generic_to_shared(&win_bar[w]));
-    if (lane == 0) {
-        mbar_init(bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
+    const WarpWindow ww = warp_window(me_win, win_bar, ptab, bal);
+    MbScratch& ws = scratch[threadIdx.x >> 5];
     uint32_t parity = 0;
     for (;;) {
         int t = 0;
         if (lane == 0) t = atomicAdd(counter, 1);
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= total) return;
-        int s = 0;
-        while (s + 1 < ns && __ldg(seg_start + s + 1) <= t) s++;
-        const int j = __ldg(seg_j + s);
-        const long long u = t - __ldg(seg_start + s);
+        int sg = 0;
+        while (sg + 1 < ns && __ldg(seg_start + sg + 1) <= t) sg++;
+        const int j = __ldg(seg_j + sg);
+        const long long u = t - __ldg(seg_start + sg);
         const int nxt = j + 1 < nf ? fds[j + 1].mb_w * fds[j + 1].mb_h : 0;
         const FrameDescMR& fd = fds[int(u % (j + 1))];
         const int k = nxt + int(u / (j + 1));
@@ -3007,10 +2053,14 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW)
         const int m = mby * fd.mb_w + mbx;
         int* fl = flags + fd.flag_base;
         const int lx = mbx * 16, ly = mby * 16;
-        uint32_t src4[4];
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-            src4[r] = ld4u(fd.src + (long long)(ly + ((lane >> 2) & 3) * 4 + r) * fd.cw + lx + (lane & 3) * 4);
+        MbLane s;
+        mb_load_src(s, fd.src, fd.cw, lx, ly);
+        if (lane == 0) {
+            ws.src = fd.src;
+            ws.bw = nullptr;
+            ws.pw = fd.cw + 2 * fd.pad; ws.ph = fd.ch + 2 * fd.pad;
+            ws.pad = fd.pad; ws.cw = fd.cw; ws.ch = fd.ch;
+        }
         if (lane == 0) {
             if (mbx > 0) wait_flag(fl + m - 1, epoch, status, 1, spin_limit);
             if (mby > 0) wait_flag(fl + m - fd.mb_w + (mbx < fd.mb_w - 1 ? 1 : 0), epoch, status, 1, spin_limit);
@@ -3024,72 +2074,52 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW)
         if (ca) c = pick_mr_at(fd.picks, m - fd.mb_w + 1, 0, 3, rc);
         else if (da) c = pick_mr_at(fd.picks, m - fd.mb_w - 1, 3, 3, rc);
         const bool cav = ca || da;
-        const int pw = fd.cw + 2 * fd.pad, ph = fd.ch + 2 * fd.pad;
         // best_part of the 16x16 over the references, then, J above the gate,
         // of each partition (lane group g = partition g) over the references
+        mb_lane_16x16(s, lx, ly, ww.win);
         int evals = 0, shape = 0;
         int ref16 = 0, mv16x = 0, mv16y = 0;
         long long c16 = LLONG_MAX;
         int pref = 0, pmx = 0, pmy = 0;  // the lane's partition's best (mode 1)
         long long pcost = LLONG_MAX;
+#pragma unroll 1
         for (int mode = 0; mode < 2; mode++) {
-            if (mode == 1 && !(fd.split_gate >= 0 && c16 > fd.split_gate)) break;
+            if (mode == 1) {
+                if (!(fd.split_gate >= 0 && c16 > fd.split_gate)) break;
+                mb_lane_parts(s);
+            }
             for (int r = 0; r < fd.nref; r++) {
                 const int2 pmv = predict_mv_ref(aa, a, ra, ba, bb, rb, cav, c, rc, r);
-                h264a_picture pc{fd.src, fd.planes[r], fd.cw, fd.ch, fd.pad};
-                const bool win_ok = STAGE && ((reinterpret_cast<uintptr_t>(pc.d_planes) | uintptr_t(pw)) & 15) == 0 &&
-                                    pw >= WIN_W && ph >= WIN_H;
-                if (win_ok) {
-                    const int wx0 = min(max((lx + pc.pad + (pmv.x >> 2) - WIN_R) & ~15, 0), pw - WIN_W);
-                    const int wy0 = min(max(ly + pc.pad + (pmv.y >> 2) - WIN_R, 0), ph - WIN_H);
-                    if (lane == 0) {
-                        scratch[w].wx0 = wx0;
-                        scratch[w].wy0 = wy0;
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        if (fd.tmap_ok) {
-                            mbar_expect_tx(bar, uint32_t(WIN_BYTES));
-                            // a tensor map written to device memory by the host since an
-                            // earlier launch read that address: acquire it for the copy
-                            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&fd.tmap[r])
-                                         : "memory");
-                            tma_load_3d(win, &fd.tmap[r], wx0, wy0, 0, bar);
-                        } else {
-                            mbar_expect_tx(bar, uint32_t(4 * WIN_H * WIN_W));
-                        }
-                    }
-                    __syncwarp();
-                    if (!fd.tmap_ok) {
-                        const long long ps = (long long)pw * ph;
-                        for (int i = lane; i < 4 * WIN_H; i += 32) {
-                            const int pl = i / WIN_H, rr = i - pl * WIN_H;
-                            bulk_g2s(win + uint32_t(pl * WIN_PLANE + rr * WIN_STRIDE),
-                                     pc.d_planes + ps * pl + (long long)(wy0 + rr) * pw + wx0, WIN_W, bar);
-                        }
-                    }
-                }
-                if (lane == 0) scratch[w].win_ok = win_ok;
+                if (lane == 0) ws.base = fd.planes[r];
                 __syncwarp();
-                GroupGeom qg;
-                group_geom_init(qg, scratch[w], pc, lx, ly, mode, win, mode == 0 ? src4 : nullptr);
+                const bool win_ok = STAGE && stage_window(ws, &fd.tmap[r], fd.tmap_ok != 0, true, lx, ly, pmv, ww.win, ww.bar);
+                mb_lane_window(s, ws, win_ok);
                 if (win_ok) {
-                    wait_window(bar, parity, status, 3, spin_limit);
+                    wait_window(ww.bar, parity, status, 3, spin_limit);
                     parity ^= 1u;
                 }
-                int preds[4] = {pmv.x, pmv.y, mv16x, mv16y};
-                int rx, ry, ev;
-                long long cst;
-                motion_search_group<BAL>(qg, prm, scratch[w], preds, mode == 0 ? 1 : 2, fd.lambda_me, rx, ry, cst, ev);
-                cst += __double2ll_rz(__dmul_rn(fd.lambda_me, double(ref_bits_of(r, fd.nref))));
+                SearchOut o;
+                const int2 mv16 = make_int2(mv16x, mv16y);
+                if constexpr (BAL) {
+                    if (mode == 0)
+                        o = search16_bal<false, STAGE>(s, ws, bal[threadIdx.x >> 5], ww.lut, pmv, fd.lambda_me, false, pmv, pmv, 0,
+                                                       nullptr);
+                    else
+                        o = search_parts_bal<false, STAGE>(s, ws, bal[threadIdx.x >> 5], ww.lut, pmv, mv16, fd.lambda_me, false, mv16);
+                } else {
+                    o = mode == 0 ? mb_search<0, false>(s, prm, ws, ww.lut, pmv, pmv, 1, fd.lambda_me)
+                                  : mb_search<1, false>(s, prm, ws, ww.lut, pmv, mv16, 2, fd.lambda_me);
+                }
+                const long long cst = o.cost + __double2ll_rz(__dmul_rn(fd.lambda_me, double(ref_bits_of(r, fd.nref))));
                 if (mode == 0) {
-                    evals += ev << 4;
-                    if (cst < c16) { c16 = cst; ref16 = r; mv16x = rx; mv16y = ry; }
+                    evals += o.evals << 4;
+                    if (cst < c16) { c16 = cst; ref16 = r; mv16x = o.x; mv16y = o.y; }
                 } else {
                     // every lane of group g holds partition g's result
-                    evals += (__shfl_sync(0xffffffffu, ev, 0) + __shfl_sync(0xffffffffu, ev, 8) +
-                              __shfl_sync(0xffffffffu, ev, 16) + __shfl_sync(0xffffffffu, ev, 24)) << 3;
-                    if (cst < pcost) { pcost = cst; pref = r; pmx = rx; pmy = ry; }
+                    evals += (__shfl_sync(0xffffffffu, o.evals, 0) + __shfl_sync(0xffffffffu, o.evals, 8) +
+                              __shfl_sync(0xffffffffu, o.evals, 16) + __shfl_sync(0xffffffffu, o.evals, 24)) << 3;
+                    if (cst < pcost) { pcost = cst; pref = r; pmx = o.x; pmy = o.y; }
                 }
-                __syncwarp();  // the window's reads are done before the next copy
             }
         }
         // the shape decision (mb16.rs:8869-8913)
@@ -3208,6 +2238,7 @@ int h264a::mr_table_build(const h264a_me_mr_frame* h_frames, int nframes, MrTabl
         d.mb_w = f.cw / 16;
         d.mb_h = f.ch / 16;
         d.flag_base = int(total);
+        t.lam_ok = t.lam_ok && balanced_lambda(f.lambda_me);
         segd[k].mb_w = d.mb_w;
         segd[k].mb_h = d.mb_h;
         total += (long long)d.mb_w * d.mb_h;
@@ -3238,7 +2269,7 @@ int h264a::mr_launch(h264a_ctx* ctx, int variant, const MeParamsDev& prm, const 
     std::call_once(once, [] { setup_rc = me_mr_setup_once(); });
     if (setup_rc) return setup_rc;
     const char* dv = static_cast<const char*>(d_table);
-    if (!balanced_preset(prm)) return mr_launch_t<false, 4, true>(ctx, prm, dv, t, counter, flags, epoch, st);
+    if (!balanced_preset(prm, t.lam_ok)) return mr_launch_t<false, 4, true>(ctx, prm, dv, t, counter, flags, epoch, st);
     switch (variant) {
         case 1: return mr_launch_t<true, 2, true>(ctx, prm, dv, t, counter, flags, epoch, st);
         case 2: return mr_launch_t<true, 8, true>(ctx, prm, dv, t, counter, flags, epoch, st);

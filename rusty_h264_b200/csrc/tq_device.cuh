@@ -96,25 +96,10 @@ __device__ __forceinline__ void tq4x4_store(const uint32_t s[4], const uint32_t 
 static __constant__ int kLevelScale[6][3] = {{160, 256, 208}, {176, 288, 224}, {208, 320, 256},
                                       {224, 368, 288}, {256, 400, 320}, {288, 464, 368}};
 
-// The inter MB's luma reconstruction of one 4x4 block (mb16.rs:3575-3605):
-// dequantize (transform.rs:233-284, flat scaling) each level, cast it to i16
-// as the reference does, inverse core transform rows then columns with
-// (x + 32) >> 6 (transform_quant.rs:30-35, 56-69), add the prediction and
-// clamp (idct_four_t4_rec, transform_quant.rs:96-119).  Four packed rows out.
-// dc_override (the chroma DC from inverse_quant_chroma_dc) replaces the
-// dequantized coefficient 0 when given.
-__device__ __forceinline__ void rec4x4(const int lv[16], const uint32_t p[4], int qp, uint32_t out[4],
-                                       int dc_override = INT_MIN) {
-    const int m6 = qp % 6, shift = qp / 6;
-    int m[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        const int g = ((i >> 2) & 1) == (i & 1) ? ((i & 1) ? 1 : 0) : 2;
-        const int ls = kLevelScale[m6][g];
-        const int d = qp >= 24 ? int(uint32_t(lv[i] * ls) << (shift - 4)) : (lv[i] * ls + (1 << (3 - shift))) >> (4 - shift);
-        m[i] = int(int16_t(d));
-    }
-    if (dc_override != INT_MIN) m[0] = int(int16_t(dc_override));
+// The inverse core transform of dequantized coefficients m (rows then columns,
+// (x + 32) >> 6, transform_quant.rs:30-35, 56-69), added to the prediction and
+// clamped (idct_four_t4_rec, transform_quant.rs:96-119).
+__device__ __forceinline__ void idct4_add(int m[16], const uint32_t p[4], uint32_t out[4]) {
 #pragma unroll
     for (int r = 0; r < 4; r++) {
         const int d0 = m[r * 4], d1 = m[r * 4 + 1], d2 = m[r * 4 + 2], d3 = m[r * 4 + 3];
@@ -137,6 +122,26 @@ __device__ __forceinline__ void rec4x4(const int lv[16], const uint32_t p[4], in
         }
         out[r] = w;
     }
+}
+
+// The inter MB's luma reconstruction of one 4x4 block (mb16.rs:3575-3605):
+// dequantize (transform.rs:233-284, flat scaling) each level, cast it to i16
+// as the reference does, then idct4_add.  Four packed rows out.
+// dc_override (the chroma DC from inverse_quant_chroma_dc) replaces the
+// dequantized coefficient 0 when given.
+__device__ __forceinline__ void rec4x4(const int lv[16], const uint32_t p[4], int qp, uint32_t out[4],
+                                       int dc_override = INT_MIN) {
+    const int m6 = qp % 6, shift = qp / 6;
+    int m[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const int g = ((i >> 2) & 1) == (i & 1) ? ((i & 1) ? 1 : 0) : 2;
+        const int ls = kLevelScale[m6][g];
+        const int d = qp >= 24 ? int(uint32_t(lv[i] * ls) << (shift - 4)) : (lv[i] * ls + (1 << (3 - shift))) >> (4 - shift);
+        m[i] = int(int16_t(d));
+    }
+    if (dc_override != INT_MIN) m[0] = int(int16_t(dc_override));
+    idct4_add(m, p, out);
 }
 
 // ---- the inter MB's chroma block --------------------------------------------
@@ -237,6 +242,120 @@ __device__ __forceinline__ void chroma_tq_rec(const uint8_t* src, const uint8_t*
     const int rdc = int(uint32_t(gk * kLevelScale[m6][0]) << (q / 6)) >> 5;
     lv[0] = 0;
     rec4x4(lv, p, q, r4, rdc);
+}
+
+// ---- luma and chroma blocks of one MB side by side ---------------------------
+// mb_code_block codes one 4x4 block per lane, luma and chroma lanes together
+// (the closed loop's fused reconstruction): a lane's source and predicted
+// rows in, levels and reconstructed rows out, the arithmetic of tq4x4_store +
+// rec4x4 for luma and of chroma_tq_rec for chroma (the four blocks of a plane
+// in an aligned quad of lanes).  One pass over the transform code for all 24
+// blocks: the kernel it runs in is bound by latency and by its instruction
+// footprint.
+struct BlockQuant {
+    int ff[8], mf[8];      // by position slot (row & 1) * 4 + column
+    int ls[3];             // LevelScale by position group
+    int add, right, left;  // dequantize: ((level * ls + add) >> right) << left
+    int m_dc, q;           // chroma: the DC multiplier and the QP
+};
+__device__ __forceinline__ BlockQuant block_quant(const int16_t* ff, const int16_t* mf, int qp) {
+    BlockQuant b;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        b.ff[i] = ff[i];
+        b.mf[i] = mf[i];
+    }
+    const int m6 = qp % 6, shift = qp / 6;
+#pragma unroll
+    for (int i = 0; i < 3; i++) b.ls[i] = kLevelScale[m6][i];
+    b.right = qp >= 24 ? 0 : 4 - shift;
+    b.left = qp >= 24 ? shift - 4 : 0;
+    b.add = qp >= 24 ? 0 : 1 << (3 - shift);
+    b.m_dc = kQuantMfDc[m6];
+    b.q = qp;
+    return b;
+}
+// Returns whether any level is non-zero (luma).  Every lane of the warp calls this.
+__device__ __forceinline__ bool mb_code_block(const uint32_t s[4], const uint32_t p[4], const BlockQuant& bq, bool chroma, int k,
+                                              int16_t* co, uint32_t r4[4]) {
+    int m[16];
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) m[r * 4 + c] = byte_of(s[r], c) - byte_of(p[r], c);
+    forward_core4(m);
+    // the 2x2 chroma DC (forward_quant_chroma_dc, inverse_quant_chroma_dc):
+    // |f| <= 16,320, so 32 bits hold every product
+    const int base = int(threadIdx.x & 31) & ~3;
+    const int dc = int(int16_t(m[0]));
+    const int d0 = __shfl_sync(0xffffffffu, dc, base + 0), d1 = __shfl_sync(0xffffffffu, dc, base + 1);
+    const int d2 = __shfl_sync(0xffffffffu, dc, base + 2), d3 = __shfl_sync(0xffffffffu, dc, base + 3);
+    const int sb = k & 1 ? -1 : 1, sc = k & 2 ? -1 : 1;
+    const int f = d0 + sb * d1 + sc * d2 + sb * sc * d3;
+    const int qbits = 15 + bq.q / 6;
+    const int la = (abs(f) * bq.m_dc + 2 * ((1 << qbits) / 6)) >> (qbits + 1);
+    const int dl = f < 0 ? -la : la;
+    const int l0 = __shfl_sync(0xffffffffu, dl, base + 0), l1 = __shfl_sync(0xffffffffu, dl, base + 1);
+    const int l2 = __shfl_sync(0xffffffffu, dl, base + 2), l3 = __shfl_sync(0xffffffffu, dl, base + 3);
+    const int rdc = int(uint32_t((l0 + sb * l1 + sc * l2 + sb * sc * l3) * bq.ls[0]) << (bq.q / 6)) >> 5;
+    int any = 0;
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const int pos = ((i >> 2) & 1) * 4 + (i & 3);
+        const int c = int(int16_t(m[i]));
+        const int l = ((abs(c) + bq.ff[pos]) * bq.mf[pos]) >> 16;
+        int lv = int(int16_t(c < 0 ? -l : l));
+        any |= lv;
+        const int out = i == 0 && chroma ? dl : lv;
+        w[i >> 1] = (i & 1) ? w[i >> 1] | (uint32_t(uint16_t(out)) << 16) : uint32_t(uint16_t(out));
+        const int g = ((i >> 2) & 1) == (i & 1) ? ((i & 1) ? 1 : 0) : 2;
+        m[i] = int(int16_t(int(uint32_t((lv * bq.ls[g] + bq.add) >> bq.right) << bq.left)));
+    }
+    if (chroma) m[0] = int(int16_t(rdc));
+    if (co != nullptr) {
+        uint4* o = reinterpret_cast<uint4*>(co);
+        o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+    idct4_add(m, p, r4);
+    return any != 0;
+}
+
+// Four packed rows of mc_chroma (inter.rs:1268-1361) of the 4x4 block whose
+// top-left reference sample is (x, y): inside the plane five rows of two
+// aligned words, all in flight together; elsewhere row by row (chroma_row).
+__device__ __noinline__ static uint4 chroma_rows_edge(const uint8_t* ref, int w, int h, int x, int y, int fx, int fy, bool cg) {
+    const int wa = (8 - fx) * (8 - fy), wb = fx * (8 - fy), wc = (8 - fx) * fy, wd = fx * fy;
+    return make_uint4(chroma_row(ref, w, h, x, y, wa, wb, wc, wd, cg), chroma_row(ref, w, h, x, y + 1, wa, wb, wc, wd, cg),
+                      chroma_row(ref, w, h, x, y + 2, wa, wb, wc, wd, cg), chroma_row(ref, w, h, x, y + 3, wa, wb, wc, wd, cg));
+}
+__device__ __forceinline__ void chroma_rows(const uint8_t* ref, int w, int h, int x, int y, int fx, int fy, uint32_t p[4]) {
+    if (!(x >= 0 && y >= 0 && x + 8 <= w && y + 5 <= h)) {
+        const uint4 v = chroma_rows_edge(ref, w, h, x, y, fx, fy, true);
+        p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w;
+        return;
+    }
+    // the plane is 4-byte aligned and w a multiple of 8
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(ref + (long long)y * w + (x & ~3));
+    const uint32_t sh = uint32_t(x & 3) * 8u;
+    uint32_t a[5], b[5];
+#pragma unroll
+    for (int r = 0; r < 5; r++) {
+        const uint32_t w0 = __ldcg(q + (long long)r * (w >> 2)), w1 = __ldcg(q + (long long)r * (w >> 2) + 1);
+        a[r] = __funnelshift_r(w0, w1, sh);             // samples x .. x+3
+        b[r] = uint32_t((((unsigned long long)w1 << 32) | w0) >> (sh + 8));  // x+1 .. x+4
+    }
+    const int wa = (8 - fx) * (8 - fy), wb = fx * (8 - fy), wc = (8 - fx) * fy, wd = fx * fy;
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        uint32_t o = 0;
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            o |= uint32_t((wa * byte_of(a[r], c) + wb * byte_of(b[r], c) + wc * byte_of(a[r + 1], c) + wd * byte_of(b[r + 1], c) + 32) >> 6)
+                 << (8 * c);
+        p[r] = o;
+    }
 }
 
 }  // namespace h264a
