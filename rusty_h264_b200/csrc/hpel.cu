@@ -29,7 +29,7 @@ namespace h264a {
 __global__ void __launch_bounds__(32 * HP_WARPS) hpel_build_kernel(const uint8_t* __restrict__ ref, int cw, int ch,
                                                                    int pad, size_t ref_fstride,
                                                                    uint8_t* __restrict__ planes, int pw, int ph,
-                                                                   int strips, int bands, long long nwarps,
+                                                                   int strips, int bands, int band_rows, long long nwarps,
                                                                    int word_in, int word_out) {
     const long long wid = (long long)blockIdx.x * HP_WARPS + (threadIdx.x >> 5);
     if (wid >= nwarps) return;  // warp-uniform
@@ -37,10 +37,10 @@ __global__ void __launch_bounds__(32 * HP_WARPS) hpel_build_kernel(const uint8_t
     const int pic = int(wid / per_pic);
     const int rem = int(wid - per_pic * pic);
     const int band = rem / strips, strip = rem - band * strips;
-    const int y0 = band * HP_BAND;
+    const int y0 = band * band_rows;
     hpel_strip_rows(ref + ref_fstride * pic, cw, ch, pad, planes + 4LL * pw * ph * pic, pw, ph,
                     strip * HP_STRIP, y0,
-                    y0 + HP_BAND < ph ? y0 + HP_BAND : ph, word_in, word_out);
+                    y0 + band_rows < ph ? y0 + band_rows : ph, word_in, word_out);
 }
 
 }  // namespace h264a
@@ -58,10 +58,18 @@ extern "C" int h264a_hpel_build(h264a_ctx* ctx, const uint8_t* d_ref, int cw, in
     const int word_in = (cw % 4 == 0) && (pad % 4 == 0) && (ref_frame_stride % 4 == 0) &&
                         ((reinterpret_cast<uintptr_t>(d_ref) & 3) == 0);
     const int word_out = (pw % 4 == 0) && ((reinterpret_cast<uintptr_t>(d_planes) & 3) == 0);
-    const int strips = (pw + HP_STRIP - 1) / HP_STRIP, bands = (ph + HP_BAND - 1) / HP_BAND;
+    const int strips = (pw + HP_STRIP - 1) / HP_STRIP;
+    // rows per warp: a warp walks its rows one after another, so a small call
+    // takes short bands (more warps, the halo rows from L2) and a large one the
+    // longest.  One CIF picture at 48, 24, 12, 6 rows: 20.6, 11.4, 7.0, 4.7 us;
+    // one 1080p 21.2, 12.8, 8.5, 7.3; four 25.2, 20.3, 19.3, 19.9; eight 37.5,
+    // 34.6, 33.7, 36.6; 59 211.7, 210.1, 223.4, 258.3
+    const long long cells = (long long)strips * ph * n;  // strips of one row
+    const int rows = cells < 25000LL ? 6 : (cells < 250000LL ? 12 : HP_BAND);
+    const int bands = (ph + rows - 1) / rows;
     const long long nwarps = (long long)strips * bands * n;
     const long long blocks = (nwarps + HP_WARPS - 1) / HP_WARPS;
     hpel_build_kernel<<<unsigned(blocks), 32 * HP_WARPS, 0, pick_stream(ctx, stream)>>>(
-        d_ref, cw, ch, pad, ref_frame_stride, d_planes, pw, ph, strips, bands, nwarps, word_in, word_out);
+        d_ref, cw, ch, pad, ref_frame_stride, d_planes, pw, ph, strips, bands, rows, nwarps, word_in, word_out);
     return check_launch("hpel_build_kernel");
 }

@@ -10,7 +10,7 @@
 namespace h264a {
 
 constexpr int HP_STRIP = 120;  // output columns per warp (30 lanes x 4)
-constexpr int HP_BAND = 48;    // output rows per warp, a multiple of 6
+constexpr int HP_BAND = 24;    // output rows per warp of a large call, a multiple of 6
 constexpr int HP_WARPS = 4;
 constexpr uint32_t HP_BIAS = 0x20102010u;  // 8208 = 256 * 32 + 16 in each half
 
