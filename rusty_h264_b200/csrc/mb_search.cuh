@@ -207,23 +207,30 @@ __device__ __forceinline__ void mb_lane_parts(MbLane& s) {
     for (int i = 0; i < 8; i++) s.src[i] = t[i];
 }
 
-// Where candidates are read: the MB's window in shared memory, or (launch
-// shapes without a window) the reference's planes in global memory.
-template <bool STAGE>
+// Where candidates are read: the MB's window in shared memory, the reference's
+// planes in global memory through L1 (launch shapes without a window), or
+// through L2 (passes that leave the window: the planes may be written during
+// the launch).
+constexpr int REF_WINDOW = 1, REF_PLANES = 0, REF_PLANES_L2 = 2;
+template <int REF>
 struct RefSrc;
 template <>
-struct RefSrc<true> {
+struct RefSrc<REF_WINDOW> {
     using Addr = uint32_t;
     static __device__ __forceinline__ uint32_t ld(Addr a) { return lds_u32(a); }
     static __device__ __forceinline__ uint32_t stride(const MbScratch&) { return WIN_STRIDE; }
-    static __device__ __forceinline__ Addr safe(const MbLane& s, const MbScratch&) { return s.winq; }
 };
 template <>
-struct RefSrc<false> {
+struct RefSrc<REF_PLANES> {
     using Addr = const uint8_t*;
     static __device__ __forceinline__ uint32_t ld(Addr a) { return __ldg(reinterpret_cast<const uint32_t*>(a)); }
     static __device__ __forceinline__ uint32_t stride(const MbScratch& ws) { return uint32_t(ws.pw); }
-    static __device__ __forceinline__ Addr safe(const MbLane& s, const MbScratch& ws) { return ws.base + (long long)(s.lane & 3) * ws.pw; }
+};
+template <>
+struct RefSrc<REF_PLANES_L2> {
+    using Addr = const uint8_t*;
+    static __device__ __forceinline__ uint32_t ld(Addr a) { return __ldcg(reinterpret_cast<const unsigned int*>(a)); }
+    static __device__ __forceinline__ uint32_t stride(const MbScratch& ws) { return uint32_t(ws.pw); }
 };
 __device__ __forceinline__ uint32_t align4(uint32_t a) { return a & ~3u; }
 __device__ __forceinline__ const uint8_t* align4(const uint8_t* a) {
@@ -235,15 +242,15 @@ __device__ __forceinline__ uint32_t shift8(const uint8_t* a) { return uint32_t(r
 // A candidate's operands: byte addresses a (and b, equal to a at one-plane
 // phases) of the lane's row of the partition's first block; a safe address
 // when the reads are not covered (the window, or the planes, do not hold them).
-template <bool STAGE>
+template <int REF>
 struct CandAddr {
-    typename RefSrc<STAGE>::Addr a, b;
+    typename RefSrc<REF>::Addr a, b;
     bool covered;
 };
-template <bool STAGE>
-__device__ __forceinline__ CandAddr<STAGE> cand_addr(const MbLane& s, const MbScratch& ws, uint32_t lut, int mvx, int mvy) {
-    CandAddr<STAGE> t;
-    if constexpr (STAGE) {
+template <int REF>
+__device__ __forceinline__ CandAddr<REF> cand_addr(const MbLane& s, const MbScratch& ws, uint32_t lut, int mvx, int mvy) {
+    CandAddr<REF> t;
+    if constexpr (REF == REF_WINDOW) {
         uint2 ent;
         asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(ent.x), "=r"(ent.y) : "r"(lut + uint32_t(((mvx & 3) * 4 + (mvy & 3)) * 8)));
         const int wx = s.wox + (mvx >> 2), wy = s.woy + (mvy >> 2);
@@ -305,45 +312,13 @@ __device__ __noinline__ static uint4 plane_rows(const MbScratch* ws, int x, int 
     return r;
 }
 
-// A pass some of whose candidates' reads are not covered, word by word from
-// the planes; ax, ay / bx, by: the column's MVs in tiles A and B (mode 0: A)
-// of the rw-wide partition at (px, py).  Returns the shares of the column sums
-// as a0 | a1 << 16, b0 | b1 << 16 (each below 2^16: 8 blocks of at most 2 x
-// 4,080), and the row SADs of both tiles.  Out of line, with nothing of the
-// search's state in memory: about one pass in a hundred needs it.
-template <int MODE>
-__device__ __noinline__ int4 slow_pass(MbScratch* ws, int px, int py, int rw, int ax, int ay, int bx, int by, bool wait) {
-    const int lane = threadIdx.x & 31, rh = MODE == 0 ? 16 : 24 - rw;
-    if (wait) band_wait_px(ws->bw, &ws->bready, py + (max(ay, by) >> 2) + rh + 1, px + (max(ax, bx) >> 2) + rw + 1);
-    __syncwarp();
-    const HadFrag had = had_frag(lane);
-    int4 out = make_int4(0, 0, 0, 0);
-#pragma unroll 1
-    for (int j = 0; j < 16; j++) {
-        const bool second = j >= 8;
-        const int k = MODE == 0 ? j : j & 7;
-        // block k of the pass: 16 wide, four a row; 8 wide, two
-        const int xo = MODE == 0 || rw == 16 ? 4 * (k & 3) : 4 * (k & 1), yo = MODE == 0 || rw == 16 ? 4 * (k >> 2) : 4 * (k >> 1);
-        const int x = px + xo, y = py + yo + (lane & 3);
-        const uint32_t sw = ld4u(ws->src + (long long)y * ws->cw + x);
-        const uint32_t pw = plane_word(*ws, x, y, MODE == 1 && second ? bx : ax, MODE == 1 && second ? by : ay);
-        __syncwarp();
-        int t0 = 0, t1 = 0;
-        had_mma(had, pw, sw, t0, t1);
-        const int t = t0 | (t1 << 16), sd = int(__vsadu4(pw, sw));
-        if (second) { out.y += t; out.w += sd; }
-        else { out.x += t; out.z += sd; }
-    }
-    return out;
-}
-
 // The sixteen words of a pass: mode 0 the candidate's (four block rows of
 // five aligned words), mode 1 tile A's and tile B's eight (four pairs of
 // adjacent blocks, three words each).
-template <int MODE, bool STAGE>
-__device__ __forceinline__ void pass_words(const MbLane& s, const MbScratch& ws, typename RefSrc<STAGE>::Addr a0,
-                                           typename RefSrc<STAGE>::Addr b0, uint32_t p[16]) {
-    using R = RefSrc<STAGE>;
+template <int MODE, int REF>
+__device__ __forceinline__ void pass_words(const MbLane& s, const MbScratch& ws, typename RefSrc<REF>::Addr a0,
+                                           typename RefSrc<REF>::Addr b0, uint32_t p[16]) {
+    using R = RefSrc<REF>;
     const auto a = align4(a0);
     const uint32_t sa = shift8(a0);
     if constexpr (MODE == 0) {
@@ -369,21 +344,79 @@ __device__ __forceinline__ void pass_words(const MbLane& s, const MbScratch& ws,
     }
 }
 
+// A pass some of whose candidates' reads the window does not cover, from the
+// planes; ax, ay / bx, by: the column's MVs in tiles A and B (mode 0: A) of
+// the rw-wide partition at (px, py).  Returns the shares of the column sums as
+// a0 | a1 << 16, b0 | b1 << 16 (each below 2^16: 8 blocks of at most 2 x
+// 4,080), and the row SADs of both tiles.  Out of line, with nothing of the
+// search's state in memory: between one pass in a hundred and one in ten
+// needs it (at the edges of fast objects), and the wavefront may wait for it,
+// so all its loads are in flight together unless a read leaves the planes.
+template <int MODE>
+__device__ __noinline__ int4 slow_pass(MbScratch* ws, int px, int py, int rw, int ax, int ay, int bx, int by, bool wait) {
+    const int lane = threadIdx.x & 31, rh = MODE == 0 ? 16 : 24 - rw;
+    if (wait) band_wait_px(ws->bw, &ws->bready, py + (max(ay, by) >> 2) + rh + 1, px + (max(ax, bx) >> 2) + rw + 1);
+    __syncwarp();
+    MbLane s;
+    s.lane = lane;
+    s.px = px; s.py = py; s.rw = rw; s.rh = rh;
+    s.had = had_frag(lane);
+    // block k of the pass: 16 wide, four a row; 8 wide, two
+    const bool wide = MODE == 0 || rw == 16;
+    auto src_word = [&](int k) {
+        const int xo = wide ? 4 * (k & 3) : 4 * (k & 1), yo = wide ? 4 * (k >> 2) : 4 * (k >> 1);
+        return ld4u(ws->src + (long long)(py + yo + (lane & 3)) * ws->cw + px + xo);
+    };
+    const CandAddr<REF_PLANES_L2> ta = cand_addr<REF_PLANES_L2>(s, *ws, 0u, ax, ay), tb = cand_addr<REF_PLANES_L2>(s, *ws, 0u, bx, by);
+    int a0 = 0, a1 = 0, b0 = 0, b1 = 0, sa = 0, sb = 0;
+    if (__all_sync(0xffffffffu, ta.covered && tb.covered)) {
+        uint32_t sw[16], p[16], r[16];
+#pragma unroll
+        for (int k = 0; k < (MODE == 0 ? 16 : 8); k++) sw[k] = src_word(k);
+        pass_words<MODE, REF_PLANES_L2>(s, *ws, ta.a, tb.a, p);
+        pass_words<MODE, REF_PLANES_L2>(s, *ws, ta.b, tb.b, r);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t wa = avg_up4(p[i], r[i]), wb = avg_up4(p[8 + i], r[8 + i]), va = sw[i], vb = sw[MODE == 0 ? 8 + i : i];
+            had_mma(s.had, wa, va, a0, a1);
+            had_mma(s.had, wb, vb, b0, b1);
+            sa += int(__vsadu4(wa, va));
+            sb += int(__vsadu4(wb, vb));
+        }
+    } else {
+#pragma unroll 1
+        for (int j = 0; j < 16; j++) {
+            const bool second = MODE == 1 && j >= 8;
+            const int k = MODE == 0 ? j : j & 7;
+            const int xo = wide ? 4 * (k & 3) : 4 * (k & 1), yo = wide ? 4 * (k >> 2) : 4 * (k >> 1);
+            const uint32_t sw = src_word(k);
+            const uint32_t pw = plane_word(*ws, px + xo, py + yo + (lane & 3), second ? bx : ax, second ? by : ay);
+            __syncwarp();
+            int t0 = 0, t1 = 0;
+            had_mma(s.had, pw, sw, t0, t1);
+            const int sd = int(__vsadu4(pw, sw));
+            if (j >= 8) { b0 += t0; b1 += t1; sb += sd; }
+            else { a0 += t0; a1 += t1; sa += sd; }
+        }
+    }
+    return make_int4(a0 | (a1 << 16), b0 | (b1 << 16), sa, sb);
+}
+
 // One pass: the lane's column's candidates at ta (tile A) and, mode 1, tb
 // (tile B) -- MVs ax, ay and bx, by -- give the lane's shares of
 // the column sums in a0, a1 (columns 2q, 2q+1 of tile A; mode 0: of the whole
 // candidate) and b0, b1 (tile B), and with SADS the lane's row SADs in sa, sb.
 // two: a two-plane phase is possible.  idle: the group has no slots (its
 // addresses are safe and its sums are not used).
-template <int MODE, bool STAGE, bool SADS>
-__device__ __forceinline__ void price_pass(const MbLane& s, MbScratch& ws, const CandAddr<STAGE>& ta, const CandAddr<STAGE>& tb,
+template <int MODE, int REF, bool SADS>
+__device__ __forceinline__ void price_pass(const MbLane& s, MbScratch& ws, const CandAddr<REF>& ta, const CandAddr<REF>& tb,
                                            int ax, int ay, int bx, int by, bool two, bool idle, int& a0, int& a1, int& b0,
                                            int& b1, int& sa, int& sb) {
     uint32_t p[16];
-    pass_words<MODE, STAGE>(s, ws, ta.a, tb.a, p);
+    pass_words<MODE, REF>(s, ws, ta.a, tb.a, p);
     if (two) {
         uint32_t r[16];
-        pass_words<MODE, STAGE>(s, ws, ta.b, tb.b, r);
+        pass_words<MODE, REF>(s, ws, ta.b, tb.b, r);
 #pragma unroll
         for (int i = 0; i < 16; i++) p[i] = avg_up4(p[i], r[i]);
     }
@@ -428,10 +461,10 @@ __device__ __forceinline__ int price_slots(const MbLane& s, MbScratch& ws, uint3
         cb = cb < n ? cb : 0;
         const int ax = __shfl_sync(0xffffffffu, mvx, s.gb + ca), ay = __shfl_sync(0xffffffffu, mvy, s.gb + ca);
         const int bx = __shfl_sync(0xffffffffu, mvx, s.gb + cb), by = __shfl_sync(0xffffffffu, mvy, s.gb + cb);
-        const CandAddr<true> ta = cand_addr<true>(s, ws, lut, ax, ay), tb = cand_addr<true>(s, ws, lut, bx, by);
+        const CandAddr<REF_WINDOW> ta = cand_addr<REF_WINDOW>(s, ws, lut, ax, ay), tb = cand_addr<REF_WINDOW>(s, ws, lut, bx, by);
         const bool two = __any_sync(0xffffffffu, ta.a != ta.b || (!one && tb.a != tb.b));
         int a0, a1, b0, b1, sa, sb;
-        price_pass<MODE, true, true>(s, ws, ta, tb, ax, ay, bx, by, two, n == 0, a0, a1, b0, b1, sa, sb);
+        price_pass<MODE, REF_WINDOW, true>(s, ws, ta, tb, ax, ay, bx, by, two, n == 0, a0, a1, b0, b1, sa, sb);
         // columns 2q, 2q+1 of tiles A and B, summed over the lanes of each
         // column: lane bit 4 keeps the odd column, in mode 1 bit 3 tile B
         const bool hi = (s.lane & 16) != 0, up = (s.lane & 8) != 0;
@@ -843,7 +876,7 @@ __device__ __forceinline__ int bal_rate_cost(const BalScratch& b, double lam, in
 // The 16x16 search of the Balanced preset (predictor p0 the mvd centre), warp-uniform.
 // LEARN with use_prop: as mb_search's.  propc / propg: proposals lane / 4 and
 // lane % 8.
-template <bool LEARN, bool STAGE>
+template <bool LEARN, int REF>
 __device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws, BalScratch& bs, uint32_t lut, int2 p0,
                                                   double lambda_me, bool use_prop, int2 propc, int2 propg, int prop_t,
                                                   int* fell) {
@@ -878,13 +911,13 @@ __device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws
             }
             if (LEARN && kind == PROP) { mx = propc.x; my = propc.y; rx = propg.x; ry = propg.y; }
         }
-        const CandAddr<STAGE> ta = cand_addr<STAGE>(s, ws, lut, mx, my);
+        const CandAddr<REF> ta = cand_addr<REF>(s, ws, lut, mx, my);
         const int rc = bal_rate_cost(bs, lambda_me, rx - p0.x, ry - p0.y);
         int a0, a1, b0, b1, sa, sb;
         // a two-plane phase is possible among the seeds, at quarter-pel steps
         // and, from a start vector, around a quarter-pel centre
         const bool two = kind == SEED || step == 1 || (LEARN && (kind == PROP || ((cx | cy) & 1)));
-        price_pass<0, STAGE, false>(s, ws, ta, ta, mx, my, mx, my, two, false, a0, a1, b0, b1, sa, sb);
+        price_pass<0, REF, false>(s, ws, ta, ta, mx, my, mx, my, two, false, a0, a1, b0, b1, sa, sb);
         // column sums through shared memory: slot gl's eight shares
         *reinterpret_cast<int2*>(&bs.red[0][col][2 * (lane & 3)]) = make_int2(a0, a1);
         __syncwarp();
@@ -1004,7 +1037,7 @@ __device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws
 // The four partitions of the Balanced preset, group g of eight lanes searching
 // partition g (mode 1): seeds (0,0), p0 (the mvd centre), p1, then as
 // search16_bal, four slots a round.  use_start: refine-only from `start`.
-template <bool LEARN, bool STAGE>
+template <bool LEARN, int REF>
 __device__ __forceinline__ SearchOut search_parts_bal(const MbLane& s, MbScratch& ws, BalScratch& bs, uint32_t lut, int2 p0,
                                                       int2 p1, double lambda_me, bool use_start, int2 start) {
     constexpr int SEED = 0, DIA = 1, RING = 2, SNAP = 3, START = 4, DONE = 5;
@@ -1047,11 +1080,11 @@ __device__ __forceinline__ SearchOut search_parts_bal(const MbLane& s, MbScratch
         slot_mv(half, ax, ay);
         slot_mv(half + 2, bx, by);
         slot_mv(sl, rx, ry);
-        const CandAddr<STAGE> ta = cand_addr<STAGE>(s, ws, lut, ax, ay), tb = cand_addr<STAGE>(s, ws, lut, bx, by);
+        const CandAddr<REF> ta = cand_addr<REF>(s, ws, lut, ax, ay), tb = cand_addr<REF>(s, ws, lut, bx, by);
         const int rc = bal_rate_cost(bs, lambda_me, rx - p0.x, ry - p0.y);
         const bool planes2 = __any_sync(FULL, ta.a != ta.b || tb.a != tb.b);
         int a0, a1, b0, b1, sa, sb;
-        price_pass<1, STAGE, false>(s, ws, ta, tb, ax, ay, bx, by, planes2, kind == DONE, a0, a1, b0, b1, sa, sb);
+        price_pass<1, REF, false>(s, ws, ta, tb, ax, ay, bx, by, planes2, kind == DONE, a0, a1, b0, b1, sa, sb);
         // column sums through shared memory: columns 2g, 2g+1 of tile A are
         // slots 0, 1 of group g, of tile B slots 2, 3
         *reinterpret_cast<int2*>(&bs.red[0][s.lane >> 2][2 * (s.lane & 3)]) = make_int2(a0, a1);

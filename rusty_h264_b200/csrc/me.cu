@@ -809,7 +809,7 @@ __device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp
     int shape = 0, fell = 0;
     SearchOut r16;
     if constexpr (BAL)
-        r16 = search16_bal<LEARN, true>(s, ws, bs, ww.lut, pmv, fd.lambda_me, LEARN, propc, prop, fd.prop_t, &fell);
+        r16 = search16_bal<LEARN, REF_WINDOW>(s, ws, bs, ww.lut, pmv, fd.lambda_me, LEARN, propc, prop, fd.prop_t, &fell);
     else
         r16 = mb_search<0, LEARN>(s, prm, ws, ww.lut, pmv, pmv, 1, fd.lambda_me, LEARN, prop, fd.prop_t, &fell);
     int evals = r16.evals << 4;  // 4x4-block evaluations
@@ -823,7 +823,7 @@ __device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp
         const int2 mv16 = make_int2(mv0x, mv0y);
         SearchOut r;
         if constexpr (BAL)
-            r = search_parts_bal<LEARN, true>(s, ws, bs, ww.lut, pmv, mv16, fd.lambda_me, LEARN && !fell, mv16);
+            r = search_parts_bal<LEARN, REF_WINDOW>(s, ws, bs, ww.lut, pmv, mv16, fd.lambda_me, LEARN && !fell, mv16);
         else
             r = mb_search<1, LEARN>(s, prm, ws, ww.lut, pmv, mv16, 2, fd.lambda_me, false, prop, 0, nullptr, LEARN && !fell, mv16);
         int px[4], py[4];
@@ -2102,10 +2102,10 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW)
                 const int2 mv16 = make_int2(mv16x, mv16y);
                 if constexpr (BAL) {
                     if (mode == 0)
-                        o = search16_bal<false, STAGE>(s, ws, bal[threadIdx.x >> 5], ww.lut, pmv, fd.lambda_me, false, pmv, pmv, 0,
+                        o = search16_bal<false, STAGE ? REF_WINDOW : REF_PLANES>(s, ws, bal[threadIdx.x >> 5], ww.lut, pmv, fd.lambda_me, false, pmv, pmv, 0,
                                                        nullptr);
                     else
-                        o = search_parts_bal<false, STAGE>(s, ws, bal[threadIdx.x >> 5], ww.lut, pmv, mv16, fd.lambda_me, false, mv16);
+                        o = search_parts_bal<false, STAGE ? REF_WINDOW : REF_PLANES>(s, ws, bal[threadIdx.x >> 5], ww.lut, pmv, mv16, fd.lambda_me, false, mv16);
                 } else {
                     o = mode == 0 ? mb_search<0, false>(s, prm, ws, ww.lut, pmv, pmv, 1, fd.lambda_me)
                                   : mb_search<1, false>(s, prm, ws, ww.lut, pmv, mv16, 2, fd.lambda_me);
