@@ -91,22 +91,6 @@ __device__ __forceinline__ void chroma_line(uint8_t* q, int step, int alpha, int
     q[0] = uint8_t(clip1(q0 - delta));
 }
 
-// MV and coefficient flag of 4x4 block (bx, by) of MB m (coefficients in the
-// reference's dct[256] order: 8x8 region, then 4x4 sub-block), read through L2
-// (the MB may have been written by another CTA of the same launch).
-__device__ __forceinline__ void block_state_at(const int32_t* picks, const int16_t* coeffs, int m, int bx, int by,
-                                               int& mvx, int& mvy, bool& nz) {
-    const int32_t* pk = picks + 6 * m;
-    const int shape = __ldcg(pk);
-    const int part = shape == 1 ? (by >= 2) : (shape == 2 ? (bx >= 2) : 0);
-    mvx = __ldcg(pk + 1 + 2 * part);
-    mvy = __ldcg(pk + 2 + 2 * part);
-    const int qi = (by >= 2 ? 2 : 0) + (bx >= 2 ? 1 : 0), k = (by & 1) * 2 + (bx & 1);
-    const uint4* c = reinterpret_cast<const uint4*>(coeffs + (long long)m * 256 + (qi * 4 + k) * 16);
-    const uint4 a = __ldcg(c), b = __ldcg(c + 1);
-    nz = (a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) != 0u;
-}
-
 // The bS of one MB's 32 edge segments from the two blocks' MVs and
 // coefficient flags; e == 0 segments on the picture border have none.
 __device__ __forceinline__ int bs_of(bool pnz, bool qnz, int pmx, int pmy, int qmx, int qmy) {
