@@ -118,15 +118,19 @@ __device__ __forceinline__ void db_filter(const DbLine& d, int bs, int p2, int& 
 // The edges of one direction of the lane's line px[0..19] (luma edges at 4, 8,
 // 12, 16; chroma at 4 and 8); bits: two per edge.
 __device__ __forceinline__ void db_line(const DbLine& d, unsigned bits, int px[20]) {
+    const unsigned any = __reduce_or_sync(0xffffffffu, bits);  // edges no line of the MB filters are skipped
 #pragma unroll
     for (int e = 0; e < 4; e++)
-        db_filter(d, int((bits >> (2 * e)) & 3u), px[4 * e + 1], px[4 * e + 2], px[4 * e + 3], px[4 * e + 4], px[4 * e + 5],
-                  px[4 * e + 6]);
+        if ((any >> (2 * e)) & 3u)
+            db_filter(d, int((bits >> (2 * e)) & 3u), px[4 * e + 1], px[4 * e + 2], px[4 * e + 3], px[4 * e + 4],
+                      px[4 * e + 5], px[4 * e + 6]);
 }
 
+// (eight 1080p pictures with 4, 6, 8, 16 rows a CTA: 529, 520, 524, 565 us for
+// luma and chroma T/Q and this; publishing every 1, 2, 4 MBs: 532, 524, 534)
 constexpr int DB_ROWS = 8;              // MB rows (warps) per CTA
 constexpr int DB_STRIP = 80;            // a finished MB's bottom rows: luma 3 x 16, chroma 2 x 2 x 8
-constexpr int DB_PUBLISH = 4;           // MBs between releases of a CTA's last row
+constexpr int DB_PUBLISH = 2;           // MBs between releases of a CTA's last row
 constexpr int DB_MAX_SMEM = 200 * 1024; // a CTA's strips; wider pictures take fewer rows per CTA
 struct DbTiles {
     uint8_t lt[LT * LT];
@@ -207,6 +211,18 @@ __global__ void __launch_bounds__(32 * DB_ROWS) deblock_rows_kernel(const __grid
             if (has_c) nc = ldw32(cown + (long long)cr * ccw + 4 * cwd);
             DbStrength ns = st[0];
             int avail = 0;  // MBs of the row above seen ready
+            // a row whose upper neighbour is another CTA's: the lane's word of
+            // the next MB's top strip, fetched a step ahead when it is ready
+            uint32_t tw = 0;
+            bool tw_ok = false;
+            auto top_word = [&](int mb) -> uint32_t {
+                if (lane < 12) return ldw32(Y + (long long)((lane >> 2) - 3) * cw + 16 * mb + 4 * (lane & 3));
+                if (lane < 20 && has_c) {
+                    const int i = lane - 12;
+                    return ldw32(((i >> 2) ? C1 : C0) + (long long)(((i >> 1) & 1) - 2) * ccw + 8 * mb + 4 * (i & 1));
+                }
+                return 0u;
+            };
             for (int x = 0; x < W; x++) {
                 const DbStrength s = ns;
                 lt32[(4 + r0) * (LT / 4) + 1 + wc] = n0;
@@ -281,17 +297,16 @@ __global__ void __launch_bounds__(32 * DB_ROWS) deblock_rows_kernel(const __grid
                         avail = __shfl_sync(0xffffffffu, avail, 0);
                     }
                     // luma rows -3..-1: lanes 0..11; chroma rows -2, -1: lanes 12..19
-                    if (lane < 12) {
-                        const int r = lane >> 2;
-                        lt32[(1 + r) * (LT / 4) + 1 + (lane & 3)] =
-                            top_shared ? reinterpret_cast<const uint32_t*>(db_strips + ((long long)(w - 1) * max_w + x) * DB_STRIP)[lane]
-                                       : ldw32(Y + (long long)(r - 3) * cw + 16 * x + 4 * (lane & 3));
-                    } else if (lane < 20 && has_c) {
-                        const int i = lane - 12, p = i >> 2, r = (i >> 1) & 1, k = i & 1;
-                        *reinterpret_cast<uint32_t*>(&tl.ct[p][r * CT + 4 + 4 * k]) =
-                            top_shared ? reinterpret_cast<const uint32_t*>(db_strips + ((long long)(w - 1) * max_w + x) * DB_STRIP)[12 + i]
-                                       : ldw32((p ? C1 : C0) + (long long)(r - 2) * ccw + 8 * x + 4 * k);
+                    if (top_shared) {
+                        if (lane < 20) tw = reinterpret_cast<const uint32_t*>(db_strips + ((long long)(w - 1) * max_w + x) * DB_STRIP)[lane];
+                    } else if (!tw_ok) {
+                        tw = top_word(x);
                     }
+                    if (lane < 12) lt32[(1 + (lane >> 2)) * (LT / 4) + 1 + (lane & 3)] = tw;
+                    else if (lane < 20 && has_c)
+                        *reinterpret_cast<uint32_t*>(&tl.ct[(lane - 12) >> 2][(((lane - 12) >> 1) & 1) * CT + 4 + 4 * (lane & 1)]) = tw;
+                    tw_ok = !top_shared && avail >= x + 2;
+                    if (tw_ok) tw = top_word(x + 1);
                     __syncwarp();
                 }
                 // ---- horizontal edges ----
