@@ -23,12 +23,14 @@
 // transposed view of a weight or activation tensor, ...) and an epilogue
 // functor (bias + ReLU + bf16 store, ReLU-mask + bf16 store, or an fp32
 // atomic add for weight gradients, whose K dimension -- the batch times the
-// output positions -- is split over CTAs).  Weight gradients get their bias
-// gradient from an extra K column of ones.
+// output positions -- is split over CTAs).  Every gather moves 16 bytes: the
+// weight gradients' operands are staged as they lie in memory, M- and N-major
+// (the tensor core transposes), and the data gradients read weights that
+// prep_kernel has transposed.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
-#include <type_traits>
 #include <vector>
 
 #include "h264a_device.cuh"
@@ -52,7 +54,6 @@ constexpr int O_B5 = O_W5 + N_W5;
 constexpr int NPARAMS = O_B5 + HEAD_N;
 static_assert(NPARAMS == H264A_MVNET_NPARAMS, "parameter count");
 static_assert((O_W1 | O_W2 | O_W3 | O_W4 | O_W5) % 2 == 0, "weights start on bf16 pairs");
-
 
 typedef uint16_t bf16_t;  // raw bf16 bits
 
@@ -96,24 +97,18 @@ __device__ __forceinline__ uint32_t x0_pair(const Geo& g, int b, int iy, int ix)
     const float r = (float(p.d_ref[o]) - 128.f) * (1.f / 64.f), c = (float(p.d_cur[o]) - 128.f) * (1.f / 64.f);
     return pack2(f2bf(r), f2bf(c));  // exact: k/64 with |k| <= 128
 }
-__device__ __forceinline__ bf16_t x0_one(const Geo& g, int b, int iy, int ix, int ci) {
-    const uint32_t v = x0_pair(g, b, iy, ix);
-    return bf16_t(ci ? (v >> 16) : (v & 0xffffu));
-}
 __device__ __forceinline__ bf16_t mv_feat(const Geo& g, int m, int i) {
     const int v = min(max(int(g.nmv[6LL * m + i]), -128), 128);
     return f2bf(float(v) * (1.f / 64.f));  // exact
 }
 
 // ---- the tcgen05 GEMM: 128 x BN tiles, accumulators in tensor memory --------
-// The GEMM of every layer, C[M][N] = sum_k A[m][k] B[k][n] (op.a(m, k) /
-// op.b(k, n) gather the bf16 pair (k, k+1), zero past their tensor; op.store
-// takes each fp32 result; CTA z covers k in [z*kchunk, ...)), on the sm_100
-// tensor cores: per 64-wide K step all 256 threads gather the A (128 x 64)
-// and B (BN x 64) tiles into one of two shared-memory stages, one thread
-// issues four tcgen05.mma (M 128, N BN, K 16, bf16 in, fp32 accumulated in
-// tensor memory) and commits them to the stage's mbarrier, and the gathers of
-// the next step overlap them.  The epilogue reads the accumulator rows with
+// The GEMM of every forward layer and data gradient, C[M][N] = sum_k A[m][k]
+// B[k][n], on the sm_100 tensor cores: per 64-wide K step all 256 threads
+// gather the A (128 x 64) and B (BN x 64) tiles into one of two shared-memory
+// stages, one thread issues four tcgen05.mma (M 128, N BN, K 16, bf16 in, fp32
+// accumulated in tensor memory) and commits them to the stage's mbarrier, and
+// the gathers of the next step overlap them.  The epilogue reads the accumulator rows with
 // tcgen05.ld: warp w may read tensor-memory lanes 32(w % 4) .. +31 (its tile
 // rows), warps w and w + 4 taking half of the columns each.
 constexpr int TC_BM = 128, TC_BK = 64, TC_THREADS = 256;
@@ -159,24 +154,13 @@ __device__ __forceinline__ void tc_wait(uint32_t bar, uint32_t parity, int* stat
     }
 }
 
-// An Op with `static constexpr bool kVec = true` also gathers 8 consecutive
-// k at once (op.a8(m, k), op.b8(k, n): 16 bytes, k a multiple of 8, zero past
-// its tensor) and stores 8 consecutive n (op.store8(m, n, v)); the GEMM then
-// moves each 16-byte chunk of a stage with one load (K and N multiples of 8).
-// Such an Op also names a `Row` (what its gathers need of output row m:
-// sample, position, base offset) made once per CTA row by op.row(m), so the
-// per-chunk gather op.a8(row, k) does no division by a runtime size.
-template <class Op, class = void>
-struct VecOp : std::false_type {
-    using Row = int;
-};
-template <class Op>
-struct VecOp<Op, std::void_t<decltype(Op::kVec)>> : std::bool_constant<Op::kVec> {
-    using Row = typename Op::Row;
-};
-
+// An Op gathers 8 consecutive k at once (op.a8(row, k), op.b8(k, n): 16 bytes,
+// k a multiple of 8, zero past its tensor) and stores 8 consecutive n
+// (op.store8(row, m, n, v)).  Its `Row` is what its gathers need of output row
+// m (sample, position, base offset), made once per CTA row by op.row(m), so
+// the per-chunk gathers divide by no runtime size.  K and N are multiples of 8.
 template <int BN, class Op>
-__global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const Op op, int M, int N, int K, int kchunk, int* status) {
+__global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const Op op, int M, int N, int K, int* status) {
     static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "tcgen05 N for M = 128");
     constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2, STAGE = A_BYTES + B_BYTES;
     constexpr int NCOL = tc_cols<BN>();
@@ -184,13 +168,11 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const Op op, int M,
     extern __shared__ __align__(128) uint8_t tc_smem[];
     __shared__ __align__(8) unsigned long long tc_bar[2];
     __shared__ uint32_t tc_tmem;
-    __shared__ typename VecOp<Op>::Row tc_rows[VecOp<Op>::value ? TC_BM : 1];
+    __shared__ typename Op::Row tc_rows[TC_BM];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * TC_BM, n0 = blockIdx.y * BN;
-    if constexpr (VecOp<Op>::value) {
-        for (int i = tid; i < TC_BM; i += TC_THREADS) tc_rows[i] = op.row(min(m0 + i, M - 1));
-    }  // read after the __syncthreads below
-    const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
+    for (int i = tid; i < TC_BM; i += TC_THREADS) tc_rows[i] = op.row(min(m0 + i, M - 1));  // read after the __syncthreads below
+    const int kb = 0, ke = K;
     const uint32_t sbase = tc_smem_u32(tc_smem), bar0 = tc_smem_u32(&tc_bar[0]);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(&tc_tmem)),
@@ -213,7 +195,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const Op op, int M,
         const uint32_t sa = sbase + uint32_t(st * STAGE), sb = sa + A_BYTES;
         // consecutive threads fill consecutive 16-byte rows of a core
         // matrix, so a warp's stores meet no bank twice
-        if constexpr (VecOp<Op>::value) {
+        {
             // the step's gathers are issued before waiting for the stage, so
             // they overlap the MMAs still reading it
             constexpr int AQ = TC_BM * 8 / TC_THREADS, BQ = (BN * 8 + TC_THREADS - 1) / TC_THREADS;
@@ -246,27 +228,6 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const Op op, int M,
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sb + tc_off(row, c)), "r"(vb[j].x),
                                  "r"(vb[j].y), "r"(vb[j].z), "r"(vb[j].w)
                                  : "memory");
-            }
-        } else {
-            // the stage's previous MMAs (step it - 2) have read it
-            if (it >= 2) tc_wait(bar0 + 8 * st, uint32_t((it - 2) >> 1) & 1u, status);
-            for (int q = tid; q < TC_BM * 8; q += TC_THREADS) {
-                const int row = ((q >> 6) << 3) | (q & 7), c = (q >> 3) & 7, m = m0 + row, k = k0 + 8 * c;
-                uint32_t v[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) v[i] = (m < M && k + 2 * i < ke) ? op.a(m, k + 2 * i) : 0u;
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sa + tc_off(row, c)), "r"(v[0]),
-                             "r"(v[1]), "r"(v[2]), "r"(v[3])
-                             : "memory");
-            }
-            for (int q = tid; q < BN * 8; q += TC_THREADS) {
-                const int row = ((q >> 6) << 3) | (q & 7), c = (q >> 3) & 7, n = n0 + row, k = k0 + 8 * c;
-                uint32_t v[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) v[i] = (n < N && k + 2 * i < ke) ? op.b(k + 2 * i, n) : 0u;
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sb + tc_off(row, c)), "r"(v[0]),
-                             "r"(v[1]), "r"(v[2]), "r"(v[3])
-                             : "memory");
             }
         }
         // the tiles' generic-proxy writes, visible to the tensor cores
@@ -304,19 +265,11 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const Op op, int M,
                            "=r"(r[7])
                          : "r"(taddr + uint32_t(c0)));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if constexpr (VecOp<Op>::value) {
-                if (row < M && n0 + c0 < N) {
-                    float f[8];
+            if (row < M && n0 + c0 < N) {
+                float f[8];
 #pragma unroll
-                    for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[i]);
-                    op.store8(row, n0 + c0, f);
-                }
-            } else if (row < M) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int n = n0 + c0 + i;
-                    if (n < N) op.store(row, n, __uint_as_float(r[i]));
-                }
+                for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[i]);
+                op.store8(tc_rows[row - m0], row, n0 + c0, f);
             }
         }
     }
@@ -330,36 +283,14 @@ struct Bufs {
     const bf16_t* w;  // bf16 parameters
     float* grad;      // fp32 parameter gradients (accumulated)
     bf16_t *a1, *a2, *a3, *h, *dl, *dh, *df, *da3, *da2, *da1;
+    const bf16_t *w4t, *w5t, *wd3, *wd2;  // prep_kernel's rearranged weights
     float* logits;
 };
-
-// im2col gather of a stride-2 3x3 conv over NHWC bf16 maps of H x W x C:
-// row m = (pair, oy, ox) of the output, column k = tap*C + ci.
-template <int C>
-__device__ __forceinline__ long long im2col_off(int H, int W, int m, int k) {
-    const int OW = W >> 1, OHW = (H >> 1) * OW;
-    const int b = m / OHW, r = m - b * OHW, oy = r / OW, ox = r - oy * OW;
-    const int tap = k / C, ci = k - tap * C, ky = tap / 3, kx = tap - ky * 3;
-    const int iy = 2 * oy + ky - 1, ix = 2 * ox + kx - 1;
-    if (iy < 0 || iy >= H || ix < 0 || ix >= W) return -1;
-    return ((long long)(b * H + iy) * W + ix) * C + ci;
-}
 
 // conv1 forward: M = P*H1*W1, N = 16, K = 18 (padded to 32)
 struct Conv1Fwd {
     Geo g; Bufs z;
-    __device__ uint32_t a(int m, int k) const {
-        if (k >= 18) return 0u;
-        const int OHW = g.H1 * g.W1;
-        const int b = m / OHW, r = m - b * OHW, oy = r / g.W1, ox = r - oy * g.W1;
-        const int tap = k >> 1, ky = tap / 3, kx = tap - ky * 3;
-        return x0_pair(g, b, 2 * oy + ky - 1, 2 * ox + kx - 1);
-    }
     __device__ uint32_t b(int k, int n) const { return k < 18 ? ld_pair(z.w + O_W1 + n * 18 + k) : 0u; }
-    __device__ void store(int m, int n, float v) const {
-        z.a1[(long long)m * 16 + n] = f2bf(fmaxf(v + bf2f(z.w[O_B1 + n]), 0.f));
-    }
-    static constexpr bool kVec = true;
     struct Row {
         int b, y0, x0;  // pair, top-left input pixel of the 3x3 window
     };
@@ -383,23 +314,14 @@ struct Conv1Fwd {
         for (int i = 0; i < 4; i++) v[i] = b(k + 2 * i, n);
         return make_uint4(v[0], v[1], v[2], v[3]);
     }
-    __device__ void store8(int m, int n, const float* v) const { st8_relu(z.a1 + (long long)m * 16 + n, v, z.w + O_B1 + n); }
+    __device__ void store8(const Row&, int m, int n, const float* v) const { st8_relu(z.a1 + (long long)m * 16 + n, v, z.w + O_B1 + n); }
 };
 // conv2 / conv3 forward: im2col of the previous map
 template <int C, int OW, int OB, int WHICH>
 struct ConvFwd {
     Geo g; Bufs z;
-    __device__ uint32_t a(int m, int k) const {
-        const long long o = WHICH == 2 ? im2col_off<C>(g.H1, g.W1, m, k) : im2col_off<C>(g.H2, g.W2, m, k);
-        return o < 0 ? 0u : ld_pair((WHICH == 2 ? z.a1 : z.a2) + o);
-    }
-    __device__ uint32_t b(int k, int n) const { return ld_pair(z.w + OW + n * 9 * C + k); }
-    __device__ void store(int m, int n, float v) const {
-        (WHICH == 2 ? z.a2 : z.a3)[(long long)m * 32 + n] = f2bf(fmaxf(v + bf2f(z.w[OB + n]), 0.f));
-    }
     // k a multiple of 8 (C = 16 or 32): the chunk is 8 channels of one tap,
     // 16 contiguous bytes of the NHWC map
-    static constexpr bool kVec = true;
     struct Row {
         long long base;  // element offset of input pixel (y0, x0), channel 0 (may lie outside the map)
         int y0, x0;
@@ -418,49 +340,18 @@ struct ConvFwd {
         return ld8((WHICH == 2 ? z.a1 : z.a2) + w.base + (long long)(ky * W + kx) * C + ci);
     }
     __device__ uint4 b8(int k, int n) const { return ld8(z.w + OW + n * 9 * C + k); }
-    __device__ void store8(int m, int n, const float* v) const {
+    __device__ void store8(const Row&, int m, int n, const float* v) const {
         st8_relu((WHICH == 2 ? z.a2 : z.a3) + (long long)m * 32 + n, v, z.w + OB + n);
     }
 };
 using Conv2Fwd = ConvFwd<16, O_W2, O_B2, 2>;
 using Conv3Fwd = ConvFwd<32, O_W3, O_B3, 3>;
 
-// offset in A3 of feature k < 1152 of sample m (its MB's 6x6-cell crop), or
-// -1 outside the map
-__device__ __forceinline__ long long crop_off(const Geo& g, int m, int k) {
-    const int b = m / g.nmb, r = m - b * g.nmb, mby = r / g.mb_w, mbx = r - mby * g.mb_w;
-    const int cy = k / 192, rem = k - cy * 192, cx = rem >> 5, c = rem & 31;
-    const int y = 2 * mby - 2 + cy, x = 2 * mbx - 2 + cx;
-    if (y < 0 || y >= g.H3 || x < 0 || x >= g.W3) return -1;
-    return ((long long)(b * g.H3 + y) * g.W3 + x) * 32 + c;
-}
-// the FC1 input row of sample m, pair (k, k+1)
-__device__ __forceinline__ uint32_t feat_pair(const Geo& g, const Bufs& z, int m, int k) {
-    if (k < CONVF) {
-        const long long o = crop_off(g, m, k);
-        return o < 0 ? 0u : ld_pair(z.a3 + o);
-    }
-    if (k < CONVF + 6) return pack2(mv_feat(g, m, k - CONVF), mv_feat(g, m, k - CONVF + 1));
-    return 0u;
-}
-__device__ __forceinline__ bf16_t feat_one(const Geo& g, const Bufs& z, int m, int k) {
-    if (k < CONVF) {
-        const long long o = crop_off(g, m, k);
-        return o < 0 ? bf16_t(0) : z.a3[o];
-    }
-    if (k < CONVF + 6) return mv_feat(g, m, k - CONVF);
-    return 0;
-}
 struct Fc1Fwd {
     Geo g; Bufs z;
-    __device__ uint32_t a(int m, int k) const { return feat_pair(g, z, m, k); }
-    __device__ uint32_t b(int k, int n) const { return ld_pair(z.w + O_W4 + (long long)n * FEAT + k); }
-    __device__ void store(int m, int n, float v) const {
-        z.h[(long long)m * HID + n] = f2bf(fmaxf(v + bf2f(z.w[O_B4 + n]), 0.f));
-    }
     // k < 1152, a multiple of 8: 8 channels of one crop cell, 16 contiguous
-    // bytes of A3; then the 6 neighbour-MV features and zeros
-    static constexpr bool kVec = true;
+    // bytes of A3 (its MB's 6x6-cell crop, zero outside the map); then the 6
+    // neighbour-MV features and zeros
     struct Row {
         long long base;  // element offset of the crop's top-left cell (y0, x0), channel 0
         int m, y0, x0;
@@ -483,19 +374,15 @@ struct Fc1Fwd {
         return make_uint4(0u, 0u, 0u, 0u);
     }
     __device__ uint4 b8(int k, int n) const { return ld8(z.w + O_W4 + (long long)n * FEAT + k); }
-    __device__ void store8(int m, int n, const float* v) const { st8_relu(z.h + (long long)m * HID + n, v, z.w + O_B4 + n); }
+    __device__ void store8(const Row&, int m, int n, const float* v) const { st8_relu(z.h + (long long)m * HID + n, v, z.w + O_B4 + n); }
 };
 struct HeadFwd {
     Bufs z;
-    __device__ uint32_t a(int m, int k) const { return ld_pair(z.h + (long long)m * HID + k); }
-    __device__ uint32_t b(int k, int n) const { return ld_pair(z.w + O_W5 + n * HID + k); }
-    __device__ void store(int m, int n, float v) const { z.logits[(long long)m * HEAD_N + n] = v + bf2f(z.w[O_B5 + n]); }
-    static constexpr bool kVec = true;
     using Row = int;
     __device__ Row row(int m) const { return m; }
     __device__ uint4 a8(Row m, int k) const { return ld8(z.h + (long long)m * HID + k); }
     __device__ uint4 b8(int k, int n) const { return ld8(z.w + O_W5 + n * HID + k); }
-    __device__ void store8(int m, int n, const float* v) const {
+    __device__ void store8(const Row&, int m, int n, const float* v) const {
         float4* d = reinterpret_cast<float4*>(z.logits + (long long)m * HEAD_N + n);
         const bf16_t* bias = z.w + O_B5 + n;
         d[0] = make_float4(v[0] + bf2f(bias[0]), v[1] + bf2f(bias[1]), v[2] + bf2f(bias[2]), v[3] + bf2f(bias[3]));
@@ -503,130 +390,319 @@ struct HeadFwd {
     }
 };
 
-// ---- backward -----------------------------------------------------------------
-// Weight gradient of a layer y = W x: dW[i][j] = sum_m dy[m][i] * x[m][j], the
-// GEMM's M = output channels, N = input columns (+1 for the bias, a column of
-// ones), K = rows m (the samples, or the pairs times the map positions).
-// a(i, m) / b(m, j) pair two consecutive rows m, m+1 (zero past K).
-__device__ __forceinline__ uint32_t col_pair(const bf16_t* y, int ld, int i, int m, int K) {
-    const bf16_t lo = y[(long long)m * ld + i];
-    const bf16_t hi = m + 1 < K ? y[(long long)(m + 1) * ld + i] : bf16_t(0);
-    return pack2(lo, hi);
+// ---- data gradients ---------------------------------------------------------
+// The weights as the data gradients' GEMMs read them, K contiguous: w5t
+// [256][296] and w4t [1152][256] transposed; wd3 [128][128] and wd2 [64][128]
+// the stride-2 transposed convolutions over a 2x2 block of input pixels: row
+// n = (2 py + px) * C + ci of input pixel (2a + py, 2b + px), column k =
+// (2 ny + nx) * 32 + co of output position (a + ny, b + nx), the tap
+// (py + 1 - 2 ny, px + 1 - 2 nx) or zero.  (A GEMM over input pixels and all
+// nine taps reads four times as much and multiplies mostly zeros: 970 us
+// against 83 for conv2's on four 1080p pairs.)
+constexpr int N_W4T = CONVF * HID, N_W5T = HID * HEAD_N, N_WD3 = 128 * 128, N_WD2 = 64 * 128;
+constexpr int N_PREP = N_W4T + N_W5T + N_WD3 + N_WD2;
+__device__ __forceinline__ bf16_t wd_at(const bf16_t* w, int C, int i) {  // w [32][9][C]
+    const int n = i >> 7, k = i & 127, par = n / C, ci = n - par * C, nb = k >> 5, co = k & 31;
+    const int ky = (par >> 1) + 1 - 2 * (nb >> 1), kx = (par & 1) + 1 - 2 * (nb & 1);
+    return ky < 0 || kx < 0 ? bf16_t(0) : w[(co * 9 + ky * 3 + kx) * C + ci];
 }
-constexpr bf16_t BF_ONE = 0x3f80;
+__global__ void prep_kernel(const bf16_t* __restrict__ w, bf16_t* __restrict__ out) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < N_W4T) {
+        out[i] = w[O_W4 + (i % HID) * FEAT + i / HID];
+        return;
+    }
+    i -= N_W4T;
+    if (i < N_W5T) {
+        out[N_W4T + i] = w[O_W5 + (i % HEAD_N) * HID + i / HEAD_N];
+        return;
+    }
+    i -= N_W5T;
+    if (i < N_WD3) {
+        out[N_W4T + N_W5T + i] = wd_at(w + O_W3, 32, i);
+        return;
+    }
+    i -= N_WD3;
+    if (i < N_WD2) out[N_W4T + N_W5T + N_WD3 + i] = wd_at(w + O_W2, 16, i);
+}
 
-struct HeadBwdW {  // M = 296, N = 258 (256 + bias + pad), K = B
-    Bufs z; int B;
-    __device__ uint32_t a(int i, int m) const { return col_pair(z.dl, HEAD_N, i, m, B); }
-    __device__ uint32_t b(int m, int j) const {
-        if (j < HID) return col_pair(z.h, HID, j, m, B);
-        if (j == HID) return pack2(BF_ONE, m + 1 < B ? BF_ONE : bf16_t(0));
-        return 0u;
+__device__ __forceinline__ uint32_t mask_pair(uint32_t act, uint32_t v) {  // bf16 pair v where the activation is not zero
+    return v & ((act & 0xffffu ? 0xffffu : 0u) | (act & 0xffff0000u ? 0xffff0000u : 0u));
+}
+// 8 values rounded to bf16, stored as one 16-byte word; with act, zero where
+// the activation there is (ReLU's gradient)
+__device__ __forceinline__ void st8_mask(bf16_t* dst, const float* v, const bf16_t* act) {
+    uint4 w = make_uint4(pack2(f2bf(v[0]), f2bf(v[1])), pack2(f2bf(v[2]), f2bf(v[3])), pack2(f2bf(v[4]), f2bf(v[5])),
+                         pack2(f2bf(v[6]), f2bf(v[7])));
+    if (act != nullptr) {
+        const uint4 a = ld8(act);
+        w = make_uint4(mask_pair(a.x, w.x), mask_pair(a.y, w.y), mask_pair(a.z, w.z), mask_pair(a.w, w.w));
     }
-    __device__ void store(int i, int j, float v) const {
-        if (j < HID) atomicAdd(z.grad + O_W5 + i * HID + j, v);
-        else if (j == HID) atomicAdd(z.grad + O_B5 + i, v);
-    }
-};
+    *reinterpret_cast<uint4*>(dst) = w;
+}
+
 struct HeadBwdData {  // dh = relu'(h) * (dl W5): M = B, N = 256, K = 296
     Bufs z;
-    __device__ uint32_t a(int m, int k) const { return ld_pair(z.dl + (long long)m * HEAD_N + k); }
-    __device__ uint32_t b(int k, int n) const { return pack2(z.w[O_W5 + k * HID + n], z.w[O_W5 + (k + 1) * HID + n]); }
-    __device__ void store(int m, int n, float v) const {
+    using Row = int;
+    __device__ Row row(int m) const { return m; }
+    __device__ uint4 a8(Row m, int k) const { return ld8(z.dl + (long long)m * HEAD_N + k); }
+    __device__ uint4 b8(int k, int n) const { return ld8(z.w5t + n * HEAD_N + k); }
+    __device__ void store8(const Row&, int m, int n, const float* v) const {
         const long long o = (long long)m * HID + n;
-        z.dh[o] = z.h[o] != 0 ? f2bf(v) : bf16_t(0);
-    }
-};
-struct Fc1BwdW {  // M = 256, N = 1170, K = B
-    Geo g; Bufs z; int B;
-    __device__ uint32_t a(int i, int m) const { return col_pair(z.dh, HID, i, m, B); }
-    __device__ uint32_t b(int m, int j) const {
-        if (j < FEAT) return pack2(feat_one(g, z, m, j), m + 1 < B ? feat_one(g, z, m + 1, j) : bf16_t(0));
-        if (j == FEAT) return pack2(BF_ONE, m + 1 < B ? BF_ONE : bf16_t(0));
-        return 0u;
-    }
-    __device__ void store(int i, int j, float v) const {
-        if (j < FEAT) atomicAdd(z.grad + O_W4 + (long long)i * FEAT + j, v);
-        else if (j == FEAT) atomicAdd(z.grad + O_B4 + i, v);
+        st8_mask(z.dh + o, v, z.h + o);
     }
 };
 struct Fc1BwdData {  // df = (dh W4)[:, :1152]: M = B, N = 1152, K = 256
     Bufs z;
-    __device__ uint32_t a(int m, int k) const { return ld_pair(z.dh + (long long)m * HID + k); }
-    __device__ uint32_t b(int k, int n) const {
-        return pack2(z.w[O_W4 + (long long)k * FEAT + n], z.w[O_W4 + (long long)(k + 1) * FEAT + n]);
-    }
-    __device__ void store(int m, int n, float v) const { z.df[(long long)m * CONVF + n] = f2bf(v); }
+    using Row = int;
+    __device__ Row row(int m) const { return m; }
+    __device__ uint4 a8(Row m, int k) const { return ld8(z.dh + (long long)m * HID + k); }
+    __device__ uint4 b8(int k, int n) const { return ld8(z.w4t + n * HID + k); }
+    __device__ void store8(const Row&, int m, int n, const float* v) const { st8_mask(z.df + (long long)m * CONVF + n, v, nullptr); }
 };
-// conv weight gradient: M = CO, N = 9*C + 2 (bias column at 9*C), K = P*OH*OW
-template <int C, int CO, int OW, int OB, int WHICH>
-struct ConvBwdW {
-    Geo g; Bufs z; int K;
-    __device__ const bf16_t* dy() const { return WHICH == 1 ? z.da1 : (WHICH == 2 ? z.da2 : z.da3); }
-    __device__ bf16_t xin(int m, int j) const {
-        if (WHICH == 1) {  // the network input, read from the frames
-            const int OHW = g.H1 * g.W1;
-            const int b = m / OHW, r = m - b * OHW, oy = r / g.W1, ox = r - oy * g.W1;
-            const int tap = j >> 1, ky = tap / 3, kx = tap - ky * 3;
-            return x0_one(g, b, 2 * oy + ky - 1, 2 * ox + kx - 1, j & 1);
-        }
-        const long long o = WHICH == 2 ? im2col_off<C>(g.H1, g.W1, m, j) : im2col_off<C>(g.H2, g.W2, m, j);
-        return o < 0 ? bf16_t(0) : (WHICH == 2 ? z.a1 : z.a2)[o];
-    }
-    __device__ uint32_t a(int i, int m) const { return col_pair(dy(), CO, i, m, K); }
-    __device__ uint32_t b(int m, int j) const {
-        if (j < 9 * C) return pack2(xin(m, j), m + 1 < K ? xin(m + 1, j) : bf16_t(0));
-        if (j == 9 * C) return pack2(BF_ONE, m + 1 < K ? BF_ONE : bf16_t(0));
-        return 0u;
-    }
-    __device__ void store(int i, int j, float v) const {
-        if (j < 9 * C) atomicAdd(z.grad + OW + i * 9 * C + j, v);
-        else if (j == 9 * C) atomicAdd(z.grad + OB + i, v);
-    }
-};
-using Conv1BwdW = ConvBwdW<2, 16, O_W1, O_B1, 1>;
-using Conv2BwdW = ConvBwdW<16, 32, O_W2, O_B2, 2>;
-using Conv3BwdW = ConvBwdW<32, 32, O_W3, O_B3, 3>;
-// conv input gradient (stride-2 transposed conv): rows m = (pair, iy, ix) of
-// the H x W input, N = C input channels, K = 9 taps x CO output channels: tap
-// (ky, kx) of input (iy, ix) feeds output ((iy + 1 - ky) / 2, (ix + 1 - kx) / 2)
-// when both are even and inside the output map.
-template <int C, int CO, int OW, int WHICH>
+// conv input gradient: M = pairs x output positions (2x2 input blocks),
+// N = 4 C, K = 4 x 32 (see prep_kernel); WHICH 3: da3 -> da2, 2: da2 -> da1
+template <int C, int WHICH>
 struct ConvBwdData {
     Geo g; Bufs z;
-    __device__ uint32_t a(int m, int k) const {
-        const int H = WHICH == 3 ? g.H2 : g.H1, W = WHICH == 3 ? g.W2 : g.W1;
-        const int OH = H >> 1, OWd = W >> 1;
-        const int HW = H * W, b = m / HW, r = m - b * HW, iy = r / W, ix = r - iy * W;
-        const int tap = k / CO, co = k - tap * CO, ky = tap / 3, kx = tap - ky * 3;
-        const int ty = iy + 1 - ky, tx = ix + 1 - kx;
-        if ((ty | tx) < 0 || (ty & 1) || (tx & 1) || ty >= 2 * OH || tx >= 2 * OWd) return 0u;
-        return ld_pair((WHICH == 3 ? z.da3 : z.da2) + ((long long)(b * OH + (ty >> 1)) * OWd + (tx >> 1)) * CO + co);
+    struct Row {
+        long long in, out;  // element offsets of dy position (a, b) and of input pixel (2a, 2b)
+        bool down, right;   // (a + 1, .) and (., b + 1) lie inside the map
+    };
+    __device__ Row row(int m) const {
+        const int OH = WHICH == 3 ? g.H3 : g.H2, OW = WHICH == 3 ? g.W3 : g.W2;
+        const int ohw = OH * OW, b = m / ohw, r = m - b * ohw, a = r / OW, x = r - a * OW;
+        return Row{(long long)m * 32, ((long long)(b * 2 * OH + 2 * a) * (2 * OW) + 2 * x) * C, a + 1 < OH, x + 1 < OW};
     }
-    __device__ uint32_t b(int k, int n) const {
-        const int tap = k / CO, co = k - tap * CO;
-        return pack2(z.w[OW + co * 9 * C + tap * C + n], z.w[OW + (co + 1) * 9 * C + tap * C + n]);
+    __device__ uint4 a8(const Row& w, int k) const {
+        const int nb = k >> 5, OW = WHICH == 3 ? g.W3 : g.W2;
+        if (((nb & 2) && !w.down) || ((nb & 1) && !w.right)) return make_uint4(0u, 0u, 0u, 0u);
+        return ld8((WHICH == 3 ? z.da3 : z.da2) + w.in + ((nb & 2) ? OW * 32 : 0) + ((nb & 1) ? 32 : 0) + (k & 31));
     }
-    __device__ void store(int m, int n, float v) const {
-        const long long o = (long long)m * C + n;
-        const bf16_t* xa = WHICH == 3 ? z.a2 : z.a1;
-        (WHICH == 3 ? z.da2 : z.da1)[o] = xa[o] != 0 ? f2bf(v) : bf16_t(0);
+    __device__ uint4 b8(int k, int n) const { return ld8((WHICH == 3 ? z.wd3 : z.wd2) + n * 128 + k); }
+    __device__ void store8(const Row& w, int, int n, const float* v) const {
+        const int par = n / C, ci = n - par * C, W = WHICH == 3 ? g.W2 : g.W1;
+        const long long o = w.out + ((par & 2) ? W * C : 0) + ((par & 1) ? C : 0) + ci;
+        st8_mask((WHICH == 3 ? z.da2 : z.da1) + o, v, (WHICH == 3 ? z.a2 : z.a1) + o);
     }
 };
-using Conv3BwdData = ConvBwdData<32, 32, O_W3, 3>;
-using Conv2BwdData = ConvBwdData<16, 32, O_W2, 2>;
+
+// ---- weight gradients ---------------------------------------------------------
+// dW[i][j] = sum_m dy[m][i] x[m][j] over the rows m (samples, or the pairs'
+// map positions), split over CTAs: M = output channels, N = input columns,
+// K = rows.  Both operands lie row by row in memory, that is M- and N-major:
+// each thread moves 16-byte chunks (8 columns of one row) as they are into the
+// M/N-major no-swizzle layout -- 8 (M or N) x 8 (K) core matrices of 128 bytes,
+// a row of K each 16 bytes, the KS/8 K-blocks of an 8-column block 128 bytes
+// apart (the leading byte offset) and the blocks KS * 16 apart (the stride byte
+// offset) -- and the tensor core transposes.  (Gathering K-major tiles took
+// two 2-byte loads per pair: 791 us for FC1's gradient on four 1080p pairs,
+// 32,640 samples, against 112 this way; 577 against 58 for conv2's.)  A tile holds only the M - m0 columns there are: the MMA's
+// further rows read whatever follows in shared memory into accumulator rows
+// that nothing reads.  The bias gradient is the sum of dy's chunks as the
+// threads of the first N tile pass them on.
+//   Op: rows K; RowW row(m); uint4 a8(row, i), b8(row, j); grad offsets out
+// (with leading dimension ld) and bias; n_real columns are stored.
+template <int KS>
+constexpr uint64_t wg_sdesc_hi() {
+    return (uint64_t(128 >> 4) << 16) | (uint64_t((KS * 16) >> 4) << 32) | (1ull << 46);
+}
+__device__ __forceinline__ void red_add_v4(float* p, const float* v) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+                 : "memory");
+}
+
+template <int BN, int KS, int AQ, class Op>  // AQ: 8-column chunks of A per thread and step
+__global__ void __launch_bounds__(TC_THREADS) wgrad_tc_kernel(const Op op, int M, int N, int K, int kchunk, int* status) {
+    static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256 && KS % 16 == 0 && TC_THREADS % KS == 0, "tile shape");
+    constexpr int GR = TC_THREADS / KS;          // threads per row
+    constexpr int BLK = KS * 16;                 // bytes of one 8-column block of a tile
+    constexpr int BQ = (BN / 8 + GR - 1) / GR, A_BYTES = AQ * GR * BLK, STAGE = A_BYTES + (BN / 8) * BLK;
+    constexpr int NCOL = tc_cols<BN>();
+    constexpr uint32_t IDESC = tc_idesc<BN>() | (1u << 15) | (1u << 16);  // A and B transposed (M/N-major)
+    extern __shared__ __align__(128) uint8_t tc_smem[];
+    __shared__ __align__(8) unsigned long long tc_bar[2];
+    __shared__ uint32_t tc_tmem;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.x * TC_BM, n0 = blockIdx.y * BN;
+    const int mblk = min(TC_BM, M - m0) / 8, nblk = min(BN, N - n0) / 8;
+    const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
+    const uint32_t sbase = tc_smem_u32(tc_smem), bar0 = tc_smem_u32(&tc_bar[0]);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(&tc_tmem)),
+                     "r"(NCOL));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        mbar_init(bar0, 1);
+        mbar_init(bar0 + 8, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tc_tmem;
+    const int p = tid % KS, c0 = tid / KS;  // the thread's row of a step and its first chunk
+    const uint32_t off = uint32_t((p >> 3) * 128 + (p & 7) * 16);
+    const bool with_bias = blockIdx.y == 0;
+    float bias[AQ][8];
+#pragma unroll
+    for (int j = 0; j < AQ; j++)
+#pragma unroll
+        for (int i = 0; i < 8; i++) bias[j][i] = 0.f;
+    const int nk = ke > kb ? (ke - kb + KS - 1) / KS : 0;
+    for (int it = 0; it < nk; it++) {
+        const int st = it & 1, m = kb + it * KS + p;
+        const uint32_t sa = sbase + uint32_t(st * STAGE), sb = sa + A_BYTES;
+        const bool live = m < ke;
+        const typename Op::Row row = op.row(live ? m : ke - 1);
+        uint4 va[AQ], vb[BQ];
+#pragma unroll
+        for (int j = 0; j < AQ; j++) {
+            const int c = c0 + j * GR;
+            va[j] = live && c < mblk ? op.a8(row, m0 + 8 * c) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int j = 0; j < BQ; j++) {
+            const int c = c0 + j * GR;
+            vb[j] = live && c < nblk ? op.b8(row, n0 + 8 * c) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        if (with_bias) {
+#pragma unroll
+            for (int j = 0; j < AQ; j++) {
+                const uint32_t w[4] = {va[j].x, va[j].y, va[j].z, va[j].w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    bias[j][2 * i] += bf2f(bf16_t(w[i] & 0xffffu));
+                    bias[j][2 * i + 1] += bf2f(bf16_t(w[i] >> 16));
+                }
+            }
+        }
+        // the stage's previous MMAs (step it - 2) have read it
+        if (it >= 2) tc_wait(bar0 + 8 * st, uint32_t((it - 2) >> 1) & 1u, status);
+#pragma unroll
+        for (int j = 0; j < AQ; j++)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sa + uint32_t((c0 + j * GR) * BLK) + off), "r"(va[j].x),
+                         "r"(va[j].y), "r"(va[j].z), "r"(va[j].w)
+                         : "memory");
+#pragma unroll
+        for (int j = 0; j < BQ; j++)
+            if (c0 + j * GR < BN / 8)
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sb + uint32_t((c0 + j * GR) * BLK) + off),
+                             "r"(vb[j].x), "r"(vb[j].y), "r"(vb[j].z), "r"(vb[j].w)
+                             : "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (tid == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < KS / 16; j++) {
+                const uint64_t da = uint64_t(((sa + 256u * j) >> 4) & 0x3fffu) | wg_sdesc_hi<KS>();
+                const uint64_t db = uint64_t(((sb + 256u * j) >> 4) & 0x3fffu) | wg_sdesc_hi<KS>();
+                const uint32_t acc = (it > 0 || j > 0) ? 1u : 0u;
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem),
+                    "l"(da), "l"(db), "r"(IDESC), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+                    : "memory");
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar0 + 8 * st)
+                         : "memory");
+        }
+    }
+    if (nk > 0) {
+        tc_wait(bar0 + 8 * ((nk - 1) & 1), uint32_t((nk - 1) >> 1) & 1u, status);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int row = m0 + (warp & 3) * 32 + lane;
+        const uint32_t taddr = tmem + (uint32_t((warp & 3) * 32) << 16);
+        const int nc = min(BN, op.n_real - n0);
+        if (m0 + (warp & 3) * 32 < M) {
+#pragma unroll 1
+            for (int c = (warp >> 2) * 8; c < nc; c += 16) {
+                uint32_t r[8];
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                               "=r"(r[7])
+                             : "r"(taddr + uint32_t(c)));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (row < M) {
+                    float f[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[i]);
+                    float* d = op.z.grad + op.out + (long long)row * op.ld + n0 + c;
+                    if (op.ld % 4 == 0 && op.out % 4 == 0) {  // every column chunk is whole then
+                        red_add_v4(d, f);
+                        red_add_v4(d + 4, f + 4);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; i++)
+                            if (c + i < nc) atomicAdd(d + i, f[i]);
+                    }
+                }
+            }
+        }
+        if (with_bias) {
+#pragma unroll
+            for (int j = 0; j < AQ; j++)
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    float v = bias[j][i];
+                    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    if (lane == 0 && c0 + j * GR < mblk) atomicAdd(op.z.grad + op.bias + m0 + 8 * (c0 + j * GR) + i, v);
+                }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOL));
+}
+
+struct HeadBwdW {  // M = 296, N = 256, K = B
+    Bufs z;
+    static constexpr int out = O_W5, ld = HID, bias = O_B5, n_real = HID;
+    using Row = int;
+    __device__ Row row(int m) const { return m; }
+    __device__ uint4 a8(Row m, int i) const { return ld8(z.dl + (long long)m * HEAD_N + i); }
+    __device__ uint4 b8(Row m, int j) const { return ld8(z.h + (long long)m * HID + j); }
+};
+struct Fc1BwdW {  // M = 256, N = 1168, K = B
+    Geo g; Bufs z;
+    static constexpr int out = O_W4, ld = FEAT, bias = O_B4, n_real = FEAT;
+    using Row = Fc1Fwd::Row;
+    __device__ Row row(int m) const { return Fc1Fwd{g, z}.row(m); }
+    __device__ uint4 a8(const Row& w, int i) const { return ld8(z.dh + (long long)w.m * HID + i); }
+    __device__ uint4 b8(const Row& w, int j) const { return Fc1Fwd{g, z}.a8(w, j); }
+};
+// conv weight gradient: M = CO, N = 9 C, K = pairs x output positions
+template <class Fwd, int C, int CO, int OW, int OB, int WHICH>
+struct ConvBwdW {
+    Geo g; Bufs z;
+    static constexpr int out = OW, ld = 9 * C, bias = OB, n_real = 9 * C;
+    struct Row {
+        typename Fwd::Row r;
+        int m;
+    };
+    __device__ Row row(int m) const { return Row{Fwd{g, z}.row(m), m}; }
+    __device__ uint4 a8(const Row& w, int i) const {
+        return ld8((WHICH == 1 ? z.da1 : (WHICH == 2 ? z.da2 : z.da3)) + (long long)w.m * CO + i);
+    }
+    __device__ uint4 b8(const Row& w, int j) const { return Fwd{g, z}.a8(w.r, j); }
+};
+using Conv1BwdW = ConvBwdW<Conv1Fwd, 2, 16, O_W1, O_B1, 1>;
+using Conv2BwdW = ConvBwdW<Conv2Fwd, 16, 32, O_W2, O_B2, 2>;
+using Conv3BwdW = ConvBwdW<Conv3Fwd, 32, 32, O_W3, O_B3, 3>;
 
 // da3 = relu'(a3) * (sum of the crop gradients of the up to 9 MBs whose 6x6
-// crop holds the cell): one thread per (pair, cell, channel pair).
+// crop holds the cell): one thread per (pair, cell, 8 channels).
 __global__ void uncrop_kernel(const Geo g, const bf16_t* __restrict__ df, const bf16_t* __restrict__ a3,
                               bf16_t* __restrict__ da3) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long total = (long long)g.P * g.H3 * g.W3 * 16;
+    const long long total = (long long)g.P * g.H3 * g.W3 * 4;
     if (i >= total) return;
-    const int c = int(i & 15) * 2;
-    const long long cell = i >> 4;
-    const int x = int(cell % g.W3), y = int((cell / g.W3) % g.H3), b = int(cell / ((long long)g.W3 * g.H3));
-    float s0 = 0.f, s1 = 0.f;
+    const int c = int(i & 3) * 8;
+    const int cell = int(i >> 2), hw = g.H3 * g.W3;
+    const int b = cell / hw, r = cell - b * hw, y = r / g.W3, x = r - y * g.W3;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const int ylo = max(0, (y - 2) >> 1), yhi = min(g.mb_h - 1, (y + 2) >> 1);
     const int xlo = max(0, (x - 2) >> 1), xhi = min(g.mb_w - 1, (x + 2) >> 1);
     for (int mby = ylo; mby <= yhi; mby++) {
@@ -636,39 +712,63 @@ __global__ void uncrop_kernel(const Geo g, const bf16_t* __restrict__ df, const 
             const int cx = x - 2 * mbx + 2;
             if (cx < 0 || cx >= 6) continue;
             const long long m = (long long)b * g.nmb + mby * g.mb_w + mbx;
-            const uint32_t v = ld_pair(df + m * CONVF + cy * 192 + cx * 32 + c);
-            s0 += bf2f(bf16_t(v & 0xffffu));
-            s1 += bf2f(bf16_t(v >> 16));
+            const uint4 v = ld8(df + m * CONVF + cy * 192 + cx * 32 + c);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                s[2 * k] += bf2f(bf16_t(w[k] & 0xffffu));
+                s[2 * k + 1] += bf2f(bf16_t(w[k] >> 16));
+            }
         }
     }
-    const long long o = cell * 32 + c;
-    da3[o] = a3[o] != 0 ? f2bf(s0) : bf16_t(0);
-    da3[o + 1] = a3[o + 1] != 0 ? f2bf(s1) : bf16_t(0);
+    const long long o = (long long)cell * 32 + c;
+    st8_mask(da3 + o, s, a3 + o);
 }
 
 // ---- loss, proposals, optimiser -------------------------------------------------
 // One warp per sample: softmax over the 289 classes, the sample's share of the
 // mean cross-entropy (atomically summed into *loss) and dl = (p - onehot) / B
 // in bf16 (zero for the 7 padding logits).
+// The row stays in registers (HEAD_N = 296: ten values a lane).
 __global__ void loss_kernel(const float* __restrict__ logits, const int16_t* __restrict__ labels, int B,
                             bf16_t* __restrict__ dl, float* __restrict__ loss) {
+    __shared__ float part[8];
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= B) return;
-    const float* z = logits + (long long)w * HEAD_N;
-    float mx = -INFINITY;
-    for (int c = lane; c < NCLS; c += 32) mx = fmaxf(mx, z[c]);
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    float s = 0.f;
-    for (int c = lane; c < NCLS; c += 32) s += expf(z[c] - mx);
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const int label = min(max(int(labels[w]), 0), NCLS - 1);
-    const float inv = 1.f / s, scale = 1.f / float(B);
-    for (int c = lane; c < HEAD_N; c += 32) {
-        float d = 0.f;
-        if (c < NCLS) d = (expf(z[c] - mx) * inv - (c == label ? 1.f : 0.f)) * scale;
-        dl[(long long)w * HEAD_N + c] = f2bf(d);
+    float mine = 0.f;
+    if (w < B) {
+        const float* z = logits + (long long)w * HEAD_N;
+        float v[10], mx = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < 10; i++) {
+            const int c = lane + 32 * i;
+            v[i] = c < NCLS ? z[c] : -INFINITY;
+            mx = fmaxf(mx, v[i]);
+        }
+        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const int label = min(max(int(labels[w]), 0), NCLS - 1);
+        const float zl = z[label];
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < 10; i++) {
+            v[i] = lane + 32 * i < NCLS ? expf(v[i] - mx) : 0.f;
+            s += v[i];
+        }
+        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const float inv = 1.f / s, scale = 1.f / float(B);
+#pragma unroll
+        for (int i = 0; i < 10; i++) {
+            const int c = lane + 32 * i;
+            if (c < HEAD_N) dl[(long long)w * HEAD_N + c] = f2bf(c < NCLS ? (v[i] * inv - (c == label ? 1.f : 0.f)) * scale : 0.f);
+        }
+        mine = (logf(s) + mx - zl) * scale;
     }
-    if (lane == 0) atomicAdd(loss, (logf(s) + mx - z[label]) * scale);
+    if (lane == 0) part[threadIdx.x >> 5] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float t = 0.f;
+        for (int i = 0; i < int(blockDim.x >> 5); i++) t += part[i];
+        atomicAdd(loss, t);
+    }
 }
 
 // One warp per sample: the 8 largest logits (ties to the lower class) as
@@ -766,30 +866,36 @@ __global__ void guide_frames_kernel(const PropFrame* __restrict__ fr, int P, int
 }
 
 template <int BN, class Op>
-static void gemm(const Op& op, int M, int N, int K, cudaStream_t st, int splits = 1) {
+static void gemm(const Op& op, int M, int N, int K, cudaStream_t st) {
     constexpr int smem = 2 * (TC_BM * TC_BK * 2 + BN * TC_BK * 2);
     static const bool attr_ok = [] {  // once per instantiation (the dynamic shared memory above 48 KB)
         return cudaFuncSetAttribute(gemm_tc_kernel<BN, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
                cudaSuccess;
     }();
     (void)attr_ok;
-    int kchunk = K;
-    if (splits > 1) {
-        kchunk = (K + splits - 1) / splits;
-        kchunk = (kchunk + TC_BK - 1) / TC_BK * TC_BK;
-        splits = (K + kchunk - 1) / kchunk;
-    }
-    dim3 grid((M + TC_BM - 1) / TC_BM, (N + BN - 1) / BN, splits);
-    gemm_tc_kernel<BN, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, kchunk, nullptr);
+    dim3 grid((M + TC_BM - 1) / TC_BM, (N + BN - 1) / BN);
+    gemm_tc_kernel<BN, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, nullptr);
 }
 
-// split count of a weight-gradient GEMM: about 4 waves of CTAs
-static int wsplits(int M, int N, int BN, long long K, int sms) {
-    const long long tiles = (long long)((M + TC_BM - 1) / TC_BM) * ((N + BN - 1) / BN);
-    long long s = (4LL * sms + tiles - 1) / tiles;
-    const long long maxs = (K + 1023) / 1024;  // at least 1024 rows per CTA
-    if (s > maxs) s = maxs;
-    return int(s < 1 ? 1 : s);
+// Weight-gradient GEMM: K split over about two CTAs per SM (what its shared
+// and tensor memory hold), at least four steps each.
+template <int BN, int KS, int AQ, class Op>
+static void wgrad(const Op& op, int M, int N, int K, int sms, cudaStream_t st) {
+    constexpr int GR = TC_THREADS / KS, BLK = KS * 16, A_BYTES = AQ * GR * BLK, STAGE = A_BYTES + (BN / 8) * BLK;
+    // the MMA reads 16 blocks of A whatever there are: 16 * BLK from the last stage's start
+    constexpr int smem = STAGE + (STAGE > 16 * BLK ? STAGE : 16 * BLK);
+    static const bool attr_ok = [] {
+        return cudaFuncSetAttribute(wgrad_tc_kernel<BN, KS, AQ, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
+               cudaSuccess;
+    }();
+    (void)attr_ok;
+    const int tiles = ((M + TC_BM - 1) / TC_BM) * ((N + BN - 1) / BN);
+    int splits = (2 * sms + tiles - 1) / tiles;
+    splits = std::max(1, std::min(splits, (K + 4 * KS - 1) / (4 * KS)));
+    int kchunk = (K + splits - 1) / splits;
+    kchunk = (kchunk + KS - 1) / KS * KS;
+    dim3 grid((M + TC_BM - 1) / TC_BM, (N + BN - 1) / BN, (K + kchunk - 1) / kchunk);
+    wgrad_tc_kernel<BN, KS, AQ, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, kchunk, nullptr);
 }
 
 }  // namespace mvnet
@@ -810,6 +916,7 @@ struct h264a_mvnet {
     // maps, activations and gradients of one batch
     bf16_t *a1 = nullptr, *a2 = nullptr, *a3 = nullptr, *h = nullptr, *dl = nullptr, *dh = nullptr, *df = nullptr;
     bf16_t *da3 = nullptr, *da2 = nullptr, *da1 = nullptr;
+    bf16_t *wprep = nullptr;  // the weights as the data gradients read them
     float* logits = nullptr;
     float* loss = nullptr;
     // inference: the batch's pair table and neighbour features
@@ -831,7 +938,7 @@ int dmalloc(T** p, size_t n) {
 
 void free_net(h264a_mvnet* n) {
     void* ps[] = {n->master, n->w, n->grad, n->m1, n->m2, n->a1, n->a2, n->a3, n->h, n->dl, n->dh, n->df,
-                  n->da3, n->da2, n->da1, n->logits, n->loss, n->ipairs, n->inmv, n->iprop};
+                  n->da3, n->da2, n->da1, n->wprep, n->logits, n->loss, n->ipairs, n->inmv, n->iprop};
     for (void* p : ps)
         if (p) cudaFree(p);
     delete n;
@@ -882,6 +989,10 @@ Bufs bufs(h264a_mvnet* n) {
     z.w = n->w; z.grad = n->grad;
     z.a1 = n->a1; z.a2 = n->a2; z.a3 = n->a3; z.h = n->h; z.dl = n->dl; z.dh = n->dh; z.df = n->df;
     z.da3 = n->da3; z.da2 = n->da2; z.da1 = n->da1;
+    z.w4t = n->wprep;
+    z.w5t = z.w4t + N_W4T;
+    z.wd3 = z.w5t + N_W5T;
+    z.wd2 = z.wd3 + N_WD3;
     z.logits = n->logits;
     return z;
 }
@@ -911,8 +1022,9 @@ void trunk_forward(h264a_mvnet* n, const Geo& g, cudaStream_t st) {
     gemm<32>(Conv3Fwd{g, z}, g.P * g.H3 * g.W3, 32, 288, st);
 }
 
-void head_forward(h264a_mvnet* n, const Geo& g, cudaStream_t st) {
-    const Bufs z = bufs(n);
+void head_forward(h264a_mvnet* n, const Geo& g, float* logits, cudaStream_t st) {
+    Bufs z = bufs(n);
+    z.logits = logits;
     const int B = g.P * g.nmb;
     gemm<256>(Fc1Fwd{g, z}, B, HID, FEAT, st);
     gemm<160>(HeadFwd{z}, B, HEAD_N, HID, st);
@@ -922,17 +1034,18 @@ void backward(h264a_mvnet* n, const Geo& g, cudaStream_t st) {
     const Bufs z = bufs(n);
     const int B = g.P * g.nmb, S = n->sms;
     const int K3 = g.P * g.H3 * g.W3, K2 = g.P * g.H2 * g.W2, K1 = g.P * g.H1 * g.W1;
-    gemm<160>(HeadBwdW{z, B}, HEAD_N, HID + 2, B, st, wsplits(HEAD_N, HID + 2, 160, B, S));
+    prep_kernel<<<(N_PREP + 255) / 256, 256, 0, st>>>(n->w, n->wprep);
+    wgrad<256, 64, 4>(HeadBwdW{z}, HEAD_N, HID, B, S, st);
     gemm<256>(HeadBwdData{z}, B, HID, HEAD_N, st);
-    gemm<256>(Fc1BwdW{g, z, B}, HID, FEAT + 2, B, st, wsplits(HID, FEAT + 2, 256, B, S));
-    gemm<256>(Fc1BwdData{z}, B, CONVF, HID, st);
-    const long long cells = (long long)K3 * 16;
+    wgrad<256, 64, 4>(Fc1BwdW{g, z}, HID, FEAT, B, S, st);
+    gemm<192>(Fc1BwdData{z}, B, CONVF, HID, st);
+    const long long cells = (long long)K3 * 4;
     uncrop_kernel<<<unsigned((cells + 255) / 256), 256, 0, st>>>(g, n->df, n->a3, n->da3);
-    gemm<160>(Conv3BwdW{g, z, K3}, 32, 9 * 32 + 2, K3, st, wsplits(32, 290, 160, K3, S));
-    gemm<32>(Conv3BwdData{g, z}, K2, 32, 288, st);
-    gemm<160>(Conv2BwdW{g, z, K2}, 32, 9 * 16 + 2, K2, st, wsplits(32, 146, 160, K2, S));
-    gemm<16>(Conv2BwdData{g, z}, K1, 16, 288, st);
-    gemm<32>(Conv1BwdW{g, z, K1}, 16, 9 * 2 + 2, K1, st, wsplits(16, 20, 32, K1, S));
+    wgrad<144, 64, 1>(Conv3BwdW{g, z}, 32, 288, K3, S, st);
+    gemm<128>(ConvBwdData<32, 3>{g, z}, K3, 128, 128, st);
+    wgrad<144, 128, 2>(Conv2BwdW{g, z}, 32, 144, K2, S, st);
+    gemm<64>(ConvBwdData<16, 2>{g, z}, K2, 64, 128, st);
+    wgrad<32, 128, 1>(Conv1BwdW{g, z}, 16, 24, K1, S, st);
 }
 
 }  // namespace
@@ -961,6 +1074,7 @@ extern "C" int h264a_mvnet_create(int device, uint64_t seed, h264a_mvnet** out) 
     if (!rc) rc = dmalloc(&n->dl, size_t(MAXS * HEAD_N));
     if (!rc) rc = dmalloc(&n->df, size_t(MAXS * CONVF));
     if (!rc) rc = dmalloc(&n->logits, size_t(MAXS * HEAD_N));
+    if (!rc) rc = dmalloc(&n->wprep, size_t(N_PREP));
     if (!rc) rc = dmalloc(&n->loss, 1);
     if (!rc) rc = dmalloc(&n->inmv, size_t(MAXS * 6));
     if (!rc) rc = dmalloc(&n->ipairs, size_t(MAXPIX / 256));
@@ -1016,8 +1130,10 @@ extern "C" int h264a_mvnet_forward(h264a_mvnet* n, const h264a_mvnet_pair* d_pai
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const Geo g = make_geo(d_pairs, npairs, cw, ch, d_nmv, nullptr);
     trunk_forward(n, g, st);
-    head_forward(n, g, st);
-    if (d_logits)
+    // straight into the caller's buffer when the epilogue's 16-byte stores can
+    const bool direct = d_logits != nullptr && (reinterpret_cast<uintptr_t>(d_logits) & 15) == 0;
+    head_forward(n, g, direct ? d_logits : n->logits, st);
+    if (d_logits && !direct)
         H264A_CUDA(cudaMemcpyAsync(d_logits, n->logits, sizeof(float) * HEAD_N * npairs * g.nmb,
                                    cudaMemcpyDeviceToDevice, st));
     return check_launch("mvnet forward");
@@ -1035,7 +1151,7 @@ extern "C" int h264a_mvnet_grads(h264a_mvnet* n, const h264a_mvnet_pair* d_pairs
     H264A_CUDA(cudaMemsetAsync(n->grad, 0, sizeof(float) * NPARAMS, st));
     H264A_CUDA(cudaMemsetAsync(n->loss, 0, sizeof(float), st));
     trunk_forward(n, g, st);
-    head_forward(n, g, st);
+    head_forward(n, g, n->logits, st);
     loss_kernel<<<(B * 32 + 255) / 256, 256, 0, st>>>(n->logits, d_labels, B, n->dl, n->loss);
     backward(n, g, st);
     if (d_grads) H264A_CUDA(cudaMemcpyAsync(d_grads, n->grad, sizeof(float) * NPARAMS, cudaMemcpyDeviceToDevice, st));
@@ -1096,7 +1212,7 @@ extern "C" int h264a_mvnet_propose(h264a_mvnet* n, const h264a_mvnet_frame* h_fr
         const long long samples = (long long)P * g.nmb;
         guide_frames_kernel<<<unsigned((samples + 255) / 256), 256, 0, st>>>(n->iprop, P, g.mb_w, g.mb_h, n->inmv);
         trunk_forward(n, g, st);
-        head_forward(n, g, st);
+        head_forward(n, g, n->logits, st);
         top8_frames_kernel<<<unsigned((samples * 32 + 255) / 256), 256, 0, st>>>(n->logits, P, g.nmb, n->iprop);
         i = j;
     }
