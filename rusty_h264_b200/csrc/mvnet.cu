@@ -53,7 +53,14 @@ constexpr int O_W5 = O_B4 + HID, N_W5 = HEAD_N * HID;
 constexpr int O_B5 = O_W5 + N_W5;
 constexpr int NPARAMS = O_B5 + HEAD_N;
 static_assert(NPARAMS == H264A_MVNET_NPARAMS, "parameter count");
-static_assert((O_W1 | O_W2 | O_W3 | O_W4 | O_W5) % 2 == 0, "weights start on bf16 pairs");
+static_assert((O_W1 | O_W2 | O_W3 | O_W4 | O_W5 | O_B2 | O_B3 | O_B4 | O_B5) % 8 == 0, "16-byte weight and bias chunks");
+
+// The GEMMs' weights lie WREP times in memory, CTA x reading copy x % WREP:
+// every CTA of a layer reads the same few hundred lines at nearly the same
+// time, and one copy's lines sit in few of the L2's slices.  conv2 on four
+// 1080p pairs: 100 us from one copy, 69 from three, 66 from eight; conv3's
+// data gradient 45, 39 and 37.
+constexpr int WREP = 8, WSTRIDE = (NPARAMS + 7) / 8 * 8;
 
 typedef uint16_t bf16_t;  // raw bf16 bits
 
@@ -66,15 +73,28 @@ __device__ __forceinline__ float bf2f(bf16_t b) { return __uint_as_float(uint32_
 __device__ __forceinline__ uint32_t pack2(bf16_t lo, bf16_t hi) { return uint32_t(lo) | (uint32_t(hi) << 16); }
 __device__ __forceinline__ uint32_t ld_pair(const bf16_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
 __device__ __forceinline__ uint4 ld8(const bf16_t* p) { return *reinterpret_cast<const uint4*>(p); }
-// 8 values (bias added, ReLU) rounded to bf16 and stored as one 16-byte word
-__device__ __forceinline__ void st8_relu(bf16_t* dst, const float* v, const bf16_t* bias) {
-    uint32_t w[4];
+__device__ __forceinline__ void st8(bf16_t* p, const uint4& v) { *reinterpret_cast<uint4*>(p) = v; }
+// 8 bf16 values as floats
+__device__ __forceinline__ void unpack8(const uint4& w, float* f) {
+    const uint32_t a[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-        w[i] = pack2(f2bf(fmaxf(v[2 * i] + bf2f(bias[2 * i]), 0.f)), f2bf(fmaxf(v[2 * i + 1] + bf2f(bias[2 * i + 1]), 0.f)));
-    *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    for (int i = 0; i < 4; i++) {
+        f[2 * i] = bf2f(bf16_t(a[i] & 0xffffu));
+        f[2 * i + 1] = bf2f(bf16_t(a[i] >> 16));
+    }
 }
-
+__device__ __forceinline__ uint4 pack8(const float* v) {  // rounded to bf16
+    return make_uint4(pack2(f2bf(v[0]), f2bf(v[1])), pack2(f2bf(v[2]), f2bf(v[3])), pack2(f2bf(v[4]), f2bf(v[5])),
+                      pack2(f2bf(v[6]), f2bf(v[7])));
+}
+// 8 values, bias added, ReLU
+__device__ __forceinline__ uint4 relu8(const float* v, const bf16_t* bias) {
+    float b[8], r[8];
+    unpack8(ld8(bias), b);
+#pragma unroll
+    for (int i = 0; i < 8; i++) r[i] = fmaxf(v[i] + b[i], 0.f);
+    return pack8(r);
+}
 // ---- a batch: frame pairs of one geometry, every MB a sample ---------------
 // Trunk maps (NHWC bf16): A1 (ch/2)x(cw/2)x16, A2 (ch/4)x(cw/4)x32, A3
 // (ch/8)x(cw/8)x32 per pair; samples are the pairs' MBs, pair-major, raster
@@ -88,14 +108,14 @@ struct Geo {
     const int16_t* labels;  // 1 per sample (training)
 };
 
-// X0 pair (reference, current) at pixel (iy, ix) of pair b; zero outside the
-// frame (the conv's padding).
-__device__ __forceinline__ uint32_t x0_pair(const Geo& g, int b, int iy, int ix) {
-    if (iy < 0 || iy >= g.ch || ix < 0 || ix >= g.cw) return 0u;
-    const h264a_mvnet_pair p = g.pairs[b];
-    const long long o = (long long)iy * g.cw + ix;
-    const float r = (float(p.d_ref[o]) - 128.f) * (1.f / 64.f), c = (float(p.d_cur[o]) - 128.f) * (1.f / 64.f);
-    return pack2(f2bf(r), f2bf(c));  // exact: k/64 with |k| <= 128
+// The bf16 pair (reference, current) of two pixels, (v - 128) / 64 each: k/64
+// with |k| <= 128, so float and bf16 hold it exactly and its upper half is the
+// bf16.  The byte is the mantissa of 2^23 + v; the multiply-add takes 2^23 / 64
+// + 2 away again.
+__device__ __forceinline__ uint32_t x0_word(uint32_t r, uint32_t c) {
+    const float a = fmaf(__uint_as_float(0x4b000000u | r), 1.f / 64.f, -131074.f);
+    const float b = fmaf(__uint_as_float(0x4b000000u | c), 1.f / 64.f, -131074.f);
+    return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 __device__ __forceinline__ bf16_t mv_feat(const Geo& g, int m, int i) {
     const int v = min(max(int(g.nmv[6LL * m + i]), -128), 128);
@@ -103,19 +123,26 @@ __device__ __forceinline__ bf16_t mv_feat(const Geo& g, int m, int i) {
 }
 
 // ---- the tcgen05 GEMM: 128 x BN tiles, accumulators in tensor memory --------
-// The GEMM of every forward layer and data gradient, C[M][N] = sum_k A[m][k]
-// B[k][n], on the sm_100 tensor cores: per 64-wide K step all 256 threads
-// gather the A (128 x 64) and B (BN x 64) tiles into one of two shared-memory
-// stages, one thread issues four tcgen05.mma (M 128, N BN, K 16, bf16 in, fp32
-// accumulated in tensor memory) and commits them to the stage's mbarrier, and
-// the gathers of the next step overlap them.  The epilogue reads the accumulator rows with
-// tcgen05.ld: warp w may read tensor-memory lanes 32(w % 4) .. +31 (its tile
-// rows), warps w and w + 4 taking half of the columns each.
+// The GEMM of conv2 to the head and of every data gradient, C[M][N] = sum_k
+// A[m][k] B[k][n], on the sm_100 tensor cores: per 64-wide K step all 256
+// threads copy the A (MT x 128 x 64) and B (BN x 64) tiles by 16-byte cp.async
+// into one of ST shared-memory stages (steps it + 1 .. it + ST - 1 are in flight
+// while step it multiplies), one thread issues four tcgen05.mma (M 128, N BN,
+// K 16, bf16 in, fp32 accumulated in tensor memory) and commits them to the
+// stage's mbarrier.  The epilogue reads the accumulator rows with tcgen05.ld
+// (warp w may read tensor-memory lanes 32(w % 4) .. +31, its tile rows; warps w
+// and w + 4 take half of the columns each), puts the packed results where the
+// stages were and writes whole rows from there: stored row by row from the
+// registers, 32 rows a request, it took longer than the products (head 27,000
+// of a CTA's 45,000 cycles).  Bound by the operands' way through the L2 (five
+// or so TB/s over both dies).  Four 1080p pairs, before (operands through
+// registers) and now: FC1 85 -> 61 us, head 48 -> 32, conv3 36 -> 30, data
+// gradients of conv3 51 -> 37, FC1 128 -> 89.
 constexpr int TC_BM = 128, TC_BK = 64, TC_THREADS = 256;
 
 template <int BN>
 constexpr int tc_cols() {
-    return BN <= 32 ? 32 : (BN <= 64 ? 64 : (BN <= 128 ? 128 : 256));
+    return BN <= 32 ? 32 : (BN <= 64 ? 64 : (BN <= 128 ? 128 : (BN <= 256 ? 256 : 512)));
 }
 
 // A K-major operand tile of R rows x 64 k (bf16) in the canonical
@@ -154,25 +181,77 @@ __device__ __forceinline__ void tc_wait(uint32_t bar, uint32_t parity, int* stat
     }
 }
 
-// An Op gathers 8 consecutive k at once (op.a8(row, k), op.b8(k, n): 16 bytes,
-// k a multiple of 8, zero past its tensor) and stores 8 consecutive n
-// (op.store8(row, m, n, v)).  Its `Row` is what its gathers need of output row
-// m (sample, position, base offset), made once per CTA row by op.row(m), so
-// the per-chunk gathers divide by no runtime size.  K and N are multiples of 8.
-template <int BN, class Op>
+// 16 accumulator columns of the lane's row
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, float* f) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; i++) f[i] = __uint_as_float(r[i]);
+}
+// 16 bytes global -> shared, zeros where not ok (`any`: an address to name then)
+__device__ __forceinline__ void cp16z(uint32_t dst, const bf16_t* p, bool ok, const bf16_t* any) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(ok ? p : any), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void st16s(uint32_t dst, const uint4& v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+__device__ __forceinline__ uint4 ld16s(uint32_t src) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src) : "memory");
+    return v;
+}
+
+// An Op names the 16 bytes of 8 consecutive k of A as op.a8(row, step, p):
+// their address in p, false for zeros.  Row is what output row m gives
+// (op.row(m): base address, position) and Step what chunk k gives (op.step(k),
+// k a multiple of 8: offset, window cell).  A thread of the GEMM below keeps
+// its rows and makes one Step per K step, one of the weight gradients its
+// Steps and one row per K step, so a copy costs an add and two compares.
+// Where kCalc, op.calc(step) chunks are op.make(row, step) instead.  B is
+// op.b(copy) with op.ldb columns per row n.  op.pack(n, v) makes 8 results
+// (n ..) the 16 bytes (32 where kF32) that op.store(o, n, w) puts at n .. of a
+// row with output offset o = op.out_at(m).  K and N are multiples of 8.
+template <class Op>
+__device__ __forceinline__ void stage_a8(const Op& op, uint32_t dst, const typename Op::Row& row, const typename Op::Step& s,
+                                         bool live) {
+    if constexpr (Op::kCalc) {
+        if (live && op.calc(s)) {
+            st16s(dst, op.make(row, s));
+            return;
+        }
+    }
+    const bf16_t* p = op.z.w;
+    live = op.a8(row, s, p) && live;
+    cp16z(dst, p, live, op.z.w);
+}
+
+template <int BN, int MT, int ST, class Op>
 __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const Op op, int M, int N, int K, int* status) {
-    static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "tcgen05 N for M = 128");
-    constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2, STAGE = A_BYTES + B_BYTES;
-    constexpr int NCOL = tc_cols<BN>();
+    static_assert(BN % 32 == 0 && BN <= 256 && ST >= 2, "tcgen05 N for M = 128, halves of 16 columns");
+    constexpr int ROWS = MT * TC_BM, A_TILE = TC_BM * TC_BK * 2, A_BYTES = MT * A_TILE, STAGE = A_BYTES + BN * TC_BK * 2;
+    constexpr int NCOL = tc_cols<BN * MT>();
     constexpr uint32_t IDESC = tc_idesc<BN>();
     extern __shared__ __align__(128) uint8_t tc_smem[];
-    __shared__ __align__(8) unsigned long long tc_bar[2];
+    __shared__ __align__(8) unsigned long long tc_bar[ST];
     __shared__ uint32_t tc_tmem;
-    __shared__ typename Op::Row tc_rows[TC_BM];
+    __shared__ typename Op::Row tc_rows[ROWS];
+    __shared__ long long tc_out[ROWS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * TC_BM, n0 = blockIdx.y * BN;
-    for (int i = tid; i < TC_BM; i += TC_THREADS) tc_rows[i] = op.row(min(m0 + i, M - 1));  // read after the __syncthreads below
-    const int kb = 0, ke = K;
+    const int m0 = blockIdx.x * ROWS, n0 = blockIdx.y * BN;
+    // read after the __syncthreads below; rows past M repeat the last and are not stored
+    for (int i = tid; i < 2 * ROWS; i += TC_THREADS) {
+        const int m = min(m0 + i % ROWS, M - 1);
+        if (i < ROWS)
+            tc_rows[i] = op.row(m);
+        else
+            tc_out[i - ROWS] = op.out_at(m);
+    }
     const uint32_t sbase = tc_smem_u32(tc_smem), bar0 = tc_smem_u32(&tc_bar[0]);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(&tc_tmem)),
@@ -180,56 +259,44 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const Op op, int M,
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        mbar_init(bar0, 1);
-        mbar_init(bar0 + 8, 1);
+#pragma unroll
+        for (int s = 0; s < ST; s++) mbar_init(bar0 + 8 * s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tc_tmem;
-    const int nk = ke > kb ? (ke - kb + TC_BK - 1) / TC_BK : 0;
+    const int nk = (K + TC_BK - 1) / TC_BK;
+    // consecutive threads fill consecutive 16-byte rows of a core matrix, so
+    // a warp's stores meet no bank twice; a thread keeps one chunk column and
+    // every 32nd row
+    constexpr int AQ = ROWS * 8 / TC_THREADS, BQ = BN * 8 / TC_THREADS;
+    static_assert(AQ * TC_THREADS == ROWS * 8 && BQ * TC_THREADS == BN * 8, "whole passes");
+    const int c = (tid >> 3) & 7, r0 = ((tid >> 6) << 3) | (tid & 7);
+    typename Op::Row rows[AQ];
+#pragma unroll
+    for (int j = 0; j < AQ; j++) rows[j] = tc_rows[r0 + 32 * j];
+    const bf16_t* bp = op.b(blockIdx.x % WREP) + (long long)(n0 + r0) * Op::ldb + 8 * c;
+    const uint32_t off0 = tc_off(r0, c);
+    auto load = [&](int it) {
+        const uint32_t sa = sbase + uint32_t((it % ST) * STAGE) + off0, sb = sa + A_BYTES;
+        const bool kin = it * TC_BK + 8 * c < K;
+        const typename Op::Step s = op.step(it * TC_BK + 8 * c);
+#pragma unroll
+        for (int j = 0; j < AQ; j++) stage_a8(op, sa + 4096u * j, rows[j], s, kin);
+#pragma unroll
+        for (int j = 0; j < BQ; j++)
+            cp16z(sb + 4096u * j, bp + it * TC_BK + 32 * j * Op::ldb, kin && n0 + r0 + 32 * j < N, op.z.w);
+    };
+#pragma unroll
+    for (int s = 0; s < ST - 1; s++) {
+        if (s < nk) load(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
     for (int it = 0; it < nk; it++) {
-        const int st = it & 1;
-        const int k0 = kb + it * TC_BK;
-        const uint32_t sa = sbase + uint32_t(st * STAGE), sb = sa + A_BYTES;
-        // consecutive threads fill consecutive 16-byte rows of a core
-        // matrix, so a warp's stores meet no bank twice
-        {
-            // the step's gathers are issued before waiting for the stage, so
-            // they overlap the MMAs still reading it
-            constexpr int AQ = TC_BM * 8 / TC_THREADS, BQ = (BN * 8 + TC_THREADS - 1) / TC_THREADS;
-            uint4 va[AQ], vb[BQ];
-#pragma unroll
-            for (int j = 0; j < AQ; j++) {
-                const int q = tid + j * TC_THREADS;
-                const int row = ((q >> 6) << 3) | (q & 7), c = (q >> 3) & 7, m = m0 + row, k = k0 + 8 * c;
-                va[j] = (m < M && k < ke) ? op.a8(tc_rows[row], k) : make_uint4(0u, 0u, 0u, 0u);
-            }
-#pragma unroll
-            for (int j = 0; j < BQ; j++) {
-                const int q = tid + j * TC_THREADS;
-                const int row = ((q >> 6) << 3) | (q & 7), c = (q >> 3) & 7, n = n0 + row, k = k0 + 8 * c;
-                vb[j] = (q < BN * 8 && n < N && k < ke) ? op.b8(k, n) : make_uint4(0u, 0u, 0u, 0u);
-            }
-            // the stage's previous MMAs (step it - 2) have read it
-            if (it >= 2) tc_wait(bar0 + 8 * st, uint32_t((it - 2) >> 1) & 1u, status);
-#pragma unroll
-            for (int j = 0; j < AQ; j++) {
-                const int q = tid + j * TC_THREADS, row = ((q >> 6) << 3) | (q & 7), c = (q >> 3) & 7;
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sa + tc_off(row, c)), "r"(va[j].x),
-                             "r"(va[j].y), "r"(va[j].z), "r"(va[j].w)
-                             : "memory");
-            }
-#pragma unroll
-            for (int j = 0; j < BQ; j++) {
-                const int q = tid + j * TC_THREADS, row = ((q >> 6) << 3) | (q & 7), c = (q >> 3) & 7;
-                if (q < BN * 8)
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sb + tc_off(row, c)), "r"(vb[j].x),
-                                 "r"(vb[j].y), "r"(vb[j].z), "r"(vb[j].w)
-                                 : "memory");
-            }
-        }
+        const uint32_t sa = sbase + uint32_t((it % ST) * STAGE), sb = sa + A_BYTES;
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
         // the tiles' generic-proxy writes, visible to the tensor cores
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
@@ -237,40 +304,60 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const Op op, int M,
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int j = 0; j < TC_BK / 16; j++) {
-                const uint64_t da = tc_sdesc(sa + 256u * j), db = tc_sdesc(sb + 256u * j);
+                const uint64_t db = tc_sdesc(sb + 256u * j);
                 const uint32_t acc = (it > 0 || j > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem),
-                    "l"(da), "l"(db), "r"(IDESC), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-                    : "memory");
+#pragma unroll
+                for (int t = 0; t < MT; t++)
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem + uint32_t(t * BN)),
+                        "l"(tc_sdesc(sa + uint32_t(t * A_TILE) + 256u * j)), "l"(db), "r"(IDESC), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+                        : "memory");
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar0 +
-                                                                                                          8 * st)
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar0 + 8 * (it % ST))
                          : "memory");
         }
+        if (it + ST - 1 < nk) {
+            // the stage's previous MMAs (step it - 1) have read it
+            if (it >= 1) tc_wait(bar0 + 8 * ((it - 1) % ST), uint32_t((it - 1) / ST) & 1u, status);
+            load(it + ST - 1);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    if (nk > 0) {
-        // the last step's commit completes after every earlier MMA
-        tc_wait(bar0 + 8 * ((nk - 1) & 1), uint32_t((nk - 1) >> 1) & 1u, status);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int row = m0 + (warp & 3) * 32 + lane;
-        const uint32_t taddr = tmem + (uint32_t((warp & 3) * 32) << 16);
+    // the last step's commit completes after every earlier MMA
+    tc_wait(bar0 + 8 * ((nk - 1) % ST), uint32_t((nk - 1) / ST) & 1u, status);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    {
+        constexpr int ES = Op::kF32 ? 4 : 2, PITCH = BN * ES + 16, CH = BN * ES / 16;
+        static_assert(MT * TC_BM * PITCH <= ST * STAGE, "the results take the stages' place");
         const int cb = (warp >> 2) * (BN / 2);
 #pragma unroll 1
-        for (int c0 = cb; c0 < cb + BN / 2; c0 += 8) {
-            uint32_t r[8];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                           "=r"(r[7])
-                         : "r"(taddr + uint32_t(c0)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row < M && n0 + c0 < N) {
-                float f[8];
+        for (int t = 0; t < MT; t++) {
+            const uint32_t so = sbase + uint32_t((t * TC_BM + (warp & 3) * 32 + lane) * PITCH);
+            const uint32_t taddr = tmem + uint32_t(t * BN) + (uint32_t((warp & 3) * 32) << 16);
+#pragma unroll 1
+            for (int c0 = cb; c0 < cb + BN / 2; c0 += 16) {
+                float f[16];
+                tc_ld16(taddr + uint32_t(c0), f);
 #pragma unroll
-                for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[i]);
-                op.store8(tc_rows[row - m0], row, n0 + c0, f);
+                for (int h = 0; h < 2; h++) {
+                    const int n = min(n0 + c0 + 8 * h, N - 8);  // columns past N are not stored
+                    if constexpr (Op::kF32) {
+                        uint4 w[2];
+                        op.pack(n, f + 8 * h, w);
+                        st16s(so + uint32_t(c0 + 8 * h) * 4, w[0]);
+                        st16s(so + uint32_t(c0 + 8 * h) * 4 + 16, w[1]);
+                    } else {
+                        st16s(so + uint32_t(c0 + 8 * h) * 2, op.pack(n, f + 8 * h));
+                    }
+                }
             }
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int i = tid; i < ROWS * CH; i += TC_THREADS) {
+            const int row = i / CH, ch = i - row * CH, n = n0 + ch * (16 / ES);
+            if (m0 + row < M && n < N) op.store(tc_out[row], n, ld16s(sbase + uint32_t(row * PITCH + ch * 16)));
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -287,107 +374,234 @@ struct Bufs {
     float* logits;
 };
 
-// conv1 forward: M = P*H1*W1, N = 16, K = 18 (padded to 32)
-struct Conv1Fwd {
-    Geo g; Bufs z;
-    __device__ uint32_t b(int k, int n) const { return k < 18 ? ld_pair(z.w + O_W1 + n * 18 + k) : 0u; }
-    struct Row {
-        int b, y0, x0;  // pair, top-left input pixel of the 3x3 window
-    };
-    __device__ Row row(int m) const {
-        const int OHW = g.H1 * g.W1;
-        const int b = m / OHW, r = m - b * OHW, oy = r / g.W1, ox = r - oy * g.W1;
-        return Row{b, 2 * oy - 1, 2 * ox - 1};
-    }
-    __device__ uint4 a8(const Row& w, int k) const {
-        uint32_t v[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int tap = (k >> 1) + i, ky = (tap * 11) >> 5, kx = tap - ky * 3;  // ky = tap / 3 for tap < 9
-            v[i] = tap < 9 ? x0_pair(g, w.b, w.y0 + ky, w.x0 + kx) : 0u;
-        }
-        return make_uint4(v[0], v[1], v[2], v[3]);
-    }
-    __device__ uint4 b8(int k, int n) const {
-        uint32_t v[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = b(k + 2 * i, n);
-        return make_uint4(v[0], v[1], v[2], v[3]);
-    }
-    __device__ void store8(const Row&, int m, int n, const float* v) const { st8_relu(z.a1 + (long long)m * 16 + n, v, z.w + O_B1 + n); }
+// conv1's window of output position m: the pair's planes at its top-left pixel
+// (oy = 0 and ox = 0 reach one row and column outside the frame)
+struct Conv1Row {
+    const uint8_t *r, *c;
+    bool top, left;  // the window's first row / column lies outside
 };
-// conv2 / conv3 forward: im2col of the previous map
+__device__ __forceinline__ Conv1Row conv1_row(const Geo& g, int m) {
+    const int OHW = g.H1 * g.W1;
+    const int b = m / OHW, q = m - b * OHW, oy = q / g.W1, ox = q - oy * g.W1;
+    const h264a_mvnet_pair p = g.pairs[b];
+    const long long o = (long long)(2 * oy - 1) * g.cw + 2 * ox - 1;
+    return Conv1Row{p.d_ref + o, p.d_cur + o, oy == 0, ox == 0};
+}
+// the input pair of tap (ky, kx), zero outside the frame (the conv's padding)
+__device__ __forceinline__ uint32_t conv1_tap(const Conv1Row& w, int cw, int ky, int kx) {
+    if ((w.top && ky == 0) || (w.left && kx == 0)) return 0u;
+    const int o = ky * cw + kx;
+    return x0_word(w.r[o], w.c[o]);
+}
+
+// conv1 forward: M = P*H1*W1, N = 16, K = 18 in two K 16 steps (the rest
+// zeros).  Persistent: a thread gathers its row's nine taps (18 byte loads)
+// into the 128 x 32 A tile while the tensor core multiplies the tile before.
+// Bound by those loads' issue; 64-wide K steps of generic gathers, a CTA per
+// tile, took 165 us on four 1080p pairs, this 38.
+constexpr int C1_CTAS = 8;  // per SM
+__global__ void __launch_bounds__(128, C1_CTAS) conv1_kernel(const Geo g, const Bufs z, int M, int* status) {
+    constexpr int STAGE = 128 * 64;  // bytes: 16 row groups x 4 k-chunks x 128
+    constexpr uint64_t DESC_HI = (uint64_t(128 >> 4) << 16) | (uint64_t(512 >> 4) << 32) | (1ull << 46);
+    __shared__ __align__(128) uint8_t smem[2 * STAGE + 16 * 64];
+    __shared__ __align__(8) unsigned long long bar[2];
+    __shared__ uint32_t tmem_s;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const uint32_t sbase = tc_smem_u32(smem), sw = sbase + 2 * STAGE, bar0 = tc_smem_u32(bar);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(&tmem_s)), "r"(32));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        mbar_init(bar0, 1);
+        mbar_init(bar0 + 8, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // element offset of (row, k-chunk) of a 32-wide tile, in bytes
+    auto off = [](int row, int chunk) { return uint32_t(((row >> 3) * 4 + chunk) * 128 + (row & 7) * 16); };
+    if (tid < 64) {  // weights: 16 rows of 18, zero to 32
+        const int n = tid >> 2, ch = tid & 3;
+        uint32_t v[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = 8 * ch + 2 * i < 18 ? ld_pair(z.w + O_W1 + n * 18 + 8 * ch + 2 * i) : 0u;
+        st16s(sw + off(n, ch), make_uint4(v[0], v[1], v[2], v[3]));
+    }
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    st16s(sbase + off(tid, 3), zero);  // k 24..31 of both stages
+    st16s(sbase + STAGE + off(tid, 3), zero);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_s;
+    float bias[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) bias[i] = bf2f(z.w[O_B1 + i]);
+    const int tiles = (M + 127) / 128;
+    int prev = -1, it = 0;  // the tile whose accumulators are to be read
+    for (int t = blockIdx.x;; t += gridDim.x, it++) {
+        const int st = it & 1;
+        if (t < tiles) {
+            const Conv1Row w = conv1_row(g, min(t * 128 + tid, M - 1));
+            uint32_t v[9];
+#pragma unroll
+            for (int k = 0; k < 9; k++) v[k] = conv1_tap(w, g.cw, k / 3, k % 3);
+            const uint32_t sa = sbase + uint32_t(st * STAGE);
+            st16s(sa + off(tid, 0), make_uint4(v[0], v[1], v[2], v[3]));
+            st16s(sa + off(tid, 1), make_uint4(v[4], v[5], v[6], v[7]));
+            st16s(sa + off(tid, 2), make_uint4(v[8], 0u, 0u, 0u));
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // the reads of tile it - 2's accumulators
+            __syncthreads();
+            if (tid == 0) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const uint64_t da = uint64_t(((sa + 256u * j) >> 4) & 0x3fffu) | DESC_HI;
+                    const uint64_t db = uint64_t(((sw + 256u * j) >> 4) & 0x3fffu) | DESC_HI;
+                    const uint32_t acc = j > 0 ? 1u : 0u;
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem + 16u * st),
+                        "l"(da), "l"(db), "r"(tc_idesc<16>()), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+                        : "memory");
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar0 + 8 * st)
+                             : "memory");
+            }
+        }
+        if (prev >= 0) {
+            tc_wait(bar0 + 8 * (st ^ 1), uint32_t((it - 1) >> 1) & 1u, status);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            float f[16];
+            tc_ld16(tmem + 16u * (st ^ 1) + (uint32_t(warp * 32) << 16), f);
+            const int m = prev * 128 + tid;
+            if (m < M) {
+                uint32_t o[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    o[i] = pack2(f2bf(fmaxf(f[2 * i] + bias[2 * i], 0.f)), f2bf(fmaxf(f[2 * i + 1] + bias[2 * i + 1], 0.f)));
+                uint4* d = reinterpret_cast<uint4*>(z.a1 + (long long)m * 16);
+                d[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                d[1] = make_uint4(o[4], o[5], o[6], o[7]);
+            }
+        }
+        if (t >= tiles) break;
+        prev = t;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(32));
+}
+// A row of a window over an NHWC map: its top-left cell (which may lie outside)
+struct WinRow {
+    const bf16_t* p;
+    int y0, x0;
+};
+struct WinStep {
+    int off, dy, dx;  // element offset and cell of the chunk in the window
+};
+__device__ __forceinline__ bool win_a8(const WinRow& w, const WinStep& s, int H, int W, const bf16_t*& p) {
+    p = w.p + s.off;
+    return unsigned(w.y0 + s.dy) < unsigned(H) && unsigned(w.x0 + s.dx) < unsigned(W);
+}
+// A row of a plain matrix; its step is the column
+struct MatRow {
+    const bf16_t* p;
+};
+__device__ __forceinline__ bool mat_a8(const MatRow& w, int k, const bf16_t*& p) {
+    p = w.p + k;
+    return true;
+}
+
+// conv2 / conv3 forward: im2col of the previous map; a chunk is 8 channels of
+// one tap, 16 contiguous bytes
 template <int C, int OW, int OB, int WHICH>
 struct ConvFwd {
     Geo g; Bufs z;
-    // k a multiple of 8 (C = 16 or 32): the chunk is 8 channels of one tap,
-    // 16 contiguous bytes of the NHWC map
-    struct Row {
-        long long base;  // element offset of input pixel (y0, x0), channel 0 (may lie outside the map)
-        int y0, x0;
-    };
+    using Row = WinRow;
+    using Step = WinStep;
+    static constexpr bool kCalc = false;
+    static constexpr int ldb = 9 * C;
     __device__ Row row(int m) const {
         const int H = WHICH == 2 ? g.H1 : g.H2, W = WHICH == 2 ? g.W1 : g.W2;
         const int ow = W >> 1, ohw = (H >> 1) * ow;
         const int b = m / ohw, r = m - b * ohw, oy = r / ow, ox = r - oy * ow;
-        return Row{((long long)(b * H + 2 * oy - 1) * W + 2 * ox - 1) * C, 2 * oy - 1, 2 * ox - 1};
+        return Row{(WHICH == 2 ? z.a1 : z.a2) + ((long long)(b * H + 2 * oy - 1) * W + 2 * ox - 1) * C, 2 * oy - 1, 2 * ox - 1};
     }
-    __device__ uint4 a8(const Row& w, int k) const {
-        const int H = WHICH == 2 ? g.H1 : g.H2, W = WHICH == 2 ? g.W1 : g.W2;
-        const int tap = k / C, ci = k - tap * C, ky = (tap * 11) >> 5, kx = tap - ky * 3;
-        const int iy = w.y0 + ky, ix = w.x0 + kx;
-        if (iy < 0 || iy >= H || ix < 0 || ix >= W) return make_uint4(0u, 0u, 0u, 0u);
-        return ld8((WHICH == 2 ? z.a1 : z.a2) + w.base + (long long)(ky * W + kx) * C + ci);
+    __device__ Step step(int k) const {
+        const int tap = k / C, ci = k - tap * C, ky = (tap * 11) >> 5, kx = tap - ky * 3;  // ky = tap / 3 for tap < 16
+        return Step{(ky * (WHICH == 2 ? g.W1 : g.W2) + kx) * C + ci, ky, kx};
     }
-    __device__ uint4 b8(int k, int n) const { return ld8(z.w + OW + n * 9 * C + k); }
-    __device__ void store8(const Row&, int m, int n, const float* v) const {
-        st8_relu((WHICH == 2 ? z.a2 : z.a3) + (long long)m * 32 + n, v, z.w + OB + n);
+    __device__ bool a8(const Row& w, const Step& s, const bf16_t*& p) const {
+        return win_a8(w, s, WHICH == 2 ? g.H1 : g.H2, WHICH == 2 ? g.W1 : g.W2, p);
     }
+    __device__ const bf16_t* b(int copy) const { return z.w + OW + copy * WSTRIDE; }
+    __device__ long long out_at(int m) const { return (long long)m * 32; }
+    static constexpr bool kF32 = false;
+    __device__ uint4 pack(int n, const float* v) const { return relu8(v, z.w + OB + n); }
+    __device__ void store(long long o, int n, const uint4& w) const { st8((WHICH == 2 ? z.a2 : z.a3) + o + n, w); }
 };
 using Conv2Fwd = ConvFwd<16, O_W2, O_B2, 2>;
 using Conv3Fwd = ConvFwd<32, O_W3, O_B3, 3>;
 
+// FC1: k < 1152 are the channels of the MB's 6x6-cell crop of A3 (zero outside
+// the map), then the 6 neighbour-MV features (one chunk) and zeros
 struct Fc1Fwd {
     Geo g; Bufs z;
-    // k < 1152, a multiple of 8: 8 channels of one crop cell, 16 contiguous
-    // bytes of A3 (its MB's 6x6-cell crop, zero outside the map); then the 6
-    // neighbour-MV features and zeros
     struct Row {
-        long long base;  // element offset of the crop's top-left cell (y0, x0), channel 0
-        int m, y0, x0;
+        WinRow w;
+        int m;
     };
+    struct Step {
+        WinStep s;
+        int k;
+    };
+    static constexpr bool kCalc = true;
+    static constexpr int ldb = FEAT;
     __device__ Row row(int m) const {
         const int b = m / g.nmb, r = m - b * g.nmb, mby = r / g.mb_w, mbx = r - mby * g.mb_w;
         const int y0 = 2 * mby - 2, x0 = 2 * mbx - 2;
-        return Row{((long long)(b * g.H3 + y0) * g.W3 + x0) * 32, m, y0, x0};
+        return Row{WinRow{z.a3 + ((long long)(b * g.H3 + y0) * g.W3 + x0) * 32, y0, x0}, m};
     }
-    __device__ uint4 a8(const Row& w, int k) const {
-        if (k < CONVF) {
-            const int cy = k / 192, rem = k - cy * 192, cx = rem >> 5, c = rem & 31;
-            const int y = w.y0 + cy, x = w.x0 + cx;
-            if (y < 0 || y >= g.H3 || x < 0 || x >= g.W3) return make_uint4(0u, 0u, 0u, 0u);
-            return ld8(z.a3 + w.base + (long long)(cy * g.W3 + cx) * 32 + c);
-        }
-        if (k == CONVF)
-            return make_uint4(pack2(mv_feat(g, w.m, 0), mv_feat(g, w.m, 1)), pack2(mv_feat(g, w.m, 2), mv_feat(g, w.m, 3)),
-                              pack2(mv_feat(g, w.m, 4), mv_feat(g, w.m, 5)), 0u);
-        return make_uint4(0u, 0u, 0u, 0u);
+    __device__ Step step(int k) const {
+        const int cy = k / 192, rem = k - cy * 192, cx = rem >> 5;
+        return Step{WinStep{(cy * g.W3 + cx) * 32 + (rem & 31), cy, cx}, k};
     }
-    __device__ uint4 b8(int k, int n) const { return ld8(z.w + O_W4 + (long long)n * FEAT + k); }
-    __device__ void store8(const Row&, int m, int n, const float* v) const { st8_relu(z.h + (long long)m * HID + n, v, z.w + O_B4 + n); }
+    __device__ bool calc(const Step& s) const { return s.k == CONVF; }
+    __device__ uint4 make(const Row& w, const Step&) const {
+        return make_uint4(pack2(mv_feat(g, w.m, 0), mv_feat(g, w.m, 1)), pack2(mv_feat(g, w.m, 2), mv_feat(g, w.m, 3)),
+                          pack2(mv_feat(g, w.m, 4), mv_feat(g, w.m, 5)), 0u);
+    }
+    __device__ bool a8(const Row& w, const Step& s, const bf16_t*& p) const {
+        return win_a8(w.w, s.s, g.H3, g.W3, p) && s.k < CONVF;
+    }
+    __device__ const bf16_t* b(int copy) const { return z.w + O_W4 + copy * WSTRIDE; }
+    __device__ long long out_at(int m) const { return (long long)m * HID; }
+    static constexpr bool kF32 = false;
+    __device__ uint4 pack(int n, const float* v) const { return relu8(v, z.w + O_B4 + n); }
+    __device__ void store(long long o, int n, const uint4& w) const { st8(z.h + o + n, w); }
 };
 struct HeadFwd {
     Bufs z;
-    using Row = int;
-    __device__ Row row(int m) const { return m; }
-    __device__ uint4 a8(Row m, int k) const { return ld8(z.h + (long long)m * HID + k); }
-    __device__ uint4 b8(int k, int n) const { return ld8(z.w + O_W5 + n * HID + k); }
-    __device__ void store8(const Row&, int m, int n, const float* v) const {
-        float4* d = reinterpret_cast<float4*>(z.logits + (long long)m * HEAD_N + n);
-        const bf16_t* bias = z.w + O_B5 + n;
-        d[0] = make_float4(v[0] + bf2f(bias[0]), v[1] + bf2f(bias[1]), v[2] + bf2f(bias[2]), v[3] + bf2f(bias[3]));
-        d[1] = make_float4(v[4] + bf2f(bias[4]), v[5] + bf2f(bias[5]), v[6] + bf2f(bias[6]), v[7] + bf2f(bias[7]));
+    using Row = MatRow;
+    using Step = int;
+    static constexpr bool kCalc = false;
+    static constexpr int ldb = HID;
+    __device__ Row row(int m) const { return Row{z.h + (long long)m * HID}; }
+    __device__ Step step(int k) const { return k; }
+    __device__ bool a8(const Row& w, Step k, const bf16_t*& p) const { return mat_a8(w, k, p); }
+    __device__ const bf16_t* b(int copy) const { return z.w + O_W5 + copy * WSTRIDE; }
+    __device__ long long out_at(int m) const { return (long long)m * HEAD_N; }
+    static constexpr bool kF32 = true;
+    __device__ void pack(int n, const float* v, uint4* w) const {
+        float b[8];
+        unpack8(ld8(z.w + O_B5 + n), b);
+#pragma unroll
+        for (int i = 0; i < 8; i++) b[i] += v[i];
+        w[0] = make_uint4(__float_as_uint(b[0]), __float_as_uint(b[1]), __float_as_uint(b[2]), __float_as_uint(b[3]));
+        w[1] = make_uint4(__float_as_uint(b[4]), __float_as_uint(b[5]), __float_as_uint(b[6]), __float_as_uint(b[7]));
     }
+    __device__ void store(long long o, int n, const uint4& w) const { *reinterpret_cast<uint4*>(z.logits + o + n) = w; }
 };
 
 // ---- data gradients ---------------------------------------------------------
@@ -407,83 +621,91 @@ __device__ __forceinline__ bf16_t wd_at(const bf16_t* w, int C, int i) {  // w [
     return ky < 0 || kx < 0 ? bf16_t(0) : w[(co * 9 + ky * 3 + kx) * C + ci];
 }
 __global__ void prep_kernel(const bf16_t* __restrict__ w, bf16_t* __restrict__ out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < N_W4T) {
-        out[i] = w[O_W4 + (i % HID) * FEAT + i / HID];
-        return;
-    }
-    i -= N_W4T;
-    if (i < N_W5T) {
-        out[N_W4T + i] = w[O_W5 + (i % HEAD_N) * HID + i / HEAD_N];
-        return;
-    }
-    i -= N_W5T;
-    if (i < N_WD3) {
-        out[N_W4T + N_W5T + i] = wd_at(w + O_W3, 32, i);
-        return;
-    }
-    i -= N_WD3;
-    if (i < N_WD2) out[N_W4T + N_W5T + N_WD3 + i] = wd_at(w + O_W2, 16, i);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N_PREP) return;
+    bf16_t v;
+    if (i < N_W4T)
+        v = w[O_W4 + (i % HID) * FEAT + i / HID];
+    else if (i < N_W4T + N_W5T)
+        v = w[O_W5 + ((i - N_W4T) % HEAD_N) * HID + (i - N_W4T) / HEAD_N];
+    else if (i < N_W4T + N_W5T + N_WD3)
+        v = wd_at(w + O_W3, 32, i - N_W4T - N_W5T);
+    else
+        v = wd_at(w + O_W2, 16, i - N_W4T - N_W5T - N_WD3);
+    for (int r = 0; r < WREP; r++) out[i + r * N_PREP] = v;
 }
 
 __device__ __forceinline__ uint32_t mask_pair(uint32_t act, uint32_t v) {  // bf16 pair v where the activation is not zero
     return v & ((act & 0xffffu ? 0xffffu : 0u) | (act & 0xffff0000u ? 0xffff0000u : 0u));
 }
-// 8 values rounded to bf16, stored as one 16-byte word; with act, zero where
-// the activation there is (ReLU's gradient)
-__device__ __forceinline__ void st8_mask(bf16_t* dst, const float* v, const bf16_t* act) {
-    uint4 w = make_uint4(pack2(f2bf(v[0]), f2bf(v[1])), pack2(f2bf(v[2]), f2bf(v[3])), pack2(f2bf(v[4]), f2bf(v[5])),
-                         pack2(f2bf(v[6]), f2bf(v[7])));
-    if (act != nullptr) {
-        const uint4 a = ld8(act);
-        w = make_uint4(mask_pair(a.x, w.x), mask_pair(a.y, w.y), mask_pair(a.z, w.z), mask_pair(a.w, w.w));
-    }
-    *reinterpret_cast<uint4*>(dst) = w;
+// 8 bf16 values, zero where the activation there is (ReLU's gradient)
+__device__ __forceinline__ uint4 mask8(const uint4& a, const uint4& w) {
+    return make_uint4(mask_pair(a.x, w.x), mask_pair(a.y, w.y), mask_pair(a.z, w.z), mask_pair(a.w, w.w));
 }
 
 struct HeadBwdData {  // dh = relu'(h) * (dl W5): M = B, N = 256, K = 296
     Bufs z;
-    using Row = int;
-    __device__ Row row(int m) const { return m; }
-    __device__ uint4 a8(Row m, int k) const { return ld8(z.dl + (long long)m * HEAD_N + k); }
-    __device__ uint4 b8(int k, int n) const { return ld8(z.w5t + n * HEAD_N + k); }
-    __device__ void store8(const Row&, int m, int n, const float* v) const {
-        const long long o = (long long)m * HID + n;
-        st8_mask(z.dh + o, v, z.h + o);
-    }
+    using Row = MatRow;
+    using Step = int;
+    static constexpr bool kCalc = false;
+    static constexpr int ldb = HEAD_N;
+    __device__ Row row(int m) const { return Row{z.dl + (long long)m * HEAD_N}; }
+    __device__ Step step(int k) const { return k; }
+    __device__ bool a8(const Row& w, Step k, const bf16_t*& p) const { return mat_a8(w, k, p); }
+    __device__ const bf16_t* b(int copy) const { return z.w5t + copy * N_PREP; }
+    __device__ long long out_at(int m) const { return (long long)m * HID; }
+    static constexpr bool kF32 = false;
+    __device__ uint4 pack(int, const float* v) const { return pack8(v); }
+    __device__ void store(long long o, int n, const uint4& w) const { st8(z.dh + o + n, mask8(ld8(z.h + o + n), w)); }
 };
 struct Fc1BwdData {  // df = (dh W4)[:, :1152]: M = B, N = 1152, K = 256
     Bufs z;
-    using Row = int;
-    __device__ Row row(int m) const { return m; }
-    __device__ uint4 a8(Row m, int k) const { return ld8(z.dh + (long long)m * HID + k); }
-    __device__ uint4 b8(int k, int n) const { return ld8(z.w4t + n * HID + k); }
-    __device__ void store8(const Row&, int m, int n, const float* v) const { st8_mask(z.df + (long long)m * CONVF + n, v, nullptr); }
+    using Row = MatRow;
+    using Step = int;
+    static constexpr bool kCalc = false;
+    static constexpr int ldb = HID;
+    __device__ Row row(int m) const { return Row{z.dh + (long long)m * HID}; }
+    __device__ Step step(int k) const { return k; }
+    __device__ bool a8(const Row& w, Step k, const bf16_t*& p) const { return mat_a8(w, k, p); }
+    __device__ const bf16_t* b(int copy) const { return z.w4t + copy * N_PREP; }
+    __device__ long long out_at(int m) const { return (long long)m * CONVF; }
+    static constexpr bool kF32 = false;
+    __device__ uint4 pack(int, const float* v) const { return pack8(v); }
+    __device__ void store(long long o, int n, const uint4& w) const { st8(z.df + o + n, w); }
 };
 // conv input gradient: M = pairs x output positions (2x2 input blocks),
 // N = 4 C, K = 4 x 32 (see prep_kernel); WHICH 3: da3 -> da2, 2: da2 -> da1
 template <int C, int WHICH>
 struct ConvBwdData {
     Geo g; Bufs z;
-    struct Row {
-        long long in, out;  // element offsets of dy position (a, b) and of input pixel (2a, 2b)
-        bool down, right;   // (a + 1, .) and (., b + 1) lie inside the map
-    };
+    using Row = WinRow;  // of dy position (a, b); steps lead to (a + ny, b + nx)
+    using Step = WinStep;
+    static constexpr bool kCalc = false;
+    static constexpr int ldb = 128;
     __device__ Row row(int m) const {
-        const int OH = WHICH == 3 ? g.H3 : g.H2, OW = WHICH == 3 ? g.W3 : g.W2;
-        const int ohw = OH * OW, b = m / ohw, r = m - b * ohw, a = r / OW, x = r - a * OW;
-        return Row{(long long)m * 32, ((long long)(b * 2 * OH + 2 * a) * (2 * OW) + 2 * x) * C, a + 1 < OH, x + 1 < OW};
+        const int OW = WHICH == 3 ? g.W3 : g.W2, ohw = (WHICH == 3 ? g.H3 : g.H2) * OW;
+        const int r = m % ohw, a = r / OW;
+        return Row{(WHICH == 3 ? z.da3 : z.da2) + (long long)m * 32, a, r - a * OW};
     }
-    __device__ uint4 a8(const Row& w, int k) const {
-        const int nb = k >> 5, OW = WHICH == 3 ? g.W3 : g.W2;
-        if (((nb & 2) && !w.down) || ((nb & 1) && !w.right)) return make_uint4(0u, 0u, 0u, 0u);
-        return ld8((WHICH == 3 ? z.da3 : z.da2) + w.in + ((nb & 2) ? OW * 32 : 0) + ((nb & 1) ? 32 : 0) + (k & 31));
+    __device__ Step step(int k) const {
+        const int nb = k >> 5;
+        return Step{((nb >> 1) * (WHICH == 3 ? g.W3 : g.W2) + (nb & 1)) * 32 + (k & 31), nb >> 1, nb & 1};
     }
-    __device__ uint4 b8(int k, int n) const { return ld8((WHICH == 3 ? z.wd3 : z.wd2) + n * 128 + k); }
-    __device__ void store8(const Row& w, int, int n, const float* v) const {
+    __device__ bool a8(const Row& w, const Step& s, const bf16_t*& p) const {
+        return win_a8(w, s, WHICH == 3 ? g.H3 : g.H2, WHICH == 3 ? g.W3 : g.W2, p);
+    }
+    __device__ const bf16_t* b(int copy) const { return (WHICH == 3 ? z.wd3 : z.wd2) + copy * N_PREP; }
+    __device__ long long out_at(int m) const {  // input pixel (2a, 2b)
+        const int OW = WHICH == 3 ? g.W3 : g.W2;
+        const int y = m / OW, x = m - y * OW;  // y: pair * OH + a
+        return ((long long)(2 * y) * (2 * OW) + 2 * x) * C;
+    }
+    static constexpr bool kF32 = false;
+    __device__ uint4 pack(int, const float* v) const { return pack8(v); }
+    __device__ void store(long long o, int n, const uint4& w) const {
         const int par = n / C, ci = n - par * C, W = WHICH == 3 ? g.W2 : g.W1;
-        const long long o = w.out + ((par & 2) ? W * C : 0) + ((par & 1) ? C : 0) + ci;
-        st8_mask((WHICH == 3 ? z.da2 : z.da1) + o, v, (WHICH == 3 ? z.a2 : z.a1) + o);
+        o += ((par & 2) ? W * C : 0) + ((par & 1) ? C : 0) + ci;
+        st8((WHICH == 3 ? z.da2 : z.da1) + o, mask8(ld8((WHICH == 3 ? z.a2 : z.a1) + o), w));
     }
 };
 
@@ -499,10 +721,10 @@ struct ConvBwdData {
 // two 2-byte loads per pair: 791 us for FC1's gradient on four 1080p pairs,
 // 32,640 samples, against 112 this way; 577 against 58 for conv2's.)  A tile holds only the M - m0 columns there are: the MMA's
 // further rows read whatever follows in shared memory into accumulator rows
-// that nothing reads.  The bias gradient is the sum of dy's chunks as the
-// threads of the first N tile pass them on.
-//   Op: rows K; RowW row(m); uint4 a8(row, i), b8(row, j); grad offsets out
-// (with leading dimension ld) and bias; n_real columns are stored.
+// that nothing reads.  The bias gradient is the sum of dy's chunks, which
+// the threads of the first N tile read back.
+//   Op: dy() with lddy columns per row m; rows and steps of x as above; grad
+// offsets out (with leading dimension ld) and bias; n_real columns are stored.
 template <int KS>
 constexpr uint64_t wg_sdesc_hi() {
     return (uint64_t(128 >> 4) << 16) | (uint64_t((KS * 16) >> 4) << 32) | (1ull << 46);
@@ -512,7 +734,7 @@ __device__ __forceinline__ void red_add_v4(float* p, const float* v) {
                  : "memory");
 }
 
-template <int BN, int KS, int AQ, class Op>  // AQ: 8-column chunks of A per thread and step
+template <int BN, int KS, int AQ, int ST, class Op>  // AQ: 8-column chunks of dy per thread and step
 __global__ void __launch_bounds__(TC_THREADS) wgrad_tc_kernel(const Op op, int M, int N, int K, int kchunk, int* status) {
     static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256 && KS % 16 == 0 && TC_THREADS % KS == 0, "tile shape");
     constexpr int GR = TC_THREADS / KS;          // threads per row
@@ -521,7 +743,7 @@ __global__ void __launch_bounds__(TC_THREADS) wgrad_tc_kernel(const Op op, int M
     constexpr int NCOL = tc_cols<BN>();
     constexpr uint32_t IDESC = tc_idesc<BN>() | (1u << 15) | (1u << 16);  // A and B transposed (M/N-major)
     extern __shared__ __align__(128) uint8_t tc_smem[];
-    __shared__ __align__(8) unsigned long long tc_bar[2];
+    __shared__ __align__(8) unsigned long long tc_bar[ST];
     __shared__ uint32_t tc_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * TC_BM, n0 = blockIdx.y * BN;
@@ -534,8 +756,8 @@ __global__ void __launch_bounds__(TC_THREADS) wgrad_tc_kernel(const Op op, int M
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        mbar_init(bar0, 1);
-        mbar_init(bar0 + 8, 1);
+#pragma unroll
+        for (int s = 0; s < ST; s++) mbar_init(bar0 + 8 * s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -551,26 +773,41 @@ __global__ void __launch_bounds__(TC_THREADS) wgrad_tc_kernel(const Op op, int M
 #pragma unroll
         for (int i = 0; i < 8; i++) bias[j][i] = 0.f;
     const int nk = ke > kb ? (ke - kb + KS - 1) / KS : 0;
-    for (int it = 0; it < nk; it++) {
-        const int st = it & 1, m = kb + it * KS + p;
-        const uint32_t sa = sbase + uint32_t(st * STAGE), sb = sa + A_BYTES;
-        const bool live = m < ke;
-        const typename Op::Row row = op.row(live ? m : ke - 1);
-        uint4 va[AQ], vb[BQ];
+    typename Op::Step steps[BQ];
 #pragma unroll
-        for (int j = 0; j < AQ; j++) {
-            const int c = c0 + j * GR;
-            va[j] = live && c < mblk ? op.a8(row, m0 + 8 * c) : make_uint4(0u, 0u, 0u, 0u);
-        }
+    for (int j = 0; j < BQ; j++) steps[j] = op.step(n0 + 8 * (c0 + j * GR));
+    const bf16_t* dyp = op.dy() + m0 + 8 * c0;
+    auto load = [&](int it) {
+        const int m = kb + it * KS + p;
+        const uint32_t sa = sbase + uint32_t((it % ST) * STAGE + c0 * BLK) + off, sb = sa + A_BYTES;
+        const bool live = m < ke;
+        const int mr = live ? m : ke - 1;
+        const typename Op::Row row = op.row(mr);
+        const bf16_t* d = dyp + (long long)mr * Op::lddy;
+#pragma unroll
+        for (int j = 0; j < AQ; j++) cp16z(sa + uint32_t(j * GR * BLK), d + 8 * j * GR, live && c0 + j * GR < mblk, op.z.w);
 #pragma unroll
         for (int j = 0; j < BQ; j++) {
             const int c = c0 + j * GR;
-            vb[j] = live && c < nblk ? op.b8(row, n0 + 8 * c) : make_uint4(0u, 0u, 0u, 0u);
+            if (c < BN / 8) stage_a8(op, sb + uint32_t(j * GR * BLK), row, steps[j], live && c < nblk);
         }
+    };
+#pragma unroll
+    for (int s = 0; s < ST - 1; s++) {
+        if (s < nk) load(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int it = 0; it < nk; it++) {
+        const uint32_t sa = sbase + uint32_t((it % ST) * STAGE), sb = sa + A_BYTES;
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
         if (with_bias) {
 #pragma unroll
             for (int j = 0; j < AQ; j++) {
-                const uint32_t w[4] = {va[j].x, va[j].y, va[j].z, va[j].w};
+                uint32_t w[4];
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                             : "r"(sa + uint32_t((c0 + j * GR) * BLK) + off)
+                             : "memory");
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     bias[j][2 * i] += bf2f(bf16_t(w[i] & 0xffffu));
@@ -578,19 +815,6 @@ __global__ void __launch_bounds__(TC_THREADS) wgrad_tc_kernel(const Op op, int M
                 }
             }
         }
-        // the stage's previous MMAs (step it - 2) have read it
-        if (it >= 2) tc_wait(bar0 + 8 * st, uint32_t((it - 2) >> 1) & 1u, status);
-#pragma unroll
-        for (int j = 0; j < AQ; j++)
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sa + uint32_t((c0 + j * GR) * BLK) + off), "r"(va[j].x),
-                         "r"(va[j].y), "r"(va[j].z), "r"(va[j].w)
-                         : "memory");
-#pragma unroll
-        for (int j = 0; j < BQ; j++)
-            if (c0 + j * GR < BN / 8)
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sb + uint32_t((c0 + j * GR) * BLK) + off),
-                             "r"(vb[j].x), "r"(vb[j].y), "r"(vb[j].z), "r"(vb[j].w)
-                             : "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (tid == 0) {
@@ -606,12 +830,18 @@ __global__ void __launch_bounds__(TC_THREADS) wgrad_tc_kernel(const Op op, int M
                     "l"(da), "l"(db), "r"(IDESC), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
                     : "memory");
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar0 + 8 * st)
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar0 + 8 * (it % ST))
                          : "memory");
         }
+        if (it + ST - 1 < nk) {
+            // the stage's previous MMAs (step it - 1) have read it
+            if (it >= 1) tc_wait(bar0 + 8 * ((it - 1) % ST), uint32_t((it - 1) / ST) & 1u, status);
+            load(it + ST - 1);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
     if (nk > 0) {
-        tc_wait(bar0 + 8 * ((nk - 1) & 1), uint32_t((nk - 1) >> 1) & 1u, status);
+        tc_wait(bar0 + 8 * ((nk - 1) % ST), uint32_t((nk - 1) / ST) & 1u, status);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int row = m0 + (warp & 3) * 32 + lane;
         const uint32_t taddr = tmem + (uint32_t((warp & 3) * 32) << 16);
@@ -657,40 +887,44 @@ __global__ void __launch_bounds__(TC_THREADS) wgrad_tc_kernel(const Op op, int M
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOL));
 }
 
-struct HeadBwdW {  // M = 296, N = 256, K = B
-    Bufs z;
-    static constexpr int out = O_W5, ld = HID, bias = O_B5, n_real = HID;
-    using Row = int;
-    __device__ Row row(int m) const { return m; }
-    __device__ uint4 a8(Row m, int i) const { return ld8(z.dl + (long long)m * HEAD_N + i); }
-    __device__ uint4 b8(Row m, int j) const { return ld8(z.h + (long long)m * HID + j); }
+struct HeadBwdW : HeadFwd {  // M = 296, N = 256, K = B
+    static constexpr int out = O_W5, ld = HID, bias = O_B5, n_real = HID, lddy = HEAD_N;
+    __device__ const bf16_t* dy() const { return z.dl; }
 };
-struct Fc1BwdW {  // M = 256, N = 1168, K = B
-    Geo g; Bufs z;
-    static constexpr int out = O_W4, ld = FEAT, bias = O_B4, n_real = FEAT;
-    using Row = Fc1Fwd::Row;
-    __device__ Row row(int m) const { return Fc1Fwd{g, z}.row(m); }
-    __device__ uint4 a8(const Row& w, int i) const { return ld8(z.dh + (long long)w.m * HID + i); }
-    __device__ uint4 b8(const Row& w, int j) const { return Fc1Fwd{g, z}.a8(w, j); }
+struct Fc1BwdW : Fc1Fwd {  // M = 256, N = 1168, K = B
+    static constexpr int out = O_W4, ld = FEAT, bias = O_B4, n_real = FEAT, lddy = HID;
+    __device__ const bf16_t* dy() const { return z.dh; }
 };
-// conv weight gradient: M = CO, N = 9 C, K = pairs x output positions
-template <class Fwd, int C, int CO, int OW, int OB, int WHICH>
-struct ConvBwdW {
+// conv weight gradient: M = 32, N = 9 C, K = pairs x output positions
+template <class Fwd, int C, int OW, int OB>
+struct ConvBwdW : Fwd {
+    static constexpr int out = OW, ld = 9 * C, bias = OB, n_real = 9 * C, lddy = 32;
+    __device__ const bf16_t* dy() const { return C == 16 ? this->z.da2 : this->z.da3; }
+};
+using Conv2BwdW = ConvBwdW<Conv2Fwd, 16, O_W2, O_B2>;
+using Conv3BwdW = ConvBwdW<Conv3Fwd, 32, O_W3, O_B3>;
+struct Conv1BwdW {  // M = 16, N = 18 (24 staged)
     Geo g; Bufs z;
-    static constexpr int out = OW, ld = 9 * C, bias = OB, n_real = 9 * C;
-    struct Row {
-        typename Fwd::Row r;
-        int m;
-    };
-    __device__ Row row(int m) const { return Row{Fwd{g, z}.row(m), m}; }
-    __device__ uint4 a8(const Row& w, int i) const {
-        return ld8((WHICH == 1 ? z.da1 : (WHICH == 2 ? z.da2 : z.da3)) + (long long)w.m * CO + i);
+    static constexpr int out = O_W1, ld = 18, bias = O_B1, n_real = 18, lddy = 16;
+    using Row = Conv1Row;
+    using Step = int;
+    static constexpr bool kCalc = true;
+    __device__ Row row(int m) const { return conv1_row(g, m); }
+    __device__ Step step(int k) const { return k; }
+    __device__ bool calc(Step) const { return true; }
+    __device__ uint4 make(const Row& w, Step j) const {
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (j == 0)
+            v = make_uint4(conv1_tap(w, g.cw, 0, 0), conv1_tap(w, g.cw, 0, 1), conv1_tap(w, g.cw, 0, 2), conv1_tap(w, g.cw, 1, 0));
+        else if (j == 8)
+            v = make_uint4(conv1_tap(w, g.cw, 1, 1), conv1_tap(w, g.cw, 1, 2), conv1_tap(w, g.cw, 2, 0), conv1_tap(w, g.cw, 2, 1));
+        else
+            v.x = conv1_tap(w, g.cw, 2, 2);
+        return v;
     }
-    __device__ uint4 b8(const Row& w, int j) const { return Fwd{g, z}.a8(w.r, j); }
+    __device__ bool a8(const Row&, Step, const bf16_t*&) const { return false; }
+    __device__ const bf16_t* dy() const { return z.da1; }
 };
-using Conv1BwdW = ConvBwdW<Conv1Fwd, 2, 16, O_W1, O_B1, 1>;
-using Conv2BwdW = ConvBwdW<Conv2Fwd, 16, 32, O_W2, O_B2, 2>;
-using Conv3BwdW = ConvBwdW<Conv3Fwd, 32, 32, O_W3, O_B3, 3>;
 
 // da3 = relu'(a3) * (sum of the crop gradients of the up to 9 MBs whose 6x6
 // crop holds the cell): one thread per (pair, cell, 8 channels).
@@ -722,7 +956,7 @@ __global__ void uncrop_kernel(const Geo g, const bf16_t* __restrict__ df, const 
         }
     }
     const long long o = (long long)cell * 32 + c;
-    st8_mask(da3 + o, s, a3 + o);
+    st8(da3 + o, mask8(ld8(a3 + o), pack8(s)));
 }
 
 // ---- loss, proposals, optimiser -------------------------------------------------
@@ -832,12 +1066,13 @@ __global__ void adam_kernel(float* __restrict__ master, bf16_t* __restrict__ w, 
     m2[i] = b;
     const float nw = master[i] - lr * (a * c1) / (sqrtf(b * c2) + eps);
     master[i] = nw;
-    w[i] = f2bf(nw);
+    for (int r = 0; r < WREP; r++) w[i + r * WSTRIDE] = f2bf(nw);
 }
 
 __global__ void to_bf16_kernel(const float* __restrict__ src, bf16_t* __restrict__ dst, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = f2bf(src[i]);
+    if (i < n)
+        for (int r = 0; r < WREP; r++) dst[i + r * WSTRIDE] = f2bf(src[i]);
 }
 
 // The neighbour MV features of every MB of the P frames of a propose batch
@@ -865,37 +1100,40 @@ __global__ void guide_frames_kernel(const PropFrame* __restrict__ fr, int P, int
     }
 }
 
-template <int BN, class Op>
+template <int BN, int MT, int ST, class Op>
 static void gemm(const Op& op, int M, int N, int K, cudaStream_t st) {
-    constexpr int smem = 2 * (TC_BM * TC_BK * 2 + BN * TC_BK * 2);
+    constexpr int smem = ST * (MT * TC_BM + BN) * TC_BK * 2;
     static const bool attr_ok = [] {  // once per instantiation (the dynamic shared memory above 48 KB)
-        return cudaFuncSetAttribute(gemm_tc_kernel<BN, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
+        return cudaFuncSetAttribute(gemm_tc_kernel<BN, MT, ST, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
                cudaSuccess;
     }();
     (void)attr_ok;
-    dim3 grid((M + TC_BM - 1) / TC_BM, (N + BN - 1) / BN);
-    gemm_tc_kernel<BN, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, nullptr);
+    dim3 grid((M + MT * TC_BM - 1) / (MT * TC_BM), (N + BN - 1) / BN);
+    gemm_tc_kernel<BN, MT, ST, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, nullptr);
 }
 
-// Weight-gradient GEMM: K split over about two CTAs per SM (what its shared
-// and tensor memory hold), at least four steps each.
-template <int BN, int KS, int AQ, class Op>
+// Weight-gradient GEMM: K split over the CTAs that shared and tensor memory
+// and the threads let stay resident, at least four steps each.
+template <int BN, int KS, int AQ, int ST, class Op>
 static void wgrad(const Op& op, int M, int N, int K, int sms, cudaStream_t st) {
     constexpr int GR = TC_THREADS / KS, BLK = KS * 16, A_BYTES = AQ * GR * BLK, STAGE = A_BYTES + (BN / 8) * BLK;
     // the MMA reads 16 blocks of A whatever there are: 16 * BLK from the last stage's start
-    constexpr int smem = STAGE + (STAGE > 16 * BLK ? STAGE : 16 * BLK);
+    constexpr int smem = (ST - 1) * STAGE + (STAGE > 16 * BLK ? STAGE : 16 * BLK);
+    constexpr int by_smem = 224 * 1024 / (smem + 2048), by_tmem = 512 / tc_cols<BN>();
+    constexpr int resident = by_smem < by_tmem ? (by_smem < 4 ? by_smem : 4) : (by_tmem < 4 ? by_tmem : 4);
+    static_assert(resident >= 1, "shared memory");
     static const bool attr_ok = [] {
-        return cudaFuncSetAttribute(wgrad_tc_kernel<BN, KS, AQ, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
+        return cudaFuncSetAttribute(wgrad_tc_kernel<BN, KS, AQ, ST, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
                cudaSuccess;
     }();
     (void)attr_ok;
     const int tiles = ((M + TC_BM - 1) / TC_BM) * ((N + BN - 1) / BN);
-    int splits = (2 * sms + tiles - 1) / tiles;
+    int splits = resident * sms / tiles;
     splits = std::max(1, std::min(splits, (K + 4 * KS - 1) / (4 * KS)));
     int kchunk = (K + splits - 1) / splits;
     kchunk = (kchunk + KS - 1) / KS * KS;
     dim3 grid((M + TC_BM - 1) / TC_BM, (N + BN - 1) / BN, (K + kchunk - 1) / kchunk);
-    wgrad_tc_kernel<BN, KS, AQ, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, kchunk, nullptr);
+    wgrad_tc_kernel<BN, KS, AQ, ST, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, kchunk, nullptr);
 }
 
 }  // namespace mvnet
@@ -1017,17 +1255,25 @@ int check_geo(const h264a_mvnet* n, const h264a_mvnet_pair* d_pairs, int P, int 
 
 void trunk_forward(h264a_mvnet* n, const Geo& g, cudaStream_t st) {
     const Bufs z = bufs(n);
-    gemm<16>(Conv1Fwd{g, z}, g.P * g.H1 * g.W1, 16, 32, st);
-    gemm<32>(Conv2Fwd{g, z}, g.P * g.H2 * g.W2, 32, 144, st);
-    gemm<32>(Conv3Fwd{g, z}, g.P * g.H3 * g.W3, 32, 288, st);
+    const int m1 = g.P * g.H1 * g.W1;
+    conv1_kernel<<<std::min((m1 + 127) / 128, n->sms * C1_CTAS), 128, 0, st>>>(g, z, m1, nullptr);
+    gemm<32, 1, 3>(Conv2Fwd{g, z}, g.P * g.H2 * g.W2, 32, 144, st);
+    gemm<32, 1, 3>(Conv3Fwd{g, z}, g.P * g.H3 * g.W3, 32, 288, st);
 }
 
 void head_forward(h264a_mvnet* n, const Geo& g, float* logits, cudaStream_t st) {
     Bufs z = bufs(n);
     z.logits = logits;
     const int B = g.P * g.nmb;
-    gemm<256>(Fc1Fwd{g, z}, B, HID, FEAT, st);
-    gemm<160>(HeadFwd{z}, B, HEAD_N, HID, st);
+    // FC1's weights (600 KB) cross the L2 once per row tile: 256-row tiles halve
+    // that, and keep every SM busy from two 128-row tiles per SM on (four 1080p
+    // pairs, 32,640 samples: 76 us with 128 rows, 61 with 256; below, the
+    // smaller tile spreads the samples over more SMs)
+    if (B > TC_BM * n->sms)
+        gemm<256, 2, 3>(Fc1Fwd{g, z}, B, HID, FEAT, st);
+    else
+        gemm<256, 1, 2>(Fc1Fwd{g, z}, B, HID, FEAT, st);
+    gemm<160, 1, 3>(HeadFwd{z}, B, HEAD_N, HID, st);
 }
 
 void backward(h264a_mvnet* n, const Geo& g, cudaStream_t st) {
@@ -1035,17 +1281,17 @@ void backward(h264a_mvnet* n, const Geo& g, cudaStream_t st) {
     const int B = g.P * g.nmb, S = n->sms;
     const int K3 = g.P * g.H3 * g.W3, K2 = g.P * g.H2 * g.W2, K1 = g.P * g.H1 * g.W1;
     prep_kernel<<<(N_PREP + 255) / 256, 256, 0, st>>>(n->w, n->wprep);
-    wgrad<256, 64, 4>(HeadBwdW{z}, HEAD_N, HID, B, S, st);
-    gemm<256>(HeadBwdData{z}, B, HID, HEAD_N, st);
-    wgrad<256, 64, 4>(Fc1BwdW{g, z}, HID, FEAT, B, S, st);
-    gemm<192>(Fc1BwdData{z}, B, CONVF, HID, st);
+    wgrad<256, 64, 4, 2>(HeadBwdW{{z}}, HEAD_N, HID, B, S, st);
+    gemm<256, 1, 2>(HeadBwdData{z}, B, HID, HEAD_N, st);
+    wgrad<256, 64, 4, 2>(Fc1BwdW{{g, z}}, HID, FEAT, B, S, st);
+    gemm<192, 1, 2>(Fc1BwdData{z}, B, CONVF, HID, st);
     const long long cells = (long long)K3 * 4;
     uncrop_kernel<<<unsigned((cells + 255) / 256), 256, 0, st>>>(g, n->df, n->a3, n->da3);
-    wgrad<144, 64, 1>(Conv3BwdW{g, z}, 32, 288, K3, S, st);
-    gemm<128>(ConvBwdData<32, 3>{g, z}, K3, 128, 128, st);
-    wgrad<144, 128, 2>(Conv2BwdW{g, z}, 32, 144, K2, S, st);
-    gemm<64>(ConvBwdData<16, 2>{g, z}, K2, 64, 128, st);
-    wgrad<32, 128, 1>(Conv1BwdW{g, z}, 16, 24, K1, S, st);
+    wgrad<144, 64, 1, 3>(Conv3BwdW{{g, z}}, 32, 288, K3, S, st);
+    gemm<128, 1, 2>(ConvBwdData<32, 3>{g, z}, K3, 128, 128, st);
+    wgrad<144, 128, 2, 2>(Conv2BwdW{{g, z}}, 32, 144, K2, S, st);
+    gemm<64, 1, 2>(ConvBwdData<16, 2>{g, z}, K2, 64, 128, st);
+    wgrad<32, 128, 1, 2>(Conv1BwdW{g, z}, 16, 24, K1, S, st);
 }
 
 }  // namespace
@@ -1059,7 +1305,7 @@ extern "C" int h264a_mvnet_create(int device, uint64_t seed, h264a_mvnet** out) 
     cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, device);
     int rc = H264A_OK;
     if (!rc) rc = dmalloc(&n->master, NPARAMS);
-    if (!rc) rc = dmalloc(&n->w, NPARAMS);
+    if (!rc) rc = dmalloc(&n->w, size_t(WREP) * WSTRIDE);
     if (!rc) rc = dmalloc(&n->grad, NPARAMS);
     if (!rc) rc = dmalloc(&n->m1, NPARAMS);
     if (!rc) rc = dmalloc(&n->m2, NPARAMS);
@@ -1074,7 +1320,7 @@ extern "C" int h264a_mvnet_create(int device, uint64_t seed, h264a_mvnet** out) 
     if (!rc) rc = dmalloc(&n->dl, size_t(MAXS * HEAD_N));
     if (!rc) rc = dmalloc(&n->df, size_t(MAXS * CONVF));
     if (!rc) rc = dmalloc(&n->logits, size_t(MAXS * HEAD_N));
-    if (!rc) rc = dmalloc(&n->wprep, size_t(N_PREP));
+    if (!rc) rc = dmalloc(&n->wprep, size_t(WREP) * N_PREP);
     if (!rc) rc = dmalloc(&n->loss, 1);
     if (!rc) rc = dmalloc(&n->inmv, size_t(MAXS * 6));
     if (!rc) rc = dmalloc(&n->ipairs, size_t(MAXPIX / 256));
