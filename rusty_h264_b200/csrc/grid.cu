@@ -15,9 +15,12 @@
 //    (3 at R = 32: 975 items in four rounds of 256).  The argmin skips the
 //    lambda*rate of a candidate whose distortion alone cannot beat the
 //    thread's best (exact: a thread meets its candidates in scan order).
-//  * SATD (fullpel_satd_kernel): one CTA per MB; a thread owns four
-//    horizontally adjacent offsets, and two aligned words per window row
-//    segment yield all four candidates' rows by funnel shifts.
+//  * SATD (fullpel_satd_kernel): one CTA per MB.  The Hadamard transform is
+//    linear, so the predictions' 4x4 blocks are transformed once per window
+//    position (77^2 at R = 32) instead of once per candidate and block
+//    (16 * 65^2); a candidate's SATD is then 16 packed maxima a block.
+#include <algorithm>
+
 #include "h264a_device.cuh"
 
 namespace h264a {
@@ -176,70 +179,148 @@ __global__ void __launch_bounds__(GRID_THREADS, 2) fullpel_sad_kernel(GridArgs a
     }
 }
 
-// SATD grid and argmin, one CTA per MB; dynamic shared memory: the window.
-__global__ void __launch_bounds__(GRID_THREADS, 2) fullpel_satd_kernel(GridArgs a) {
+// The 4x4 Hadamard coefficients of a block (4 row words) as eight words of two
+// 16-bit halves, SATD_BIAS added to each: |coefficient| <= 8 * 255 but for the
+// sum of all pixels, so every half is 0 .. 6120.  Two columns' worth per 32-bit
+// integer (lo + 65536 * hi): the vertical butterflies are plain adds, and the
+// bias on row 0 reaches every output.
+constexpr int SATD_BIAS = 2040;
+__device__ __forceinline__ int dot4_us(uint32_t pix, uint32_t coef, int acc) {  // unsigned bytes x signed bytes
+    int d;
+    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(pix), "r"(coef), "r"(acc));
+    return d;
+}
+__device__ __forceinline__ void had_words(const uint32_t w[4], uint32_t o[8]) {
+    int x[4], y[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const int b = r == 0 ? SATD_BIAS : 0;
+        x[r] = dot4_us(w[r], 0x01010101u, b) + dot4_us(w[r], 0xffff0101u, b) * 65536;
+        y[r] = dot4_us(w[r], 0x01ffff01u, b) + dot4_us(w[r], 0xff01ff01u, b) * 65536;
+    }
+    const int a = x[0] + x[1], b = x[0] - x[1], c = x[2] + x[3], d = x[2] - x[3];
+    o[0] = uint32_t(a + c), o[1] = uint32_t(a - c), o[2] = uint32_t(b + d), o[3] = uint32_t(b - d);
+    const int e = y[0] + y[1], f = y[0] - y[1], g = y[2] + y[3], h = y[2] - y[3];
+    o[4] = uint32_t(e + g), o[5] = uint32_t(e - g), o[6] = uint32_t(f + h), o[7] = uint32_t(f - h);
+}
+
+// SATD grid and argmin, one CTA per MB.
+//
+// With the biased coefficients P of a prediction block and S of a source
+// block, sum |P - S| = 2 sum max(P, S) - sum P - sum S, and sum P = 16 times
+// the block's first pixel + 16 * SATD_BIAS (a Hadamard matrix's rows sum to
+// its first column).  Per (candidate, block) that is eight packed maxima, four
+// three-operand adds (a half's sum stays below 2^16; the ninth addend is the
+// first pixel's share, SATD_BIAS - 8 * pixel >= 0) and one dp2a.
+//
+// Offsets with row dy = ph (mod 4) use window rows ph (mod 4) only: a stage
+// transforms the rows of `ps` such phases and `g` runs of SATD_J candidates
+// down (4 rows apart) into shared memory, then a thread takes one column
+// offset and one run: SATD_J + 3 positions per block column, each met by up to
+// four candidates, with the column's four source blocks in registers.  Bound
+// by the integer pipes: 4 million packed operations a MB at R = 32.  3,600
+// MBs, R = 32: 1,833 us transforming every candidate's blocks, SATD_US now.
+//
+// Dynamic shared memory: the window, then per stage position two uint4 of
+// coefficients and one word.
+constexpr int SATD_J = 6;
+__host__ __device__ constexpr int satd_rows(int ps, int g) { return ps * (SATD_J * g + 3); }
+__global__ void __launch_bounds__(GRID_THREADS) fullpel_satd_kernel(GridArgs a, int ps, int g) {
     extern __shared__ __align__(16) uint8_t win[];
     __shared__ long long red_key[GRID_THREADS / 32];
+    __shared__ __align__(16) uint32_t hs[16][8];  // source blocks [4 * by + bx]
+    __shared__ int ksum;
     const int mb = blockIdx.x;
     const int lx = (mb % a.mb_w) * 16, ly = (mb / a.mb_w) * 16;
     const int R = a.R, n = 2 * R + 1;
     int cxf, cyf, pmx, pmy;
     grid_center(a, mb, cxf, cyf, pmx, pmy);
-    const int ws = 16 + 2 * R, pitch = (ws + 4 + 3) & ~3, wrows = ws + GRID_K;
-    stage_grid_window(win, a.P, lx, ly, cxf, cyf, R, ws, pitch, wrows, threadIdx.x >> 5, GRID_THREADS / 32);
-    // the source MB in shared memory (the four candidates' rows need the registers)
-    __shared__ uint32_t src_s[16][4];
-    if (threadIdx.x < 64)
-        src_s[threadIdx.x >> 2][threadIdx.x & 3] =
-            ld4u(a.src + (long long)(ly + (threadIdx.x >> 2)) * a.cw + lx + 4 * (threadIdx.x & 3));
+    const int ws = 16 + 2 * R, pitch = (ws + 4 + 3) & ~3;
+    stage_grid_window(win, a.P, lx, ly, cxf, cyf, R, ws, pitch, ws, threadIdx.x >> 5, blockDim.x >> 5);
+    if (threadIdx.x < 32) {
+        const int b = threadIdx.x & 15;
+        uint32_t w[4], o[8];
+#pragma unroll
+        for (int r = 0; r < 4; r++) w[r] = ld4u(a.src + (long long)(ly + 4 * (b >> 2) + r) * a.cw + lx + 4 * (b & 3));
+        had_words(w, o);
+#pragma unroll
+        for (int i = 0; i < 8; i++) hs[b][i] = o[i];
+        int s = int(w[0] & 0xffu);
+#pragma unroll
+        for (int i = 8; i > 0; i >>= 1) s += __shfl_xor_sync(0xffffffffu, s, i);
+        if (threadIdx.x == 0) ksum = 8 * s + 16 * (SATD_BIAS + 16 * SATD_BIAS);
+    }
+    const int wx = n + 12, prows = SATD_J * g + 3, npos = satd_rows(ps, g) * wx;
+    uint4* h0 = reinterpret_cast<uint4*>(win + ((size_t(ws) * pitch + 15) & ~size_t(15)));
+    uint4* h1 = h0 + npos;
+    uint32_t* ex = reinterpret_cast<uint32_t*>(h1 + npos);
     __syncthreads();
+    const int k_mb = ksum;
 
     long long best_key = LLONG_MAX;  // (cost << 32) | scan index; min = first-wins argmin
     const long long grid_base = (long long)mb * n * n;
-    const bool argmin = a.metric == 1;
-
-    {
-        const int gx = (n + 3) / 4;  // groups of four adjacent column offsets
-        for (int item = threadIdx.x; item < gx * n; item += blockDim.x) {
-            const int g = item % gx, dyi = item / gx;
-            const int dx0 = g * 4;
-            int acc[4] = {0, 0, 0, 0};
+    const bool argmin = a.metric == 1, rate_pos = a.lambda >= 0.0;
+    for (int ph0 = 0; ph0 < 4; ph0 += ps)
+        for (int j0 = 0; ph0 + 4 * j0 < n; j0 += SATD_J * g) {
+            for (int i = threadIdx.x; i < npos; i += blockDim.x) {
+                const int row = i / wx, x = i - row * wx, p = row / prows;
+                const int y0 = ph0 + p + 4 * (j0 + row - p * prows);
+                uint32_t w[4], o[8];
 #pragma unroll
-            for (int by = 0; by < 4; by++) {
-#pragma unroll
-                for (int bx = 0; bx < 4; bx++) {
-                    uint32_t p[4][4];  // [candidate][row]
-#pragma unroll
-                    for (int r = 0; r < 4; r++) {
-                        const uint8_t* row = win + (dyi + by * 4 + r) * pitch + dx0 + bx * 4;
-                        const uint32_t lo = win_word(row, 0), hi = win_word(row, 4);
-                        p[0][r] = lo;
-                        p[1][r] = __funnelshift_r(lo, hi, 8);
-                        p[2][r] = __funnelshift_r(lo, hi, 16);
-                        p[3][r] = __funnelshift_r(lo, hi, 24);
-                    }
-                    const uint32_t sr[4] = {src_s[by * 4][bx], src_s[by * 4 + 1][bx], src_s[by * 4 + 2][bx],
-                                            src_s[by * 4 + 3][bx]};
-#pragma unroll
-                    for (int q = 0; q < 4; q++) acc[q] += satd4x4_rows(sr, p[q]);
-                }
+                for (int r = 0; r < 4; r++) w[r] = win_word(win + min(y0 + r, ws - 1) * pitch, x);  // past the window: unused
+                had_words(w, o);
+                h0[i] = make_uint4(o[0], o[1], o[2], o[3]);
+                h1[i] = make_uint4(o[4], o[5], o[6], o[7]);
+                ex[i] = uint32_t(SATD_BIAS) - 8u * (w[0] & 0xffu);
             }
+            __syncthreads();
+            for (int item = threadIdx.x; item < ps * g * n; item += blockDim.x) {
+                const int u = item / n, dxi = item - u * n, p = u / g, c = u - p * g;
+                uint32_t acc[SATD_J];
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int dxi = dx0 + q;
-                if (dxi < n) {
-                    const int idx = dyi * n + dxi;
-                    if (a.satd_grid) a.satd_grid[grid_base + idx] = acc[q];
-                    if (argmin) {
+                for (int j = 0; j < SATD_J; j++) acc[j] = 0;
+#pragma unroll 1
+                for (int bx = 0; bx < 4; bx++) {
+                    uint4 s0[4], s1[4];
+#pragma unroll
+                    for (int by = 0; by < 4; by++) {
+                        s0[by] = *reinterpret_cast<const uint4*>(&hs[4 * by + bx][0]);
+                        s1[by] = *reinterpret_cast<const uint4*>(&hs[4 * by + bx][4]);
+                    }
+                    const int at = (p * prows + c * SATD_J) * wx + dxi + 4 * bx;
+#pragma unroll
+                    for (int k = 0; k < SATD_J + 3; k++) {
+                        const uint4 v0 = h0[at + k * wx], v1 = h1[at + k * wx];
+                        const uint32_t e = ex[at + k * wx];
+#pragma unroll
+                        for (int by = 0; by < 4; by++) {
+                            const int j = k - by;
+                            if (j < 0 || j >= SATD_J) continue;
+                            const uint32_t t = e + __vmaxu2(v0.x, s0[by].x) + __vmaxu2(v0.y, s0[by].y) +
+                                               __vmaxu2(v0.z, s0[by].z) + __vmaxu2(v0.w, s0[by].w) +
+                                               __vmaxu2(v1.x, s1[by].x) + __vmaxu2(v1.y, s1[by].y) +
+                                               __vmaxu2(v1.z, s1[by].z) + __vmaxu2(v1.w, s1[by].w);
+                            acc[j] = __dp2a_lo(t, 0x0101u, acc[j]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < SATD_J; j++) {
+                    const int dyi = ph0 + p + 4 * (j0 + c * SATD_J + j);
+                    if (dyi >= n) continue;
+                    const int idx = dyi * n + dxi, dist = 2 * (int(acc[j]) - k_mb);
+                    if (a.satd_grid) a.satd_grid[grid_base + idx] = dist;
+                    // a rate is >= 0 when lambda is: a larger distortion cannot win then
+                    if (argmin && (!rate_pos || (long long)dist <= (best_key >> 32))) {
                         const long long key =
-                            (grid_cost(a, acc[q], (cxf + dxi - R) * 4, (cyf + dyi - R) * 4, pmx, pmy) << 32) |
-                            (long long)idx;
+                            (grid_cost(a, dist, (cxf + dxi - R) * 4, (cyf + dyi - R) * 4, pmx, pmy) << 32) | (long long)idx;
                         best_key = key < best_key ? key : best_key;
                     }
                 }
             }
+            __syncthreads();
         }
-    }
+    if (!argmin) return;
     // ---- argmin over the CTA ----
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -248,9 +329,9 @@ __global__ void __launch_bounds__(GRID_THREADS, 2) fullpel_satd_kernel(GridArgs 
     }
     if ((threadIdx.x & 31) == 0) red_key[threadIdx.x >> 5] = best_key;
     __syncthreads();
-    if (threadIdx.x == 0 && a.best && argmin) {
+    if (threadIdx.x == 0 && a.best) {
         long long k = red_key[0];
-        for (int i = 1; i < GRID_THREADS / 32; i++) k = red_key[i] < k ? red_key[i] : k;
+        for (int i = 1; i < int(blockDim.x >> 5); i++) k = red_key[i] < k ? red_key[i] : k;
         grid_store_best(a, mb, k, cxf, cyf, pmx, pmy);
     }
 }
@@ -320,9 +401,21 @@ extern "C" int h264a_fullpel_grid(h264a_ctx* ctx, const h264a_picture* h_pic, in
         if (rc) return rc;
     }
     if (d_satd_grid || metric == 1) {
-        if (smem > 48 * 1024)
-            H264A_CUDA(cudaFuncSetAttribute(fullpel_satd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        fullpel_satd_kernel<<<nmb, GRID_THREADS, smem, st>>>(a);
+        // runs of SATD_J candidates and phases per stage: as many as give a
+        // thread each up to a CTA's threads and fit SATD_SMEM (R = 32: one
+        // phase's three runs, 195 threads, three CTAs per SM)
+        constexpr size_t SATD_SMEM = 72 * 1024;
+        const int n = 2 * R + 1, nj = (n + 3) / 4, runs = (nj + SATD_J - 1) / SATD_J;
+        const size_t wbytes = (size_t(ws) * pitch + 15) & ~size_t(15);
+        auto need = [&](int ps, int g) { return wbytes + size_t(satd_rows(ps, g)) * (n + 12) * 36; };
+        int ps = 1, g = 1;
+        while (g < runs && (g + 1) * n <= GRID_THREADS && need(1, g + 1) <= SATD_SMEM) g++;
+        while (g == runs && ps < 4 && 2 * ps * g * n <= GRID_THREADS && need(2 * ps, g) <= SATD_SMEM) ps *= 2;
+        const size_t sm = need(ps, g);
+        if (sm > 48 * 1024)
+            H264A_CUDA(cudaFuncSetAttribute(fullpel_satd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+        const int threads = std::min(GRID_THREADS, (ps * g * n + 31) / 32 * 32);
+        fullpel_satd_kernel<<<nmb, threads, sm, st>>>(a, ps, g);
         const int rc = check_launch("fullpel_satd_kernel");
         if (rc) return rc;
     }
