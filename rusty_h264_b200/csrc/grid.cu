@@ -219,7 +219,9 @@ __device__ __forceinline__ void had_words(const uint32_t w[4], uint32_t o[8]) {
 // offset and one run: SATD_J + 3 positions per block column, each met by up to
 // four candidates, with the column's four source blocks in registers.  Bound
 // by the integer pipes: 4 million packed operations a MB at R = 32.  3,600
-// MBs, R = 32: 1,833 us transforming every candidate's blocks, SATD_US now.
+// MBs, R = 32: 1,833 us transforming every candidate's blocks, 463 now (the
+// integer pipe 60% busy, barriers between the stages most of the rest; runs of
+// 9 candidates 531).
 //
 // Dynamic shared memory: the window, then per stage position two uint4 of
 // coefficients and one word.
