@@ -7,21 +7,20 @@
 //    (left MV, else top MV; mbtree.rs:225-231) makes every row a sequential
 //    chain that starts from column 0, and column 0 a chain down the frame.
 //    Frames are independent (source domain, f against f-1).  One persistent
-//    kernel deals the column-0 chains first (one warp per frame, publishing
-//    each MB's flag as it finishes), then the rows in row order across frames:
-//    a row's warp waits (bounded) only for its own column-0 MB, so rows start
-//    while column 0 is still walking down the frame.  Inside a search the warp prices the four ring
-//    points of the cascading diamond together and takes the first improvement,
-//    re-pricing the rest of the ring around the moved centre (the reference's
-//    evaluation order).
-//    In HalfRes mode (the default) each chain reads its block's candidates
-//    from a shared-memory window (the block +-16 rows, 48 columns), copied by
-//    TMA one block ahead; candidates outside it, or outside the picture, read
-//    the clamped picture.  The kernel is instantiated per mode.
+//    kernel deals the column-0 chains first (publishing each MB's flag as it
+//    finishes), then the rows in row order across frames: a row waits (bounded)
+//    only for its own column-0 MB, so rows start while column 0 is still
+//    walking down the frame.  Inside a search the ring points of the cascading
+//    diamond are priced together and the first improvement taken, the rest of
+//    the ring priced again around the moved centre (the reference's evaluation
+//    order).
+//    HalfRes mode (the default) has a kernel of its own, one chain per warp:
+//    see la_half_kernel.  FullRes and Hybrid walk two chains per warp.
 #include <cstring>
 #include <vector>
 
 #include "h264a_device.cuh"
+#include "satd_mma.cuh"
 
 namespace h264a {
 
@@ -93,24 +92,6 @@ __global__ void la_intra_kernel(const uint8_t* __restrict__ pics, size_t fstride
 // searches, lane group g = lane / 16 (slots 16g.. of the candidate and
 // distortion arrays), each walking its own row chain; a group prices
 // 16 / (bs/4)^2 candidates per pass (four 8x8 or one 16x16).
-// HalfRes reference windows: per chain two buffers of LA_WIN_H rows of
-// LA_WIN_W bytes (the block +-16 rows, and 48 columns from the 16-byte boundary
-// at or left of the block's x - 16), filled by a TMA copy one block ahead.
-constexpr int LA_WIN_W = 48, LA_WIN_H = 40, LA_WIN_BYTES = LA_WIN_W * LA_WIN_H;
-constexpr int LA_WIN_BUF = 2048;  // buffer stride: 128-byte aligned, with room for a row read's second word
-extern __shared__ __align__(128) uint8_t la_win[];
-
-// The four rows of a 4x4 block at window column cx, row cy of the buffer at
-// byte offset `off` of la_win (two aligned words and a funnel shift per row).
-__device__ __forceinline__ void la_win_rows(int off, int cx, int cy, uint32_t p[4]) {
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const int a = off + (cy + r) * LA_WIN_W + cx;
-        const uint32_t* wp = reinterpret_cast<const uint32_t*>(la_win + (a & ~3));
-        p[r] = __funnelshift_r(wp[0], wp[1], uint32_t(a & 3) * 8u);
-    }
-}
-
 struct LaSearch {
     const uint8_t* cur;
     const uint8_t* ref;
@@ -118,26 +99,10 @@ struct LaSearch {
     uint32_t spa[4], spb[4];  // the source rows split into column pairs (split_pairs)
     int2* cand;
     int* dist;
-    // the block's window (wbuf < 0: none): buffer offset, the lane's 4x4 block
-    // at MV (0,0) in window coordinates, and the window columns/rows a 4x4
-    // read may start at (inside the window and the picture) as bytes
-    // xlo | xhi << 8 | ylo << 16 | yhi << 24
-    int wbuf, wox, woy;
-    uint32_t wlim;
-
-    __device__ void set_window(int buf, int wx0, int wy0) {
-        wbuf = buf;
-        wox = x0 + bxo - wx0;
-        woy = y0 + byo - wy0;
-        const int xlo = max(0, -wx0), xhi = min(LA_WIN_W, w - wx0) - 4;
-        const int ylo = max(0, -wy0), yhi = min(LA_WIN_H, h - wy0) - 4;
-        wlim = uint32_t(xlo) | uint32_t(xhi) << 8 | uint32_t(ylo) << 16 | uint32_t(yhi) << 24;
-    }
 
     __device__ void init(const uint8_t* c, const uint8_t* r, int pw, int ph, int b, int bx0, int by0, int2* cs,
                          int* ds) {
         cur = c; ref = r; w = pw; h = ph; bs = b; x0 = bx0; y0 = by0; cand = cs; dist = ds;
-        wbuf = -1;
         const int lane = threadIdx.x & 31;
         gl = lane & 15;
         gb = lane & 16;
@@ -157,7 +122,7 @@ struct LaSearch {
     // SATD of each group's cand[gb..gb+n) (full-pel MVs, quarter-pel units)
     // added into dist (zeroed by the caller) by shared-memory atomics of the
     // lanes' 4x4 blocks; passes run to the larger group's need.
-    template <bool FULLPEL>  // FULLPEL: every candidate is a full-pel MV (HalfRes, FullRes)
+    template <bool FULLPEL>  // FULLPEL: every candidate is a full-pel MV (FullRes)
     __device__ void eval(int n) {
         const int cps = 4 - lg_nb;  // log2 candidates per pass of a group
         const int npass = __reduce_max_sync(0xffffffffu, (n + (1 << cps) - 1) >> cps);
@@ -167,14 +132,9 @@ struct LaSearch {
             if (c < n) {
                 const int2 mv = cand[gb + c];
                 uint32_t p[4];
-                if (FULLPEL || ((mv.x | mv.y) & 3) == 0) {
-                    const int cx = wox + (mv.x >> 2), cy = woy + (mv.y >> 2);
-                    if (wbuf >= 0 && cx >= int(wlim & 255u) && cx <= int((wlim >> 8) & 255u) &&
-                        cy >= int((wlim >> 16) & 255u) && cy <= int(wlim >> 24))
-                        la_win_rows(wbuf, cx, cy, p);
-                    else
-                        fullpel_rows_clamped(ref, w, h, x0 + bxo + (mv.x >> 2), y0 + byo + (mv.y >> 2), p);
-                } else  // a sub-pel seed (Hybrid mode halves a full-res MV): mc_luma on the plain picture
+                if (FULLPEL || ((mv.x | mv.y) & 3) == 0)
+                    fullpel_rows_clamped(ref, w, h, x0 + bxo + (mv.x >> 2), y0 + byo + (mv.y >> 2), p);
+                else  // a sub-pel seed (Hybrid mode halves a full-res MV): mc_luma on the plain picture
                     subpel_rows_clamped(ref, w, h, x0 + bxo + (mv.x >> 2), y0 + byo + (mv.y >> 2), mv.x & 3, mv.y & 3, p);
                 d = satd4x4_packed(spa, spb, p);
             }
@@ -269,8 +229,8 @@ __device__ void la_inter_cost(LaSearch& s, bool active, int seedx, int seedy, in
 }
 
 struct LaBufs {
-    CUtensorMap hmap;     // the half-res frames as (cw/2, ch/2, n), box LA_WIN_W x LA_WIN_H x 1
-    int hmap_ok;          // HalfRes mode with a valid map: searches read windows
+    CUtensorMap hmap;     // HalfRes: the half-res frames as (cw/2, ch/2, n), box LA_WIN_W x LA_WIN_H x 1
+    int hmap_ok;          // HalfRes with a valid map: searches read windows
     const uint8_t* full;  // n frames cw x ch
     const uint8_t* half;  // n frames cw/2 x ch/2 (modes 1, 2)
     int cw, ch, mb_w, mb_h, n, mode;
@@ -279,14 +239,11 @@ struct LaBufs {
     int32_t* mvs;
 };
 
-// Window origin of half-res block column mbx: 16 columns left of the block,
-// rounded down to a 16-byte boundary (the TMA x alignment).
-__device__ __forceinline__ int la_win_x0(int mbx) { return (mbx * 8 - 16) & ~15; }
-
-// frame_costs for MB (mbx, mby) of frame f >= 1 given the full-res seed.
+// frame_costs for MB (mbx, mby) of frame f >= 1 given the full-res seed
+// (MODE 0 FullRes, 1 Hybrid).
 template <int MODE>
 __device__ void la_mb(const LaBufs& b, bool active, int f, int mbx, int mby, int sfx, int sfy, int2* cs, int* ds,
-                      int wbuf, int& outx, int& outy) {
+                      int& outx, int& outy) {
     const long long nmb = (long long)b.mb_w * b.mb_h;
     const long long gm = nmb * f + (long long)mby * b.mb_w + mbx;
     const int cwh = b.cw / 2, chh = b.ch / 2;
@@ -300,16 +257,11 @@ __device__ void la_mb(const LaBufs& b, bool active, int f, int mbx, int mby, int
         la_inter_cost<true>(s, active, sfx, sfy, 8, cost, mx, my);
     } else {
         s.init(b.half + hs * f, b.half + hs * (f - 1), cwh, chh, 8, mbx * 8, mby * 8, cs, ds);
-        if (wbuf >= 0) s.set_window(wbuf, la_win_x0(mbx), mby * 8 - 16);
         int hx, hy;
-        la_inter_cost<MODE == 2>(s, active, sfx / 2, sfy / 2, 8, cost, hx, hy);
-        if (MODE == 2) {  // HalfRes
-            mx = hx * 2;
-            my = hy * 2;
-        } else {  // Hybrid: refine at full-res from the coarse MV
-            s.init(b.full + fs * f, b.full + fs * (f - 1), b.cw, b.ch, 16, mbx * 16, mby * 16, cs, ds);
-            la_inter_cost<true>(s, active, hx * 2, hy * 2, 2, cost, mx, my);
-        }
+        la_inter_cost<false>(s, active, sfx / 2, sfy / 2, 8, cost, hx, hy);
+        // refine at full-res from the coarse MV
+        s.init(b.full + fs * f, b.full + fs * (f - 1), b.cw, b.ch, 16, mbx * 16, mby * 16, cs, ds);
+        la_inter_cost<true>(s, active, hx * 2, hy * 2, 2, cost, mx, my);
     }
     if (active && s.gl == 0) {
         b.inter[gm] = cost < ic ? cost : ic;
@@ -327,10 +279,7 @@ constexpr int LA_WARPS = 4;
 // walk column 0 of frames 1+2t+g and publish flag (f-1)*mb_h + y after MB
 // (0, y); later tickets take rows 2p and 2p+1 of the row order (rows in
 // order, frames interleaved), each group waiting for its own column-0 flag
-// and walking columns 1.. seeded by the left neighbour.  In HalfRes mode each
-// chain's next block window is copied (TMA, lane 0 of the group) while the
-// current block is searched; every copy issued is waited for (bounded,
-// status 3) before the block that reads it.
+// and walking columns 1.. seeded by the left neighbour.
 // Several streams' lookaheads in one launch: stream s's column tickets are
 // col0[s] .. col0[s+1]-1, all of them before any stream's row tickets
 // (rowt0[s] .. rowt0[s+1]-1 after col0[ns]), so a row ticket's column chain
@@ -351,33 +300,9 @@ __global__ void __launch_bounds__(32 * LA_WARPS, 4) la_chains_kernel(const __gri
                                                                  int epoch, int* __restrict__ status, int spin_limit) {
     __shared__ int2 cs[LA_WARPS][32];
     __shared__ int ds[LA_WARPS][32];
-    __shared__ __align__(8) unsigned long long la_bar[LA_WARPS][2][2];
     const int w = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int grp = lane >> 4, gl = lane & 15;
-    const int buf0 = ((w * 2 + grp) * 2) * LA_WIN_BUF;  // this chain's two buffers in la_win
-    const uint32_t win0 = uint32_t(__cvta_generic_to_shared(la_win)) + uint32_t(buf0);
-    const uint32_t bar0 = uint32_t(__cvta_generic_to_shared(&la_bar[w][grp][0]));
-    if (gl == 0) {
-        mbar_init(bar0, 1);
-        mbar_init(bar0 + 8, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
-    uint32_t parity = 0;  // bit k: the phase buffer k completes next
-    // window of block (mbx, mby) of frame f into buffer k (lane 0 of the group);
-    // the group's earlier reads of the buffer are complete (converged warp)
-    auto issue = [&](const LaBufs& b, int k, int f, int mbx, int mby) {
-        if (gl == 0) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_expect_tx(bar0 + 8 * k, uint32_t(LA_WIN_BYTES));
-            tma_load_3d(win0 + uint32_t(k * LA_WIN_BUF), &b.hmap, la_win_x0(mbx), mby * 8 - 16, f - 1, bar0 + 8 * k);
-        }
-    };
-    auto wait = [&](int k) {
-        wait_window(bar0 + 8 * k, (parity >> k) & 1u, status, 3, spin_limit);
-        parity ^= 1u << k;
-    };
     const int ns = lm.ns;
     for (;;) {
         int t = 0;
@@ -391,15 +316,10 @@ __global__ void __launch_bounds__(32 * LA_WARPS, 4) la_chains_kernel(const __gri
             const int nf = b.n - 1;
             const int f = 1 + 2 * (t - lm.col0[sidx]) + grp;
             const bool active = f <= nf;
-            const bool uw = active && b.hmap_ok;
-            if (uw) issue(b, 0, f, 0, 0);
             int sx = 0, sy = 0;
             for (int mby = 0; mby < b.mb_h; mby++) {
-                const int k = mby & 1;
-                if (uw && mby + 1 < b.mb_h) issue(b, k ^ 1, f, 0, mby + 1);
-                if (uw) wait(k);
                 int mx, my;
-                la_mb<MODE>(b, active, active ? f : 1, 0, mby, sx, sy, cs[w], ds[w], uw ? buf0 + k * LA_WIN_BUF : -1, mx, my);
+                la_mb<MODE>(b, active, active ? f : 1, 0, mby, sx, sy, cs[w], ds[w], mx, my);
                 sx = mx;
                 sy = my;
                 if (active && gl == 0) st_release(flags + (f - 1) * b.mb_h + mby, epoch);  // after the lane's MV store
@@ -417,21 +337,311 @@ __global__ void __launch_bounds__(32 * LA_WARPS, 4) la_chains_kernel(const __gri
         const long long nrows = (long long)nf * b.mb_h;
         const long long r = 2 * (tr - lm.rowt0[sidx]) + grp;
         const bool active = r < nrows;
-        const bool uw = active && b.hmap_ok && b.mb_w > 1;
         const int mby = active ? int(r / nf) : 0, f = active ? 1 + int(r % nf) : 1;
-        if (uw) issue(b, 0, f, 1, mby);  // the window is an input: no need to wait for column 0
         if (active && gl == 0) wait_flag(flags + (f - 1) * b.mb_h + mby, epoch, status, 1, spin_limit);
         __syncwarp();
         const long long gm0 = (long long)b.mb_w * b.mb_h * f + (long long)mby * b.mb_w;
         int sx = active ? __ldcg(b.mvs + 2 * gm0) : 0, sy = active ? __ldcg(b.mvs + 2 * gm0 + 1) : 0;
         for (int mbx = 1; mbx < b.mb_w; mbx++) {
-            const int k = (mbx - 1) & 1;
-            if (uw && mbx + 1 < b.mb_w) issue(b, k ^ 1, f, mbx + 1, mby);
-            if (uw) wait(k);
             int mx, my;
-            la_mb<MODE>(b, active, f, mbx, mby, sx, sy, cs[w], ds[w], uw ? buf0 + k * LA_WIN_BUF : -1, mx, my);
+            la_mb<MODE>(b, active, f, mbx, mby, sx, sy, cs[w], ds[w], mx, my);
             sx = mx;
             sy = my;
+            __syncwarp();
+        }
+    }
+}
+
+// ---- HalfRes ------------------------------------------------------------------
+// The search of an 8x8 half-res block by a whole warp, eight candidates a
+// round on the tensor cores (satd_mma.cuh): candidate c is column c of four
+// mmas, one per 4x4 block, lane l holding row l % 4 of candidate l / 4's
+// blocks; a candidate's sum (<= 65,280) is half a word, so three shuffles
+// reduce two candidates at once.
+//
+// The diamond evaluates its points one after the other and moves at the first
+// improvement, so the points that follow while nothing improves are known:
+// a round prices the next eight of that list (the rest of the ring, then the
+// following steps' rings), takes its first improvement and forgets what came
+// after it.  The first round is (0,0), the seed and the first six points
+// around the seed.  A block that keeps its seed takes three rounds.
+//
+// Bound by a chain's serial latency (a 1080p frame: 68 blocks down column 0,
+// then 119 along the last row), so everything else stays off it: the next
+// block's source and intra cost are loaded a block ahead, the reference
+// windows two copies ahead (TMA; along a row two blocks share a window).  60
+// 1080p frames: 1,216 us with 16 lanes a chain through shared-memory slots,
+// one ring a round; LA_US this way.
+//
+// Windows: LA_BUFS buffers a chain of LA_WIN_H rows of LA_WIN_W bytes, the
+// block +-16 rows, and 48 columns from the 16-byte boundary at or left of the
+// block's x - 16.  A candidate outside the picture reads clamped coordinates;
+// one whose clamped rows or columns lie outside the window reads the picture.
+constexpr int LA_HWARPS = 4, LA_BUFS = 3;
+constexpr int LA_WIN_W = 48, LA_WIN_H = 40, LA_WIN_BYTES = LA_WIN_W * LA_WIN_H;
+constexpr int LA_WIN_BUF = 2048;  // buffer stride: 128-byte aligned, with room for a row read's further words
+extern __shared__ __align__(128) uint8_t la_win[];
+
+__device__ __noinline__ uint32_t la_clamped_word(const uint8_t* ref, int w, int h, int x, int y) {
+    const uint8_t* row = ref + (long long)clampi(y, 0, h - 1) * w;
+    uint32_t v = 0;
+#pragma unroll
+    for (int c = 0; c < 4; c++) v |= uint32_t(__ldg(row + clampi(x + c, 0, w - 1))) << (8 * c);
+    return v;
+}
+
+// Point `pos` of the list that follows while nothing improves, from ring point
+// 0 of the ring at `step` on; `moved`: that ring is walked again at its step.
+__device__ __forceinline__ int la_list_step(int step, bool moved, int pos) {
+    const int ring = pos >> 2;
+    return step >> (ring - (moved && ring > 0 ? 1 : 0));
+}
+
+struct LaBlock {
+    const uint8_t* ref;
+    int w, h, x0, y0;
+    const uint8_t* win;  // null: none
+    int wx0, wy0;
+    bool edge;  // the window reaches outside the picture
+    uint32_t src[4];
+};
+
+// SATD of the lane's candidate column (full-pel offset dx, dy): candidates 2q
+// (low half) and 2q + 1 (high half) of lane q = lane % 4, in every lane
+__device__ __forceinline__ uint32_t la_price(const HadFrag& hf, const LaBlock& b, int dx, int dy) {
+    const int r = threadIdx.x & 3;
+    const int x = b.x0 + dx, y = b.y0 + dy + r;
+    uint32_t p[4];
+    bool ok = false;
+    if (b.win != nullptr) {
+        if (!b.edge) {
+            const int cx = x - b.wx0, cy = y - b.wy0;
+            ok = unsigned(cx) <= unsigned(LA_WIN_W - 8) && unsigned(cy) < unsigned(LA_WIN_H - 4);
+            if (ok) {
+                const int a = cy * LA_WIN_W + cx;
+                const uint32_t* w0 = reinterpret_cast<const uint32_t*>(b.win + (a & ~3));
+                const uint32_t* w1 = w0 + LA_WIN_W;  // four rows down
+                const uint32_t sh = uint32_t(a & 3) * 8u;
+                const uint32_t m0 = w0[1], m1 = w1[1];
+                p[0] = __funnelshift_r(w0[0], m0, sh);
+                p[1] = __funnelshift_r(m0, w0[2], sh);
+                p[2] = __funnelshift_r(w1[0], m1, sh);
+                p[3] = __funnelshift_r(m1, w1[2], sh);
+            }
+        } else {
+            const int xa = clampi(x, 0, b.w - 4), xb = clampi(x + 4, 0, b.w - 4);
+            const int ya = clampi(y, 0, b.h - 1) - b.wy0, yb = clampi(y + 4, 0, b.h - 1) - b.wy0;
+            ok = unsigned(xa - b.wx0) <= unsigned(LA_WIN_W - 4) && unsigned(xb - b.wx0) <= unsigned(LA_WIN_W - 4) &&
+                 unsigned(ya) < unsigned(LA_WIN_H) && unsigned(yb) < unsigned(LA_WIN_H);
+            if (ok) {
+                // byte i of a clamped word is byte clamp(i + x - xa, 0, 3) of the word at xa
+                const uint32_t sa = __funnelshift_r(0x33210000u, 0x33u, uint32_t(4 * (clampi(x - xa, -3, 3) + 3)));
+                const uint32_t sb = __funnelshift_r(0x33210000u, 0x33u, uint32_t(4 * (clampi(x + 4 - xb, -3, 3) + 3)));
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int a = ((i & 2) ? yb : ya) * LA_WIN_W + ((i & 1) ? xb : xa) - b.wx0;
+                    const uint32_t* wp = reinterpret_cast<const uint32_t*>(b.win + (a & ~3));
+                    p[i] = __byte_perm(__funnelshift_r(wp[0], wp[1], uint32_t(a & 3) * 8u), 0u, (i & 1) ? sb : sa);
+                }
+            }
+        }
+    }
+    if (!ok) {
+#pragma unroll 1
+        for (int i = 0; i < 4; i++) {
+            const uint32_t v = la_clamped_word(b.ref, b.w, b.h, x + 4 * (i & 1), y + 4 * (i >> 1));
+            p[0] = i == 0 ? v : p[0];
+            p[1] = i == 1 ? v : p[1];
+            p[2] = i == 2 ? v : p[2];
+            p[3] = i == 3 ? v : p[3];
+        }
+    }
+    __syncwarp();
+    int s0 = 0, s1 = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) had_mma(hf, p[i], b.src[i], s0, s1);
+    uint32_t v = uint32_t(s0) | uint32_t(s1) << 16;
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// inter_cost (mbtree.rs:154-197), as la_inter_cost above; seed and result in
+// full pixels.  (The reference's bound on walks of one ring cannot be reached:
+// each follows an improvement of a cost below 2^16.)
+__device__ __forceinline__ void la_half_search(const HadFrag& hf, const LaBlock& b, int seedx, int seedy, int& cost,
+                                               int& mvx, int& mvy) {
+    const int lane = threadIdx.x & 31, c = lane >> 2, qa = 2 * (lane & 3);
+    int bx = seedx, by = seedy, step = 8, ri = 0, base = 2;
+    bool moved = false;
+    uint32_t best = 0;
+    for (bool first = true;; first = false) {
+        // the lane's candidate
+        int dx = bx, dy = by;
+        {
+            const int pos = ri + c - base, st = la_list_step(step, moved, pos), k = pos & 3;
+            if (c >= base) {
+                dx += la_ring_dx(k) * st;
+                dy += la_ring_dy(k) * st;
+            } else if (c == 0) {
+                dx = dy = 0;
+            }
+        }
+        const uint32_t v = la_price(hf, b, dx, dy);
+        if (first) {
+            const uint32_t v0 = __shfl_sync(0xffffffffu, v, 0);
+            best = v0 & 0xffffu;
+            if (best == 0) {
+                bx = by = 0;
+                break;
+            }
+            if (bx != 0 || by != 0) {
+                if ((v0 >> 16) < best) {
+                    best = v0 >> 16;
+                } else {  // the points around the seed do not count
+                    bx = by = 0;
+                    base = 0;
+                    continue;
+                }
+            }
+        }
+        // the first improvement of the list
+        const bool ha = qa >= base && la_list_step(step, moved, ri + qa - base) > 0 && (v & 0xffffu) < best;
+        const bool hb = qa + 1 >= base && la_list_step(step, moved, ri + qa + 1 - base) > 0 && (v >> 16) < best;
+        const int hit = int(__reduce_min_sync(0xffffffffu, ha ? unsigned(qa) : (hb ? unsigned(qa + 1) : 8u)));
+        const int pos = ri + hit - base;  // no improvement (8): the list's next point
+        const bool old = moved && (pos >> 2) == 0;
+        step = la_list_step(step, moved, pos);
+        ri = pos & 3;
+        moved = old;
+        if (hit < 8) {
+            const uint32_t d = __shfl_sync(0xffffffffu, v, hit >> 1);
+            best = (hit & 1) ? d >> 16 : d & 0xffffu;
+            bx += la_ring_dx(ri) * step;
+            by += la_ring_dy(ri) * step;
+            moved = ri != 3;  // after its last point the ring is walked again
+            ri = (ri + 1) & 3;
+        } else if (step == 0) {
+            break;
+        }
+        base = 0;
+    }
+    cost = int(best);
+    mvx = bx;
+    mvy = by;
+}
+
+// Column-0 chains and row chains in one persistent launch, one per warp:
+// tickets as la_chains_kernel's, chain by chain.
+__global__ void __launch_bounds__(32 * LA_HWARPS, 8) la_half_kernel(const __grid_constant__ LaMulti lm, int* __restrict__ counter,
+                                                                    int* __restrict__ flags0, int epoch,
+                                                                    int* __restrict__ status, int spin_limit) {
+    __shared__ __align__(8) unsigned long long la_bar[LA_HWARPS][LA_BUFS];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    uint8_t* win = la_win + wp * LA_BUFS * LA_WIN_BUF;
+    const uint32_t win0 = uint32_t(__cvta_generic_to_shared(win));
+    const uint32_t bar0 = uint32_t(__cvta_generic_to_shared(&la_bar[wp][0]));
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < LA_BUFS; i++) mbar_init(bar0 + 8 * i, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    const HadFrag hf = had_frag(lane);
+    uint32_t parity = 0;  // bit k: the phase buffer k completes next
+    const int ns = lm.ns;
+    for (;;) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(counter, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        const bool col = t < lm.col0[ns];
+        const long long tr = (long long)t - lm.col0[ns];
+        if (!col && tr >= lm.rowt0[ns]) return;
+        int sidx = 0;
+        if (col)
+            while (sidx + 1 < ns && lm.col0[sidx + 1] <= t) sidx++;
+        else
+            while (sidx + 1 < ns && lm.rowt0[sidx + 1] <= tr) sidx++;
+        const LaBufs& b = lm.b[sidx];
+        int* flags = flags0 + lm.flag0[sidx];
+        const int nf = b.n - 1, mbw = b.mb_w, mbh = b.mb_h;
+        const int r = col ? 0 : int(tr - lm.rowt0[sidx]);
+        const int f = col ? 1 + t - lm.col0[sidx] : 1 + r % nf, row = col ? 0 : r / nf;
+        // the chain's blocks: (0, i), or (i, row) from i = 1 on; its windows:
+        // one per block, or one per two columns
+        const int i0 = col ? 0 : 1, ni = col ? mbh : mbw, wshift = col ? 0 : 1, nw = (ni + wshift) >> wshift;
+        if (i0 >= ni) continue;
+        LaBlock blk;
+        blk.w = b.cw / 2;
+        blk.h = b.ch / 2;
+        const size_t hs = size_t(blk.w) * blk.h;
+        const uint8_t* cur = b.half + hs * f;
+        blk.ref = cur - hs;
+        const bool uw = b.hmap_ok != 0;
+        auto issue = [&](int wn) {  // window wn into its buffer, whose earlier reads are complete
+            __syncwarp();
+            if (lane == 0) {
+                const uint32_t bar = bar0 + 8 * (wn % LA_BUFS);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                mbar_expect_tx(bar, uint32_t(LA_WIN_BYTES));
+                tma_load_3d(win0 + uint32_t(wn % LA_BUFS * LA_WIN_BUF), &b.hmap, col ? -16 : 16 * wn - 16,
+                            (col ? 8 * wn : 8 * row) - 16, f - 1, bar);
+            }
+        };
+        if (uw)
+            for (int k = 0; k < LA_BUFS - 1 && k < nw; k++) issue(k);
+        const int q = lane & 3;
+        const uint8_t* sp = cur + (long long)(col ? 0 : 8 * row + 0) * blk.w + (col ? 0 : 8 * i0) + (long long)q * blk.w;
+        const long long sstep = col ? 8LL * blk.w : 8;
+        uint32_t nsrc[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) nsrc[i] = ld4u(sp + (long long)(4 * (i >> 1)) * blk.w + 4 * (i & 1));
+        const long long gm0 = (long long)mbw * mbh * f + (long long)row * mbw;
+        int nic = __ldg(b.intra + gm0 + i0);
+        int sx = 0, sy = 0;
+        if (!col) {
+            if (lane == 0) wait_flag(flags + (f - 1) * mbh + row, epoch, status, 1, spin_limit);
+            __syncwarp();
+            sx = __ldcg(b.mvs + 2 * gm0) / 8;
+            sy = __ldcg(b.mvs + 2 * gm0 + 1) / 8;
+        }
+        int wn = -1;
+        for (int i = i0; i < ni; i++) {
+            const int ic = nic;
+#pragma unroll
+            for (int k = 0; k < 4; k++) blk.src[k] = nsrc[k];
+            const long long gm = col ? gm0 + (long long)i * mbw : gm0 + i;
+            if (i + 1 < ni) {
+                sp += sstep;
+#pragma unroll
+                for (int k = 0; k < 4; k++) nsrc[k] = ld4u(sp + (long long)(4 * (k >> 1)) * blk.w + 4 * (k & 1));
+                nic = __ldg(b.intra + gm + (col ? mbw : 1));
+            }
+            blk.x0 = col ? 0 : 8 * i;
+            blk.y0 = col ? 8 * i : 8 * row;
+            if ((i >> wshift) != wn) {
+                wn = i >> wshift;
+                blk.wx0 = col ? -16 : 16 * wn - 16;
+                blk.wy0 = blk.y0 - 16;
+                blk.edge = blk.wx0 < 0 || blk.wy0 < 0 || blk.wx0 + LA_WIN_W > blk.w || blk.wy0 + LA_WIN_H > blk.h;
+                blk.win = uw ? win + wn % LA_BUFS * LA_WIN_BUF : nullptr;
+                if (uw) {
+                    if (wn + LA_BUFS - 1 < nw) issue(wn + LA_BUFS - 1);
+                    wait_window(bar0 + 8 * (wn % LA_BUFS), (parity >> (wn % LA_BUFS)) & 1u, status, 3, spin_limit);
+                    parity ^= 1u << (wn % LA_BUFS);
+                    __syncwarp();
+                }
+            }
+            int cost, mx, my;
+            la_half_search(hf, blk, sx, sy, cost, mx, my);
+            sx = mx;
+            sy = my;
+            if (lane == 0) {
+                b.inter[gm] = cost < ic ? cost : ic;
+                b.mvs[2 * gm] = mx * 8;
+                b.mvs[2 * gm + 1] = my * 8;
+                if (col) st_release(flags + (f - 1) * mbh + i, epoch);  // after the lane's MV store
+            }
             __syncwarp();
         }
     }
@@ -494,8 +704,9 @@ int la_run(h264a_ctx* ctx, const h264a_la_stream* qs, int nq, int mode, cudaStre
         const int rc = check_launch("la_intra_kernel");
         if (rc) return rc;
     }
-    const int smem = LA_WARPS * 2 * 2 * LA_WIN_BUF;  // two window buffers per chain
-    auto kern = mode == 0 ? la_chains_kernel<0> : (mode == 1 ? la_chains_kernel<1> : la_chains_kernel<2>);
+    const int smem = mode == 2 ? LA_HWARPS * LA_BUFS * LA_WIN_BUF : 0;
+    const int wpc = mode == 2 ? LA_HWARPS : LA_WARPS, cpw = mode == 2 ? 1 : 2;  // warps per CTA, chains per warp
+    auto kern = mode == 0 ? la_chains_kernel<0> : (mode == 1 ? la_chains_kernel<1> : la_half_kernel);
     for (int s0 = 0; s0 < nq; s0 += LA_MAXS) {
         LaMulti* lm = new LaMulti;
         memset(lm, 0, sizeof *lm);
@@ -506,8 +717,8 @@ int la_run(h264a_ctx* ctx, const h264a_la_stream* qs, int nq, int mode, cudaStre
             const int nf = qs[i].n - 1;
             const long long nrows = (long long)nf * (qs[i].ch / 16);
             lm->b[k] = bufs[i];
-            lm->col0[k + 1] = lm->col0[k] + (nf + 1) / 2;
-            lm->rowt0[k + 1] = lm->rowt0[k] + (nrows + 1) / 2;
+            lm->col0[k + 1] = lm->col0[k] + (nf + cpw - 1) / cpw;
+            lm->rowt0[k + 1] = lm->rowt0[k] + (nrows + cpw - 1) / cpw;
             lm->flag0[k] = flags;
             flags += nrows;
         }
@@ -515,7 +726,7 @@ int la_run(h264a_ctx* ctx, const h264a_la_stream* qs, int nq, int mode, cudaStre
             delete lm;
             continue;
         }
-        const long long chains = lm->col0[lm->ns] + lm->rowt0[lm->ns];  // two chains per warp
+        const long long chains = lm->col0[lm->ns] + lm->rowt0[lm->ns];  // tickets
         int rc = flags > (1LL << 30) ? fail(H264A_E_ARG, "lookahead_costs: too many rows") : H264A_OK;
         if (!rc) rc = ensure_me_scratch(ctx, size_t(flags), Q_LOOKAHEAD);
         if (!rc && cudaMemsetAsync(ctx->q[Q_LOOKAHEAD].d_counter, 0, sizeof(int32_t), st) != cudaSuccess)
@@ -523,13 +734,13 @@ int la_run(h264a_ctx* ctx, const h264a_la_stream* qs, int nq, int mode, cudaStre
         const int epoch = rc ? -1 : next_epoch(ctx, st, Q_LOOKAHEAD);
         if (!rc && epoch < 0) rc = H264A_E_CUDA;
         int per_sm = 0;
-        if (!rc && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * LA_WARPS, smem) != cudaSuccess)
+        if (!rc && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * wpc, smem) != cudaSuccess)
             rc = cuda_fail(cudaGetLastError(), "lookahead_costs: occupancy");
         if (!rc) {
             long long blocks = (long long)ctx->num_sms * (per_sm > 0 ? per_sm : 1);
-            const long long need = (chains + LA_WARPS - 1) / LA_WARPS;
+            const long long need = (chains + wpc - 1) / wpc;
             if (blocks > need) blocks = need;
-            kern<<<unsigned(blocks), 32 * LA_WARPS, smem, st>>>(*lm, ctx->q[Q_LOOKAHEAD].d_counter,
+            kern<<<unsigned(blocks), 32 * wpc, smem, st>>>(*lm, ctx->q[Q_LOOKAHEAD].d_counter,
                                                                 ctx->q[Q_LOOKAHEAD].d_flags, epoch, ctx->d_status,
                                                                 SPIN_LIMIT);
             rc = check_launch("la_chains_kernel");
