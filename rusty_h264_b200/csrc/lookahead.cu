@@ -371,7 +371,8 @@ __global__ void __launch_bounds__(32 * LA_WARPS, 4) la_chains_kernel(const __gri
 // block's source and intra cost are loaded a block ahead, the reference
 // windows two copies ahead (TMA; along a row two blocks share a window).  60
 // 1080p frames: 1,216 us with 16 lanes a chain through shared-memory slots,
-// one ring a round; LA_US this way.
+// one ring a round; 451 this way (five CTAs an SM; eight, with 64 registers a
+// thread, 631: every row resident, most of them waiting).
 //
 // Windows: LA_BUFS buffers a chain of LA_WIN_H rows of LA_WIN_W bytes, the
 // block +-16 rows, and 48 columns from the 16-byte boundary at or left of the
@@ -390,11 +391,18 @@ __device__ __noinline__ uint32_t la_clamped_word(const uint8_t* ref, int w, int 
     return v;
 }
 
-// Point `pos` of the list that follows while nothing improves, from ring point
-// 0 of the ring at `step` on; `moved`: that ring is walked again at its step.
+// Point `pos` (0 .. 10) of the list that follows while nothing improves, from
+// ring point 0 of the ring at `step` on: its step (0 past the end).  `moved`:
+// that ring is walked again at its step.
 __device__ __forceinline__ int la_list_step(int step, bool moved, int pos) {
     const int ring = pos >> 2;
-    return step >> (ring - (moved && ring > 0 ? 1 : 0));
+    return step >> (moved && ring > 0 ? ring - 1 : ring);
+}
+// Adds ring point k at step st
+__device__ __forceinline__ void la_ring_add(int k, int st, int& x, int& y) {
+    const int s = (k & 1) ? -st : st;
+    x += (k & 2) ? 0 : s;
+    y += (k & 2) ? s : 0;
 }
 
 struct LaBlock {
@@ -402,19 +410,18 @@ struct LaBlock {
     int w, h, x0, y0;
     const uint8_t* win;  // null: none
     int wx0, wy0;
-    bool edge;  // the window reaches outside the picture
+    int mode;  // 0 no window, 1 the window reaches outside the picture, 2 it does not
     uint32_t src[4];
 };
 
 // SATD of the lane's candidate column (full-pel offset dx, dy): candidates 2q
 // (low half) and 2q + 1 (high half) of lane q = lane % 4, in every lane
 __device__ __forceinline__ uint32_t la_price(const HadFrag& hf, const LaBlock& b, int dx, int dy) {
-    const int r = threadIdx.x & 3;
-    const int x = b.x0 + dx, y = b.y0 + dy + r;
+    const int x = b.x0 + dx, y = b.y0 + dy + int(threadIdx.x & 3);
     uint32_t p[4];
     bool ok = false;
-    if (b.win != nullptr) {
-        if (!b.edge) {
+    if (b.mode != 0) {
+        if (b.mode == 2) {
             const int cx = x - b.wx0, cy = y - b.wy0;
             ok = unsigned(cx) <= unsigned(LA_WIN_W - 8) && unsigned(cy) < unsigned(LA_WIN_H - 4);
             if (ok) {
@@ -466,65 +473,59 @@ __device__ __forceinline__ uint32_t la_price(const HadFrag& hf, const LaBlock& b
     return v;
 }
 
+// Takes the first improvement of a round's list, whose point 0 is candidate
+// `base`, or goes past it.  (Candidates before `base` and past the list's end
+// cost no less than `best`: they are what `best` is the least of, and the
+// centre again.)
+__device__ __forceinline__ void la_take(uint32_t v, int qa, int base, int& bx, int& by, int& step, int& ri, bool& moved,
+                                        uint32_t& best) {
+    const unsigned mine = (v & 0xffffu) < best ? unsigned(qa) : ((v >> 16) < best ? unsigned(qa + 1) : 8u);
+    const int hit = int(__reduce_min_sync(0xffffffffu, mine));
+    const int pos = ri + hit - base;
+    step = la_list_step(step, moved, pos);
+    moved = moved && pos < 4;
+    ri = pos & 3;
+    if (hit < 8) {
+        const uint32_t d = __shfl_sync(0xffffffffu, v, hit >> 1);
+        best = (hit & 1) ? d >> 16 : d & 0xffffu;
+        la_ring_add(ri, step, bx, by);
+        moved = ri != 3;  // after its last point the ring is walked again
+        ri = (ri + 1) & 3;
+    }
+}
+
 // inter_cost (mbtree.rs:154-197), as la_inter_cost above; seed and result in
 // full pixels.  (The reference's bound on walks of one ring cannot be reached:
 // each follows an improvement of a cost below 2^16.)
 __device__ __forceinline__ void la_half_search(const HadFrag& hf, const LaBlock& b, int seedx, int seedy, int& cost,
                                                int& mvx, int& mvy) {
     const int lane = threadIdx.x & 31, c = lane >> 2, qa = 2 * (lane & 3);
-    int bx = seedx, by = seedy, step = 8, ri = 0, base = 2;
+    int bx = seedx, by = seedy, step = 8, ri = 0;
     bool moved = false;
     uint32_t best = 0;
-    for (bool first = true;; first = false) {
-        // the lane's candidate
-        int dx = bx, dy = by;
-        {
-            const int pos = ri + c - base, st = la_list_step(step, moved, pos), k = pos & 3;
-            if (c >= base) {
-                dx += la_ring_dx(k) * st;
-                dy += la_ring_dy(k) * st;
-            } else if (c == 0) {
-                dx = dy = 0;
-            }
-        }
+    {
+        const int pos = max(c - 2, 0);
+        int dx = c == 0 ? 0 : bx, dy = c == 0 ? 0 : by;
+        la_ring_add(pos & 3, c < 2 ? 0 : 8 >> (pos >> 2), dx, dy);
         const uint32_t v = la_price(hf, b, dx, dy);
-        if (first) {
-            const uint32_t v0 = __shfl_sync(0xffffffffu, v, 0);
-            best = v0 & 0xffffu;
-            if (best == 0) {
-                bx = by = 0;
-                break;
-            }
-            if (bx != 0 || by != 0) {
-                if ((v0 >> 16) < best) {
-                    best = v0 >> 16;
-                } else {  // the points around the seed do not count
-                    bx = by = 0;
-                    base = 0;
-                    continue;
-                }
-            }
+        const uint32_t v0 = __shfl_sync(0xffffffffu, v, 0);
+        best = v0 & 0xffffu;
+        if (best == 0) {
+            cost = mvx = mvy = 0;
+            return;
         }
-        // the first improvement of the list
-        const bool ha = qa >= base && la_list_step(step, moved, ri + qa - base) > 0 && (v & 0xffffu) < best;
-        const bool hb = qa + 1 >= base && la_list_step(step, moved, ri + qa + 1 - base) > 0 && (v >> 16) < best;
-        const int hit = int(__reduce_min_sync(0xffffffffu, ha ? unsigned(qa) : (hb ? unsigned(qa + 1) : 8u)));
-        const int pos = ri + hit - base;  // no improvement (8): the list's next point
-        const bool old = moved && (pos >> 2) == 0;
-        step = la_list_step(step, moved, pos);
-        ri = pos & 3;
-        moved = old;
-        if (hit < 8) {
-            const uint32_t d = __shfl_sync(0xffffffffu, v, hit >> 1);
-            best = (hit & 1) ? d >> 16 : d & 0xffffu;
-            bx += la_ring_dx(ri) * step;
-            by += la_ring_dy(ri) * step;
-            moved = ri != 3;  // after its last point the ring is walked again
-            ri = (ri + 1) & 3;
-        } else if (step == 0) {
-            break;
+        if ((bx | by) == 0 || (v0 >> 16) < best) {
+            best = min(best, v0 >> 16);
+            la_take(v, qa, 2, bx, by, step, ri, moved, best);
+        } else {
+            bx = by = 0;  // the points around the seed do not count
         }
-        base = 0;
+    }
+    while (step > 0) {
+        const int pos = ri + c;
+        int dx = bx, dy = by;
+        la_ring_add(pos & 3, la_list_step(step, moved, pos), dx, dy);
+        la_take(la_price(hf, b, dx, dy), qa, 0, bx, by, step, ri, moved, best);
     }
     cost = int(best);
     mvx = bx;
@@ -533,7 +534,7 @@ __device__ __forceinline__ void la_half_search(const HadFrag& hf, const LaBlock&
 
 // Column-0 chains and row chains in one persistent launch, one per warp:
 // tickets as la_chains_kernel's, chain by chain.
-__global__ void __launch_bounds__(32 * LA_HWARPS, 8) la_half_kernel(const __grid_constant__ LaMulti lm, int* __restrict__ counter,
+__global__ void __launch_bounds__(32 * LA_HWARPS, 5) la_half_kernel(const __grid_constant__ LaMulti lm, int* __restrict__ counter,
                                                                     int* __restrict__ flags0, int epoch,
                                                                     int* __restrict__ status, int spin_limit) {
     __shared__ __align__(8) unsigned long long la_bar[LA_HWARPS][LA_BUFS];
@@ -623,8 +624,9 @@ __global__ void __launch_bounds__(32 * LA_HWARPS, 8) la_half_kernel(const __grid
                 wn = i >> wshift;
                 blk.wx0 = col ? -16 : 16 * wn - 16;
                 blk.wy0 = blk.y0 - 16;
-                blk.edge = blk.wx0 < 0 || blk.wy0 < 0 || blk.wx0 + LA_WIN_W > blk.w || blk.wy0 + LA_WIN_H > blk.h;
-                blk.win = uw ? win + wn % LA_BUFS * LA_WIN_BUF : nullptr;
+                blk.mode = !uw ? 0
+                           : blk.wx0 < 0 || blk.wy0 < 0 || blk.wx0 + LA_WIN_W > blk.w || blk.wy0 + LA_WIN_H > blk.h ? 1 : 2;
+                blk.win = win + wn % LA_BUFS * LA_WIN_BUF;
                 if (uw) {
                     if (wn + LA_BUFS - 1 < nw) issue(wn + LA_BUFS - 1);
                     wait_window(bar0 + 8 * (wn % LA_BUFS), (parity >> (wn % LA_BUFS)) & 1u, status, 3, spin_limit);
