@@ -123,8 +123,8 @@ __device__ __forceinline__ bf16_t mv_feat(const Geo& g, int m, int i) {
 }
 
 // ---- the tcgen05 GEMM: 128 x BN tiles, accumulators in tensor memory --------
-// The GEMM of conv2 to the head and of every data gradient, C[M][N] = sum_k
-// A[m][k] B[k][n], on the sm_100 tensor cores: per 64-wide K step all 256
+// The GEMM of FC1, the head and their data gradients, C[M][N] = sum_k A[m][k]
+// B[k][n], on the sm_100 tensor cores: per 64-wide K step all 256
 // threads copy the A (MT x 128 x 64) and B (BN x 64) tiles by 16-byte cp.async
 // into one of ST shared-memory stages (steps it + 1 .. it + ST - 1 are in flight
 // while step it multiplies), one thread issues four tcgen05.mma (M 128, N BN,
@@ -136,8 +136,8 @@ __device__ __forceinline__ bf16_t mv_feat(const Geo& g, int m, int i) {
 // registers, 32 rows a request, it took longer than the products (head 27,000
 // of a CTA's 45,000 cycles).  Bound by the operands' way through the L2 (five
 // or so TB/s over both dies).  Four 1080p pairs, before (operands through
-// registers) and now: FC1 85 -> 61 us, head 48 -> 32, conv3 36 -> 30, data
-// gradients of conv3 51 -> 37, FC1 128 -> 89.
+// registers) and now: FC1 85 -> 61 us, head 48 -> 32, FC1's data gradient
+// 128 -> 89.
 constexpr int TC_BM = 128, TC_BK = 64, TC_THREADS = 256;
 
 template <int BN>
@@ -360,6 +360,141 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const Op op, int M,
             if (m0 + row < M && n < N) op.store(tc_out[row], n, ld16s(sbase + uint32_t(row * PITCH + ch * 16)));
         }
     }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOL));
+}
+
+// The GEMMs of few columns and a short K (conv2, conv3 and their data
+// gradients: N <= 128, at most KT = 2 .. 5 steps), persistent: a CTA keeps the
+// whole B in shared memory and walks row tiles, its ring of ST stages of A
+// running on from one tile into the next and its accumulators in two sets, so
+// a tile's loads, products and results overlap its neighbours'.  (A CTA per
+// tile spent most of its time on its own start: row table, tensor memory,
+// first loads, then results with nothing behind them.)  Bound by the 16-byte
+// gathers (conv2 reads each input cell 2.25 times).  Four 1080p pairs, a CTA
+// per tile and persistent: conv2 67 -> 57 us, conv3 30 -> 29, conv3's data
+// gradient 37 -> 32, conv2's 83 -> 84.
+template <int BN, int KT, int ST>
+constexpr int conv_smem() {
+    return KT * BN * TC_BK * 2 + ST * TC_BM * TC_BK * 2 + TC_BM * (BN * 2 + 16);
+}
+template <int BN, int KT, int ST, class Op>
+__global__ void __launch_bounds__(TC_THREADS) conv_tc_kernel(const Op op, int M, int K, int* status) {
+    static_assert(BN % 32 == 0 && BN <= 128 && ST >= 2 && !Op::kCalc && !Op::kF32, "tile shape");
+    constexpr int A_BYTES = TC_BM * TC_BK * 2, B_STEP = BN * TC_BK * 2, NCOL = tc_cols<2 * BN>();
+    constexpr uint32_t IDESC = tc_idesc<BN>();
+    extern __shared__ __align__(128) uint8_t tc_smem[];
+    __shared__ __align__(8) unsigned long long tc_bar[ST + 2];  // stages, accumulator sets
+    __shared__ uint32_t tc_tmem;
+    __shared__ long long tc_out[2][TC_BM];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t sw = tc_smem_u32(tc_smem), sbase = sw + KT * B_STEP, sres = sbase + ST * A_BYTES;
+    const uint32_t bar0 = tc_smem_u32(&tc_bar[0]), tbar = bar0 + 8 * ST;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(&tc_tmem)),
+                     "r"(NCOL));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+#pragma unroll
+        for (int s = 0; s < ST + 2; s++) mbar_init(bar0 + 8 * s, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tc_tmem;
+    const int tiles = (M + TC_BM - 1) / TC_BM;
+    const int nt = (tiles - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x), steps = nt * KT;  // grid <= tiles: nt >= 1
+    auto tile_m0 = [&](int i) { return (int(blockIdx.x) + i * int(gridDim.x)) * TC_BM; };
+    constexpr int AQ = TC_BM * 8 / TC_THREADS;
+    const int c = (tid >> 3) & 7, r0 = ((tid >> 6) << 3) | (tid & 7);
+    const uint32_t off0 = tc_off(r0, c);
+    {
+        const bf16_t* bp = op.b(blockIdx.x % WREP);
+        for (int i = tid; i < BN * 8 * KT; i += TC_THREADS) {
+            const int n = ((i >> 6) << 3 | (i & 7)) % BN, ks = i / (BN * 8), ch = (i >> 3) & 7, k = ks * TC_BK + 8 * ch;
+            cp16z(sw + uint32_t(ks * B_STEP) + tc_off(n, ch), bp + n * Op::ldb + k, k < K, op.z.w);
+        }
+    }
+    typename Op::Row rows[AQ];
+    auto load = [&](int g) {  // in order of g
+        const int ks = g % KT;
+        if (ks == 0) {
+            const int m0 = tile_m0(g / KT);
+#pragma unroll
+            for (int j = 0; j < AQ; j++) rows[j] = op.row(min(m0 + r0 + 32 * j, M - 1));
+        }
+        const uint32_t sa = sbase + uint32_t((g % ST) * A_BYTES) + off0;
+        const int k = ks * TC_BK + 8 * c;
+        const typename Op::Step s = op.step(k);
+#pragma unroll
+        for (int j = 0; j < AQ; j++) stage_a8(op, sa + 4096u * j, rows[j], s, k < K);
+    };
+    auto results = [&](int i) {  // of the CTA's tile i, whose products are committed
+        constexpr int PITCH = BN * 2 + 16, CH = BN / 8;
+        tc_wait(tbar + 8 * (i & 1), uint32_t(i >> 1) & 1u, status);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t so = sres + uint32_t(((warp & 3) * 32 + lane) * PITCH);
+        const uint32_t taddr = tmem + uint32_t((i & 1) * BN) + (uint32_t((warp & 3) * 32) << 16);
+        const int cb = (warp >> 2) * (BN / 2);
+#pragma unroll 1
+        for (int c0 = cb; c0 < cb + BN / 2; c0 += 16) {
+            float f[16];
+            tc_ld16(taddr + uint32_t(c0), f);
+            st16s(so + uint32_t(c0) * 2, op.pack(c0, f));
+            st16s(so + uint32_t(c0) * 2 + 16, op.pack(c0 + 8, f + 8));
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        const int m0 = tile_m0(i);
+#pragma unroll 4
+        for (int j = tid; j < TC_BM * CH; j += TC_THREADS) {
+            const int row = j / CH, ch = j - row * CH;
+            if (m0 + row < M) op.store(tc_out[i & 1][row], 8 * ch, ld16s(sres + uint32_t(row * PITCH + ch * 16)));
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < ST - 1; s++) {
+        if (s < steps) load(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int i = 0, g = 0; i < nt; i++) {
+        for (int ks = 0; ks < KT; ks++, g++) {
+            const uint32_t sa = sbase + uint32_t((g % ST) * A_BYTES), sb = sw + uint32_t(ks * B_STEP);
+            asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();  // also: everyone has read tile i - 2's accumulators and results
+            if (tid == 0) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < TC_BK / 16; j++)
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(
+                            tmem + uint32_t((i & 1) * BN)),
+                        "l"(tc_sdesc(sa + 256u * j)), "l"(tc_sdesc(sb + 256u * j)), "r"(IDESC), "r"((ks > 0 || j > 0) ? 1u : 0u),
+                        "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+                        : "memory");
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar0 + 8 * (g % ST))
+                             : "memory");
+                if (ks == KT - 1)
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tbar + 8 * (i & 1))
+                                 : "memory");
+            }
+            if (ks == 0 && tid < TC_BM) tc_out[i & 1][tid] = op.out_at(min(tile_m0(i) + tid, M - 1));
+            if (g + ST - 1 < steps) {
+                // the stage's previous MMAs (step g - 1) have read it
+                if (g >= 1) tc_wait(bar0 + 8 * ((g - 1) % ST), uint32_t((g - 1) / ST) & 1u, status);
+                load(g + ST - 1);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        if (i > 0) results(i - 1);
+    }
+    __syncthreads();  // the last tile's row offsets, where KT = 1
+    results(nt - 1);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOL));
@@ -1112,6 +1247,19 @@ static void gemm(const Op& op, int M, int N, int K, cudaStream_t st) {
     gemm_tc_kernel<BN, MT, ST, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, nullptr);
 }
 
+template <int BN, int KT, int ST, class Op>
+static void conv_gemm(const Op& op, int M, int K, int sms, cudaStream_t st) {
+    constexpr int smem = conv_smem<BN, KT, ST>(), fit = 226 * 1024 / (smem + 4096), per_sm = fit < 4 ? fit : 4;
+    static_assert(per_sm >= 1 && per_sm * tc_cols<2 * BN>() <= 512, "shared and tensor memory");
+    static const bool attr_ok = [] {
+        return cudaFuncSetAttribute(conv_tc_kernel<BN, KT, ST, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
+               cudaSuccess;
+    }();
+    (void)attr_ok;
+    const int tiles = (M + TC_BM - 1) / TC_BM;
+    conv_tc_kernel<BN, KT, ST, Op><<<std::min(tiles, per_sm * sms), TC_THREADS, smem, st>>>(op, M, K, nullptr);
+}
+
 // Weight-gradient GEMM: K split over the CTAs that shared and tensor memory
 // and the threads let stay resident, at least four steps each.
 template <int BN, int KS, int AQ, int ST, class Op>
@@ -1257,8 +1405,8 @@ void trunk_forward(h264a_mvnet* n, const Geo& g, cudaStream_t st) {
     const Bufs z = bufs(n);
     const int m1 = g.P * g.H1 * g.W1;
     conv1_kernel<<<std::min((m1 + 127) / 128, n->sms * C1_CTAS), 128, 0, st>>>(g, z, m1, nullptr);
-    gemm<32, 1, 3>(Conv2Fwd{g, z}, g.P * g.H2 * g.W2, 32, 144, st);
-    gemm<32, 1, 3>(Conv3Fwd{g, z}, g.P * g.H3 * g.W3, 32, 288, st);
+    conv_gemm<32, 3, 3>(Conv2Fwd{g, z}, g.P * g.H2 * g.W2, 144, n->sms, st);
+    conv_gemm<32, 5, 3>(Conv3Fwd{g, z}, g.P * g.H3 * g.W3, 288, n->sms, st);
 }
 
 void head_forward(h264a_mvnet* n, const Geo& g, float* logits, cudaStream_t st) {
@@ -1288,9 +1436,9 @@ void backward(h264a_mvnet* n, const Geo& g, cudaStream_t st) {
     const long long cells = (long long)K3 * 4;
     uncrop_kernel<<<unsigned((cells + 255) / 256), 256, 0, st>>>(g, n->df, n->a3, n->da3);
     wgrad<144, 64, 1, 3>(Conv3BwdW{{g, z}}, 32, 288, K3, S, st);
-    gemm<128, 1, 2>(ConvBwdData<32, 3>{g, z}, K3, 128, 128, st);
+    conv_gemm<128, 2, 2>(ConvBwdData<32, 3>{g, z}, K3, 128, S, st);
     wgrad<144, 128, 2, 2>(Conv2BwdW{{g, z}}, 32, 144, K2, S, st);
-    gemm<64, 1, 2>(ConvBwdData<16, 2>{g, z}, K2, 64, 128, st);
+    conv_gemm<64, 2, 3>(ConvBwdData<16, 2>{g, z}, K2, 128, S, st);
     wgrad<32, 128, 1, 2>(Conv1BwdW{g, z}, 16, 24, K1, S, st);
 }
 
