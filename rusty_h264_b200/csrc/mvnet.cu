@@ -1096,11 +1096,11 @@ __global__ void uncrop_kernel(const Geo g, const bf16_t* __restrict__ df, const 
 
 // ---- loss, proposals, optimiser -------------------------------------------------
 // One warp per sample: softmax over the 289 classes, the sample's share of the
-// mean cross-entropy (atomically summed into *loss) and dl = (p - onehot) / B
+// mean cross-entropy (atomically summed into *loss, in 64 bits) and dl = (p - onehot) / B
 // in bf16 (zero for the 7 padding logits).
 // The row stays in registers (HEAD_N = 296: ten values a lane).
 __global__ void loss_kernel(const float* __restrict__ logits, const int16_t* __restrict__ labels, int B,
-                            bf16_t* __restrict__ dl, float* __restrict__ loss) {
+                            bf16_t* __restrict__ dl, double* __restrict__ loss) {
     __shared__ float part[8];
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     float mine = 0.f;
@@ -1134,11 +1134,12 @@ __global__ void loss_kernel(const float* __restrict__ logits, const int16_t* __r
     if (lane == 0) part[threadIdx.x >> 5] = mine;
     __syncthreads();
     if (threadIdx.x == 0) {
-        float t = 0.f;
-        for (int i = 0; i < int(blockDim.x >> 5); i++) t += part[i];
+        double t = 0.0;
+        for (int i = 0; i < int(blockDim.x >> 5); i++) t += double(part[i]);
         atomicAdd(loss, t);
     }
 }
+__global__ void loss_out_kernel(const double* __restrict__ loss, float* __restrict__ out) { *out = float(*loss); }
 
 // One warp per sample: the 8 largest logits (ties to the lower class) as
 // quarter-pel MVs, 16 i32 per sample; sample i of a batch is MB mb0 + i of
@@ -1304,7 +1305,7 @@ struct h264a_mvnet {
     bf16_t *da3 = nullptr, *da2 = nullptr, *da1 = nullptr;
     bf16_t *wprep = nullptr;  // the weights as the data gradients read them
     float* logits = nullptr;
-    float* loss = nullptr;
+    double* loss = nullptr;
     // inference: the batch's pair table and neighbour features
     h264a_mvnet_pair* ipairs = nullptr;
     PropFrame* iprop = nullptr;  // a propose batch's frames: guide MVs and proposals
@@ -1543,13 +1544,13 @@ extern "C" int h264a_mvnet_grads(h264a_mvnet* n, const h264a_mvnet_pair* d_pairs
     const Geo g = make_geo(d_pairs, npairs, cw, ch, d_nmv, d_labels);
     const int B = npairs * g.nmb;
     H264A_CUDA(cudaMemsetAsync(n->grad, 0, sizeof(float) * NPARAMS, st));
-    H264A_CUDA(cudaMemsetAsync(n->loss, 0, sizeof(float), st));
+    H264A_CUDA(cudaMemsetAsync(n->loss, 0, sizeof(double), st));
     trunk_forward(n, g, st);
     head_forward(n, g, n->logits, st);
     loss_kernel<<<(B * 32 + 255) / 256, 256, 0, st>>>(n->logits, d_labels, B, n->dl, n->loss);
     backward(n, g, st);
     if (d_grads) H264A_CUDA(cudaMemcpyAsync(d_grads, n->grad, sizeof(float) * NPARAMS, cudaMemcpyDeviceToDevice, st));
-    if (d_loss) H264A_CUDA(cudaMemcpyAsync(d_loss, n->loss, sizeof(float), cudaMemcpyDeviceToDevice, st));
+    if (d_loss) loss_out_kernel<<<1, 1, 0, st>>>(n->loss, d_loss);
     return check_launch("mvnet grads");
 }
 
