@@ -742,11 +742,15 @@ def cpu_baseline(frames: np.ndarray, nthreads: int, lam: float, gate: int):
 
 def _grid_roofline(nmb: int, R: int, grid_ms: dict, int32_peak: float) -> dict:
     """INT32 roofline of the exhaustive grid on one frame: SAD is 2 lane-ops
-    per 4 pixels (__vsadu4 + accumulate), SATD 112 per 4x4 block."""
+    per 4 pixels (__vsadu4 + accumulate), SATD 112 per 4x4 block (what a
+    transform per candidate and block takes; the kernel transforms each window
+    position once, so its fraction may exceed 1)."""
     cands = nmb * (2 * R + 1) ** 2
     ops = {"sad": cands * 256 // 2, "satd": cands * 16 * SATD_OPS_PER_4X4}
     out = {"kernels": {"sad": "fullpel_sad_kernel", "satd": "fullpel_satd_kernel"}, "bound": "int32", "R": R,
-           "unit": "Gop/s", "peak": round(int32_peak, 1), "frame": "one 1920x1088 frame"}
+           "unit": "Gop/s", "peak": round(int32_peak, 1), "frame": "one 1920x1088 frame",
+           "note": "satd: operations of one transform per candidate and block; the kernel transforms each window "
+                   "position once"}
     for k, ms in grid_ms.items():
         g = ops[k] / (ms * 1e-3) / 1e9
         out[k] = {"ms": round(ms, 4), "ops": ops[k], "achieved": round(g, 1), "frac": round(g / int32_peak, 4)}
@@ -1112,7 +1116,7 @@ def run_ours(args, ws, rank, local):
     cwork = int(cb.picks[1:, :, 5].sum().item())
     c_achieved = cwork * SATD_OPS_PER_4X4 / (pipe_ms * 1e-3) / 1e9
     croof = {
-        "kernel": "closed_pipe_kernel (one launch over every P frame: a CTA per MB, its search, MC + T/Q, "
+        "kernel": "closed_pipe_kernel (one launch over every P frame: a warp per MB, its search, MC + T/Q, "
                   "reconstruction and deblocking, each reconstruction's planes built band by band; consecutive "
                   "frames overlap)", "bound": "int32",
         "achieved": round(c_achieved, 1), "peak": round(int32_peak, 1), "unit": "Gop/s",

@@ -125,8 +125,8 @@ struct MeLearnIn {
     int32_t *fallback;
     int32_t prop_t;
 };
-// Per-frame reconstruction fused into the wide plain-ME kernel (the closed
-// loop): the frame's chroma source, the previous frame's chroma
+// Per-frame reconstruction fused into the plain-ME kernel of one or two frames
+// (me_step_kernel): the frame's chroma source, the previous frame's chroma
 // reconstruction, the frame's reconstruction planes (written, then deblocked
 // in place) and chroma levels (128 i16 per MB, 16-byte aligned).  Luma levels
 // and the QP come from the frame's MeTqOut.
