@@ -546,8 +546,8 @@ H264A_API int h264a_batch_variant_shape(int variant, int *mbs_per_cta, int *stag
  * the search prices them on the reconstruction),
  * MC + T/Q and reconstruction of luma and chroma, and deblocking.  Each
  * frame's MBs run as a wavefront, and consecutive frames overlap in one
- * launch: an MB of frame f waits only for the segments (16 rows by 7 MB
- * columns) of rec(f-1) its search reads, whose planes are built as those
+ * launch: an MB of frame f waits only for the segments (16 rows by one to
+ * seven MB columns) of rec(f-1) its search reads, whose planes are built as those
  * MBs are deblocked, so about ten frames run at once.  From host buffers the
  * sources of frames 1.. are uploaded beside the launch and each frame's
  * outputs come down as it becomes final.

@@ -7,7 +7,7 @@
 // every P frame in one launch of the pipelined kernel (closed_pipe_kernel,
 // me.cu): each MB's search, its MC + T/Q and reconstruction of luma and
 // chroma and its in-loop deblocking by the same warp, and the planes of each
-// reconstruction built segment by segment (16 picture rows by 7 MB columns) as
+// reconstruction built segment by segment (16 picture rows by one to seven MB columns) as
 // its MBs are deblocked, so that about ten frames' wavefronts run at once, each
 // a few MBs behind the one before.  With a proposal net the
 // proposals of all frames come first, in one batched h264a_mvnet_propose pass

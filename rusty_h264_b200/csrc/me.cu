@@ -519,18 +519,29 @@ constexpr int ME_MAXF = 96;
 // Launches of at most this many frames use the work queue of the closed loop
 // (Q_WIDE), larger ones Q_MAIN.
 constexpr int ME_FEW_FRAMES = 2;
-// The pipelined closed loop: the width of a band's column segments in MBs (112
-// pixels: one strip of the plane builder; the next frame follows closer than
-// with 16 MBs: 46.1 -> 43.7 ms for 59 1080p P frames when it was changed) and
-// the number of warp pools (frames dealt round-robin to them).  The launch
-// takes as many CTAs per SM as give a pool about one warp per ready MB of its
-// frame's wavefront: more only hold MBs that wait, and slow the warps that
-// run (59 1080p P frames at 1, 2, 3, 4 CTAs per SM: 27.1, 29.2, 31.0, 32.4 ms,
-// with 10, 12, 12, 16 pools; at one CTA, 8 pools take 28.7 and 16 pools more).
+// The pipelined closed loop: the width of a band's column segments in MBs, the
+// number of warp pools (frames dealt round-robin to them) and the CTAs per SM,
+// by the picture's size.  A narrower segment is final sooner, so the next frame
+// follows closer; it also means more tickets and plane strips with idle lanes.
+// So a 24th of the width: what the wavefront of a small picture waits for is
+// the frame before, a large one's segments are too many (30 frames, segments
+// of 1, 2, 3, 4, 7 MBs: 640x360 7.9, 8.4, 8.9, 9.3, 10.4 ms; 960x540 9.7, 8.1,
+// 8.4, 8.8, 10.1; 1920x1080, 60 frames, -, 29.4, 28.4, 27.5, 27.7; 3840x2160,
+// 16 frames, 4 and 7: 20.0, 18.8).  Pools: about the frames whose wavefronts
+// fit one after another; more pools only hold warps that wait (learned 720p at
+// 6, 8, 10, 13: 7.5, 6.8, 7.0, 8.0 ms; 1080p at 8, 10, 13: 28.4, 26.5, 27.1).
+// CTAs: about a warp per MB of the pools' longest anti-diagonals: more hold MBs
+// that wait, and slow the warps that run (1080p at 1 and 2: 26.5 and 27.5 ms;
+// 2560x1440 18.9 and 17.0; 3840x2160 27.0 and 20.0, 4 MBs a segment).
 constexpr int PIPE_SEGW = 7, PIPE_POOLS = 10;
+static inline int pipe_segw(int mb_w) { return std::min(std::max(mb_w / 24, 1), PIPE_SEGW); }
+static inline int pipe_pools(int mb_w, int mb_h) {
+    return std::min(std::max((mb_w + 2 * mb_h) / 16, 6), PIPE_POOLS);
+}
 static inline int pipe_ctas_per_sm(int mb_w, int mb_h, int pools, int num_sms, int most) {
     const int wave = std::min((mb_w + 1) / 2, mb_h);  // MBs of the longest anti-diagonal
-    const int n = (pools * wave + ME_WARPS * num_sms - 1) / (ME_WARPS * num_sms);
+    const int warps = ME_WARPS * num_sms;
+    const int n = (pools * wave + warps * 3 / 4 - 1) / warps;  // a quarter short is near enough
     return std::min(std::max(n, 1), most);
 }
 struct FrameBatch {
@@ -1838,8 +1849,8 @@ int h264a::closed_pipe_run(h264a_ctx* ctx, const ClosedPipeIn& in, const h264a_m
     // the plane buffers (frame h's planes in buffer h % nbuf), the column
     // segments of the bands, the warp pools
     const int nbuf = std::min(n, H264A_CLOSED_PLANE_PICTURES);
-    const int segw = PIPE_SEGW, nseg = (mb_w + segw - 1) / segw;
-    const int pools = std::min(PIPE_POOLS, n - 1);
+    const int segw = pipe_segw(mb_w), nseg = (mb_w + segw - 1) / segw;
+    const int pools = std::min(pipe_pools(mb_w, mb_h), n - 1);
     if (pad % 4) return fail(H264A_E_ARG, "closed loop: the plane padding must be a multiple of 4");
     std::vector<CUtensorMap> maps(nbuf);
     std::vector<int> maps_ok(nbuf);
