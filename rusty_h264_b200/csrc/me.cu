@@ -534,14 +534,14 @@ constexpr int ME_FEW_FRAMES = 2;
 // that wait, and slow the warps that run (1080p at 1 and 2: 26.5 and 27.5 ms;
 // 2560x1440 18.9 and 17.0; 3840x2160 27.0 and 20.0, 4 MBs a segment).
 constexpr int PIPE_SEGW = 7, PIPE_POOLS = 10;
+static inline int wave_mbs(int mb_w, int mb_h) { return std::min((mb_w + 1) / 2, mb_h); }  // of the longest anti-diagonal
 static inline int pipe_segw(int mb_w) { return std::min(std::max(mb_w / 24, 1), PIPE_SEGW); }
 static inline int pipe_pools(int mb_w, int mb_h) {
     return std::min(std::max((mb_w + 2 * mb_h) / 16, 6), PIPE_POOLS);
 }
 static inline int pipe_ctas_per_sm(int mb_w, int mb_h, int pools, int num_sms, int most) {
-    const int wave = std::min((mb_w + 1) / 2, mb_h);  // MBs of the longest anti-diagonal
     const int warps = ME_WARPS * num_sms;
-    const int n = (pools * wave + warps * 3 / 4 - 1) / warps;  // a quarter short is near enough
+    const int n = (pools * wave_mbs(mb_w, mb_h) + warps * 3 / 4 - 1) / warps;  // a quarter short is near enough
     return std::min(std::max(n, 1), most);
 }
 struct FrameBatch {
@@ -1353,6 +1353,19 @@ static int make_segments(const FrameDesc* f, int nf, long long* start, int* segj
     return ns;
 }
 
+// CTAs of a frame launch: of those that fit (per_sm on each SM), as many as
+// give a warp to every MB of the frames' longest anti-diagonals.  More hold MBs
+// that wait: 1, 2, 4 CTAs an SM, one 720p frame with its reconstruction 1,806,
+// 1,847, 1,858 us; five 1080p frames (300 MBs, 592 warps) 2,565, 2,579, 2,605;
+// fifteen (900) 3,191, 3,177, 3,168; 75 of mixed sizes (2,430) 4,981, 4,494,
+// 4,360.
+static long long frame_ctas(const FrameDesc* f, int n, long long total, int num_sms, int per_sm) {
+    long long wave = 0;
+    for (int i = 0; i < n; i++) wave += wave_mbs(f[i].mb_w, f[i].mb_h);
+    const long long warps = (long long)ME_WARPS * num_sms, want = std::max(1LL, (wave + warps - 1) / warps);
+    return std::min(num_sms * std::min<long long>(per_sm, want), (total + ME_WARPS - 1) / ME_WARPS);
+}
+
 // fb.nseg and the segment arrays of a batch of fb.n sorted frames; returns the
 // ticket count.
 static long long fill_segments(FrameBatch& fb) {
@@ -1580,9 +1593,7 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
     if (words) H264A_CUDA(cudaMemsetAsync(words, 0, sizeof(unsigned long long) * EW_PER_MB * size_t(total), st));
     const int epoch = next_epoch(ctx, st, qi);
     if (epoch < 0) return H264A_E_CUDA;
-    long long blocks = (long long)ctx->num_sms * per_sm;
-    const long long need = (total + ME_WARPS - 1) / ME_WARPS;
-    if (blocks > need) blocks = need;
+    const long long blocks = frame_ctas(desc.data(), nframes, total, ctx->num_sms, per_sm);
     if (rec) {
         StepBatch sb;
         memset(&sb, 0, sizeof sb);
@@ -1783,9 +1794,7 @@ extern "C" int h264a_me_frames_noalloc(const h264a_me_frame* h_frames, int nfram
     const int rc0 = me_frames_setup(per_sm);
     if (rc0) return rc0;
     H264A_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    long long blocks = (long long)sms * per_sm;
-    const long long need = (total + ME_WARPS - 1) / ME_WARPS;
-    if (blocks > need) blocks = need;
+    const long long blocks = frame_ctas(fb.f, fb.n, total, sms, per_sm);
     const MeParamsDev prm = to_dev(*params);
     launch_me_frames(prm, unsigned(blocks), st, fb, total, scratch, scratch + 1, nullptr, kNoallocFlag, d_status, lam_ok);
     return check_launch("me_frames_kernel (no-alloc)");
