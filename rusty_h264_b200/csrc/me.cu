@@ -544,6 +544,16 @@ static inline int pipe_ctas_per_sm(int mb_w, int mb_h, int pools, int num_sms, i
     const int n = (pools * wave_mbs(mb_w, mb_h) + warps * 3 / 4 - 1) / warps;  // a quarter short is near enough
     return std::min(std::max(n, 1), most);
 }
+// Dynamic shared memory of such a launch: its windows, or as much as keeps one
+// CTA more than its share off an SM.  Beside another kernel (the lookahead of
+// the next frames on its own stream) the CTAs would otherwise crowd onto the
+// SMs that are free first (60 1080p frames with their lookahead: 64.8 ms, the
+// loop alone 41.7).
+constexpr int SM_SHARED = 228 * 1024, FRAME_SMEM_MAX = SM_SHARED / 2;
+static inline size_t frame_smem(long long blocks, int num_sms) {
+    const long long share = (blocks + num_sms - 1) / num_sms;
+    return std::max<size_t>(ME_WARPS * WIN_BYTES, size_t(SM_SHARED / (share + 1)));
+}
 struct FrameBatch {
     FrameDesc f[ME_MAXF];
     long long seg_start[ME_MAXF + 1];
@@ -1297,18 +1307,18 @@ static int me_frames_setup(int& per_sm, bool learn = false) {
 
 static int me_frames_setup_once(int& per_sm, bool learn) {
     const int smem = ME_WARPS * WIN_BYTES;
-    H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_frames_dkernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_frames_dkernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_frames_dkernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_frames_dkernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_frames_dkernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_frames_dkernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_frames_dkernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_frames_dkernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
     per_sm = 0;
     if (learn)
         H264A_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, me_frames_kernel<false, true>, 32 * ME_WARPS,
@@ -1373,11 +1383,10 @@ static long long fill_segments(FrameBatch& fb) {
     return fb.seg_start[fb.nseg];
 }
 
-static void launch_me_frames_dtab(const MeParamsDev& prm, unsigned blocks, cudaStream_t st, const FrameDesc* frames,
+static void launch_me_frames_dtab(const MeParamsDev& prm, unsigned blocks, size_t sm, cudaStream_t st, const FrameDesc* frames,
                                   const long long* seg_start, const int* seg_j, int nframes, int nseg, long long total,
                                   int* counter, int* flags, unsigned long long* words, int epoch, int* status,
                                   bool lam_ok, bool learn = false) {
-    const size_t sm = ME_WARPS * WIN_BYTES;
     const bool bal = balanced_preset(prm, lam_ok);
     if (learn && bal)
         me_frames_dkernel<true, true><<<blocks, 32 * ME_WARPS, sm, st>>>(frames, seg_start, seg_j, nframes, nseg, total,
@@ -1393,19 +1402,17 @@ static void launch_me_frames_dtab(const MeParamsDev& prm, unsigned blocks, cudaS
                                                                    counter, flags, words, epoch, status, SPIN_LIMIT);
 }
 
-static void launch_me_step(const MeParamsDev& prm, unsigned blocks, cudaStream_t st, const StepBatch& sb, long long total,
+static void launch_me_step(const MeParamsDev& prm, unsigned blocks, size_t sm, cudaStream_t st, const StepBatch& sb, long long total,
                            int* counter, int* flags, unsigned long long* words, int epoch, int* status, bool lam_ok,
                            bool learn) {
-    const size_t sm = ME_WARPS * WIN_BYTES;
     auto kern = balanced_preset(prm, lam_ok) ? (learn ? me_step_kernel<true, true> : me_step_kernel<true, false>)
                                      : (learn ? me_step_kernel<false, true> : me_step_kernel<false, false>);
     kern<<<blocks, 32 * ME_WARPS, sm, st>>>(sb, total, prm, counter, flags, words, epoch, status, SPIN_LIMIT);
 }
 
-static void launch_me_frames(const MeParamsDev& prm, unsigned blocks, cudaStream_t st, const FrameBatch& fb,
+static void launch_me_frames(const MeParamsDev& prm, unsigned blocks, size_t sm, cudaStream_t st, const FrameBatch& fb,
                              long long total, int* counter, int* flags, unsigned long long* words, int epoch,
                              int* status, bool lam_ok, bool learn = false) {
-    const size_t sm = ME_WARPS * WIN_BYTES;
     const bool bal = balanced_preset(prm, lam_ok);
     if (learn && bal)
         me_frames_kernel<true, true><<<blocks, 32 * ME_WARPS, sm, st>>>(fb, total, prm, counter, flags, words, epoch, status,
@@ -1606,7 +1613,7 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
         }
         sb.nseg = make_segments(sb.f, sb.n, sb.seg_start, sb.seg_j);
         if (sb.seg_start[sb.nseg] != total) return fail(H264A_E_ARG, "me_frames: internal queue layout error");
-        launch_me_step(prm, unsigned(blocks), st, sb, total, qw.d_counter, qw.d_flags, words, epoch, ctx->d_status,
+        launch_me_step(prm, unsigned(blocks), frame_smem(blocks, ctx->num_sms), st, sb, total, qw.d_counter, qw.d_flags, words, epoch, ctx->d_status,
                        lam_ok, learn != nullptr);
         return check_launch("me_step_kernel");
     }
@@ -1616,7 +1623,7 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
         fb.n = nframes;
         memcpy(fb.f, desc.data(), sizeof(FrameDesc) * nframes);
         if (fill_segments(fb) != total) return fail(H264A_E_ARG, "me_frames: internal queue layout error");
-        launch_me_frames(prm, unsigned(blocks), st, fb, total, qw.d_counter, qw.d_flags, words, epoch, ctx->d_status,
+        launch_me_frames(prm, unsigned(blocks), frame_smem(blocks, ctx->num_sms), st, fb, total, qw.d_counter, qw.d_flags, words, epoch, ctx->d_status,
                          lam_ok, learn != nullptr);
         return check_launch("me_frames_kernel");
     }
@@ -1632,7 +1639,7 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
     rc = table_upload(ctx, bytes, st);
     if (rc) return rc;
     char* dv = static_cast<char*>(ctx->me_tab);
-    launch_me_frames_dtab(prm, unsigned(blocks), st, reinterpret_cast<const FrameDesc*>(dv),
+    launch_me_frames_dtab(prm, unsigned(blocks), frame_smem(blocks, ctx->num_sms), st, reinterpret_cast<const FrameDesc*>(dv),
                           reinterpret_cast<const long long*>(dv + b_desc), reinterpret_cast<const int*>(dv + b_desc + b_seg),
                           nframes, nseg, total, qw.d_counter, qw.d_flags, words, epoch, ctx->d_status,
                           lam_ok, learn != nullptr);
@@ -1796,7 +1803,7 @@ extern "C" int h264a_me_frames_noalloc(const h264a_me_frame* h_frames, int nfram
     H264A_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const long long blocks = frame_ctas(fb.f, fb.n, total, sms, per_sm);
     const MeParamsDev prm = to_dev(*params);
-    launch_me_frames(prm, unsigned(blocks), st, fb, total, scratch, scratch + 1, nullptr, kNoallocFlag, d_status, lam_ok);
+    launch_me_frames(prm, unsigned(blocks), frame_smem(blocks, sms), st, fb, total, scratch, scratch + 1, nullptr, kNoallocFlag, d_status, lam_ok);
     return check_launch("me_frames_kernel (no-alloc)");
 }
 
@@ -1805,11 +1812,10 @@ extern "C" int h264a_me_frames_noalloc(const h264a_me_frame* h_frames, int nfram
 // ---------------------------------------------------------------------------
 
 static int closed_pipe_setup_once() {
-    const int smem = ME_WARPS * WIN_BYTES;
-    H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
+    H264A_CUDA(cudaFuncSetAttribute(closed_pipe_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
     return H264A_OK;
 }
 
@@ -1978,7 +1984,7 @@ int h264a::closed_pipe_run(h264a_ctx* ctx, const ClosedPipeIn& in, const h264a_m
     const bool bal = balanced_preset(prm, balanced_lambda(in.lambda_me)), learn = in.props != nullptr;
     auto kern = bal ? (learn ? closed_pipe_kernel<true, true> : closed_pipe_kernel<true, false>)
                     : (learn ? closed_pipe_kernel<false, true> : closed_pipe_kernel<false, false>);
-    kern<<<unsigned(blocks), 32 * ME_WARPS, ME_WARPS * WIN_BYTES, st>>>(pp, prm, epoch, ctx->d_status, SPIN_LIMIT);
+    kern<<<unsigned(blocks), 32 * ME_WARPS, frame_smem(blocks, ctx->num_sms), st>>>(pp, prm, epoch, ctx->d_status, SPIN_LIMIT);
     rc = check_launch("closed_pipe_kernel");
     if (rc) return rc;
     return table_done(ctx, st);
