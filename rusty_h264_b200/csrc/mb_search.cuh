@@ -928,6 +928,7 @@ __device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws
         int d = 0;
 #pragma unroll
         for (int g = 0; g < 8; g++) d += bs.red[0][g][gl];
+        __syncwarp();  // read by every lane: the next round stores its own
         const int cc = d + rc;
         if (kind == RING) {
             const unsigned hit = __ballot_sync(FULL, gl < rn - ri && cc < best) & 0xffu;

@@ -1,0 +1,40 @@
+"""Properties of the kernels' sources that no run can show: an ordering that one
+machine happens to give, a limit that no test may wait for, an attribute of a
+device that is not there."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "rusty_h264_b200", "csrc")
+
+
+def source(name):
+    """A source file without its comments, white space folded."""
+    with open(os.path.join(CSRC, name)) as f:
+        t = f.read()
+    t = re.sub(r"/\*.*?\*/", " ", t, flags=re.S)
+    return re.sub(r"\s+", " ", re.sub(r"//[^\n]*", " ", t))
+
+
+def body(name, head):
+    """The text from `head` to the end of the braces that follow it."""
+    t = source(name)
+    i = t.index(head)
+    j = t.index("{", i)
+    depth = 0
+    for k in range(j, len(t)):
+        depth += (t[k] == "{") - (t[k] == "}")
+        if depth == 0:
+            return t[i:k + 1]
+    raise AssertionError(head)
+
+
+def test_column_sums_are_read_before_the_next_round_stores():
+    """The lanes of a search exchange column sums through the warp's shared
+    scratch: a __syncwarp between every read of a round and the next store."""
+    for head in ("SearchOut search16_bal(", "SearchOut search_parts_bal("):
+        b = body("mb_search.cuh", head)
+        loop = b[b.index("bs.red"):]  # store, sync, read, ... and round again
+        last = [m.end() for m in re.finditer(r"d \+= bs\.red\[[^;]*;", loop)][-1]
+        # nothing but unconditional statements up to the __syncwarp
+        m = re.match(r"((?:(?!\bif\b|\bcontinue\b|\bbreak\b|\bfor\b|\bwhile\b).)*?)__syncwarp\(\);", loop[last:])
+        assert m, head
