@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(32 * DB_ROWS) deblock_rows_kernel(const __grid
                             }
                             if (top_shared) __threadfence_block();
                         }
+                        __syncwarp();  // what lane 0 has seen is every lane's to read
                         avail = __shfl_sync(0xffffffffu, avail, 0);
                     }
                     // luma rows -3..-1: lanes 0..11; chroma rows -2, -1: lanes 12..19

@@ -38,3 +38,13 @@ def test_column_sums_are_read_before_the_next_round_stores():
         # nothing but unconditional statements up to the __syncwarp
         m = re.match(r"((?:(?!\bif\b|\bcontinue\b|\bbreak\b|\bfor\b|\bwhile\b).)*?)__syncwarp\(\);", loop[last:])
         assert m, head
+
+
+def test_deblocking_rows_wait_with_the_whole_warp():
+    """Lane 0 alone acquires the row above's progress: a __syncwarp before the
+    other lanes read that row's samples."""
+    b = body("deblock.cu", "deblock_rows_kernel(")
+    i = b.index("ld_acquire(gprog - 1)")
+    reads = min(b.index("top_word(x)", i), b.index("db_strips + ((long long)(w - 1)", i))
+    branch = b[i:reads]
+    assert "__syncwarp();" in branch[branch.index("avail = W"):branch.index("if (top_shared) { if (lane < 20)")]
