@@ -891,24 +891,34 @@ __device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp
     const int mvx = part ? mv1x : mv0x, mvy = part ? mv1y : mv0y;
     const int cx0 = mbx * 8, cy0 = mby * 8;
     uint32_t sr[4], prd[4];
+    const int ccw = pc.cw / 2, cch = pc.ch / 2;
+    const int wx = lx + bx + pc.pad - ws.wx0 + (mvx >> 2), wy = ly + by + pc.pad - ws.wy0 + (mvy >> 2);
+    const bool in_win = win_ok && win_covers(wx, wy);
+    if constexpr (REC) {
+        if (sy.bw != nullptr) {
+            // the rows of the previous reconstruction that the lane reads
+            // outside the window are final, then the warp together: a lane may
+            // have it from another that its segment was seen ready
+            if (chroma)
+                band_wait_px(sy.bw, &ws.bready, 2 * min(cy0 + cby + 4 + (mvy >> 3), cch - 1) + 1,
+                             2 * min(cx0 + cbx + 4 + (mvx >> 3), ccw - 1) + 1);
+            else if (!in_win)
+                band_wait_px(sy.bw, &ws.bready, ly + by + (mvy >> 2) + 5, lx + bx + (mvx >> 2) + 5);
+            __syncwarp();
+        }
+    }
     if (chroma) {
-        const int ccw = pc.cw / 2, cch = pc.ch / 2;
         const uint8_t* sp = rdp->src_c[cpl] + (long long)(cy0 + cby) * ccw + cx0 + cbx;
 #pragma unroll
         for (int r = 0; r < 4; r++) sr[r] = __ldg(reinterpret_cast<const uint32_t*>(sp + (long long)r * ccw));
-        // the previous reconstruction's chroma rows it reads are final
-        band_wait_px(sy.bw, &ws.bready, 2 * min(cy0 + cby + 4 + (mvy >> 3), cch - 1) + 1,
-                     2 * min(cx0 + cbx + 4 + (mvx >> 3), ccw - 1) + 1);
         chroma_rows(rdp->ref_c[cpl], ccw, cch, cx0 + cbx + (mvx >> 3), cy0 + cby + (mvy >> 3), mvx & 7, mvy & 7, prd);
     } else if (lane < 16) {
         const int x = lx + bx, y = ly + by;
 #pragma unroll
         for (int r = 0; r < 4; r++) sr[r] = ld4u(pc.d_src + (long long)(y + r) * pc.cw + x);
-        const int wx = x + pc.pad - ws.wx0 + (mvx >> 2), wy = y + pc.pad - ws.wy0 + (mvy >> 2);
-        if (win_ok && win_covers(wx, wy)) {
+        if (in_win) {
             win_rows(win, wx, wy, mvx & 3, mvy & 3, prd);
         } else {
-            band_wait_px(sy.bw, &ws.bready, y + (mvy >> 2) + 5, x + (mvx >> 2) + 5);
             const uint4 r = plane_rows(&ws, x, y, mvx, mvy);
             prd[0] = r.x; prd[1] = r.y; prd[2] = r.z; prd[3] = r.w;
         }

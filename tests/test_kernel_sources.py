@@ -48,3 +48,13 @@ def test_deblocking_rows_wait_with_the_whole_warp():
     reads = min(b.index("top_word(x)", i), b.index("db_strips + ((long long)(w - 1)", i))
     branch = b[i:reads]
     assert "__syncwarp();" in branch[branch.index("avail = W"):branch.index("if (top_shared) { if (lane < 20)")]
+
+
+def test_motion_compensation_waits_with_the_whole_warp():
+    """A lane may find in shared memory that another lane has seen a reference
+    segment ready: a __syncwarp between those waits and the reads."""
+    b = body("me.cu", "void frame_mb(")
+    last = [m.end() for m in re.finditer(r"band_wait_px\(", b)][-1]
+    for read in ("chroma_rows(", "plane_rows("):
+        assert last < b.index(read), read
+        assert "__syncwarp();" in b[last:b.index(read)], read
