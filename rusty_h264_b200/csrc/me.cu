@@ -882,7 +882,10 @@ __device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp
     // luma 4x4 blocks, the prediction from the staged window when it covers
     // the block's MV; with REC, lanes 16..23 the chroma blocks (plane, block k
     // in SUBBLOCKS order; lanes 24..31 shadow them) and the reconstruction of both
-    if (!REC && fd.coeffs == nullptr) return;
+    if (!REC && fd.coeffs == nullptr) {
+        __syncwarp();  // the warp's scratch is read: lane 0 writes the next MB's
+        return;
+    }
     const bool chroma = REC && lane >= 16;
     const int bx = (lane & 3) * 4, by = ((lane >> 2) & 3) * 4;             // luma block
     const int cpl = (lane >> 2) & 1, kb = lane & 3, cbx = (kb & 1) * 4, cby = (kb >> 1) * 4;  // chroma block

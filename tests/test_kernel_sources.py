@@ -58,3 +58,12 @@ def test_motion_compensation_waits_with_the_whole_warp():
     for read in ("chroma_rows(", "plane_rows("):
         assert last < b.index(read), read
         assert "__syncwarp();" in b[last:b.index(read)], read
+
+
+def test_an_mb_leaves_its_warp_scratch_to_the_next():
+    """Lane 0 writes the warp's scratch for the next MB: a __syncwarp before
+    every way out of an MB."""
+    b = body("me.cu", "void frame_mb(")
+    outs = [m.start() for m in re.finditer(r"\breturn;", b)] + [len(b) - 1]
+    for o in outs:
+        assert b[:o].rstrip().endswith("__syncwarp();"), b[max(0, o - 80):o + 8]
