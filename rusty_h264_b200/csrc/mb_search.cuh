@@ -528,8 +528,9 @@ struct SearchOut {
 // saturates and comparisons match the reference's i64.
 //
 // LEARN with use_prop (the learned-proposal kernels' 16x16 search): after the
-// seeds, the 8 proposals (lane gl: proposal gl in `prop`) are priced with the
-// search's own cost; when the best proposal's distortion exceeds the
+// seeds, the 8 proposals (lane gl: proposal gl in `prop`) are priced, both with
+// `cost` (SATD and λ also where the full-pel phase has a cost of its own, so
+// that predictor and proposals compare); when the best proposal's distortion exceeds the
 // predictor's by more than prop_t the plain search goes on from the seeds
 // (fell = 1), otherwise it continues as motion_search with the cheapest of
 // predictor and proposals as its start vector (mb16.rs:2445, 2579-2596:
@@ -578,6 +579,7 @@ __device__ __forceinline__ SearchOut mb_search(const MbLane& s, const MeParamsDe
     int best_c = 0, seed_c = 0;
     int cp = 0, dp = 0;  // the predictor's cost and distortion (learned search)
     int phase = use_start ? PH_START : PH_SEEDS;
+    bool prop_next = use_prop;  // the proposals are still to be priced
     int si = -1, sk = -1, loops = 0, iter = 0, step = 0;
     bool ring_open = false, ring_improved = false;
     int ring_i = 0, ring_n = 0;
@@ -588,7 +590,8 @@ __device__ __forceinline__ SearchOut mb_search(const MbLane& s, const MeParamsDe
         double lam = lam_r;
         while (kind < 0 && phase != PH_DONE) {
             if (phase == PH_SEEDS) {
-                kind = EV_SEEDS; n = n_seed; metric = m_fp; lam = l_fp;
+                kind = EV_SEEDS; n = n_seed;
+                if (!(LEARN && prop_next)) { metric = m_fp; lam = l_fp; }
                 mx = my = 0;
                 if (gl == 1) { mx = p0.x; my = p0.y; }
                 if (two && gl == 2) { mx = p1.x; my = p1.y; }
@@ -740,7 +743,7 @@ __device__ __forceinline__ SearchOut mb_search(const MbLane& s, const MeParamsDe
                 best_c = k == 2 ? c_seed[2] : (k == 3 ? c_seed[3] : c_seed[4]);
                 evals += 1;
             }
-            phase = LEARN && use_prop ? PH_PROP : PH_DIA;
+            phase = LEARN && prop_next ? PH_PROP : PH_DIA;
         } else if (kind == EV_START) {
             // a refine-only search (mb16.rs:2580-2582): the start vector
             // priced with `cost`, no full-pel phase, the sub-pel steps from it
@@ -759,10 +762,14 @@ __device__ __forceinline__ SearchOut mb_search(const MbLane& s, const MeParamsDe
             const int vx = __shfl_sync(0xffffffffu, prop.x, gb + bi), vy = __shfl_sync(0xffffffffu, prop.y, gb + bi);
             const bool fb = (long long)dprop > (long long)dp + prop_t;
             if (fell) *fell = fb ? 1 : 0;
-            evals += fb ? N_PROP + 1 : N_PROP + 1 - evals;
+            prop_next = false;
             if (fb) {
-                phase = PH_DIA;  // the plain search goes on from its seeds
+                // the plain search goes on from its seeds, priced again where
+                // its full-pel cost is another than `cost`
+                evals = sadfp ? N_PROP + 1 : evals + N_PROP + 1;
+                phase = sadfp ? PH_SEEDS : PH_DIA;
             } else {
+                evals = N_PROP + 1;
                 best_c = cp;
                 bx = p0.x; by = p0.y;
                 if (m < best_c) { best_c = m; bx = vx; by = vy; }
