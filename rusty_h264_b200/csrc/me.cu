@@ -634,15 +634,19 @@ struct RecDesc {
 // right, lower (and lower-left) and lower-right neighbours' median predictors
 // read (mv_neighbors_block, mb16.rs:1871).  A waiting MB polls the words it
 // needs until their epoch is the launch's, so the flag and the data arrive in
-// one load and no release fence orders anything else.  MVs fit i16 because
-// the search keeps every block inside the padded picture, at most 8191 samples
-// wide or high; larger pictures, and launches whose scratch holds one flag per
-// MB (h264a_me_frames_noalloc), publish a flag after the pick instead.
+// one load and no release fence orders anything else.  An MV that does not fit
+// (a caller's proposal may lie anywhere, and a search walks on from it) is the
+// word MV_FAR: the pick is in memory before it, for the reader to take from
+// there.  Pictures more than 8191 samples wide or high, whose MVs seldom fit,
+// and launches whose scratch holds one flag per MB (h264a_me_frames_noalloc),
+// publish a flag after the pick instead.
 constexpr int EW_PER_MB = 3;
 // Nanoseconds between polls of a warp diagonals ahead of the wavefront, and of
 // one waiting for its left or top-right neighbour.
 constexpr unsigned POLL_FAR_NS = 1000, POLL_NEAR_NS = 40;
 constexpr int EW_MAX_SIDE = 8191;
+constexpr int MV_FAR = -32768;  // both components of the word of an MV beyond +-32767
+__device__ __forceinline__ bool mv_far(int v) { return v < -32767 || v > 32767; }
 __device__ __forceinline__ unsigned long long mv_word(int epoch, int x, int y) {
     return ((unsigned long long)(unsigned)epoch << 32) | (uint32_t(uint16_t(x)) | (uint32_t(uint16_t(y)) << 16));
 }
@@ -798,10 +802,14 @@ __device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp
     const bool need = lane < 4 && (lane == 0 ? aa : (lane == 1 ? ba : (lane == 2 ? ca : (!ca && da))));
     const int nb = m + (lane == 0 ? -1 : (lane == 1 ? -mb_w : (lane == 2 ? 1 - mb_w : -1 - mb_w)));
     auto fetch = [&](unsigned ns) {
-        if (sy.ew != nullptr)
-            return wait_mv_word(sy.ew + EW_PER_MB * (long long)nb + (lane == 0 ? 0 : (lane == 3 ? 2 : 1)), sy.epoch, sy.status,
-                                sy.limit, ns);
-        wait_flag(sy.flags + nb, sy.epoch, sy.status, 1, sy.limit);
+        if (sy.ew != nullptr) {
+            const int2 v = wait_mv_word(sy.ew + EW_PER_MB * (long long)nb + (lane == 0 ? 0 : (lane == 3 ? 2 : 1)), sy.epoch,
+                                        sy.status, sy.limit, ns);
+            if (v.x != MV_FAR) return v;
+            __threadfence();  // the word first, then the pick
+        } else {
+            wait_flag(sy.flags + nb, sy.epoch, sy.status, 1, sy.limit);
+        }
         return pick_mv_at(fd.picks, nb, lane == 0 || lane == 3 ? 3 : 0, lane == 0 ? 0 : 3);
     };
     // most resident warps hold MBs some diagonals ahead of the wavefront: they
@@ -865,13 +873,20 @@ __device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp
             mv0x = px[2]; mv0y = py[2]; mv1x = px[3]; mv1y = py[3];
         }
     }
-    if (sy.ew != nullptr && lane < EW_PER_MB) {
+    int32_t* const p = fd.picks + 6LL * m;
+    if (sy.ew != nullptr) {
         // the pick to the wavefront: blocks (3,0), (0,3), (3,3)
         const bool second = lane == 0 ? shape == 2 : (lane == 1 ? shape == 1 : shape != 0);
-        st_relaxed_u64(sy.ew + EW_PER_MB * (long long)m + lane, mv_word(sy.epoch, second ? mv1x : mv0x, second ? mv1y : mv0y));
+        int wx = second ? mv1x : mv0x, wy = second ? mv1y : mv0y;
+        if (mv_far(mv0x) || mv_far(mv0y) || mv_far(mv1x) || mv_far(mv1y)) {  // warp-uniform
+            if (lane == 0) { p[0] = shape; p[1] = mv0x; p[2] = mv0y; p[3] = mv1x; p[4] = mv1y; }
+            __syncwarp();
+            __threadfence();  // the pick before the words
+            if (mv_far(wx) || mv_far(wy)) wx = wy = MV_FAR;
+        }
+        if (lane < EW_PER_MB) st_relaxed_u64(sy.ew + EW_PER_MB * (long long)m + lane, mv_word(sy.epoch, wx, wy));
     }
     if (lane == 0) {
-        int32_t* p = fd.picks + 6LL * m;
         p[0] = shape; p[1] = mv0x; p[2] = mv0y; p[3] = mv1x; p[4] = mv1y; p[5] = evals;
         fd.costs[2LL * m] = best;
         fd.costs[2LL * m + 1] = c16;
@@ -979,6 +994,7 @@ __device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp
         if (edge) {
             const int qbx = hor ? sg : e, qby = hor ? e : sg;
             int2 pm = make_int2(int(int16_t(nw & 0xffffu)), int(int16_t((nw >> 16) & 0xffffu)));
+            if (e == 0 && pm.x == MV_FAR) pm = pick_mv_at(fd.picks, hor ? m - mb_w : m - 1, hor ? sg : 3, hor ? 3 : sg);
             if (e > 0) {
                 const int pbx = hor ? sg : e - 1, pby = hor ? e - 1 : sg;
                 pm = own(pbx, pby);
