@@ -261,7 +261,9 @@ __global__ void __launch_bounds__(GRID_THREADS) fullpel_satd_kernel(GridArgs a, 
 
     long long best_key = LLONG_MAX;  // (cost << 32) | scan index; min = first-wins argmin
     const long long grid_base = (long long)mb * n * n;
-    const bool argmin = a.metric == 1, rate_pos = a.lambda >= 0.0;
+    // rates are below 2^17: up to this lambda a cost is its distortion and a
+    // product >= 0, and fits 31 bits
+    const bool argmin = a.metric == 1, rate_pos = a.lambda >= 0.0 && a.lambda <= 8192.0;
     for (int ph0 = 0; ph0 < 4; ph0 += ps)
         for (int j0 = 0; ph0 + 4 * j0 < n; j0 += SATD_J * g) {
             for (int i = threadIdx.x; i < npos; i += blockDim.x) {
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(GRID_THREADS) fullpel_satd_kernel(GridArgs a, 
                     if (dyi >= n) continue;
                     const int idx = dyi * n + dxi, dist = 2 * (int(acc[j]) - k_mb);
                     if (a.satd_grid) a.satd_grid[grid_base + idx] = dist;
-                    // a rate is >= 0 when lambda is: a larger distortion cannot win then
+                    // a larger distortion than the best cost cannot win then
                     if (argmin && (!rate_pos || (long long)dist <= (best_key >> 32))) {
                         const long long key =
                             (grid_cost(a, dist, (cxf + dxi - R) * 4, (cyf + dyi - R) * 4, pmx, pmy) << 32) | (long long)idx;
