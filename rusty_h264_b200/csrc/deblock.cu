@@ -211,6 +211,8 @@ __global__ void __launch_bounds__(32 * DB_ROWS) deblock_rows_kernel(const __grid
             if (has_c) nc = ldw32(cown + (long long)cr * ccw + 4 * cwd);
             DbStrength ns = st[0];
             int avail = 0;  // MBs of the row above seen ready
+            const unsigned poll_ns = top_shared ? 20 : 100;
+            const int polls = poll_limit(spin_limit, poll_ns);
             // a row whose upper neighbour is another CTA's: the lane's word of
             // the next MB's top strip, fetched a step ahead when it is ready
             uint32_t tw = 0;
@@ -285,12 +287,12 @@ __global__ void __launch_bounds__(32 * DB_ROWS) deblock_rows_kernel(const __grid
                             for (;; it++) {
                                 avail = top_shared ? *reinterpret_cast<volatile int*>(&done[w - 1]) : ld_acquire(gprog - 1);
                                 if (avail >= x + 1) break;
-                                if (it >= spin_limit || ((it & 255) == 255 && *reinterpret_cast<volatile int*>(status) != 0)) {
+                                if (it >= polls || ((it & 255) == 255 && *reinterpret_cast<volatile int*>(status) != 0)) {
                                     atomicCAS(status, 0, 1);
                                     avail = W;
                                     break;
                                 }
-                                __nanosleep(top_shared ? 20 : 100);
+                                __nanosleep(poll_ns);
                             }
                             if (top_shared) __threadfence_block();
                         }

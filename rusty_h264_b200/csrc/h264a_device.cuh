@@ -357,7 +357,12 @@ __device__ __forceinline__ long long lam_cost(double lam, uint32_t rate) {
 // both neighbours lie on earlier diagonals.  Readiness is a per-MB flag set to
 // the launch's epoch with release semantics and polled with acquire loads.
 
-constexpr int SPIN_LIMIT = 1000 * 1000;  // ~0.5 s of polling at a 200 ns sleep per poll
+// A wait's limit counts polls SPIN_NS apart (a poll itself takes about as long
+// again, so SPIN_LIMIT is some 0.5 s); a wait that sleeps for another time
+// scales it, so that none gives up before the waits it depends on.
+constexpr unsigned SPIN_NS = 200;
+constexpr int SPIN_LIMIT = 1000 * 1000;
+__host__ __device__ constexpr int poll_limit(int limit, unsigned ns) { return int((long long)limit * SPIN_NS / ns); }
 
 // Number of MBs (x, y) of a W x H frame with x + 2y < t: rows y < a are
 // full (t - 2y >= W), rows a <= y < b hold t - 2y MBs.
@@ -411,10 +416,11 @@ __device__ __forceinline__ void st_release(int* p, int v) {
 // timeout records `code` in status.
 // Once any wait of the launch has timed out (status non-zero, checked every
 // 256 polls) the others give up too, so a failed launch ends promptly.
-static __device__ void wait_flag(const int* flag, int epoch, int* status, int code, int limit, unsigned ns = 200) {
+static __device__ void wait_flag(const int* flag, int epoch, int* status, int code, int limit, unsigned ns = SPIN_NS) {
+    const int polls = poll_limit(limit, ns);
     for (int it = 0;; it++) {
         if (ld_acquire(flag) == epoch) return;
-        if (it >= limit || ((it & 255) == 255 && *reinterpret_cast<volatile int*>(status) != 0)) {
+        if (it >= polls || ((it & 255) == 255 && *reinterpret_cast<volatile int*>(status) != 0)) {
             atomicCAS(status, 0, code);
             return;
         }

@@ -657,10 +657,11 @@ __device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned l
 // every `ns` nanoseconds; returns its MV.
 __device__ __forceinline__ int2 wait_mv_word(const unsigned long long* p, int epoch, int* status, int limit, unsigned ns) {
     unsigned long long v = 0;
+    const int polls = poll_limit(limit, ns);
     for (int it = 0;; it++) {
         asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
         if (int(v >> 32) == epoch) break;
-        if (it >= limit || ((it & 255) == 255 && *reinterpret_cast<volatile int*>(status) != 0)) {
+        if (it >= polls || ((it & 255) == 255 && *reinterpret_cast<volatile int*>(status) != 0)) {
             atomicCAS(status, 0, 1);
             break;
         }
@@ -1175,7 +1176,7 @@ __device__ __forceinline__ void pipe_band(const PipeParams& pp, int h, int b, in
                     atomicCAS(status, 0, 1);
                     break;
                 }
-                __nanosleep(200);
+                __nanosleep(SPIN_NS);
             }
         }
     }
@@ -1237,7 +1238,7 @@ __global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
                         atomicCAS(status, 0, 1);
                         break;
                     }
-                    __nanosleep(200);
+                    __nanosleep(SPIN_NS);
                 }
             }
             if (fenced != h)

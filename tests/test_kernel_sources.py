@@ -67,3 +67,26 @@ def test_an_mb_leaves_its_warp_scratch_to_the_next():
     outs = [m.start() for m in re.finditer(r"\breturn;", b)] + [len(b) - 1]
     for o in outs:
         assert b[:o].rstrip().endswith("__syncwarp();"), b[max(0, o - 80):o + 8]
+
+
+def test_wait_limits_are_times():
+    """A wait's limit stands for polls SPIN_NS apart, about half a second: a
+    loop that sleeps for another time scales it."""
+    dev = source("h264a_device.cuh")
+    ns = int(re.search(r"constexpr unsigned SPIN_NS = (\d+);", dev).group(1))
+    limit = eval(re.search(r"constexpr int SPIN_LIMIT = ([\d *]+);", dev).group(1))
+    scaled = re.search(r"int poll_limit\(int limit, unsigned ns\) \{ return int\((.*?)\); \}", dev).group(1)
+    scaled = scaled.replace("(long long)", "").replace("/", "//")
+    for every in (20, 40, 100, 200, 1000):
+        polls = eval(scaled, {"limit": limit, "SPIN_NS": ns, "ns": every})
+        assert polls * every == limit * ns >= 200_000_000
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        t = source(name)
+        for m in re.finditer(r"__nanosleep\(([^;]*)\);", t):
+            sleep = m.group(1)
+            if sleep == "SPIN_NS":
+                continue
+            before = t[max(0, m.start() - 6000):m.start()]
+            assert re.search(r"poll_limit\((spin_)?limit, %s\)" % re.escape(sleep), before), (name, sleep)
