@@ -1247,46 +1247,56 @@ __global__ void guide_frames_kernel(const PropFrame* __restrict__ fr, int P, int
     }
 }
 
+// Each launcher has its kernel's opt-in to dynamic shared memory above 48 KB, an
+// attribute of the current device (opt_in_kernels).
+template <int BN, int MT, int ST>
+constexpr int gemm_smem() {
+    return ST * (MT * TC_BM + BN) * TC_BK * 2;
+}
+template <int BN, int MT, int ST, class Op>
+static cudaError_t gemm_opt_in() {
+    return cudaFuncSetAttribute(gemm_tc_kernel<BN, MT, ST, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                gemm_smem<BN, MT, ST>());
+}
 template <int BN, int MT, int ST, class Op>
 static void gemm(const Op& op, int M, int N, int K, cudaStream_t st) {
-    constexpr int smem = ST * (MT * TC_BM + BN) * TC_BK * 2;
-    static const bool attr_ok = [] {  // once per instantiation (the dynamic shared memory above 48 KB)
-        return cudaFuncSetAttribute(gemm_tc_kernel<BN, MT, ST, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
-               cudaSuccess;
-    }();
-    (void)attr_ok;
+    constexpr int smem = gemm_smem<BN, MT, ST>();
     dim3 grid((M + MT * TC_BM - 1) / (MT * TC_BM), (N + BN - 1) / BN);
     gemm_tc_kernel<BN, MT, ST, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, nullptr);
 }
 
 template <int BN, int KT, int ST, class Op>
+static cudaError_t conv_gemm_opt_in() {
+    return cudaFuncSetAttribute(conv_tc_kernel<BN, KT, ST, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                conv_smem<BN, KT, ST>());
+}
+template <int BN, int KT, int ST, class Op>
 static void conv_gemm(const Op& op, int M, int K, int sms, cudaStream_t st) {
     constexpr int smem = conv_smem<BN, KT, ST>(), fit = 226 * 1024 / (smem + 4096), per_sm = fit < 4 ? fit : 4;
     static_assert(per_sm >= 1 && per_sm * tc_cols<2 * BN>() <= 512, "shared and tensor memory");
-    static const bool attr_ok = [] {
-        return cudaFuncSetAttribute(conv_tc_kernel<BN, KT, ST, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
-               cudaSuccess;
-    }();
-    (void)attr_ok;
     const int tiles = (M + TC_BM - 1) / TC_BM;
     conv_tc_kernel<BN, KT, ST, Op><<<std::min(tiles, per_sm * sms), TC_THREADS, smem, st>>>(op, M, K, nullptr);
 }
 
 // Weight-gradient GEMM: K split over the CTAs that shared and tensor memory
 // and the threads let stay resident, at least four steps each.
-template <int BN, int KS, int AQ, int ST, class Op>
-static void wgrad(const Op& op, int M, int N, int K, int sms, cudaStream_t st) {
+template <int BN, int KS, int AQ, int ST>
+constexpr int wgrad_smem() {
     constexpr int GR = TC_THREADS / KS, BLK = KS * 16, A_BYTES = AQ * GR * BLK, STAGE = A_BYTES + (BN / 8) * BLK;
     // the MMA reads 16 blocks of A whatever there are: 16 * BLK from the last stage's start
-    constexpr int smem = (ST - 1) * STAGE + (STAGE > 16 * BLK ? STAGE : 16 * BLK);
+    return (ST - 1) * STAGE + (STAGE > 16 * BLK ? STAGE : 16 * BLK);
+}
+template <int BN, int KS, int AQ, int ST, class Op>
+static cudaError_t wgrad_opt_in() {
+    return cudaFuncSetAttribute(wgrad_tc_kernel<BN, KS, AQ, ST, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                wgrad_smem<BN, KS, AQ, ST>());
+}
+template <int BN, int KS, int AQ, int ST, class Op>
+static void wgrad(const Op& op, int M, int N, int K, int sms, cudaStream_t st) {
+    constexpr int smem = wgrad_smem<BN, KS, AQ, ST>();
     constexpr int by_smem = 224 * 1024 / (smem + 2048), by_tmem = 512 / tc_cols<BN>();
     constexpr int resident = by_smem < by_tmem ? (by_smem < 4 ? by_smem : 4) : (by_tmem < 4 ? by_tmem : 4);
     static_assert(resident >= 1, "shared memory");
-    static const bool attr_ok = [] {
-        return cudaFuncSetAttribute(wgrad_tc_kernel<BN, KS, AQ, ST, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
-               cudaSuccess;
-    }();
-    (void)attr_ok;
     const int tiles = ((M + TC_BM - 1) / TC_BM) * ((N + BN - 1) / BN);
     int splits = resident * sms / tiles;
     splits = std::max(1, std::min(splits, (K + 4 * KS - 1) / (4 * KS)));
@@ -1454,16 +1464,36 @@ void backward(h264a_mvnet* n, const Geo& g, cudaStream_t st) {
     wgrad<32, 128, 1, 2>(Conv1BwdW{g, z}, 16, 24, K1, S, st);
 }
 
+// Every instantiation launched above, on the current device.
+static int opt_in_kernels() {
+    H264A_CUDA((conv_gemm_opt_in<32, 3, 3, Conv2Fwd>()));
+    H264A_CUDA((conv_gemm_opt_in<32, 5, 3, Conv3Fwd>()));
+    H264A_CUDA((gemm_opt_in<256, 2, 3, Fc1Fwd>()));
+    H264A_CUDA((gemm_opt_in<256, 1, 2, Fc1Fwd>()));
+    H264A_CUDA((gemm_opt_in<160, 1, 3, HeadFwd>()));
+    H264A_CUDA((wgrad_opt_in<256, 64, 4, 2, HeadBwdW>()));
+    H264A_CUDA((gemm_opt_in<256, 1, 2, HeadBwdData>()));
+    H264A_CUDA((wgrad_opt_in<256, 64, 4, 2, Fc1BwdW>()));
+    H264A_CUDA((gemm_opt_in<192, 1, 2, Fc1BwdData>()));
+    H264A_CUDA((wgrad_opt_in<144, 64, 1, 3, Conv3BwdW>()));
+    H264A_CUDA((conv_gemm_opt_in<128, 2, 2, ConvBwdData<32, 3>>()));
+    H264A_CUDA((wgrad_opt_in<144, 128, 2, 2, Conv2BwdW>()));
+    H264A_CUDA((conv_gemm_opt_in<64, 2, 3, ConvBwdData<16, 2>>()));
+    H264A_CUDA((wgrad_opt_in<32, 128, 1, 2, Conv1BwdW>()));
+    return H264A_OK;
+}
+
 }  // namespace
 
 extern "C" int h264a_mvnet_create(int device, uint64_t seed, h264a_mvnet** out) {
     if (!out) return fail(H264A_E_ARG, "mvnet_create: null out");
     *out = nullptr;
     H264A_CUDA(cudaSetDevice(device));
+    int rc = opt_in_kernels();
+    if (rc) return rc;
     h264a_mvnet* n = new h264a_mvnet();
     n->device = device;
     cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, device);
-    int rc = H264A_OK;
     if (!rc) rc = dmalloc(&n->master, NPARAMS);
     if (!rc) rc = dmalloc(&n->w, size_t(WREP) * WSTRIDE);
     if (!rc) rc = dmalloc(&n->grad, NPARAMS);

@@ -90,3 +90,17 @@ def test_wait_limits_are_times():
                 continue
             before = t[max(0, m.start() - 6000):m.start()]
             assert re.search(r"poll_limit\((spin_)?limit, %s\)" % re.escape(sleep), before), (name, sleep)
+
+
+def test_network_kernels_opt_in_on_their_nets_device():
+    """Dynamic shared memory above 48 KB is an attribute of a kernel on a
+    device: mvnet_create sets it for every instantiation that is launched."""
+    t = source("mvnet.cu")
+    assert not re.search(r"static (const )?(bool|std::once_flag)", t)
+    launched = {(k, re.sub(r"\s", "", a), op) for k, a, op in
+                re.findall(r"\b(gemm|conv_gemm|wgrad)<([\d, ]+)>\((\w+(?:<[\d, ]+>)?)\{", t)}
+    setup = body("mvnet.cu", "static int opt_in_kernels(")
+    listed = {(k, re.sub(r"\s", "", a), op) for k, a, op in
+              re.findall(r"H264A_CUDA\(\((\w+)_opt_in<((?:\d+, )*\d+), (\w+(?:<[\d, ]+>)?)>\(\)\)\)", setup)}
+    assert len(launched) >= 12 and launched == listed
+    assert "opt_in_kernels()" in body("mvnet.cu", "int h264a_mvnet_create(")
