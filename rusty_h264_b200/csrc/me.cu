@@ -2233,6 +2233,22 @@ static int me_mr_setup_once() {
     if (!rc) rc = mr_attr<true, 8, true>();
     return rc;
 }
+// Once per device, as me_frames_setup.
+static int me_mr_setup() {
+    constexpr int kMaxDev = 64;
+    static bool done[kMaxDev];
+    static std::mutex mu;
+    int dev = 0;
+    H264A_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDev) return me_mr_setup_once();
+    std::lock_guard<std::mutex> lock(mu);
+    if (!done[dev]) {
+        const int rc = me_mr_setup_once();
+        if (rc) return rc;
+        done[dev] = true;
+    }
+    return H264A_OK;
+}
 
 template <bool BAL, int NW, bool STAGE>
 static int mr_launch_t(h264a_ctx* ctx, const MeParamsDev& prm, const char* dv, const MrTable& t, int32_t* counter,
@@ -2320,10 +2336,8 @@ int h264a::mr_table_build(const h264a_me_mr_frame* h_frames, int nframes, MrTabl
 int h264a::mr_launch(h264a_ctx* ctx, int variant, const MeParamsDev& prm, const void* d_table, const MrTable& t,
                      int32_t* counter, int32_t* flags, int epoch, cudaStream_t st) {
     if (variant < 0 || variant >= H264A_BATCH_VARIANTS) return fail(H264A_E_ARG, "me_frames_multiref: no such launch shape");
-    static std::once_flag once;
-    static int setup_rc = 0;
-    std::call_once(once, [] { setup_rc = me_mr_setup_once(); });
-    if (setup_rc) return setup_rc;
+    const int rc = me_mr_setup();
+    if (rc) return rc;
     const char* dv = static_cast<const char*>(d_table);
     if (!balanced_preset(prm, t.lam_ok)) return mr_launch_t<false, 4, true>(ctx, prm, dv, t, counter, flags, epoch, st);
     switch (variant) {

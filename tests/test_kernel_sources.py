@@ -104,3 +104,12 @@ def test_network_kernels_opt_in_on_their_nets_device():
               re.findall(r"H264A_CUDA\(\((\w+)_opt_in<((?:\d+, )*\d+), (\w+(?:<[\d, ]+>)?)>\(\)\)\)", setup)}
     assert len(launched) >= 12 and launched == listed
     assert "opt_in_kernels()" in body("mvnet.cu", "int h264a_mvnet_create(")
+
+
+def test_multi_reference_kernels_opt_in_on_every_device():
+    """As above for the frame kernels: no once-per-process opt-in."""
+    t = source("me.cu")
+    assert "once_flag" not in t and "call_once" not in t
+    b = body("me.cu", "int h264a::mr_launch(")
+    assert "me_mr_setup(" in b
+    assert "cudaGetDevice(&dev)" in body("me.cu", "static int me_mr_setup(")
