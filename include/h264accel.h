@@ -370,7 +370,9 @@ H264A_API int h264a_pixel_path_prefetch(h264a_ctx *ctx, const uint8_t *h_frames,
  * them, pair-major, raster order within a pair: d_nmv holds 6 i16 per MB
  * (the neighbour MVs, quarter-pel), d_labels 1 i16 per MB (class 0..288).
  * A net owns its parameters, optimiser state and the workspace of one batch;
- * calls on one net must not overlap. */
+ * calls on one net must not overlap.  Its kernels' waits are bounded: once one
+ * has run out, every further call returns H264A_E_TIMEOUT (get_params
+ * after a synchronisation) until set_params. */
 #define H264A_MVNET_NPARAMS 389528
 #define H264A_MVNET_MAX_PIXELS 8388608
 typedef struct h264a_mvnet h264a_mvnet;

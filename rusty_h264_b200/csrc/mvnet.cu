@@ -171,12 +171,13 @@ constexpr uint32_t tc_idesc() {
 __device__ __forceinline__ uint32_t tc_smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
 // Waits (bounded) for phase `parity` of an mbarrier; on timeout records 4 in
-// status and keeps waiting up to twice as long, so that no tensor-core work
-// is left reading a stage or writing tensor memory.
+// status (the net's host word, see check_waits) and keeps waiting up to twice
+// as long, so that no tensor-core work is left reading a stage or writing
+// tensor memory.
 __device__ __forceinline__ void tc_wait(uint32_t bar, uint32_t parity, int* status) {
     constexpr int kLimit = 1 << 22;
     for (int it = 0; !mbar_try_wait(bar, parity); it++) {
-        if (it == kLimit && status != nullptr) atomicCAS(status, 0, 4);
+        if (it == kLimit) *reinterpret_cast<volatile int*>(status) = 4;
         if (it >= 2 * kLimit) break;
     }
 }
@@ -507,6 +508,7 @@ struct Bufs {
     bf16_t *a1, *a2, *a3, *h, *dl, *dh, *df, *da3, *da2, *da1;
     const bf16_t *w4t, *w5t, *wd3, *wd2;  // prep_kernel's rearranged weights
     float* logits;
+    int* status;  // the net's status word
 };
 
 // conv1's window of output position m: the pair's planes at its top-left pixel
@@ -1262,7 +1264,7 @@ template <int BN, int MT, int ST, class Op>
 static void gemm(const Op& op, int M, int N, int K, cudaStream_t st) {
     constexpr int smem = gemm_smem<BN, MT, ST>();
     dim3 grid((M + MT * TC_BM - 1) / (MT * TC_BM), (N + BN - 1) / BN);
-    gemm_tc_kernel<BN, MT, ST, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, nullptr);
+    gemm_tc_kernel<BN, MT, ST, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, op.z.status);
 }
 
 template <int BN, int KT, int ST, class Op>
@@ -1275,7 +1277,7 @@ static void conv_gemm(const Op& op, int M, int K, int sms, cudaStream_t st) {
     constexpr int smem = conv_smem<BN, KT, ST>(), fit = 226 * 1024 / (smem + 4096), per_sm = fit < 4 ? fit : 4;
     static_assert(per_sm >= 1 && per_sm * tc_cols<2 * BN>() <= 512, "shared and tensor memory");
     const int tiles = (M + TC_BM - 1) / TC_BM;
-    conv_tc_kernel<BN, KT, ST, Op><<<std::min(tiles, per_sm * sms), TC_THREADS, smem, st>>>(op, M, K, nullptr);
+    conv_tc_kernel<BN, KT, ST, Op><<<std::min(tiles, per_sm * sms), TC_THREADS, smem, st>>>(op, M, K, op.z.status);
 }
 
 // Weight-gradient GEMM: K split over the CTAs that shared and tensor memory
@@ -1303,7 +1305,7 @@ static void wgrad(const Op& op, int M, int N, int K, int sms, cudaStream_t st) {
     int kchunk = (K + splits - 1) / splits;
     kchunk = (kchunk + KS - 1) / KS * KS;
     dim3 grid((M + TC_BM - 1) / TC_BM, (N + BN - 1) / BN, (K + kchunk - 1) / kchunk);
-    wgrad_tc_kernel<BN, KS, AQ, ST, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, kchunk, nullptr);
+    wgrad_tc_kernel<BN, KS, AQ, ST, Op><<<grid, TC_THREADS, smem, st>>>(op, M, N, K, kchunk, op.z.status);
 }
 
 }  // namespace mvnet
@@ -1327,6 +1329,7 @@ struct h264a_mvnet {
     bf16_t *wprep = nullptr;  // the weights as the data gradients read them
     float* logits = nullptr;
     double* loss = nullptr;
+    int* status = nullptr;  // mapped host word: non-zero once a kernel's wait has run out
     // inference: the batch's pair table and neighbour features
     h264a_mvnet_pair* ipairs = nullptr;
     PropFrame* iprop = nullptr;  // a propose batch's frames: guide MVs and proposals
@@ -1349,7 +1352,17 @@ void free_net(h264a_mvnet* n) {
                   n->da3, n->da2, n->da1, n->wprep, n->logits, n->loss, n->ipairs, n->inmv, n->iprop};
     for (void* p : ps)
         if (p) cudaFree(p);
+    if (n->status) cudaFreeHost(n->status);
     delete n;
+}
+
+// An earlier batch's kernel may have given up a wait: its results are not to be
+// used, and the net says so at the next call (no synchronisation here).
+// h264a_mvnet_set_params starts afresh.
+int check_waits(const h264a_mvnet* n) {
+    if (n && *const_cast<const volatile int*>(n->status) != 0)
+        return fail(H264A_E_TIMEOUT, "mvnet: a wait of an earlier batch ran out (status 4); its results are not valid");
+    return H264A_OK;
 }
 
 uint64_t splitmix(uint64_t& s) {
@@ -1402,6 +1415,7 @@ Bufs bufs(h264a_mvnet* n) {
     z.wd3 = z.w5t + N_W5T;
     z.wd2 = z.wd3 + N_WD3;
     z.logits = n->logits;
+    z.status = n->status;  // mapped: one address on host and device
     return z;
 }
 
@@ -1426,7 +1440,7 @@ int check_geo(const h264a_mvnet* n, const h264a_mvnet_pair* d_pairs, int P, int 
 void trunk_forward(h264a_mvnet* n, const Geo& g, cudaStream_t st) {
     const Bufs z = bufs(n);
     const int m1 = g.P * g.H1 * g.W1;
-    conv1_kernel<<<std::min((m1 + 127) / 128, n->sms * C1_CTAS), 128, 0, st>>>(g, z, m1, nullptr);
+    conv1_kernel<<<std::min((m1 + 127) / 128, n->sms * C1_CTAS), 128, 0, st>>>(g, z, m1, z.status);
     conv_gemm<32, 3, 3>(Conv2Fwd{g, z}, g.P * g.H2 * g.W2, 144, n->sms, st);
     conv_gemm<32, 5, 3>(Conv3Fwd{g, z}, g.P * g.H3 * g.W3, 288, n->sms, st);
 }
@@ -1512,6 +1526,11 @@ extern "C" int h264a_mvnet_create(int device, uint64_t seed, h264a_mvnet** out) 
     if (!rc) rc = dmalloc(&n->logits, size_t(MAXS * HEAD_N));
     if (!rc) rc = dmalloc(&n->wprep, size_t(WREP) * N_PREP);
     if (!rc) rc = dmalloc(&n->loss, 1);
+    if (!rc && cudaHostAlloc(reinterpret_cast<void**>(&n->status), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        rc = fail(H264A_E_NOMEM, "mvnet: cudaHostAlloc failed");
+    }
+    if (!rc) *n->status = 0;
     if (!rc) rc = dmalloc(&n->inmv, size_t(MAXS * 6));
     if (!rc) rc = dmalloc(&n->ipairs, size_t(MAXPIX / 256));
     if (!rc) rc = dmalloc(&n->iprop, size_t(MAXPIX / 256));
@@ -1545,6 +1564,7 @@ extern "C" int h264a_mvnet_set_params(h264a_mvnet* n, const float* h_params) {
     H264A_CUDA(cudaSetDevice(n->device));
     const int rc = upload_params(n, h_params);
     if (rc) return rc;
+    *n->status = 0;  // the device is idle here
     H264A_CUDA(cudaMemset(n->m1, 0, sizeof(float) * NPARAMS));
     H264A_CUDA(cudaMemset(n->m2, 0, sizeof(float) * NPARAMS));
     n->step = 0;
@@ -1555,6 +1575,8 @@ extern "C" int h264a_mvnet_get_params(h264a_mvnet* n, float* h_params) {
     if (!n || !h_params) return fail(H264A_E_ARG, "mvnet_get_params: null pointer");
     H264A_CUDA(cudaSetDevice(n->device));
     H264A_CUDA(cudaDeviceSynchronize());
+    const int rc = check_waits(n);
+    if (rc) return rc;
     H264A_CUDA(cudaMemcpy(h_params, n->master, sizeof(float) * NPARAMS, cudaMemcpyDeviceToHost));
     return H264A_OK;
 }
@@ -1562,6 +1584,7 @@ extern "C" int h264a_mvnet_get_params(h264a_mvnet* n, float* h_params) {
 extern "C" int h264a_mvnet_forward(h264a_mvnet* n, const h264a_mvnet_pair* d_pairs, int npairs, int cw, int ch,
                                    const int16_t* d_nmv, float* d_logits, void* stream) {
     int rc = check_geo(n, d_pairs, npairs, cw, ch, d_nmv);
+    if (!rc) rc = check_waits(n);
     if (rc) return rc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const Geo g = make_geo(d_pairs, npairs, cw, ch, d_nmv, nullptr);
@@ -1581,6 +1604,8 @@ extern "C" int h264a_mvnet_grads(h264a_mvnet* n, const h264a_mvnet_pair* d_pairs
     int rc = check_geo(n, d_pairs, npairs, cw, ch, d_nmv);
     if (rc) return rc;
     if (!d_labels) return fail(H264A_E_ARG, "mvnet_grads: null labels");
+    rc = check_waits(n);
+    if (rc) return rc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const Geo g = make_geo(d_pairs, npairs, cw, ch, d_nmv, d_labels);
     const int B = npairs * g.nmb;
@@ -1621,6 +1646,8 @@ extern "C" int h264a_mvnet_propose(h264a_mvnet* n, const h264a_mvnet_frame* h_fr
             (long long)f.cw * f.ch > MAXPIX)
             return fail(H264A_E_ARG, "mvnet_propose: frames must be MB-aligned, at most 8192 pixels a side");
     }
+    const int wrc = check_waits(n);
+    if (wrc) return wrc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     // consecutive frames of one geometry, up to MAXPIX pixels, form a batch:
     // their trunk maps in one pass, then FC1 + head over their MBs, then each

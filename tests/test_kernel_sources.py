@@ -113,3 +113,13 @@ def test_multi_reference_kernels_opt_in_on_every_device():
     b = body("me.cu", "int h264a::mr_launch(")
     assert "me_mr_setup(" in b
     assert "cudaGetDevice(&dev)" in body("me.cu", "static int me_mr_setup(")
+
+
+def test_network_waits_that_run_out_are_reported():
+    """Every kernel that waits for the tensor cores has the net's status word,
+    and every call on the net looks at it first."""
+    t = source("mvnet.cu")
+    for m in re.finditer(r"\b(\w+_tc_kernel|conv1_kernel)(<[^;{}]*?>)? ?<<<[^;]*;", t):
+        assert m.group(0).endswith("z.status);"), m.group(0)[-60:]
+    for call in ("forward", "grads", "propose", "get_params"):  # train_step calls grads
+        assert "check_waits(" in body("mvnet.cu", "int h264a_mvnet_%s(" % call), call
