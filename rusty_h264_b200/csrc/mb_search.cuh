@@ -28,6 +28,8 @@
 // five mixed streams (one launch): 8.3 and 4.0 ms.
 #pragma once
 
+#include <cstddef>
+
 #include "satd_mma.cuh"
 
 namespace h264a {
@@ -121,23 +123,6 @@ __device__ __forceinline__ void win_rows(uint32_t win, int wx, int wy, int fx, i
 __device__ __forceinline__ bool win_covers(int wx, int wy) {
     return wx >= 0 && ((wx + 1) & ~3) <= WIN_W - 8 && wy >= 0 && wy + 5 <= WIN_H;
 }
-
-// The preset's knobs as the general search reads them.
-struct Knobs {
-    const MeParamsDev& p;
-    // the next enabled rung of the diamond ladder after si (5: none)
-    __device__ __forceinline__ int next_rung(int si) const {
-        if (p.fast) return si + 1 >= 2 ? 5 : si + 1;
-        int n = si + 1;
-        while (n < 5 && !(p.dia_mask & (1u << n))) n++;
-        return n;
-    }
-    __device__ __forceinline__ int rung_step(int si) const {
-        return p.fast ? (si == 0 ? 16 : 4) : (64 >> si);  // rungs [64,32,16,8,4] quarter-pel
-    }
-    // rate of an MV against the mvd centre (mb16.rs:2454-2482)
-    __device__ __forceinline__ uint32_t rate(int dx, int dy) const { return mvbits(p.kind, p.tab, dx) + mvbits(p.kind, p.tab, dy); }
-};
 
 // ---------------------------------------------------------------------------
 // Pricing
@@ -348,44 +333,65 @@ __device__ __forceinline__ void pass_words(const MbLane& s, const MbScratch& ws,
     }
 }
 
-// A pass some of whose candidates' reads the window does not cover, from the
-// planes; ax, ay / bx, by: the column's MVs in tiles A and B (mode 0: A) of
-// the rw-wide partition at (px, py).  Returns the shares of the column sums as
-// a0 | a1 << 16, b0 | b1 << 16 (each below 2^16: 8 blocks of at most 2 x
-// 4,080), and the row SADs of both tiles.  Out of line, with nothing of the
-// search's state in memory: between one pass in a hundred and one in ten
-// needs it (at the edges of fast objects), and the wavefront may wait for it,
-// so all its loads are in flight together unless a read leaves the planes.
-template <int MODE>
-__device__ __noinline__ int4 slow_pass(MbScratch* ws, int px, int py, int rw, int ax, int ay, int bx, int by, bool wait) {
+// The columns of a pass whose candidates' reads the window does not cover
+// (`miss`: the lane's), from the planes; ax, ay / bx, by: the column's MVs in
+// tiles A and B (mode 0: A) of the rw-wide partition at (px, py).  Returns the
+// shares of the column sums as a0 | a1 << 16, b0 | b1 << 16 (each below 2^16:
+// 8 blocks of at most 2 x 4,080), and the row SADs of both tiles, put in their
+// places among the other columns' in `part`.  Out of line, with nothing of the search's state
+// in memory: between one pass in a hundred and one in ten needs it (at the
+// edges of fast objects; one in four with 16-pixel steps), and the wavefront
+// may wait for it, so only the missing columns are read, the second plane only
+// where a phase has one, and all loads are in flight together unless a read
+// leaves the planes.  (A pass that read every column from both operands through
+// L2, and the source beside them, took 3,900 cycles, 5,400 for the partitions;
+// this one 2,600 and 2,800.)  Inlined for the presets other than Balanced, whose
+// steps leave the window more often and whose kernels have the registers: `own`
+// the lane's source words then.
+template <int MODE, bool CG>
+__device__ __forceinline__ int4 slow_columns(MbScratch* ws, const HadFrag& had, const uint32_t* own, int px, int py, int rw, int ax, int ay,
+                                             int bx, int by, bool miss, int4 part) {
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int REF = CG ? REF_PLANES_L2 : REF_PLANES;
     const int lane = threadIdx.x & 31, rh = MODE == 0 ? 16 : 24 - rw;
-    if (wait) band_wait_px(ws->bw, &ws->bready, py + (max(ay, by) >> 2) + rh + 1, px + (max(ax, bx) >> 2) + rw + 1);
+    if (CG && miss) band_wait_px(ws->bw, &ws->bready, py + (max(ay, by) >> 2) + rh + 1, px + (max(ax, bx) >> 2) + rw + 1);
     __syncwarp();
     MbLane s;
     s.lane = lane;
     s.px = px; s.py = py; s.rw = rw; s.rh = rh;
-    s.had = had_frag(lane);
     // block k of the pass: 16 wide, four a row; 8 wide, two
     const bool wide = MODE == 0 || rw == 16;
-    auto src_word = [&](int k) {
-        const int xo = wide ? 4 * (k & 3) : 4 * (k & 1), yo = wide ? 4 * (k >> 2) : 4 * (k >> 1);
-        return ld4u(ws->src + (long long)(py + yo + (lane & 3)) * ws->cw + px + xo);
-    };
-    const CandAddr<REF_PLANES_L2> ta = cand_addr<REF_PLANES_L2>(s, *ws, 0u, ax, ay), tb = cand_addr<REF_PLANES_L2>(s, *ws, 0u, bx, by);
+    const uint8_t* const src = ws->src + (long long)(py + (lane & 3)) * ws->cw + px;
+    const long long sstep = 4LL * ws->cw;
+    const CandAddr<REF> ta = cand_addr<REF>(s, *ws, 0u, ax, ay), tb = cand_addr<REF>(s, *ws, 0u, bx, by);
     int a0 = 0, a1 = 0, b0 = 0, b1 = 0, sa = 0, sb = 0;
-    if (__all_sync(0xffffffffu, ta.covered && tb.covered)) {
-        uint32_t sw[16], p[16], r[16];
+    if (__all_sync(FULL, !miss || (ta.covered && tb.covered))) {
+        uint32_t p[16];
 #pragma unroll
-        for (int k = 0; k < (MODE == 0 ? 16 : 8); k++) sw[k] = src_word(k);
-        pass_words<MODE, REF_PLANES_L2>(s, *ws, ta.a, tb.a, p);
-        pass_words<MODE, REF_PLANES_L2>(s, *ws, ta.b, tb.b, r);
+        for (int i = 0; i < 16; i++) p[i] = 0;
+        if (__any_sync(FULL, miss && ((ax | ay | bx | by) & 1))) {  // quarter phases have two operands
+            if (miss) {
+                uint32_t r[16];
+                pass_words<MODE, REF>(s, *ws, ta.a, tb.a, p);
+                pass_words<MODE, REF>(s, *ws, ta.b, tb.b, r);
+#pragma unroll
+                for (int i = 0; i < 16; i++) p[i] = avg_up4(p[i], r[i]);
+            }
+        } else if (miss) {
+            pass_words<MODE, REF>(s, *ws, ta.a, tb.a, p);
+        }
+        __syncwarp();
+        uint32_t sw[MODE == 0 ? 16 : 8];
+#pragma unroll
+        for (int k = 0; k < (MODE == 0 ? 16 : 8); k++)
+            sw[k] = own != nullptr ? own[k] : ld4u(src + (wide ? k >> 2 : k >> 1) * sstep + 4 * (wide ? k & 3 : k & 1));  // (from L1)
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const uint32_t wa = avg_up4(p[i], r[i]), wb = avg_up4(p[8 + i], r[8 + i]), va = sw[i], vb = sw[MODE == 0 ? 8 + i : i];
-            had_mma(s.had, wa, va, a0, a1);
-            had_mma(s.had, wb, vb, b0, b1);
-            sa += int(__vsadu4(wa, va));
-            sb += int(__vsadu4(wb, vb));
+            const uint32_t va = sw[i], vb = sw[MODE == 0 ? 8 + i : i];
+            had_mma(had, p[i], va, a0, a1);
+            had_mma(had, p[8 + i], vb, b0, b1);
+            sa += int(__vsadu4(p[i], va));
+            sb += int(__vsadu4(p[8 + i], vb));
         }
     } else {
 #pragma unroll 1
@@ -393,29 +399,41 @@ __device__ __noinline__ int4 slow_pass(MbScratch* ws, int px, int py, int rw, in
             const bool second = MODE == 1 && j >= 8;
             const int k = MODE == 0 ? j : j & 7;
             const int xo = wide ? 4 * (k & 3) : 4 * (k & 1), yo = wide ? 4 * (k >> 2) : 4 * (k >> 1);
-            const uint32_t sw = src_word(k);
-            const uint32_t pw = plane_word(*ws, px + xo, py + yo + (lane & 3), second ? bx : ax, second ? by : ay);
+            const uint32_t sw = ld4u(src + (wide ? k >> 2 : k >> 1) * sstep + xo);
+            uint32_t pw = 0;
+            if (miss) pw = plane_word(*ws, px + xo, py + yo + (lane & 3), second ? bx : ax, second ? by : ay);
             __syncwarp();
             int t0 = 0, t1 = 0;
-            had_mma(s.had, pw, sw, t0, t1);
+            had_mma(had, pw, sw, t0, t1);
             const int sd = int(__vsadu4(pw, sw));
             if (j >= 8) { b0 += t0; b1 += t1; sb += sd; }
             else { a0 += t0; a1 += t1; sa += sd; }
         }
     }
-    return make_int4(a0 | (a1 << 16), b0 | (b1 << 16), sa, sb);
+    // columns 2q and 2q + 1 (four lanes each) and the lane's own, as they missed
+    const unsigned m = __ballot_sync(FULL, miss) >> (8 * (lane & 3));
+    const int keep = ((m & 1u) ? 0 : 0xffff) | ((m & 16u) ? 0 : int(0xffff0000u));
+    part.x = (part.x & keep) | ((a0 | (a1 << 16)) & ~keep);
+    part.y = (part.y & keep) | ((b0 | (b1 << 16)) & ~keep);
+    if (miss) { part.z = sa; part.w = sb; }
+    return part;
+}
+template <int MODE, bool CG>
+__device__ __noinline__ int4 slow_pass(MbScratch* ws, int px, int py, int rw, int ax, int ay, int bx, int by, bool miss, int4 part) {
+    return slow_columns<MODE, CG>(ws, had_frag(threadIdx.x & 31), nullptr, px, py, rw, ax, ay, bx, by, miss, part);
 }
 
 // One pass: the lane's column's candidates at ta (tile A) and, mode 1, tb
 // (tile B) -- MVs ax, ay and bx, by -- give the lane's shares of
 // the column sums in a0, a1 (columns 2q, 2q+1 of tile A; mode 0: of the whole
-// candidate) and b0, b1 (tile B), and with SADS the lane's row SADs in sa, sb.
-// two: a two-plane phase is possible.  idle: the group has no slots (its
+// candidate) and b0, b1 (tile B), and the lane's row SADs in sa, sb; of these
+// what `satd` and `sad` ask for.  CG: planes written during the launch are read
+// through L2.  two: a two-plane phase is possible.  idle: the group has no slots (its
 // addresses are safe and its sums are not used).
-template <int MODE, int REF, bool SADS>
+template <int MODE, int REF, bool CG, bool INL>
 __device__ __forceinline__ void price_pass(const MbLane& s, MbScratch& ws, const CandAddr<REF>& ta, const CandAddr<REF>& tb,
-                                           int ax, int ay, int bx, int by, bool two, bool idle, int& a0, int& a1, int& b0,
-                                           int& b1, int& sa, int& sb) {
+                                           int ax, int ay, int bx, int by, bool two, bool idle, bool satd, bool sad, int& a0,
+                                           int& a1, int& b0, int& b1, int& sa, int& sb) {
     uint32_t p[16];
     pass_words<MODE, REF>(s, ws, ta.a, tb.a, p);
     if (two) {
@@ -425,12 +443,14 @@ __device__ __forceinline__ void price_pass(const MbLane& s, MbScratch& ws, const
         for (int i = 0; i < 16; i++) p[i] = avg_up4(p[i], r[i]);
     }
     a0 = a1 = b0 = b1 = sa = sb = 0;
+    if (satd) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        had_mma(s.had, p[i], s.src[i], a0, a1);
-        had_mma(s.had, p[8 + i], s.src[MODE == 0 ? 8 + i : i], b0, b1);
+        for (int i = 0; i < 8; i++) {
+            had_mma(s.had, p[i], s.src[i], a0, a1);
+            had_mma(s.had, p[8 + i], s.src[MODE == 0 ? 8 + i : i], b0, b1);
+        }
     }
-    if (SADS) {
+    if (sad) {
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             sa += int(__vsadu4(p[i], s.src[i]));
@@ -439,55 +459,16 @@ __device__ __forceinline__ void price_pass(const MbLane& s, MbScratch& ws, const
     }
     const bool miss = !idle && !(ta.covered && (MODE == 0 || tb.covered));
     if (__any_sync(0xffffffffu, miss)) {
-        const int4 r = slow_pass<MODE>(&ws, s.px, s.py, s.rw, ax, ay, bx, by, miss);
+        int4 r = make_int4(a0 | (a1 << 16), b0 | (b1 << 16), sa, sb);
+        if constexpr (INL)
+            r = slow_columns<MODE, CG>(&ws, s.had, s.src, s.px, s.py, s.rw, ax, ay, bx, by, miss, r);
+        else
+            r = slow_pass<MODE, CG>(&ws, s.px, s.py, s.rw, ax, ay, bx, by, miss, r);
         a0 = r.x & 0xffff; a1 = int(uint32_t(r.x) >> 16);
         b0 = r.y & 0xffff; b1 = int(uint32_t(r.y) >> 16);
         sa = r.z; sb = r.w;
     }
     if (MODE == 0) { a0 += b0; a1 += b1; sa += sb; }
-}
-
-// Distortions of the group's slots 0..n-1 (nmax: the largest n of the
-// groups, nmax <= 8; n = 0: none) under the MVs the lanes hold (lane gl of a
-// group: slot gl), returned to the slots' lanes.  `sad`: this group's metric
-// is SAD.
-template <int MODE>
-__device__ __forceinline__ int price_slots(const MbLane& s, MbScratch& ws, uint32_t lut, int mvx, int mvy, int n, int nmax,
-                                           bool sad) {
-    constexpr bool one = MODE == 0;
-    int out = 0;
-#pragma unroll 1
-    for (int tp = 0; tp < (one ? 1 : (nmax + 3) >> 2); tp++) {
-        // the column's slots in tiles A and B (unused ones repeat slot 0)
-        int ca = one ? s.lane >> 2 : 4 * tp + ((s.lane >> 2) & 1);
-        int cb = ca + 2;
-        ca = ca < n ? ca : 0;
-        cb = cb < n ? cb : 0;
-        const int ax = __shfl_sync(0xffffffffu, mvx, s.gb + ca), ay = __shfl_sync(0xffffffffu, mvy, s.gb + ca);
-        const int bx = __shfl_sync(0xffffffffu, mvx, s.gb + cb), by = __shfl_sync(0xffffffffu, mvy, s.gb + cb);
-        const CandAddr<REF_WINDOW> ta = cand_addr<REF_WINDOW>(s, ws, lut, ax, ay), tb = cand_addr<REF_WINDOW>(s, ws, lut, bx, by);
-        const bool two = __any_sync(0xffffffffu, ta.a != ta.b || (!one && tb.a != tb.b));
-        int a0, a1, b0, b1, sa, sb;
-        price_pass<MODE, REF_WINDOW, true>(s, ws, ta, tb, ax, ay, bx, by, two, n == 0, a0, a1, b0, b1, sa, sb);
-        // columns 2q, 2q+1 of tiles A and B, summed over the lanes of each
-        // column: lane bit 4 keeps the odd column, in mode 1 bit 3 tile B
-        const bool hi = (s.lane & 16) != 0, up = (s.lane & 8) != 0;
-        const int ka = (hi ? a1 : a0) + __shfl_xor_sync(0xffffffffu, hi ? a0 : a1, 16);
-        const int kb = one ? ka : (hi ? b1 : b0) + __shfl_xor_sync(0xffffffffu, hi ? b0 : b1, 16);
-        int v = (up ? kb : ka) + __shfl_xor_sync(0xffffffffu, up ? ka : kb, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        v = __shfl_sync(0xffffffffu, v, s.gather);
-        // SAD of a column: its four lanes' rows
-        sa += __shfl_xor_sync(0xffffffffu, sa, 1);
-        sa += __shfl_xor_sync(0xffffffffu, sa, 2);
-        sb += __shfl_xor_sync(0xffffffffu, sb, 1);
-        sb += __shfl_xor_sync(0xffffffffu, sb, 2);
-        const int at = one ? 4 * s.gl : s.gb + 4 * (s.gl & 1);
-        const int va = __shfl_sync(0xffffffffu, sa, at), vb = __shfl_sync(0xffffffffu, sb, at);
-        if (sad) v = one || !(s.gl & 2) ? va : vb;
-        if (one || (s.gl >> 2) == tp) out = v;
-    }
-    return out;
 }
 
 // The eight ring points (dx, dy) in the reference's order: (1,0) (-1,0) (0,1)
@@ -509,352 +490,61 @@ struct SearchOut {
     int x, y, cost, evals;
 };
 
-// motion_search (mb16.rs:2433-3302) of each group's partition, every group at
-// once (mode 0: four copies of one search).  preds p0 (the mvd centre) and,
-// with npred 2, p1.  Returns the reference's evaluation count in evals.
+// ---------------------------------------------------------------------------
+// The searches
+// ---------------------------------------------------------------------------
+// motion_search (mb16.rs:2433-3302) as a loop of rounds, each of a kind: the
+// seeds (with the integer snaps of sub-pel predictors, mb16.rs:2597-2607), the
+// learned search's proposals, a fixed-centre diamond of the full-pel ladder
+// (all four points, first strict minimum, as the reference's argmin loops), a
+// cascading ring (the centre moves mid-ring: the points left are priced
+// around the current centre, the first improvement moves it, and the rest are
+// priced again around the new one, the order in which the reference evaluates
+// them), the B2 reprice, or a fixed-centre sub-pel ring (sp_fc).  The centre,
+// `step` (quarter-pels; STEP_REPRICE between the ladder and the sub-pel steps)
+// and the kind are the state; evals counts what the reference evaluates.
 //
-// One loop around one pricing site: each iteration plans the next slots from
-// the phase state (seeds together with the snaps of sub-pel predictors,
-// diamond ladder, B2 reprice, sub-pel rings), prices them, and folds the
-// result back into the state.
-//  * fixed-centre batches (the FC diamond, sp_fc rings) price all points and
-//    take the first strict minimum, like the reference's argmin loops;
-//  * cascading rings (the centre moves mid-ring) price the remaining points
-//    against the current centre; at the first improvement the centre moves and
-//    the points after it are priced again around the new centre, which is the
-//    order in which the reference evaluates them.
 // Costs are dist + (λ·rate) as i64 held in 32 bits: distortions are below
 // 2^21 and λ·rate below 2^28 for every λ the encoder forms, so the sum never
 // saturates and comparisons match the reference's i64.
 //
-// LEARN with use_prop (the learned-proposal kernels' 16x16 search): after the
-// seeds, the 8 proposals (lane gl: proposal gl in `prop`) are priced, both with
-// `cost` (SATD and λ also where the full-pel phase has a cost of its own, so
-// that predictor and proposals compare); when the best proposal's distortion exceeds the
-// predictor's by more than prop_t the plain search goes on from the seeds
-// (fell = 1), otherwise it continues as motion_search with the cheapest of
-// predictor and proposals as its start vector (mb16.rs:2445, 2579-2596:
-// refine-only, no full-pel phase).  use_start: a refine-only search from
-// `start`.
-template <int MODE, bool LEARN>
-__device__ __forceinline__ SearchOut mb_search(const MbLane& s, const MeParamsDev& prm, MbScratch& ws, uint32_t lut, int2 p0, int2 p1,
-                                               int npred, double lambda_me, bool use_prop = false,
-                                               int2 prop = make_int2(0, 0), int prop_t = 0, int* fell = nullptr,
-                                               bool use_start = false, int2 start = make_int2(0, 0)) {
-    const Knobs kn{prm};
-    const int gl = s.gl, gb = s.gb;
-    constexpr bool one = MODE == 0;
-    const int rmax = one ? 8 : 4;      // points of a cascading ring priced per round: one pass
-    const bool sadfp = !prm.fast && prm.sadfp;
-    const int m_main = prm.use_sad ? MET_SAD : MET_SATD;
-    const int m_fp = sadfp ? MET_SAD : m_main;
-    const double lam_r = prm.kind != 0 ? lambda_me * 0.25 : lambda_me;  // cost's λ
-    const double lam_fp = lambda_me * (sadfp ? prm.sadfp_lambda : 1.0); // cost_fp's λ under the 16-wide FC diamond
-    const double l_fp = sadfp ? lam_fp : lam_r;
-    const bool fc = !prm.fast && prm.fc;
-    const int spat = prm.subpel_pat >= 0 ? prm.subpel_pat : (prm.sp_single_pass ? 2 : 0);
-    const bool sp_fc = prm.sp_fc && !prm.fast;
-    const int sp_nring = (spat & 1) ? 4 : 8;
-    const int rw = s.rw, rh = s.rh, cw = ws.cw, ch = ws.ch;
-
-    // Seed slots: 0 the zero MV, 1 p0, 2 p1 when it differs, then with the
-    // integer snap on the snapped positions of the sub-pel predictors
-    // (mb16.rs:2597-2607); equal positions share a slot (equal costs).
-    const bool two = npred > 1 && (p1.x != p0.x || p1.y != p0.y);
-    const int2 q0 = make_int2(((p0.x + 2) >> 2) * 4, ((p0.y + 2) >> 2) * 4);
-    const int2 q1 = make_int2(((p1.x + 2) >> 2) * 4, ((p1.y + 2) >> 2) * 4);
-    const bool snap0 = prm.me_snap && ((p0.x | p0.y) & 3) != 0;
-    const bool snap1 = two && prm.me_snap && ((p1.x | p1.y) & 3) != 0;
-    const int i_q0 = two ? 3 : 2;
-    const bool q_same = snap0 && q0.x == q1.x && q0.y == q1.y;
-    const int i_q1 = q_same ? i_q0 : i_q0 + (snap0 ? 1 : 0);
-    const int n_seed = i_q0 + (snap0 ? 1 : 0) + (snap1 && !q_same ? 1 : 0);
-    auto inside = [&](int x, int y, int step) {  // every point of the ring at full-pel distance inside the picture
-        const int st = step >> 2, px = s.px + (x >> 2), py = s.py + (y >> 2);
-        return px - st >= 0 && py - st >= 0 && px + st + rw <= cw && py + st + rh <= ch;
-    };
-
-    int evals = 0;
-    int bx = 0, by = 0, seed_x = 0, seed_y = 0;
-    int best_c = 0, seed_c = 0;
-    int cp = 0, dp = 0;  // the predictor's cost and distortion (learned search)
-    int phase = use_start ? PH_START : PH_SEEDS;
-    bool prop_next = use_prop;  // the proposals are still to be priced
-    int si = -1, sk = -1, loops = 0, iter = 0, step = 0;
-    bool ring_open = false, ring_improved = false;
-    int ring_i = 0, ring_n = 0;
-    for (;;) {
-        // ---------- plan (per group) ----------
-        int kind = -1, n = 0, metric = m_main;
-        int mx = bx, my = by;  // the lane's slot
-        double lam = lam_r;
-        while (kind < 0 && phase != PH_DONE) {
-            if (phase == PH_SEEDS) {
-                kind = EV_SEEDS; n = n_seed;
-                if (!(LEARN && prop_next)) { metric = m_fp; lam = l_fp; }
-                mx = my = 0;
-                if (gl == 1) { mx = p0.x; my = p0.y; }
-                if (two && gl == 2) { mx = p1.x; my = p1.y; }
-                if (snap0 && gl == i_q0) { mx = q0.x; my = q0.y; }
-                else if (snap1 && gl == i_q1) { mx = q1.x; my = q1.y; }
-            } else if (LEARN && phase == PH_PROP) {
-                mx = prop.x; my = prop.y;
-                kind = EV_PROP; n = N_PROP;
-            } else if (phase == PH_START) {
-                mx = start.x; my = start.y;
-                kind = EV_START; n = 1;
-            } else if (phase == PH_DIA) {
-                if (ring_open) {
-                    kind = EV_RING; n = min(ring_n - ring_i, rmax); metric = m_fp; lam = l_fp;
-                    break;
-                }
-                if (si < 0 || loops >= LOOP_GUARD) {
-                    const int nsi = kn.next_rung(si);
-                    if (nsi >= 5) {
-                        phase = PH_REPRICE;
-                        continue;
-                    }
-                    si = nsi;
-                    step = kn.rung_step(si);
-                    loops = 0;
-                }
-                loops++;
-                if (fc && ((bx | by) & 3) == 0 && inside(bx, by, step)) {
-                    kind = EV_FIXED; n = 4;
-                    metric = rw == 16 ? (sadfp ? MET_SAD : MET_SATD) : m_fp;
-                    lam = rw == 16 ? lam_fp : l_fp;
-                    mx = bx + ring_dx(gl & 3) * step;
-                    my = by + ring_dy(gl & 3) * step;
-                } else {
-                    ring_open = true; ring_improved = false; ring_i = 0; ring_n = 4;
-                    kind = EV_RING; n = 4; metric = m_fp; lam = l_fp;
-                }
-            } else if (phase == PH_REPRICE) {
-                if (sadfp) {
-                    if (gl == 1) { mx = seed_x; my = seed_y; }
-                    kind = EV_REPRICE; n = 2;
-                } else {
-                    phase = PH_SUB;
-                }
-            } else {  // PH_SUB
-                if (ring_open) {
-                    kind = EV_RING; n = min(ring_n - ring_i, rmax);
-                    break;
-                }
-                if (!prm.subpel) {
-                    phase = PH_DONE;
-                    continue;
-                }
-                if (sk < 0 || loops >= LOOP_GUARD) {
-                    if (++sk >= 2) {
-                        phase = PH_DONE;
-                        continue;
-                    }
-                    step = sk == 0 ? 2 : 1;
-                    loops = 0;
-                    iter = 0;
-                }
-                loops++;
-                iter++;
-                if (sp_fc && (spat & 1) == 0 && (step == 1 || ((bx | by) & 3) == 0)) {
-                    // hpel_qpel_refs / hpel_ref resolve every ring point (inter.rs:1015, 1060):
-                    // inside the +1-slack window, and at step 1 a quarter phase
-                    bool all = true;
-                    for (int i = 0; i < 8; i++) {
-                        const int rx = bx + ring_dx(i) * step, ry = by + ring_dy(i) * step;
-                        const int px = s.px + (rx >> 2) + ws.pad, py = s.py + (ry >> 2) + ws.pad;
-                        all = all && px >= 0 && py >= 0 && px + rw + 1 <= ws.pw && py + rh + 1 <= ws.ph &&
-                              (step == 2 || ((rx | ry) & 1));
-                    }
-                    if (all) {
-                        mx = bx + ring_dx(gl) * step;
-                        my = by + ring_dy(gl) * step;
-                        kind = EV_FIXED; n = 8;
-                        metric = rw == 16 ? MET_SATD : m_main;
-                        lam = rw == 16 ? lambda_me : lam_r;
-                        break;
-                    }
-                }
-                ring_open = true; ring_improved = false; ring_i = 0; ring_n = sp_nring;
-                kind = EV_RING; n = min(sp_nring, rmax);
-            }
-        }
-        if (kind == EV_RING && gl < n) {
-            mx = bx + ring_dx(ring_i + gl) * step;
-            my = by + ring_dy(ring_i + gl) * step;
-        }
-        if (kind < 0) n = 0;
-        if (__all_sync(0xffffffffu, kind < 0)) break;
-        const int nmax = one ? n : __reduce_max_sync(0xffffffffu, n);
-        // which collectives this round's folds need (warp-uniform)
-        const bool need_min = __any_sync(0xffffffffu, kind == EV_FIXED || kind == EV_PROP);
-        const bool need_hit = __any_sync(0xffffffffu, kind == EV_RING);
-        const bool need_seed = __any_sync(0xffffffffu, kind == EV_SEEDS || kind == EV_REPRICE || kind == EV_START);
-
-        // ---------- price ----------
-        const long long rc = lam_cost(lam, kn.rate(mx - p0.x, my - p0.y));
-        const int d = price_slots<MODE>(s, ws, lut, mx, my, n, nmax, metric == MET_SAD);
-        int cc = INT_MAX;  // dist + λ·rate of the lane's slot
-        if (gl < n) {
-            const long long c = (long long)d + rc;
-            cc = c > INT_MAX - 1 ? INT_MAX - 1 : int(c);
-        }
-        // group-wide collectives, taken by every lane: the first minimum of
-        // slots 0..3 and of 4..7, the first improving slot, the seed slots
-        int m0 = INT_MAX, m1 = INT_MAX;
-        unsigned at = 0;
-        if (need_min) {
-            int t = min(cc, __shfl_xor_sync(0xffffffffu, cc, 1));
-            t = min(t, __shfl_xor_sync(0xffffffffu, t, 2));
-            m0 = __shfl_sync(0xffffffffu, t, gb);
-            m1 = __shfl_sync(0xffffffffu, t, gb + 4);
-            at = (__ballot_sync(0xffffffffu, cc == t) >> gb) & 0xffu;
-        }
-        unsigned hit = 0;
-        int jhit = 0, cj = 0;
-        if (need_hit) {
-            hit = (__ballot_sync(0xffffffffu, gl < n && cc < best_c) >> gb) & 0xffu;
-            jhit = hit ? __ffs(hit) - 1 : 0;
-            cj = __shfl_sync(0xffffffffu, cc, gb + jhit);
-        }
-        int c_seed[5] = {0, 0, 0, 0, 0};
-        if (need_seed) {
-#pragma unroll
-            for (int i = 0; i < 5; i++) c_seed[i] = __shfl_sync(0xffffffffu, cc, gb + i);
-            if (LEARN) dp = __shfl_sync(0xffffffffu, d, gb + 1);
-        }
-
-        // ---------- fold (per group) ----------
-        if (kind == EV_SEEDS) {
-            // sequential strict-< scan: (0,0) first, then the predictors in order
-            best_c = c_seed[0];
-            bx = 0; by = 0;
-            int wi = 0;
-            if (c_seed[1] < best_c) { best_c = c_seed[1]; bx = p0.x; by = p0.y; wi = 1; }
-            if (two && c_seed[2] < best_c) { best_c = c_seed[2]; bx = p1.x; by = p1.y; wi = 2; }
-            cp = c_seed[1];
-            evals += npred + 1;
-            seed_x = bx; seed_y = by; seed_c = best_c;
-            if ((wi == 1 && snap0) || (wi == 2 && snap1)) {
-                // the winner is a sub-pel predictor: take its snap, priced in this round
-                bx = wi == 1 ? q0.x : q1.x;
-                by = wi == 1 ? q0.y : q1.y;
-                const int k = wi == 1 ? i_q0 : i_q1;
-                best_c = k == 2 ? c_seed[2] : (k == 3 ? c_seed[3] : c_seed[4]);
-                evals += 1;
-            }
-            phase = LEARN && prop_next ? PH_PROP : PH_DIA;
-        } else if (kind == EV_START) {
-            // a refine-only search (mb16.rs:2580-2582): the start vector
-            // priced with `cost`, no full-pel phase, the sub-pel steps from it
-            best_c = c_seed[0];
-            bx = start.x;
-            by = start.y;
-            seed_x = bx; seed_y = by; seed_c = best_c;
-            evals += 1;
-            phase = PH_SUB;
-        } else if (LEARN && kind == EV_PROP) {
-            // the cheapest proposal (first wins) and its distortion against the predictor's
-            const int m = min(m0, m1);
-            const unsigned bits = m0 == m ? at & 0xfu : at & 0xf0u;
-            const int bi = __ffs(bits) - 1;
-            const int dprop = __shfl_sync(0xffffffffu, d, gb + bi);  // mode 0: every lane is here
-            const int vx = __shfl_sync(0xffffffffu, prop.x, gb + bi), vy = __shfl_sync(0xffffffffu, prop.y, gb + bi);
-            const bool fb = (long long)dprop > (long long)dp + prop_t;
-            if (fell) *fell = fb ? 1 : 0;
-            prop_next = false;
-            if (fb) {
-                // the plain search goes on from its seeds, priced again where
-                // its full-pel cost is another than `cost`
-                evals = sadfp ? N_PROP + 1 : evals + N_PROP + 1;
-                phase = sadfp ? PH_SEEDS : PH_DIA;
-            } else {
-                evals = N_PROP + 1;
-                best_c = cp;
-                bx = p0.x; by = p0.y;
-                if (m < best_c) { best_c = m; bx = vx; by = vy; }
-                seed_x = bx; seed_y = by; seed_c = best_c;
-                phase = PH_SUB;  // a start vector: no full-pel phase, no B2 reprice
-            }
-        } else if (kind == EV_REPRICE) {
-            best_c = c_seed[0];
-            seed_c = c_seed[1];
-            evals += 2;
-            phase = PH_SUB;
-        } else if (kind == EV_FIXED) {
-            if (phase == PH_DIA) {
-                evals += 4;
-                if (m0 < best_c) {
-                    const int bi = __ffs(at & 0xfu) - 1;
-                    best_c = m0;
-                    bx += ring_dx(bi) * step;
-                    by += ring_dy(bi) * step;
-                } else {
-                    loops = LOOP_GUARD;  // rung done
-                }
-            } else {
-                evals += n;
-                const int m = min(m0, m1);
-                const int bi = m < best_c ? __ffs(m0 == m ? at & 0xfu : at & 0xf0u) - 1 : -1;
-                if (bi >= 0) {
-                    best_c = m;
-                    bx += ring_dx(bi) * step;
-                    by += ring_dy(bi) * step;
-                }
-                if (bi < 0 || !prm.me_subpel_iter || (spat & 2) || (prm.sp_maxit != 0 && iter >= prm.sp_maxit))
-                    loops = LOOP_GUARD;
-            }
-        } else if (kind == EV_RING) {
-            if (hit == 0) {
-                evals += n;
-                ring_i += n;
-            } else {
-                best_c = cj;
-                evals += jhit + 1;
-                bx += ring_dx(ring_i + jhit) * step;
-                by += ring_dy(ring_i + jhit) * step;
-                ring_improved = true;
-                ring_i += jhit + 1;
-            }
-            ring_open = ring_i < ring_n;
-            if (!ring_open) {
-                if (phase == PH_DIA) {
-                    if (!ring_improved) loops = LOOP_GUARD;
-                } else if (!ring_improved || !prm.me_subpel_iter || (spat & 2) ||
-                           (prm.sp_maxit != 0 && iter >= prm.sp_maxit)) {
-                    loops = LOOP_GUARD;
-                }
-            }
-        }
-        __syncwarp();
-    }
-    // ---- seed restore (mb16.rs:3297-3300) ----
-    if (prm.me_snap && seed_c < best_c) {
-        bx = seed_x; by = seed_y; best_c = seed_c;
-    }
-    return SearchOut{bx, by, best_c, evals};
-}
-
-// ---------------------------------------------------------------------------
-// The Balanced preset's searches
-// ---------------------------------------------------------------------------
-// mb_search above runs any preset.  The Balanced preset's 16x16 search, which
-// every MB runs and the wavefront waits for, has its own form, in which every
-// decision is warp-uniform: costs are compared through redux and ballots, a
+// BAL: the Balanced preset's knobs as constants, and the λ·rate products from
+// a table per λ.  Host rule (balanced_preset): the preset's knobs and
+// 0 <= λ < 2^23, so that every table entry and cost fits 31 bits.  Any other
+// preset, or λ, runs the same rounds with its knobs read.  (One CIF frame,
+// fast / walk to convergence / full ladder: 493, 1,607 and 1,641 us with four
+// warps an MB and butterflies; 593, 2,004 and 2,852 with one warp and a search
+// of their own for both modes, its state per lane and its sums by shuffles;
+// 414, 1,472 and 1,615 this way, with the registers for it, see ME_ANY_BLOCKS.)
+//
+// Every decision of the 16x16 search, which every MB runs and the wavefront
+// waits for, is warp-uniform: costs are compared through redux and ballots, a
 // lane forms its column's candidate from the round's centre, step and ring
-// index, the operand addresses come from a 16-entry table and the
-// λ·rate products from a table per λ, and one pass's column sums cross the
-// lanes through shared memory.  Host rule (balanced_search_ok): the preset's
-// knobs and 0 <= λ < 2^23, so that every table entry and cost fits 31 bits.
+// index, the operand addresses come from a 16-entry table, and a pass's
+// column sums cross the lanes through shared memory.
+//
+// LEARN with use_prop (the learned-proposal kernels' 16x16 search): after the
+// seeds, the 8 proposals are priced, both with `cost` (SATD and λ also where
+// the full-pel phase has a cost of its own, so that predictor and proposals
+// compare); when the best proposal's distortion exceeds the predictor's by
+// more than prop_t the plain search goes on from the seeds (fell = 1),
+// otherwise it continues as motion_search with the cheapest of predictor and
+// proposals as its start vector (mb16.rs:2445, 2579-2596: refine-only, no
+// full-pel phase).  use_start: a refine-only search from `start`.
 
 constexpr int LAM_TAB = 48;  // (λ·rate) as i64 for rates below LAM_TAB
+constexpr double LAM_TAB_MAX = 8388608.0;  // of a λ whose products fit 31 bits (rates up to 126)
+constexpr int STEP_REPRICE = 3;
 
-// Per-warp tables and scratch of the Balanced searches.
-struct BalScratch {
+// Per-warp tables and scratch of the searches.
+struct SearchScratch {
     double lam;             // the λ the table holds (NaN: none)
+    double lam_main, lam_dia;  // not BAL: the λ of `cost` and of the fixed diamond
     int lamtab[LAM_TAB];
-    int red[2][8][8];       // column sums' shares: [tile][lane / 4][column]
+    // a pass's shares, 64 words a tile: SATD [lane / 4][column], then SAD [column][lane % 4]
+    alignas(16) int red[128];
 };
+static_assert(offsetof(SearchScratch, red) % 16 == 0 && sizeof(SearchScratch) % 16 == 0, "16-byte reads of the shares");
 // Per-CTA operand table: byte offsets in the window of both operands of each
 // quarter phase fx * 4 + fy (equal at one-plane phases).
 struct PhaseTab {
@@ -867,7 +557,7 @@ __device__ __forceinline__ void phase_tab_init(PhaseTab& t, int i) {
     const uint32_t b = ((pb >> 2) & 3u) * WIN_PLANE + ((pb >> 7) & 1u) * WIN_STRIDE + ((pb >> 6) & 1u);
     t.e[i] = make_uint2(a, ((pb >> 2) & 3u) ? b : a);
 }
-__device__ __forceinline__ void bal_lambda(BalScratch& b, double lambda_me) {
+__device__ __forceinline__ void bal_lambda(SearchScratch& b, double lambda_me) {
     if (b.lam == lambda_me) return;  // warp-uniform
     __syncwarp();
     for (int r = int(threadIdx.x & 31); r < LAM_TAB; r += 32) b.lamtab[r] = int(lam_cost(lambda_me, uint32_t(r)));
@@ -879,41 +569,131 @@ __device__ __forceinline__ uint32_t eg_bits(int d) {
     const uint32_t v = uint32_t(d > 0 ? 2 * d : 1 - 2 * d);
     return 63u - 2u * uint32_t(__clz(int(v)));
 }
-__device__ __forceinline__ int bal_rate_cost(const BalScratch& b, double lam, int dx, int dy) {
+__device__ __forceinline__ int bal_rate_cost(const SearchScratch& b, double lam, int dx, int dy) {
     const uint32_t r = eg_bits(dx) + eg_bits(dy);
     return r < LAM_TAB ? b.lamtab[r] : int(lam_cost(lam, r));
 }
 
-// The 16x16 search of the Balanced preset (predictor p0 the mvd centre), warp-uniform.
-// LEARN with use_prop: as mb_search's.  propc / propg: proposals lane / 4 and
-// lane % 8.
-template <bool LEARN, int REF>
-__device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws, BalScratch& bs, uint32_t lut, int2 p0,
-                                                  double lambda_me, bool use_prop, int2 propc, int2 propg, int prop_t,
-                                                  int* fell) {
-    constexpr int SEED = 0, DIA = 1, RING = 2, PROP = 3;
+// A preset's knobs as the searches read them: constants for BAL, else worked
+// out once a search.  A round's cost is one of four: `cost`, the full-pel
+// phase's cost_fp, the 16-wide fixed diamond's and the 16-wide sub-pel ring's.
+constexpr int C_MAIN = 0, C_FP = 1, C_DIA = 2, C_SPFC = 3;
+template <bool BAL>
+struct Knobs {
+    static constexpr bool kSnap = true, kFc = true, kSadfp = false, kSpFc = false;
+    static constexpr int kFirst = 16, kSub = 2, kRing = 8, sads = 0, tabs = 15;
+    __device__ __forceinline__ Knobs(const MeParamsDev&, double lambda_me, SearchScratch& b) { bal_lambda(b, lambda_me); }
+    __device__ __forceinline__ int next_step(int step) const { return step >> 1; }
+    __device__ __forceinline__ bool again(int) const { return false; }
+    __device__ __forceinline__ bool sad(int) const { return false; }
+};
+template <>
+struct Knobs<false> {
+    bool kSnap, kFc, kSadfp, kSpFc, iterate;
+    int kFirst, kSub, kRing;
+    int ladder;  // the steps of the full-pel ladder, one bit each (64 .. 4 quarter-pels by dia_mask's bits 0..4)
+    int maxit, sads, tabs;  // sads, tabs: a bit per cost
+    __device__ __forceinline__ Knobs(const MeParamsDev& p, double lambda_me, SearchScratch& b) {
+        const bool full = !p.fast;
+        const int pat = p.subpel_pat >= 0 ? p.subpel_pat : (p.sp_single_pass ? 2 : 0);
+        kSnap = p.me_snap;
+        kFc = full && p.fc;
+        kSadfp = full && p.sadfp;
+        kSpFc = full && p.sp_fc && (pat & 1) == 0;
+        iterate = p.me_subpel_iter && !(pat & 2);
+        maxit = p.sp_maxit != 0 ? p.sp_maxit : INT_MAX;
+        kRing = (pat & 1) ? 4 : 8;
+        kSub = p.subpel ? 2 : 0;
+        ladder = full ? int(__brev(p.dia_mask & 0x1fu) >> 25) : 16 + 4;
+        kFirst = lower(128);
+        const int m = p.use_sad ? 1 : 0, f = kSadfp ? 1 : 0;
+        sads = m << C_MAIN | (f | m) << C_FP | f << C_DIA;
+        // Exp-Golomb rates: the costs whose λ is λ itself read its table
+        const bool tab = p.kind == 0 && lambda_me >= 0.0 && lambda_me < LAM_TAB_MAX;
+        tabs = tab ? (kSadfp ? 1 << C_MAIN | 1 << C_SPFC : 15) : 0;
+        if (b.lam != lambda_me) {  // warp-uniform
+            __syncwarp();
+            if ((threadIdx.x & 31) == 0) {
+                b.lam_main = p.kind != 0 ? lambda_me * 0.25 : lambda_me;
+                b.lam_dia = kSadfp ? lambda_me * p.sadfp_lambda : lambda_me;
+            }
+            if (!tab && (threadIdx.x & 31) == 0) b.lam = lambda_me;
+            __syncwarp();
+            if (tab) bal_lambda(b, lambda_me);
+        }
+    }
+    __device__ __forceinline__ int lower(int step) const {
+        const int r = ladder & (step - 1);
+        return r ? 1 << (31 - __clz(r)) : (kSadfp ? STEP_REPRICE : kSub);
+    }
+    // the step after `step` (0: the search is done)
+    __device__ __forceinline__ int next_step(int step) const {
+        return step > STEP_REPRICE ? lower(step) : (step == STEP_REPRICE ? kSub : step >> 1);
+    }
+    // another sub-pel ring at the step after `iter` of them, the last of which improved
+    __device__ __forceinline__ bool again(int iter) const { return iterate && iter < maxit; }
+    __device__ __forceinline__ bool sad(int cost) const { return (sads >> cost) & 1; }
+};
+// (λ·rate) of an mvd, and a cost
+template <bool BAL>
+__device__ __forceinline__ long long rate_cost(const MeParamsDev& p, const SearchScratch& b, double lambda_me, int tabs, bool sadfp,
+                                               int cost, int dx, int dy) {
+    if (BAL || tabs == 15 || (tabs >> cost) & 1) return bal_rate_cost(b, lambda_me, dx, dy);
+    const double l = cost == C_MAIN || (cost == C_FP && !sadfp) ? b.lam_main : (cost == C_SPFC ? lambda_me : b.lam_dia);
+    return lam_cost(l, mvbits(p.kind, p.tab, dx) + mvbits(p.kind, p.tab, dy));
+}
+template <bool BAL>
+__device__ __forceinline__ int cost_sum(int d, long long rc) {
+    if constexpr (BAL) return d + int(rc);
+    const long long c = (long long)d + rc;
+    return c > INT_MAX - 1 ? INT_MAX - 1 : int(c);
+}
+
+// Every point of the w x h block's ring at full-pel distance st inside the picture.
+__device__ __forceinline__ bool ring_inside(const MbLane& s, int cw, int ch, int x, int y, int st) {
+    const int ox = s.px + (x >> 2), oy = s.py + (y >> 2);
+    return ox - st >= 0 && oy - st >= 0 && ox + st + s.rw <= cw && oy + st + s.rh <= ch;
+}
+// hpel_qpel_refs / hpel_ref resolve the ring point (inter.rs:1015, 1060): inside
+// the planes with a slack of 1, and at step 1 a quarter phase
+__device__ __forceinline__ bool point_resolves(const MbLane& s, const MbScratch& ws, int x, int y, int step) {
+    const int ox = s.px + (x >> 2) + ws.pad, oy = s.py + (y >> 2) + ws.pad;
+    return ox >= 0 && oy >= 0 && ox + s.rw + 1 <= ws.pw && oy + s.rh + 1 <= ws.ph && (step == 2 || ((x | y) & 1));
+}
+
+// The 16x16 search (predictor p0 the mvd centre), warp-uniform.  propc / propg:
+// proposals lane / 4 and lane % 8.
+template <bool BAL, bool LEARN, int REF, bool CG>
+__device__ __forceinline__ SearchOut search16(const MbLane& s, const MeParamsDev& prm, MbScratch& ws, SearchScratch& bs, uint32_t lut,
+                                              int2 p0, double lambda_me, bool use_prop, int2 propc, int2 propg, int prop_t,
+                                              int* fell) {
+    constexpr int SEED = 0, DIA = 1, RING = 2, PROP = 3, SPFC = 4, REPRICE = 5;
     constexpr unsigned FULL = 0xffffffffu;
-    const int lane = s.lane, gl = s.gl, col = lane >> 2;
-    const int px = s.px, py = s.py, cw = ws.cw, ch = ws.ch;
-    bal_lambda(bs, lambda_me);
-    auto inside = [&](int x, int y, int st) {  // the ring's points at full-pel distance st inside the picture
-        const int ox = px + (x >> 2), oy = py + (y >> 2);
-        return ox - st >= 0 && oy - st >= 0 && ox + st + 16 <= cw && oy + st + 16 <= ch;
-    };
+    const Knobs<BAL> kn(prm, lambda_me, bs);
+    const int lane = s.lane, gl = s.gl, col = lane >> 2, cw = ws.cw, ch = ws.ch;
     const int2 q0 = make_int2(((p0.x + 2) >> 2) * 4, ((p0.y + 2) >> 2) * 4);  // its integer snap
     const bool sub = ((p0.x | p0.y) & 3) != 0;
-    const bool seed_ring = !(LEARN && use_prop) && inside(q0.x, q0.y, 4);
+    const int step0 = kn.kFirst;
+    bool prop_next = LEARN && use_prop;  // the proposals are still to be priced
+    // the first rung's ring around p0's (snapped) position in the seeds' round, where both have one cost
+    const bool seed_ring = !prop_next && step0 >= 4 && kn.kFc && (kn.kSnap || !sub) && (BAL || kn.kSadfp || (!prm.use_sad && prm.kind == 0)) &&
+                           ring_inside(s, cw, ch, q0.x, q0.y, step0 >> 2);
     int evals = 0, best = 0, seed_c = 0, seed_x = 0, seed_y = 0, cp = 0, dp = 0;
-    int cx = q0.x, cy = q0.y, step = 16, kind = SEED, ri = 0, rn = 4;
+    int cx = q0.x, cy = q0.y, step = step0, kind = SEED, ri = 0, rn = 4;
+    int iter = 0, loops = 0;  // rings at this step (not counted for BAL, whose steps end by themselves)
+    int low = step0, cost = prop_next ? C_MAIN : C_FP;  // DIA: the next rung where it is >= 4; the round's cost
     bool improved = false;
     for (;;) {
         // the candidates of the lane's mma column and of its cost slot: SEED
         // 0 the zero MV, 1 p0, 2 its snap, 4..7 the first rung's ring around
-        // the snap; DIA this rung's ring and the next's; RING the points from ri
+        // the snap; DIA this rung's ring and the next's; RING and SPFC the
+        // points from ri; REPRICE the centre and the seed
         int mx, my, rx, ry;
         {
-            const int ic = kind == RING ? min(ri + col, 7) : col & 3, ig = kind == RING ? min(ri + gl, 7) : gl & 3;
-            const int sc = kind == DIA && col >= 4 ? step >> 1 : step, sg = kind == DIA && gl >= 4 ? step >> 1 : step;
+            const int ic = kind == RING ? min(ri + col, 7) : (kind == SPFC ? col : col & 3),
+                      ig = kind == RING ? min(ri + gl, 7) : (kind == SPFC ? gl : gl & 3);
+            const int lw = BAL ? step >> 1 : low;
+            const int sc = kind == DIA && col >= 4 ? lw : step, sg = kind == DIA && gl >= 4 ? lw : step;
             mx = cx + ring_dx(ic) * sc; my = cy + ring_dy(ic) * sc;
             rx = cx + ring_dx(ig) * sg; ry = cy + ring_dy(ig) * sg;
             if (kind == SEED) {
@@ -921,22 +701,35 @@ __device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws
                 if (gl < 4 || !seed_ring) { rx = gl == 0 ? 0 : (gl == 1 ? p0.x : q0.x); ry = gl == 0 ? 0 : (gl == 1 ? p0.y : q0.y); }
             }
             if (LEARN && kind == PROP) { mx = propc.x; my = propc.y; rx = propg.x; ry = propg.y; }
+            if (!BAL && kind == REPRICE) {
+                mx = col == 1 ? seed_x : cx; my = col == 1 ? seed_y : cy;
+                rx = gl == 1 ? seed_x : cx; ry = gl == 1 ? seed_y : cy;
+            }
         }
+        const bool sad = kn.sad(cost);
         const CandAddr<REF> ta = cand_addr<REF>(s, ws, lut, mx, my);
-        const int rc = bal_rate_cost(bs, lambda_me, rx - p0.x, ry - p0.y);
+        const long long rc = rate_cost<BAL>(prm, bs, lambda_me, kn.tabs, kn.kSadfp, cost, rx - p0.x, ry - p0.y);
         int a0, a1, b0, b1, sa, sb;
         // a two-plane phase is possible among the seeds, at quarter-pel steps
         // and, from a start vector, around a quarter-pel centre
-        const bool two = kind == SEED || step == 1 || (LEARN && (kind == PROP || ((cx | cy) & 1)));
-        price_pass<0, REF, false>(s, ws, ta, ta, mx, my, mx, my, two, false, a0, a1, b0, b1, sa, sb);
-        // column sums through shared memory: slot gl's eight shares
-        *reinterpret_cast<int2*>(&bs.red[0][col][2 * (lane & 3)]) = make_int2(a0, a1);
-        __syncwarp();
+        const bool two = BAL ? kind == SEED || step == 1 || (LEARN && (kind == PROP || ((cx | cy) & 1))) : __any_sync(FULL, (mx | my) & 1);
+        price_pass<0, REF, CG, !BAL>(s, ws, ta, ta, mx, my, mx, my, two, false, !sad, sad, a0, a1, b0, b1, sa, sb);
+        // column sums through shared memory: slot gl's eight shares, or four rows' SADs
         int d = 0;
+        if (!sad) {
+            *reinterpret_cast<int2*>(&bs.red[8 * col + 2 * (lane & 3)]) = make_int2(a0, a1);
+            __syncwarp();
 #pragma unroll
-        for (int g = 0; g < 8; g++) d += bs.red[0][g][gl];
+            for (int g = 0; g < 8; g++) d += bs.red[8 * g + gl];
+        } else {
+            bs.red[lane] = sa;
+            __syncwarp();
+            const int4 r = *reinterpret_cast<const int4*>(&bs.red[4 * gl]);
+            d = r.x + r.y + r.z + r.w;
+        }
         __syncwarp();  // read by every lane: the next round stores its own
-        const int cc = d + rc;
+        const int cc = cost_sum<BAL>(d, rc);
+        bool stay = false;  // another ring at this step
         if (kind == RING) {
             const unsigned hit = __ballot_sync(FULL, gl < rn - ri && cc < best) & 0xffu;
             if (hit) {
@@ -952,7 +745,7 @@ __device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws
                 ri = rn;
             }
             if (ri < rn) continue;  // the rest of the ring around the moved centre
-            if (!(step >= 4 && improved)) step >>= 1;
+            stay = improved && (step >= 4 || kn.again(iter));
         } else {
             // the minima of slots 0..3 and 4..7 and their first slots
             const int m0 = __reduce_min_sync(FULL, gl < 4 ? cc : INT_MAX), m1 = __reduce_min_sync(FULL, gl < 4 ? INT_MAX : cc);
@@ -960,22 +753,24 @@ __device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws
             const int j0 = __ffs(at) - 1, j1 = __ffs(at >> 4) - 1;
             if (kind == DIA) {
                 evals += 4;
+                stay = true;
                 if (m0 < best) {
                     best = m0;
                     cx += ring_dx(j0) * step;
                     cy += ring_dy(j0) * step;
-                } else {
-                    step >>= 1;
-                    if (step >= 4) {  // the next rung's first ring, priced beside it
-                        evals += 4;
-                        if (m1 < best) {
-                            best = m1;
-                            cx += ring_dx(j1) * step;
-                            cy += ring_dy(j1) * step;
-                        } else {
-                            step >>= 1;
-                        }
+                } else if ((BAL ? step >> 1 : low) >= 4) {  // the next rung's first ring, priced beside it
+                    step = BAL ? step >> 1 : low;
+                    loops = 0;
+                    evals += 4;
+                    if (m1 < best) {
+                        best = m1;
+                        cx += ring_dx(j1) * step;
+                        cy += ring_dy(j1) * step;
+                    } else {
+                        stay = false;
                     }
+                } else {
+                    stay = false;
                 }
             } else if (kind == SEED) {
                 // sequential strict-< scan: (0,0), then the predictor; the
@@ -986,40 +781,57 @@ __device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws
                     cp = c1;
                     dp = __reduce_min_sync(FULL, gl == 1 ? d : INT_MAX);
                 }
-                evals = 2;
+                evals += 2;
                 if (c1 < c0) {
                     best = seed_c = c1;
                     seed_x = p0.x; seed_y = p0.y;
-                    if (sub) {
+                    if (sub && kn.kSnap) {
                         best = c2;
-                        evals = 3;
+                        evals += 1;
+                    } else if (!BAL) {
+                        cx = p0.x; cy = p0.y;
                     }
                 } else {
                     best = seed_c = c0;
+                    seed_x = seed_y = 0;
                     cx = cy = 0;
                 }
-                if (LEARN && use_prop) {
+                if (LEARN && (BAL ? use_prop : prop_next)) {  // (the seeds come once for BAL)
                     kind = PROP;
                     continue;
                 }
+                stay = true;
                 if (seed_ring && cx == q0.x && cy == q0.y) {
                     evals += 4;
                     if (m1 < best) {
                         best = m1;
-                        cx += ring_dx(j1) * 16;
-                        cy += ring_dy(j1) * 16;
+                        cx += ring_dx(j1) * step;
+                        cy += ring_dy(j1) * step;
                     } else {
-                        step = 8;
+                        stay = false;
                     }
                 }
+            } else if (!BAL && kind == SPFC) {
+                const int m = min(m0, m1), j = m0 == m ? j0 : 4 + j1;
+                evals += 8;
+                if (m < best) {
+                    best = m;
+                    cx += ring_dx(j) * step;
+                    cy += ring_dy(j) * step;
+                    stay = kn.again(iter);
+                }
+            } else if (!BAL && kind == REPRICE) {
+                best = __reduce_min_sync(FULL, gl == 0 ? cc : INT_MAX);
+                seed_c = __reduce_min_sync(FULL, gl == 1 ? cc : INT_MAX);
+                evals += 2;
             } else {  // PROP: the cheapest proposal (first wins) against the predictor
                 const int m = min(m0, m1), j = m0 == m ? j0 : 4 + j1;
                 const int dprop = __reduce_min_sync(FULL, gl == j ? d : INT_MAX);
                 const bool fb = dprop - dp > prop_t;
                 *fell = fb ? 1 : 0;
-                if (fb) {
-                    evals += N_PROP + 1;  // the plain search goes on from its seeds
-                } else {
+                prop_next = false;
+                stay = true;
+                if (!fb) {
                     evals = N_PROP + 1;
                     best = cp;
                     cx = p0.x; cy = p0.y;
@@ -1029,83 +841,137 @@ __device__ __forceinline__ SearchOut search16_bal(const MbLane& s, MbScratch& ws
                         cy = __shfl_sync(FULL, propg.y, j);
                     }
                     seed_c = best; seed_x = cx; seed_y = cy;
-                    step = 2;  // a start vector: the sub-pel steps only
+                    step = kn.kSub;  // a start vector: the sub-pel steps only
+                } else if (kn.kSadfp) {
+                    // the plain search's seeds, priced again with its full-pel cost
+                    evals = N_PROP + 1;
+                    cx = q0.x; cy = q0.y;
+                    kind = SEED;
+                    cost = C_FP;
+                    continue;
+                } else {
+                    evals += N_PROP + 1;  // the plain search goes on from its seeds
                 }
             }
+        }
+        if (BAL) {
+            if (!stay) step >>= 1;
+        } else if (!stay || ++loops >= LOOP_GUARD) {
+            step = kn.next_step(step);
+            iter = loops = 0;
         }
         if (step == 0) break;
         improved = false;
         ri = 0;
-        rn = step >= 4 ? 4 : 8;
-        kind = step >= 4 && inside(cx, cy, step >> 2) ? DIA : RING;
+        rn = step >= 4 ? 4 : kn.kRing;
+        kind = RING;
+        if constexpr (BAL) {
+            if (step >= 4 && ring_inside(s, cw, ch, cx, cy, step >> 2)) kind = DIA;
+        } else {
+            iter++;
+            cost = C_MAIN;
+            if (step >= 4) {
+                cost = C_FP;
+                if (kn.kFc && ((cx | cy) & 3) == 0 && ring_inside(s, cw, ch, cx, cy, step >> 2)) {
+                    kind = DIA;
+                    cost = C_DIA;
+                    low = kn.lower(step);
+                }
+            } else if (step == STEP_REPRICE) {
+                kind = REPRICE;
+            } else if (kn.kSpFc && (step == 1 || ((cx | cy) & 3) == 0) &&
+                       __all_sync(FULL, point_resolves(s, ws, cx + ring_dx(gl) * step, cy + ring_dy(gl) * step, step))) {
+                kind = SPFC;
+                cost = C_SPFC;
+            }
+        }
     }
     // ---- seed restore (mb16.rs:3297-3300) ----
-    if (seed_c < best) {
+    if (kn.kSnap && seed_c < best) {
         cx = seed_x; cy = seed_y; best = seed_c;
     }
     return SearchOut{cx, cy, best, evals};
 }
 
-// The four partitions of the Balanced preset, group g of eight lanes searching
-// partition g (mode 1): seeds (0,0), p0 (the mvd centre), p1, then as
-// search16_bal, four slots a round.  use_start: refine-only from `start`.
-template <bool LEARN, int REF>
-__device__ __forceinline__ SearchOut search_parts_bal(const MbLane& s, MbScratch& ws, BalScratch& bs, uint32_t lut, int2 p0,
-                                                      int2 p1, double lambda_me, bool use_start, int2 start) {
-    constexpr int SEED = 0, DIA = 1, RING = 2, SNAP = 3, START = 4, DONE = 5;
+// The four partitions, group g of eight lanes searching partition g (mode 1):
+// seeds (0,0), p0 (the mvd centre), p1, then as search16, four slots a round
+// (a fixed-centre ring of eight takes two).  use_start: refine-only from `start`.
+template <bool BAL, bool LEARN, int REF, bool CG>
+__device__ __forceinline__ SearchOut search_parts(const MbLane& s, const MeParamsDev& prm, MbScratch& ws, SearchScratch& bs, uint32_t lut,
+                                                  int2 p0, int2 p1, double lambda_me, bool use_start, int2 start) {
+    constexpr int SEED = 0, DIA = 1, RING = 2, SNAP = 3, START = 4, DONE = 5, SPFC = 6, REPRICE = 7;
     constexpr unsigned FULL = 0xffffffffu;
-    const int gl = s.gl, gb = s.gb, sl = gl & 3, grp = gb >> 3, half = (s.lane >> 2) & 1;
-    const int px = s.px, py = s.py, cw = ws.cw, ch = ws.ch;
-    bal_lambda(bs, lambda_me);
-    auto inside = [&](int x, int y, int st) {
-        const int ox = px + (x >> 2), oy = py + (y >> 2);
-        return ox - st >= 0 && oy - st >= 0 && ox + st + s.rw <= cw && oy + st + s.rh <= ch;
-    };
+    const Knobs<BAL> kn(prm, lambda_me, bs);
+    const int gl = s.gl, gb = s.gb, sl = gl & 3, grp = gb >> 3, half = (s.lane >> 2) & 1, cw = ws.cw, ch = ws.ch;
     auto snap = [](int v) { return ((v + 2) >> 2) * 4; };
     const bool two = p1.x != p0.x || p1.y != p0.y;  // equal predictors: p1 cannot win
     // seed slots: 0 the zero MV, 1 p0, 2 p1, 3 the snap of p1 (the likely winner)
     const int2 q0 = make_int2(snap(p0.x), snap(p0.y)), q1 = make_int2(snap(p1.x), snap(p1.y));
     const bool sub1 = ((p1.x | p1.y) & 3) != 0;
     int evals = 0, best = 0, seed_c = 0, seed_x = 0, seed_y = 0;
-    int cx = 0, cy = 0, step = 16, kind = SEED, ri = 0, rn = 4;
+    int cx = 0, cy = 0, step = kn.kFirst, kind = SEED, ri = 0, rn = 4;
+    int iter = 0, loops = 0, fm = 0, fj = 0;  // SPFC: the first four points' minimum and its point
+    int cost = C_FP;
     bool improved = false;
     if (LEARN && use_start) {
         kind = START;
+        cost = C_MAIN;
         cx = seed_x = start.x;
         cy = seed_y = start.y;
     }
     while (!__all_sync(FULL, kind == DONE)) {
         // the MV of slot i of this round
         auto slot_mv = [&](int i, int& x, int& y) {
-            const int ir = kind == RING ? min(ri + i, 7) : i;
+            const int ir = kind == RING || (!BAL && kind == SPFC) ? min(ri + i, 7) : i;
             x = cx + ring_dx(ir) * step;
             y = cy + ring_dy(ir) * step;
             if (kind == SEED) {
                 x = i == 0 ? 0 : (i == 1 ? p0.x : (i == 2 ? p1.x : q1.x));
                 y = i == 0 ? 0 : (i == 1 ? p0.y : (i == 2 ? p1.y : q1.y));
-            } else if (kind >= SNAP) {  // (DONE: a position the window covers)
+            } else if (kind >= SNAP && (BAL || kind <= DONE)) {  // (DONE: a position the window covers)
                 x = cx;
                 y = cy;
+            } else if (!BAL && kind == REPRICE) {
+                x = i == 1 ? seed_x : cx;
+                y = i == 1 ? seed_y : cy;
             }
         };
         int ax, ay, bx, by, rx, ry;
         slot_mv(half, ax, ay);
         slot_mv(half + 2, bx, by);
         slot_mv(sl, rx, ry);
+        const bool sad = kn.sad(cost);
+        bool any_satd = true, any_sad = false;
+        if (!BAL && kn.sads != 0) {
+            any_satd = __any_sync(FULL, kind != DONE && !sad);
+            any_sad = __any_sync(FULL, kind != DONE && sad);
+        }
         const CandAddr<REF> ta = cand_addr<REF>(s, ws, lut, ax, ay), tb = cand_addr<REF>(s, ws, lut, bx, by);
-        const int rc = bal_rate_cost(bs, lambda_me, rx - p0.x, ry - p0.y);
-        const bool planes2 = __any_sync(FULL, ta.a != ta.b || tb.a != tb.b);
+        const long long rc = rate_cost<BAL>(prm, bs, lambda_me, kn.tabs, kn.kSadfp, cost, rx - p0.x, ry - p0.y);
+        const bool planes2 = __any_sync(FULL, ((ax | ay | bx | by) & 1) != 0 && kind != DONE);  // quarter phases
         int a0, a1, b0, b1, sa, sb;
-        price_pass<1, REF, false>(s, ws, ta, tb, ax, ay, bx, by, planes2, kind == DONE, a0, a1, b0, b1, sa, sb);
+        price_pass<1, REF, CG, !BAL>(s, ws, ta, tb, ax, ay, bx, by, planes2, kind == DONE, any_satd, any_sad, a0, a1, b0, b1, sa, sb);
         // column sums through shared memory: columns 2g, 2g+1 of tile A are
         // slots 0, 1 of group g, of tile B slots 2, 3
-        *reinterpret_cast<int2*>(&bs.red[0][s.lane >> 2][2 * (s.lane & 3)]) = make_int2(a0, a1);
-        *reinterpret_cast<int2*>(&bs.red[1][s.lane >> 2][2 * (s.lane & 3)]) = make_int2(b0, b1);
-        __syncwarp();
         int d = 0;
+        if (any_satd) {
+            int* const mine = &bs.red[8 * (s.lane >> 2) + 2 * (s.lane & 3)];
+            *reinterpret_cast<int2*>(mine) = make_int2(a0, a1);
+            *reinterpret_cast<int2*>(mine + 64) = make_int2(b0, b1);
+            __syncwarp();
 #pragma unroll
-        for (int g = 0; g < 8; g++) d += bs.red[sl >> 1][g][2 * grp + (sl & 1)];
-        const int cc = d + rc;
+            for (int g = 0; g < 8; g++) d += bs.red[64 * (sl >> 1) + 8 * g + 2 * grp + (sl & 1)];
+            __syncwarp();  // as in search16
+        }
+        if (any_sad) {
+            bs.red[s.lane] = sa;
+            bs.red[64 + s.lane] = sb;
+            __syncwarp();
+            const int4 r = *reinterpret_cast<const int4*>(&bs.red[64 * (sl >> 1) + 4 * (2 * grp + (sl & 1))]);
+            if (sad) d = r.x + r.y + r.z + r.w;
+            __syncwarp();
+        }
+        const int cc = cost_sum<BAL>(d, rc);
         // collectives of every group's fold
         const int n = rn - ri < 4 ? rn - ri : 4;
         const unsigned hit = (__ballot_sync(FULL, sl < n && cc < best) >> gb) & 0xfu;
@@ -1116,8 +982,7 @@ __device__ __forceinline__ SearchOut search_parts_bal(const MbLane& s, MbScratch
         const int cj = __shfl_sync(FULL, cc, gb + jh);
         const int c0 = __shfl_sync(FULL, cc, gb), c1 = __shfl_sync(FULL, cc, gb + 1), c2 = __shfl_sync(FULL, cc, gb + 2),
                   c3 = __shfl_sync(FULL, cc, gb + 3);
-        __syncwarp();
-        bool next = false;  // the round's ring or rung is done
+        bool next = false, stay = false;  // the round's ring or rung is done; another at its step
         if (kind == RING) {
             if (hit) {
                 best = cj;
@@ -1131,15 +996,14 @@ __device__ __forceinline__ SearchOut search_parts_bal(const MbLane& s, MbScratch
                 ri += n;
             }
             next = ri >= rn;
-            if (next && !(step >= 4 && improved)) step >>= 1;
+            stay = improved && (step >= 4 || kn.again(iter));
         } else if (kind == DIA) {
             evals += 4;
             if (m < best) {
                 best = m;
                 cx += ring_dx(jm) * step;
                 cy += ring_dy(jm) * step;
-            } else {
-                step >>= 1;
+                stay = true;
             }
             next = true;
         } else if (kind == SEED) {
@@ -1147,14 +1011,14 @@ __device__ __forceinline__ SearchOut search_parts_bal(const MbLane& s, MbScratch
             // integer snap is the centre
             evals = 3;
             best = seed_c = c0;
-            next = true;
+            next = stay = true;
             if (c1 < best) { best = seed_c = c1; cx = seed_x = p0.x; cy = seed_y = p0.y; }
             if (two && c2 < best) { best = seed_c = c2; cx = seed_x = p1.x; cy = seed_y = p1.y; }
-            if (best == c2 && two && cx == p1.x && cy == p1.y && sub1) {
+            if (kn.kSnap && best == c2 && two && cx == p1.x && cy == p1.y && sub1) {
                 best = c3;
                 cx = q1.x; cy = q1.y;
                 evals = 4;
-            } else if ((cx | cy) & 3) {  // p0 won
+            } else if (kn.kSnap && ((cx | cy) & 3)) {  // p0 won
                 evals = 4;
                 cx = q0.x; cy = q0.y;
                 if (cx == q1.x && cy == q1.y) {
@@ -1166,21 +1030,69 @@ __device__ __forceinline__ SearchOut search_parts_bal(const MbLane& s, MbScratch
             }
         } else if (kind == SNAP) {
             best = c0;
-            next = true;
+            next = stay = true;
         } else if (LEARN && kind == START) {
             best = seed_c = c0;
             evals = 1;
-            step = 2;
+            step = kn.kSub;
+            next = stay = true;
+        } else if (!BAL && kind == SPFC) {
+            if (ri == 0) {
+                fm = m; fj = jm;
+                ri = 4;
+            } else {
+                if (m < fm) { fm = m; fj = 4 + jm; }
+                evals += 8;
+                next = true;
+                if (fm < best) {
+                    best = fm;
+                    cx += ring_dx(fj) * step;
+                    cy += ring_dy(fj) * step;
+                    stay = kn.again(iter);
+                }
+            }
+        } else if (!BAL && kind == REPRICE) {
+            best = c0;
+            seed_c = c1;
+            evals += 2;
             next = true;
         }
         if (next) {
+            if (BAL) {
+                if (!stay) step >>= 1;
+            } else if (!stay || ++loops >= LOOP_GUARD) {
+                step = kn.next_step(step);
+                iter = loops = 0;
+            }
             improved = false;
             ri = 0;
-            rn = step >= 4 ? 4 : 8;
-            kind = step == 0 ? DONE : (step >= 4 && inside(cx, cy, step >> 2) ? DIA : RING);
+            rn = step >= 4 ? 4 : kn.kRing;
+            if constexpr (BAL) {
+                kind = step == 0 ? DONE : (step >= 4 && ring_inside(s, cw, ch, cx, cy, step >> 2) ? DIA : RING);
+            } else {
+                iter++;
+                kind = step == 0 ? DONE : (step == STEP_REPRICE ? REPRICE : RING);
+                cost = C_MAIN;
+                if (step >= 4) {
+                    cost = C_FP;
+                    if (kn.kFc && ((cx | cy) & 3) == 0 && ring_inside(s, cw, ch, cx, cy, step >> 2)) {
+                        kind = DIA;
+                        if (s.rw == 16) cost = C_DIA;
+                    }
+                }
+            }
+        }
+        if (!BAL && kn.kSpFc) {
+            // a sub-pel ring about to start: all its points resolve
+            const bool r = point_resolves(s, ws, cx + ring_dx(gl) * step, cy + ring_dy(gl) * step, step);
+            const unsigned all = (__ballot_sync(FULL, r) >> gb) & 0xffu;
+            if (next && kind == RING && step < STEP_REPRICE && (step == 1 || ((cx | cy) & 3) == 0) && all == 0xffu) {
+                kind = SPFC;
+                if (s.rw == 16) cost = C_SPFC;
+            }
         }
     }
-    if (seed_c < best) {
+    if (kn.kSnap && seed_c < best) {
         cx = seed_x; cy = seed_y; best = seed_c;
     }
     return SearchOut{cx, cy, best, evals};

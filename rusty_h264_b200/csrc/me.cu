@@ -433,7 +433,14 @@ __device__ __forceinline__ bool job_shape_ok(int w, int h) {
            (w == 4 && (h == 8 || h == 4));
 }
 
-constexpr int ME_MIN_BLOCKS = 4;  // CTAs per SM of the frame kernels (their windows fill the shared memory)
+// CTAs per SM that the frame kernels' registers allow: three with Balanced,
+// whose searches need some 140 registers a thread; at the 128 of four CTAs their
+// reloads cost more than the further warps give (1080p closed loop 25.4 and 24.1
+// ms, one 720p frame with its reconstruction 1.88 and 1.78, 75 mixed frames
+// 4.52 and 4.12).  Two with other presets, whose searches hold more: reloads at
+// 128 and 168 registers cost a round 20% and 5%, also in calls of many frames
+// (fifteen 720p frames walked to convergence: 4.24, 3.72 and 3.65 ms).
+constexpr int ME_MIN_BLOCKS = 3, ME_ANY_BLOCKS = 2;
 
 __global__ void __launch_bounds__(32 * ME_WARPS) me_search_kernel(const h264a_picture* __restrict__ pics, int npics,
                                                                  const __grid_constant__ MeParamsDev prm,
@@ -744,7 +751,7 @@ struct WarpWindow {
     uint8_t* p;
     uint32_t win, bar, lut;
 };
-__device__ __forceinline__ WarpWindow warp_window(uint8_t* dyn, unsigned long long* bars, PhaseTab& pt, BalScratch* bs) {
+__device__ __forceinline__ WarpWindow warp_window(uint8_t* dyn, unsigned long long* bars, PhaseTab& pt, SearchScratch* bs) {
     const int w = threadIdx.x >> 5;
     WarpWindow o;
     o.p = dyn + w * WIN_BYTES;
@@ -771,9 +778,9 @@ __device__ __forceinline__ WarpWindow warp_window(uint8_t* dyn, unsigned long lo
 // the wavefront's path.  So the window's origin comes from the top MB's MV
 // and its copy overlaps the wait for the left MB; any origin gives the same
 // picks, as candidates the window misses read the planes.
-template <bool BAL, bool LEARN, bool REC>
+template <bool BAL, bool LEARN, bool REC, bool PIPE>
 __device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp, int mbx, int mby,
-                                         const MeParamsDev& prm, const MbSync& sy, MbScratch& ws, BalScratch& bs,
+                                         const MeParamsDev& prm, const MbSync& sy, MbScratch& ws, SearchScratch& bs,
                                          const WarpWindow& ww, uint32_t& parity, bool tmap_global) {
     const uint32_t win = ww.win, bar = ww.bar;
     uint8_t* const winp = ww.p;
@@ -837,11 +844,8 @@ __device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp
     // best_part for 16x16, then, J above the gate, the four partitions seeded
     // [pmv, mv16] side by side
     int shape = 0, fell = 0;
-    SearchOut r16;
-    if constexpr (BAL)
-        r16 = search16_bal<LEARN, REF_WINDOW>(s, ws, bs, ww.lut, pmv, fd.lambda_me, LEARN, propc, prop, fd.prop_t, &fell);
-    else
-        r16 = mb_search<0, LEARN>(s, prm, ws, ww.lut, pmv, pmv, 1, fd.lambda_me, LEARN, prop, fd.prop_t, &fell);
+    const SearchOut r16 =
+        search16<BAL, LEARN, REF_WINDOW, PIPE>(s, prm, ws, bs, ww.lut, pmv, fd.lambda_me, LEARN, propc, prop, fd.prop_t, &fell);
     int evals = r16.evals << 4;  // 4x4-block evaluations
     const int c16 = r16.cost;
     long long best = c16;
@@ -851,11 +855,8 @@ __device__ __forceinline__ void frame_mb(const FrameDesc& fd, const RecDesc* rdp
         // the learned search's partitions, when its 16x16 search took a
         // proposal: refine-only from the 16x16 MV
         const int2 mv16 = make_int2(mv0x, mv0y);
-        SearchOut r;
-        if constexpr (BAL)
-            r = search_parts_bal<LEARN, REF_WINDOW>(s, ws, bs, ww.lut, pmv, mv16, fd.lambda_me, LEARN && !fell, mv16);
-        else
-            r = mb_search<1, LEARN>(s, prm, ws, ww.lut, pmv, mv16, 2, fd.lambda_me, false, prop, 0, nullptr, LEARN && !fell, mv16);
+        const SearchOut r =
+            search_parts<BAL, LEARN, REF_WINDOW, PIPE>(s, prm, ws, bs, ww.lut, pmv, mv16, fd.lambda_me, LEARN && !fell, mv16);
         int px[4], py[4];
         long long pcost[4];
 #pragma unroll
@@ -1025,11 +1026,11 @@ __device__ __forceinline__ void me_frames_body(const TAB& tab, long long total, 
                                                unsigned long long* __restrict__ words, int epoch,
                                                int* __restrict__ status, int spin_limit) {
     __shared__ MbScratch scratch[ME_WARPS];
-    __shared__ __align__(16) BalScratch bal[ME_WARPS];
+    __shared__ __align__(16) SearchScratch scr[ME_WARPS];
     __shared__ PhaseTab ptab;
     __shared__ __align__(8) unsigned long long win_bar[ME_WARPS];
     extern __shared__ __align__(128) uint8_t me_win[];
-    const WarpWindow ww = warp_window(me_win, win_bar, ptab, bal);
+    const WarpWindow ww = warp_window(me_win, win_bar, ptab, scr);
     MbScratch& ws = scratch[threadIdx.x >> 5];
     uint32_t parity = 0;
     for (;;) {
@@ -1053,12 +1054,12 @@ __device__ __forceinline__ void me_frames_body(const TAB& tab, long long total, 
         const MbSync sy{words ? words + EW_PER_MB * (long long)fd.flag_base : nullptr, flags + fd.flag_base,
                         REC ? flags + rd->dflag_base : nullptr, REC ? flags + rd->nz_base : nullptr, nullptr, epoch,
                         status, spin_limit};
-        frame_mb<BAL, LEARN, REC>(fd, rd, mbx, mby, prm, sy, ws, bal[threadIdx.x >> 5], ww, parity, TAB::kGlobal);
+        frame_mb<BAL, LEARN, REC, false>(fd, rd, mbx, mby, prm, sy, ws, scr[threadIdx.x >> 5], ww, parity, TAB::kGlobal);
     }
 }
 
 template <bool BAL, bool LEARN = false>
-__global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
+__global__ void __launch_bounds__(32 * ME_WARPS, BAL ? ME_MIN_BLOCKS : ME_ANY_BLOCKS)
     me_frames_kernel(const __grid_constant__ FrameBatch batch, long long total, const __grid_constant__ MeParamsDev prm,
                      int* __restrict__ counter, int* __restrict__ flags, unsigned long long* __restrict__ words,
                      int epoch, int* __restrict__ status, int spin_limit) {
@@ -1068,7 +1069,7 @@ __global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
 // The same kernel over a frame table in device memory (more than ME_MAXF
 // frames in one wavefront launch); the frames' tensor maps are read there.
 template <bool BAL, bool LEARN = false>
-__global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
+__global__ void __launch_bounds__(32 * ME_WARPS, BAL ? ME_MIN_BLOCKS : ME_ANY_BLOCKS)
     me_frames_dkernel(const FrameDesc* __restrict__ frames, const long long* __restrict__ seg_start,
                       const int* __restrict__ seg_j, int nframes, int nseg, long long total,
                       const __grid_constant__ MeParamsDev prm, int* __restrict__ counter, int* __restrict__ flags,
@@ -1097,7 +1098,7 @@ struct StepTable {
     __device__ __forceinline__ const RecDesc* rec(int i) const { return &b.rec[i]; }
 };
 template <bool BAL, bool LEARN>
-__global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
+__global__ void __launch_bounds__(32 * ME_WARPS, BAL ? ME_MIN_BLOCKS : ME_ANY_BLOCKS)
     me_step_kernel(const __grid_constant__ StepBatch batch, long long total, const __grid_constant__ MeParamsDev prm,
                    int* __restrict__ counter, int* __restrict__ flags, unsigned long long* __restrict__ words, int epoch,
                    int* __restrict__ status, int spin_limit) {
@@ -1202,17 +1203,17 @@ __device__ __forceinline__ void pipe_band(const PipeParams& pp, int h, int b, in
 }
 
 template <bool BAL, bool LEARN>
-__global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
+__global__ void __launch_bounds__(32 * ME_WARPS, BAL ? ME_MIN_BLOCKS : ME_ANY_BLOCKS)
     closed_pipe_kernel(const __grid_constant__ PipeParams pp, const __grid_constant__ MeParamsDev prm, int epoch,
                        int* __restrict__ status, int spin_limit) {
     __shared__ MbScratch scratch[ME_WARPS];
-    __shared__ __align__(16) BalScratch bal[ME_WARPS];
+    __shared__ __align__(16) SearchScratch scr[ME_WARPS];
     __shared__ PhaseTab ptab;
     __shared__ __align__(8) unsigned long long win_bar[ME_WARPS];
     __shared__ BandWait bwait[ME_WARPS];
     extern __shared__ __align__(128) uint8_t me_win[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const WarpWindow ww = warp_window(me_win, win_bar, ptab, bal);
+    const WarpWindow ww = warp_window(me_win, win_bar, ptab, scr);
     uint32_t parity = 0;
     int fenced = -1;   // the frame whose tensor map this warp has acquired and whose sources it has seen
     int h = 1 + int((blockIdx.x * ME_WARPS + w) % unsigned(pp.pools));  // this warp's pool: frames h, h + pools, ...
@@ -1249,7 +1250,7 @@ __global__ void __launch_bounds__(32 * ME_WARPS, ME_MIN_BLOCKS)
         // frame 1's reference (frame 0) is built before the launch
         const MbSync sy{reinterpret_cast<unsigned long long*>(ff + pp.ew_off), nullptr, ff + pp.dfl_off, ff + pp.nz_off,
                         h > 1 ? &bwait[w] : nullptr, epoch, status, spin_limit};
-        frame_mb<BAL, LEARN, true>(pp.fds[h], pp.rds + h, item % pp.mb_w, item / pp.mb_w, prm, sy, scratch[w], bal[w], ww,
+        frame_mb<BAL, LEARN, true, true>(pp.fds[h], pp.rds + h, item % pp.mb_w, item / pp.mb_w, prm, sy, scratch[w], scr[w], ww,
                                    parity, fenced != h);
         fenced = h;
         if (lane == 0 && pp.frame_words == nullptr) {
@@ -1314,20 +1315,20 @@ static int encode_window_map(CUtensorMap* map, const uint8_t* planes, int pw, in
 
 // Dynamic shared memory of me_frames_kernel, its opt-in above 48 KB, and the
 // CTAs per SM it reaches.
-static int me_frames_setup_once(int& per_sm, bool learn);
+static int me_frames_setup_once(int& per_sm, bool bal, bool learn);
 // Cached per device: the attributes and the occupancy of the frame kernels
 // (queried once, not on every launch).
-static int me_frames_setup(int& per_sm, bool learn = false) {
+static int me_frames_setup(int& per_sm, bool bal, bool learn = false) {
     constexpr int kMaxDev = 64;
-    static int cached[kMaxDev][2];  // CTAs per SM + 1, 0 while unknown
+    static int cached[kMaxDev][4];  // CTAs per SM + 1, 0 while unknown
     static std::mutex mu;
     int dev = 0;
     H264A_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDev) return me_frames_setup_once(per_sm, learn);
+    if (dev < 0 || dev >= kMaxDev) return me_frames_setup_once(per_sm, bal, learn);
     std::lock_guard<std::mutex> lock(mu);
-    int& c = cached[dev][learn ? 1 : 0];
+    int& c = cached[dev][(bal ? 2 : 0) + (learn ? 1 : 0)];
     if (!c) {
-        const int rc = me_frames_setup_once(per_sm, learn);
+        const int rc = me_frames_setup_once(per_sm, bal, learn);
         if (rc) return rc;
         c = per_sm + 1;
     }
@@ -1335,7 +1336,7 @@ static int me_frames_setup(int& per_sm, bool learn = false) {
     return H264A_OK;
 }
 
-static int me_frames_setup_once(int& per_sm, bool learn) {
+static int me_frames_setup_once(int& per_sm, bool bal, bool learn) {
     const int smem = ME_WARPS * WIN_BYTES;
     H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
     H264A_CUDA(cudaFuncSetAttribute(me_frames_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
@@ -1350,11 +1351,9 @@ static int me_frames_setup_once(int& per_sm, bool learn) {
     H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
     H264A_CUDA(cudaFuncSetAttribute(me_step_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRAME_SMEM_MAX));
     per_sm = 0;
-    if (learn)
-        H264A_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, me_frames_kernel<false, true>, 32 * ME_WARPS,
-                                                                 smem));
-    else
-        H264A_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, me_frames_kernel<false>, 32 * ME_WARPS, smem));
+    auto kern = bal ? (learn ? me_frames_kernel<true, true> : me_frames_kernel<true, false>)
+                    : (learn ? me_frames_kernel<false, true> : me_frames_kernel<false, false>);
+    H264A_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * ME_WARPS, smem));
     if (per_sm < 1) per_sm = 1;
     return H264A_OK;
 }
@@ -1362,7 +1361,7 @@ static int me_frames_setup_once(int& per_sm, bool learn) {
 // A λ that the Balanced searches' tables hold: every (λ·rate) as i64 (rates
 // up to 126) and every cost (distortions below 2^21) fits 31 bits.  The
 // encoder's are below 1,500; others run the general search.
-static bool balanced_lambda(double lam) { return lam >= 0.0 && lam < 8388608.0; }
+static bool balanced_lambda(double lam) { return lam >= 0.0 && lam < LAM_TAB_MAX; }
 // True when the parameters are the Balanced preset's (h264a_me_params_default)
 // and the frames' λ allow it (lam_ok): the frame kernels then run the searches
 // written for it.
@@ -1533,9 +1532,6 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
     }
     cudaStream_t st = pick_stream(ctx, stream);
     const MeParamsDev prm = to_dev(*params);
-    int per_sm = 0;
-    int rc0 = me_frames_setup(per_sm, learn != nullptr);
-    if (rc0) return rc0;
     // One wavefront launch over all frames, largest first: the frame table in
     // the kernel's parameters up to ME_MAXF frames, in device memory beyond.
     std::vector<int> order(nframes);
@@ -1602,6 +1598,9 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
         total += (long long)d.mb_w * d.mb_h;
         if (total >= (1LL << 31)) return fail(H264A_E_ARG, "me_frames: too many macroblocks in one call");
     }
+    int per_sm = 0;
+    int rc = me_frames_setup(per_sm, balanced_preset(prm, lam_ok), learn != nullptr);
+    if (rc) return rc;
     std::vector<long long> seg(nframes + 1);
     std::vector<int> segj(nframes);
     const int nseg = make_segments(desc.data(), nframes, seg.data(), segj.data());
@@ -1621,7 +1620,7 @@ int h264a::me_frames_run(h264a_ctx* ctx, const h264a_me_frame* h_frames, int nfr
     const int qi = few ? Q_WIDE : Q_MAIN;
     WorkQueue& qw = ctx->q[qi];
     const size_t nflags = size_t(rec ? 3 * total : total);  // with rec: then deblocking flags and coefficient masks
-    int rc = ensure_me_scratch(ctx, nflags, qi);
+    rc = ensure_me_scratch(ctx, nflags, qi);
     if (!rc && words_ok) rc = ensure_me_words(ctx, size_t(EW_PER_MB) * size_t(total), qi);
     if (rc) return rc;
     H264A_CUDA(cudaMemsetAsync(qw.d_counter, 0, sizeof(int32_t), st));
@@ -1828,11 +1827,11 @@ extern "C" int h264a_me_frames_noalloc(const h264a_me_frame* h_frames, int nfram
     H264A_CUDA(cudaMemsetAsync(scratch, 0, sizeof(int) * size_t(1 + total), st));
     H264A_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int32_t), st));
     int per_sm = 0, sms = 0;
-    const int rc0 = me_frames_setup(per_sm);
+    const MeParamsDev prm = to_dev(*params);
+    const int rc0 = me_frames_setup(per_sm, balanced_preset(prm, lam_ok));
     if (rc0) return rc0;
     H264A_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const long long blocks = frame_ctas(fb.f, fb.n, total, sms, per_sm);
-    const MeParamsDev prm = to_dev(*params);
     launch_me_frames(prm, unsigned(blocks), frame_smem(blocks, sms), st, fb, total, scratch, scratch + 1, nullptr, kNoallocFlag, d_status, lam_ok);
     return check_launch("me_frames_kernel (no-alloc)");
 }
@@ -1850,27 +1849,24 @@ static int closed_pipe_setup_once() {
 }
 
 // The per-device kernel attributes and the CTAs per SM of the pipelined loop.
-static int closed_pipe_setup(int& per_sm) {
+static int closed_pipe_setup(int& per_sm, bool bal) {
     constexpr int kMaxDev = 64;
-    static int cached[kMaxDev];
+    static int cached[kMaxDev][2];
     static std::mutex mu;
     int dev = 0;
     H264A_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(mu);
-    if (dev < 0 || dev >= kMaxDev || !cached[dev]) {
-        int rc = closed_pipe_setup_once();
-        if (rc) return rc;
-        int p = 0;
-        H264A_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, closed_pipe_kernel<false, true>,
-                                                                 32 * ME_WARPS, ME_WARPS * WIN_BYTES));
-        if (p < 1) p = 1;
-        if (dev < 0 || dev >= kMaxDev) {
-            per_sm = p;
-            return H264A_OK;
-        }
-        cached[dev] = p;
+    const bool known = dev >= 0 && dev < kMaxDev;
+    if (known && cached[dev][bal]) {
+        per_sm = cached[dev][bal];
+        return H264A_OK;
     }
-    per_sm = cached[dev];
+    const int rc = closed_pipe_setup_once();
+    if (rc) return rc;
+    auto kern = bal ? closed_pipe_kernel<true, true> : closed_pipe_kernel<false, true>;
+    H264A_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * ME_WARPS, ME_WARPS * WIN_BYTES));
+    if (per_sm < 1) per_sm = 1;
+    if (known) cached[dev][bal] = per_sm;
     return H264A_OK;
 }
 
@@ -1883,8 +1879,9 @@ int h264a::closed_pipe_run(h264a_ctx* ctx, const ClosedPipeIn& in, const h264a_m
     const int mb_w = cw / 16, mb_h = ch / 16, nmb = mb_w * mb_h, nbands = mb_h;
     const long long fs = (long long)cw * ch, cs = fs / 4, pbytes = 4LL * pw * ph;
     const MeParamsDev prm = to_dev(*params);
+    const bool bal = balanced_preset(prm, balanced_lambda(in.lambda_me)), learn = in.props != nullptr;
     int per_sm = 0;
-    int rc = closed_pipe_setup(per_sm);
+    int rc = closed_pipe_setup(per_sm, bal);
     if (rc) return rc;
     // the frame and reconstruction descriptors (entry 0 unused)
     std::vector<FrameDesc> fds(n);
@@ -2011,7 +2008,6 @@ int h264a::closed_pipe_run(h264a_ctx* ctx, const ClosedPipeIn& in, const h264a_m
     const int epoch = next_epoch(ctx, st, Q_WIDE);
     if (epoch < 0) return H264A_E_CUDA;
     const long long blocks = (long long)ctx->num_sms * pipe_ctas_per_sm(mb_w, mb_h, pools, ctx->num_sms, per_sm);
-    const bool bal = balanced_preset(prm, balanced_lambda(in.lambda_me)), learn = in.props != nullptr;
     auto kern = bal ? (learn ? closed_pipe_kernel<true, true> : closed_pipe_kernel<true, false>)
                     : (learn ? closed_pipe_kernel<false, true> : closed_pipe_kernel<false, false>);
     kern<<<unsigned(blocks), 32 * ME_WARPS, frame_smem(blocks, ctx->num_sms), st>>>(pp, prm, epoch, ctx->d_status, SPIN_LIMIT);
@@ -2078,18 +2074,18 @@ __device__ __forceinline__ int2 pick_mr_at(const int32_t* picks, int m, int bx4,
 // staged in shared memory by TMA, or every candidate read from L2 through the
 // search's global path (no window, no shared memory, the same results).
 template <bool BAL, int NW, bool STAGE>
-__global__ void __launch_bounds__(32 * NW, 16 / NW)
+__global__ void __launch_bounds__(32 * NW, (BAL ? 16 : 4 * ME_ANY_BLOCKS) / NW)
     me_frames_mr_kernel(const FrameDescMR* __restrict__ fds, const long long* __restrict__ seg_start,
                         const int* __restrict__ seg_j, int nf, int ns, long long total,
                         const __grid_constant__ MeParamsDev prm, int* __restrict__ counter, int* __restrict__ flags,
                         int epoch, int* __restrict__ status, int spin_limit) {
     __shared__ MbScratch scratch[NW];
-    __shared__ __align__(16) BalScratch bal[NW];
+    __shared__ __align__(16) SearchScratch scr[NW];
     __shared__ PhaseTab ptab;
     __shared__ __align__(8) unsigned long long win_bar[NW];
     extern __shared__ __align__(128) uint8_t me_win[];
     const int lane = threadIdx.x & 31;
-    const WarpWindow ww = warp_window(me_win, win_bar, ptab, bal);
+    const WarpWindow ww = warp_window(me_win, win_bar, ptab, scr);
     MbScratch& ws = scratch[threadIdx.x >> 5];
     uint32_t parity = 0;
     for (;;) {
@@ -2154,18 +2150,12 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW)
                     wait_window(ww.bar, parity, status, 3, spin_limit);
                     parity ^= 1u;
                 }
-                SearchOut o;
+                constexpr int REF = STAGE ? REF_WINDOW : REF_PLANES;
+                SearchScratch& bs = scr[threadIdx.x >> 5];
                 const int2 mv16 = make_int2(mv16x, mv16y);
-                if constexpr (BAL) {
-                    if (mode == 0)
-                        o = search16_bal<false, STAGE ? REF_WINDOW : REF_PLANES>(s, ws, bal[threadIdx.x >> 5], ww.lut, pmv, fd.lambda_me, false, pmv, pmv, 0,
-                                                       nullptr);
-                    else
-                        o = search_parts_bal<false, STAGE ? REF_WINDOW : REF_PLANES>(s, ws, bal[threadIdx.x >> 5], ww.lut, pmv, mv16, fd.lambda_me, false, mv16);
-                } else {
-                    o = mode == 0 ? mb_search<0, false>(s, prm, ws, ww.lut, pmv, pmv, 1, fd.lambda_me)
-                                  : mb_search<1, false>(s, prm, ws, ww.lut, pmv, mv16, 2, fd.lambda_me);
-                }
+                const SearchOut o =
+                    mode == 0 ? search16<BAL, false, REF, false>(s, prm, ws, bs, ww.lut, pmv, fd.lambda_me, false, pmv, pmv, 0, nullptr)
+                              : search_parts<BAL, false, REF, false>(s, prm, ws, bs, ww.lut, pmv, mv16, fd.lambda_me, false, mv16);
                 const long long cst = o.cost + __double2ll_rz(__dmul_rn(fd.lambda_me, double(ref_bits_of(r, fd.nref))));
                 if (mode == 0) {
                     evals += o.evals << 4;

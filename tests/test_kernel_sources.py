@@ -31,7 +31,7 @@ def body(name, head):
 def test_column_sums_are_read_before_the_next_round_stores():
     """The lanes of a search exchange column sums through the warp's shared
     scratch: a __syncwarp between every read of a round and the next store."""
-    for head in ("SearchOut search16_bal(", "SearchOut search_parts_bal("):
+    for head in ("SearchOut search16(", "SearchOut search_parts("):
         b = body("mb_search.cuh", head)
         loop = b[b.index("bs.red"):]  # store, sync, read, ... and round again
         last = [m.end() for m in re.finditer(r"d \+= bs\.red\[[^;]*;", loop)][-1]
