@@ -384,12 +384,13 @@ extern "C" int h264a_fullpel_grid(h264a_ctx* ctx, const h264a_picture* h_pic, in
     // one launch per metric wanted (its grid, or the argmin's metric)
     if (d_sad_grid || metric == 0) {
         // MBs per CTA: the most even fill of whole rounds of GRID_THREADS
-        // items, at most SAD_MAX_MBS windows and 100 KB (two CTAs per SM)
+        // items, at most SAD_MAX_MBS windows and SAD_SMEM (two CTAs per SM)
+        constexpr size_t SAD_SMEM = 100 * 1024;
         const int n = 2 * R + 1, per_mb = n * ((n + GRID_K - 1) / GRID_K);
         const int win_bytes = int((smem + 15) & ~size_t(15));
         int mbs = 1;
         double best_fill = 0.0;
-        for (int m = 1; m <= SAD_MAX_MBS && size_t(m) * win_bytes <= 100 * 1024; m++) {
+        for (int m = 1; m <= SAD_MAX_MBS && size_t(m) * win_bytes <= SAD_SMEM; m++) {
             const int rounds = (m * per_mb + GRID_THREADS - 1) / GRID_THREADS;
             const double fill = double(m * per_mb) / double(rounds * GRID_THREADS);
             if (fill > best_fill + 1e-9) {
@@ -399,7 +400,7 @@ extern "C" int h264a_fullpel_grid(h264a_ctx* ctx, const h264a_picture* h_pic, in
         }
         const size_t sm = size_t(mbs) * win_bytes;
         if (sm > 48 * 1024)
-            H264A_CUDA(cudaFuncSetAttribute(fullpel_sad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+            H264A_CUDA(cudaFuncSetAttribute(fullpel_sad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SAD_SMEM)));
         fullpel_sad_kernel<<<unsigned((nmb + mbs - 1) / mbs), GRID_THREADS, sm, st>>>(a, mbs, nmb, win_bytes);
         const int rc = check_launch("fullpel_sad_kernel");
         if (rc) return rc;
@@ -417,7 +418,7 @@ extern "C" int h264a_fullpel_grid(h264a_ctx* ctx, const h264a_picture* h_pic, in
         while (g == runs && ps < 4 && 2 * ps * g * n <= GRID_THREADS && need(2 * ps, g) <= SATD_SMEM) ps *= 2;
         const size_t sm = need(ps, g);
         if (sm > 48 * 1024)
-            H264A_CUDA(cudaFuncSetAttribute(fullpel_satd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+            H264A_CUDA(cudaFuncSetAttribute(fullpel_satd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SATD_SMEM)));
         const int threads = std::min(GRID_THREADS, (ps * g * n + 31) / 32 * 32);
         fullpel_satd_kernel<<<nmb, threads, sm, st>>>(a, ps, g);
         const int rc = check_launch("fullpel_satd_kernel");

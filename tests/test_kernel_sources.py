@@ -123,3 +123,10 @@ def test_network_waits_that_run_out_are_reported():
         assert m.group(0).endswith("z.status);"), m.group(0)[-60:]
     for call in ("forward", "grads", "propose", "get_params"):  # train_step calls grads
         assert "check_waits(" in body("mvnet.cu", "int h264a_mvnet_%s(" % call), call
+
+
+def test_grid_opt_ins_do_not_depend_on_the_call():
+    """Two threads' calls of different radius: the opt-in of one must not fall
+    below what the other is about to launch with."""
+    for m in re.finditer(r"cudaFuncSetAttribute\(fullpel_\w+, cudaFuncAttributeMaxDynamicSharedMemorySize, ([^)]*\)?)\)", source("grid.cu")):
+        assert re.fullmatch(r"int\([A-Z_]+\)|[A-Z_]+", m.group(1)), m.group(1)
