@@ -1036,10 +1036,12 @@ def run_ours(args, ws, rank, local):
         "kernel": "me_frames_kernel (persistent plain-ME)", "bound": "int32", "achieved": round(achieved, 1),
         "peak": round(int32_peak, 1), "unit": "Gop/s", "frac": round(achieved / int32_peak, 4),
         "peak_source": "measured live by h264a_measure_int32_peak (INT32 is not in MEASURED_PEAKS.json)",
-        # dram__bytes_read.sum + dram__bytes_write.sum of one launch (ncu --set full of the
-        # 60-frame step: 481,440 MBs, 1374.5 MB + 42.6 MB), scaled by MBs to this launch
-        "traffic": int(1415.2e6 / 481440 * (n - 1) * nmb),
-        "traffic_source": "ncu capture of the 60-frame 1080p launch, scaled by macroblocks",
+        # dram__bytes_read.sum + dram__bytes_write.sum of one launch (ncu, 15 1080p P frames:
+        # 122,400 MBs, 171.4 MB + 8.4 MB), scaled by MBs to this launch
+        "traffic": int(179.8e6 / 122400 * (n - 1) * nmb),
+        "traffic_source": "ncu capture of 15 1080p P frames, scaled by macroblocks",
+        "note": "operations of the reference's transforms (112 INT32 operations per 4x4 block); the kernel does them "
+                "as tensor-core products, so frac compares work and is no share of the INT32 pipe's issue",
         "work": {"satd_4x4_evals_per_step": work4x4, "ops_per_4x4": SATD_OPS_PER_4X4},
         "critical_path": {"me_ms_all_frames": round(stage["me"], 3), "frames": n - 1,
                           "me_ms_third_of_frames": round(float(np.mean(sub_ms)), 3), "frames_in_third": sub_n,
@@ -1122,15 +1124,17 @@ def run_ours(args, ws, rank, local):
         "achieved": round(c_achieved, 1), "peak": round(int32_peak, 1), "unit": "Gop/s",
         "frac": round(c_achieved / int32_peak, 4),
         "peak_source": "measured live by h264a_measure_int32_peak (INT32 is not in MEASURED_PEAKS.json)",
-        "traffic": int(1415.2e6 / 481440 * nmb * (n - 1)),
-        "traffic_source": "ncu capture of the 60-frame source-model launch (1415.2 MB over 481,440 MBs), scaled "
-                          "by macroblocks to the launch's 59 P frames",
+        "traffic": int(170.9e6 / 57120 * nmb * (n - 1)),
+        "traffic_source": "ncu capture of the launch over 7 1080p P frames (88.7 MB read, 82.2 MB written, 57,120 "
+                          "MBs), scaled by macroblocks to the launch's 59 P frames",
         "work": {"satd_4x4_evals_per_step": cwork, "ops_per_4x4": SATD_OPS_PER_4X4,
                  "launch_ms": round(pipe_ms, 3), "launches": 1,
                  "timing": "CUDA events around h264a_closed_frames alone (memsets, the planes of rec(0), the "
                            "pipelined kernel), median of 3"},
         "note": "each frame is a wavefront of 254 anti-diagonals bound by its critical path; the pipelined launch "
-                "overlaps a frame with the rows of the previous one its searches do not read",
+                "overlaps a frame with the rows of the previous one its searches do not read.  The operations are the "
+                "reference's transforms (112 per 4x4 block), done as tensor-core products: frac compares work and is "
+                "no share of the INT32 pipe's issue",
     }
     closed_launches = 2 + 3  # the planes of rec(0) and the pipelined kernel; lookahead 3
     line = {

@@ -23,11 +23,13 @@ struct WorkQueue {
     size_t words_cap = 0;
     int32_t epoch = 0;
 };
-// Q_MAIN serves plain-ME, deblocking and the bounded-wait self-test (flags
-// that only ever hold an epoch); Q_LOOKAHEAD the lookahead, which can
-// therefore run on another stream beside them; Q_WIDE the wide and pipelined
-// closed-loop kernels, whose flag space also holds MV words and counters and
-// is cleared before each of their launches.  The counters sit 128 bytes apart.
+// Q_MAIN serves plain-ME of more than two frames, deblocking and the
+// bounded-wait self-test (flags that only ever hold an epoch; its words also
+// hold a deblocking call's edge strengths); Q_LOOKAHEAD the lookahead, which can
+// therefore run on another stream beside them; Q_WIDE plain-ME of one or two
+// frames, the step and the pipelined closed loop, whose flag space also holds
+// other layouts (the pipelined loop's MV words and counters) and is cleared
+// before each of their launches.  The counters sit 128 bytes apart.
 constexpr int Q_MAIN = 0, Q_LOOKAHEAD = 1, Q_WIDE = 2, NUM_QUEUES = 3, Q_COUNTER_STRIDE = 32;
 // h264a_pixel_path_host: PP_CHUNKS upload chunks; its events are the
 // uploads, planes and half-res frames ready, ME + T/Q done, lookahead done.

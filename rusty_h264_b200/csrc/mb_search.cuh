@@ -20,12 +20,12 @@
 //
 // The bound is the wavefront's latency: each MB's rounds depend on one
 // another, and a round is a chain of shared-memory reads, mma and shuffles.
-// Measured inside the closed loop's launch: a 16x16 round takes 1,330-1,500
-// cycles, where the butterflies on 32 lanes (satd4x4_packed, two 16x16
-// candidates or one per partition a pass, four warps a MB) took about 3,000,
-// and a partition round 1,900-2,400; an MB has about 7.7 and 11.4 of them.  59
-// 1080p P frames of the closed loop: 46.6 ms before, 26.8 now; 15 P frames of
-// five mixed streams (one launch): 8.3 and 4.0 ms.
+// Measured with Balanced inside the closed loop's launch (and in the step's): a
+// 16x16 round takes 1,230 (1,160) cycles, where the butterflies on 32 lanes
+// (satd4x4_packed, two 16x16 candidates or one per partition a pass, four warps
+// a MB) took about 3,000, and a partition round 1,980 (1,510); an MB has about
+// 6.5 to 7.8 and 11 to 12 of them.  59 1080p P frames of the closed loop: 46.6 ms
+// before, 24.9 now; 15 P frames of five mixed streams (one launch): 8.3 and 3.8.
 #pragma once
 
 #include <cstddef>

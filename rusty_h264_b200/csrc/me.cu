@@ -538,8 +538,11 @@ constexpr int ME_FEW_FRAMES = 2;
 // fit one after another; more pools only hold warps that wait (learned 720p at
 // 6, 8, 10, 13: 7.5, 6.8, 7.0, 8.0 ms; 1080p at 8, 10, 13: 28.4, 26.5, 27.1).
 // CTAs: about a warp per MB of the pools' longest anti-diagonals: more hold MBs
-// that wait, and slow the warps that run (1080p at 1 and 2: 26.5 and 27.5 ms;
-// 2560x1440 18.9 and 17.0; 3840x2160 27.0 and 20.0, 4 MBs a segment).
+// that wait, and slow the warps that run (60 1080p frames at 1 and 2 an SM: 24.1
+// and 26.1 ms; 30 of 2560x1440 at 2 and 3: 19.4 and 20.9; 16 of 3840x2160: 18.3
+// and 19.6).  (The segment and pool sweeps, and fewer CTAs than that -- 2560x1440
+// at 1 and 2: 18.9 and 17.0, 3840x2160 27.0 and 20.0 -- on an earlier build at
+// 128 registers a thread.)
 constexpr int PIPE_SEGW = 7, PIPE_POOLS = 10;
 static inline int wave_mbs(int mb_w, int mb_h) { return std::min((mb_w + 1) / 2, mb_h); }  // of the longest anti-diagonal
 static inline int pipe_segw(int mb_w) { return std::min(std::max(mb_w / 24, 1), PIPE_SEGW); }
@@ -555,7 +558,8 @@ static inline int pipe_ctas_per_sm(int mb_w, int mb_h, int pools, int num_sms, i
 // CTA more than its share off an SM.  Beside another kernel (the lookahead of
 // the next frames on its own stream) the CTAs would otherwise crowd onto the
 // SMs that are free first (60 1080p frames with their lookahead: 64.8 ms, the
-// loop alone 41.7).
+// loop alone 41.7).  The price: launches of one CTA an SM from two contexts do
+// not share SMs, although one of them keeps 5% of an SM's warps active.
 constexpr int SM_SHARED = 228 * 1024, FRAME_SMEM_MAX = SM_SHARED / 2;
 static inline size_t frame_smem(long long blocks, int num_sms) {
     const long long share = (blocks + num_sms - 1) / num_sms;
@@ -2026,8 +2030,8 @@ int h264a::closed_pipe_run(h264a_ctx* ctx, const ClosedPipeIn& in, const h264a_m
 // cheapest kept (references in order).  An MV predicts only from neighbours
 // of the same reference (inter.rs:36-69), so a pick carries each half's
 // reference index: 8 i32 per MB (shape, ref0, mv0x, mv0y, ref1, mv1x, mv1y,
-// 4x4-block evaluations).  One warp per MB, the narrow kernel's queue and
-// wavefront; the window is staged again for each reference.
+// 4x4-block evaluations).  One warp per MB, tickets in the frame kernels'
+// order, readiness by a flag per MB; the window is staged again for each reference.
 constexpr int ME_MAXREF = 4;
 struct FrameDescMR {
     CUtensorMap tmap[ME_MAXREF];  // each reference's planes as the window's 3D tensor
