@@ -34,9 +34,6 @@
 
 namespace h264a {
 
-constexpr int MET_SATD = 0;
-constexpr int MET_SAD = 1;
-
 // The reference picture's readiness in the pipelined closed loop: its planes
 // are built segment by segment (16 picture rows by segw picture columns;
 // segment (b, s)'s flag == epoch means every segment up and left of it is
@@ -479,9 +476,6 @@ constexpr uint32_t kRingXP = 0x2252u, kRingYP = 0x8225u;
 __device__ __forceinline__ int ring_dx(int i) { return int((kRingXP >> (2 * i)) & 3u) - 1; }
 __device__ __forceinline__ int ring_dy(int i) { return int((kRingYP >> (2 * i)) & 3u) - 1; }
 
-// Search phases and what an evaluation round's results are for.
-constexpr int PH_SEEDS = 0, PH_PROP = 1, PH_DIA = 2, PH_REPRICE = 3, PH_SUB = 4, PH_DONE = 5, PH_START = 6;
-constexpr int EV_START = 0, EV_SEEDS = 1, EV_PROP = 2, EV_FIXED = 3, EV_RING = 4, EV_REPRICE = 5;
 // Proposals of the learned search's 16x16 search.
 constexpr int N_PROP = 8;
 constexpr int LOOP_GUARD = 1 << 20;  // iterations of one rung / sub-pel step

@@ -37,6 +37,12 @@ namespace h264a {
 // Warps per CTA of the frame kernels (one MB per warp).
 constexpr int ME_WARPS = 4;
 
+// Of h264a_me_search's jobs: metrics, search phases and what an evaluation
+// round's results are for.
+constexpr int MET_SATD = 0, MET_SAD = 1;
+constexpr int PH_SEEDS = 0, PH_DIA = 1, PH_REPRICE = 2, PH_SUB = 3, PH_DONE = 4;
+constexpr int EV_START = 0, EV_SEEDS = 1, EV_FIXED = 2, EV_RING = 3, EV_REPRICE = 4;
+
 // Per-warp shared state of an h264a_me_search job: the round's candidates and
 // distortions, and the search's cold parameters (read a few times per round,
 // so they live here rather than in registers).

@@ -1,5 +1,5 @@
-"""Every preset knob through the frame searches (mb_search, which runs all but
-the Balanced preset there), and one preset each through the step, the closed
+"""Every preset knob through the frame searches (which run all but the Balanced
+preset in an instance of their own), and some presets each through the step, the closed
 loop, the learned and the multi-reference calls.  Bit-exact with the oracle."""
 import numpy as np
 import pytest
